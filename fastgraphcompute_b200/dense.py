@@ -73,9 +73,11 @@ def _full_precision() -> bool:
 def fused_ok(linear, x) -> bool:
     """Whether ``linear(x)`` may take the fused form: plain fp32 matrices on one GPU, fp32 arithmetic asked
     for, no hooks and no tracing that would have to see the module called."""
-    if type(x) is not torch.Tensor or x.dim() != 2 or x.shape[0] < min_rows:
-        return False
+    # before any look at the shape: a tracer would record the comparison with min_rows as a condition on a dynamic row
+    # count (an export then fails, a compiled module gets a second graph)
     if torch.jit.is_tracing() or torch.compiler.is_compiling() or torch._C._are_functorch_transforms_active():
+        return False
+    if type(x) is not torch.Tensor or x.dim() != 2 or x.shape[0] < min_rows:
         return False
     if nn.modules.module._has_any_global_hook() or not _plain_linear(linear):
         return False

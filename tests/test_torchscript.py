@@ -14,6 +14,7 @@ from fastgraphcompute_b200.extensions.binned_select_knn import binned_select_knn
 from fastgraphcompute_b200.extensions.bin_by_coordinates import bin_by_coordinates
 from fastgraphcompute_b200.extensions.index_replacer import index_replacer
 from fastgraphcompute_b200.gnn_ops import GravNetOp
+from fastgraphcompute_b200.gravnet_model import GravNetModel
 
 
 class BinnedSelectKnnModule(torch.nn.Module):
@@ -60,6 +61,18 @@ def test_everything_compiles_without_a_gpu():
 def test_ops_reject_cpu_tensors_through_the_dispatcher():
     with pytest.raises(RuntimeError, match="CUDA tensors only"):
         torch.ops.fgc_b200.knn_forward(torch.rand(10, 3), torch.tensor([0, 10]), 4, None, False)
+
+
+@pytest.mark.parametrize("n", [1000, 40000])
+@pytest.mark.parametrize("module", [GravNetOp(8, 8, 3, 8, 8), GravNetModel(8, 8, 3, 8, 16, 4, 1)],
+                         ids=lambda m: type(m).__name__)
+def test_strict_export_with_a_dynamic_row_count(module, n):
+    """The row count stays free whatever the example's, below or above the one from which the eager dense layers
+    leave their modules."""
+    rows = torch.export.Dim("N", min=2, max=1 << 24)
+    program = torch.export.export(module, (torch.randn(n, 8), torch.tensor([0, n])), dynamic_shapes=({0: rows}, None),
+                                  strict=True)
+    assert "linear" in program.graph_module.code
 
 
 def _roundtrip(scripted):
