@@ -5,6 +5,7 @@ usual wherever the plain form is not given: see ``_plain_linear`` and ``fused_ok
 """
 import torch
 from torch import nn
+from torch.autograd import forward_ad
 
 from . import _cabi
 
@@ -80,6 +81,8 @@ def fused_ok(linear, x) -> bool:
     if type(x) is not torch.Tensor or x.dim() != 2 or x.shape[0] < min_rows:
         return False
     if nn.modules.module._has_any_global_hook() or not _plain_linear(linear):
+        return False
+    if forward_ad.unpack_dual(x).tangent is not None:        # forward-mode derivatives: the modules have them
         return False
     w = linear.weight
     return (x.is_cuda and x.shape[0] > 0 and x.dtype == torch.float32 and w.dtype == torch.float32

@@ -77,3 +77,24 @@ def test_dense_layer_special_values_and_plain_calls(monkeypatch):
     with torch.autocast("cuda", dtype=torch.bfloat16):
         assert not dense.fused_ok(lin, xs)
     assert not torch.vmap(lambda v: torch.tensor(float(dense.fused_ok(lin, v))))(xs[:, None, :]).any()
+
+
+def test_forward_mode_derivatives_of_dense_layers(monkeypatch):
+    """An input that carries a tangent goes through the modules, which have forward-mode derivatives: as one layer, and
+    where the tangent starts at an inner layer's weight."""
+    import torch.autograd.forward_ad as fwad
+    from fastgraphcompute_b200 import dense
+    monkeypatch.setattr(dense, "min_rows", 1)
+    torch.manual_seed(0)
+    stack = nn.Sequential(nn.Linear(8, 16), nn.ReLU(), nn.Linear(16, 4)).to(DEV)
+    x, t = torch.randn((100, 8), device=DEV), torch.randn((100, 8), device=DEV)
+    with fwad.dual_level():
+        got = fwad.unpack_dual(dense.sequential(stack, fwad.make_dual(x, t))).tangent
+        ref = fwad.unpack_dual(stack(fwad.make_dual(x, t))).tangent
+        assert torch.equal(got, ref)
+        w = stack[0].weight.detach()
+        del stack[0]._parameters["weight"]
+        stack[0].weight = fwad.make_dual(w, torch.ones_like(w))
+        got = fwad.unpack_dual(dense.sequential(stack, x)).tangent
+        ref = fwad.unpack_dual(stack(x)).tangent
+        assert ref is not None and torch.equal(got, ref)
