@@ -14,17 +14,28 @@ from . import _cabi
 # with ReLU take 0.153 ms as modules and 0.169 fused at 10 000 rows, 0.578 and 0.322 at 200 000.
 min_rows = 32768
 
+# Results of this many entries or more get bias and ReLU in a pass of their own: the library's product with the bias in
+# it is then slower than the plain product and the pass (forward alone, module / pass, us: 200 000 rows, 64 to 128
+# without ReLU 230 / 160, with it 264 / 161; 131 072 rows, 128 to 64 98 / 95 and 106 / 96).  Below, the pass and its
+# launch cost more than they save (200 000 rows, 128 to 10 85 / 91; 32 768 rows, 128 to 128 59 / 64).
+pass_from = 1 << 23
+
 
 class _Linear(torch.autograd.Function):
-    """act(x @ weight^T + bias): GEMMs from the library, bias and ReLU in one pass over the result, their
+    """act(x @ weight^T + bias): GEMMs from the library, bias and ReLU in one pass over a large result, their
     gradients and the weight's in one pass over the incoming gradient (csrc/dense.cu)."""
 
     @staticmethod
     def forward(ctx, x, weight, bias, relu):
-        y = torch.mm(x, weight.t())
-        with _cabi.on_device(x.device):
-            _cabi.check(_cabi.lib.fgc_bias_act(_cabi.ptr(y), _cabi.ptr(bias.contiguous()), y.shape[0], y.shape[1], int(relu),
-                                               _cabi.current_stream(x.device)), "fgc_bias_act")
+        if x.shape[0] * weight.shape[0] < pass_from:
+            y = torch.addmm(bias, x, weight.t())
+            if relu:
+                y.relu_()
+        else:
+            y = torch.mm(x, weight.t())
+            with _cabi.on_device(x.device):
+                _cabi.check(_cabi.lib.fgc_bias_act(_cabi.ptr(y), _cabi.ptr(bias.contiguous()), y.shape[0], y.shape[1],
+                                                   int(relu), _cabi.current_stream(x.device)), "fgc_bias_act")
         ctx.save_for_backward(x, weight, y if relu else None)
         return y
 
@@ -71,14 +82,16 @@ def _full_precision() -> bool:
         return False
 
 
+def _traced() -> bool:
+    """Asked before any look at a shape: a tracer would record the comparison of the row count with a threshold as a
+    condition on a dynamic size (an export then fails, a compiled module gets a second graph)."""
+    return torch.jit.is_tracing() or torch.compiler.is_compiling() or torch._C._are_functorch_transforms_active()
+
+
 def fused_ok(linear, x) -> bool:
     """Whether ``linear(x)`` may take the fused form: plain fp32 matrices on one GPU, fp32 arithmetic asked
     for, no hooks and no tracing that would have to see the module called."""
-    # before any look at the shape: a tracer would record the comparison with min_rows as a condition on a dynamic row
-    # count (an export then fails, a compiled module gets a second graph)
-    if torch.jit.is_tracing() or torch.compiler.is_compiling() or torch._C._are_functorch_transforms_active():
-        return False
-    if type(x) is not torch.Tensor or x.dim() != 2 or x.shape[0] < min_rows:
+    if _traced() or type(x) is not torch.Tensor or x.dim() != 2 or x.shape[0] < min_rows:
         return False
     if nn.modules.module._has_any_global_hook() or not _plain_linear(linear):
         return False

@@ -98,3 +98,18 @@ def test_forward_mode_derivatives_of_dense_layers(monkeypatch):
         got = fwad.unpack_dual(dense.sequential(stack, x)).tangent
         ref = fwad.unpack_dual(stack(x)).tangent
         assert ref is not None and torch.equal(got, ref)
+
+
+@pytest.mark.parametrize("n,n_out", [(1, 1), (1, 4), (255, 4), (257, 12), (1000, 7), (20011, 64), (3, 4100), (300000, 33)])
+@pytest.mark.parametrize("relu", [False, True])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_bias_and_relu_pass(n, n_out, relu, offset):
+    """One addition and one comparison per entry: the same bits as torch, on and off 16-byte alignment."""
+    from fastgraphcompute_b200 import _cabi
+    torch.manual_seed(n)
+    y = torch.randn(n * n_out + offset, device=DEV)[offset:].view(n, n_out)
+    bias = torch.randn(n_out + offset, device=DEV)[offset:]
+    ref = y + bias
+    ref = ref.relu() if relu else ref
+    assert _cabi.lib.fgc_bias_act(_cabi.ptr(y), _cabi.ptr(bias), n, n_out, int(relu), _cabi.current_stream(y.device)) == 0
+    assert torch.equal(y, ref)
