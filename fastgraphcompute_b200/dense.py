@@ -104,16 +104,42 @@ def fused_ok(linear, x) -> bool:
             and not torch.is_autocast_enabled("cuda") and _full_precision())
 
 
+def _pays(linear, x) -> bool:
+    """Whether the fused form is the faster one of those that ``fused_ok`` allows (B200, forward and backward, modules /
+    fused, us)."""
+    if _traced() or type(linear) is not nn.Linear or x.dim() != 2 or x.shape[0] < min_rows:
+        return False
+    n, n_in, n_out = x.shape[0], linear.in_features, linear.out_features
+    if not (torch.is_grad_enabled() and (x.requires_grad or linear.weight.requires_grad)):
+        return n * n_out >= pass_from            # nothing but the forward's pass to gain
+    # A small weight: the library's product for its gradient is a good one.  800 000 rows, 64 to 4 451 / 560 and 32 to 16
+    # 470 / 547; 200 000 rows, 32 to 32 710 / 239.
+    if n_in * n_out < min_rows // 32:
+        return False
+    # Few outputs fill a sixth of a tile, which takes twice the rows to pay: 128 to 10 at 32 768 rows 165 / 177, at
+    # 65 536 214 / 188; 64 to 24 at 32 768 226 / 198.
+    if n_out < 24 and (n + 1) // 2 < min_rows:
+        return False
+    # Many tiles of a weight read x and the gradient again and again: 200 000 rows, 256 to 256 2129 / 1956, 512 to 128 2048 /
+    # 1974, but 384 to 160 (padded to 384 x 256) 2196 / 2370, 2048 to 64 3490 / 3798, 512 to 512 6591 / 6891.
+    return _padded(n_in) * _padded(n_out) <= 65536
+
+
+def _padded(columns: int) -> int:
+    return 64 if columns <= 64 else -(-columns // 128) * 128
+
+
 def linear_relu(linear: nn.Module, relu: nn.Module, x: torch.Tensor) -> torch.Tensor:
     """relu(linear(x))."""
-    if type(relu) is nn.ReLU and _no_hooks(relu) and "forward" not in relu.__dict__ and fused_ok(linear, x):
+    if type(relu) is nn.ReLU and _no_hooks(relu) and "forward" not in relu.__dict__ and _pays(linear, x) \
+            and fused_ok(linear, x):
         return _Linear.apply(x, linear.weight, linear.bias, True)
     return relu(linear(x))
 
 
 def linear(module: nn.Module, x: torch.Tensor) -> torch.Tensor:
     """module(x)."""
-    if fused_ok(module, x):
+    if _pays(module, x) and fused_ok(module, x):
         return _Linear.apply(x, module.weight, module.bias, False)
     return module(x)
 

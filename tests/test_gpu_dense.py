@@ -113,3 +113,20 @@ def test_bias_and_relu_pass(n, n_out, relu, offset):
     ref = ref.relu() if relu else ref
     assert _cabi.lib.fgc_bias_act(_cabi.ptr(y), _cabi.ptr(bias), n, n_out, int(relu), _cabi.current_stream(y.device)) == 0
     assert torch.equal(y, ref)
+
+
+def test_dense_layer_is_fused_only_where_it_pays():
+    """Small weights, few outputs, weights of many tiles and forwards without a large result stay modules."""
+    from fastgraphcompute_b200 import dense
+    rows = dense.min_rows
+
+    def fused(n, n_in, n_out, grad=True):
+        lin = nn.Linear(n_in, n_out).to(DEV).requires_grad_(grad)
+        out = dense.linear(lin, torch.zeros((n, n_in), device=DEV))
+        assert type(out.grad_fn).__name__ == ("_LinearBackward" if out.grad_fn is not None and dense._pays(
+            lin, torch.empty((n, n_in), device=DEV)) else ("AddmmBackward0" if grad else "NoneType"))
+        return dense._pays(lin, torch.empty((n, n_in), device=DEV))
+    assert fused(rows, 128, 64) and fused(rows, 64, 24) and fused(2 * rows, 128, 10) and fused(rows, 256, 256)
+    assert not fused(rows, 128, 10) and not fused(4 * rows, 32, 16) and not fused(4 * rows, 64, 4)
+    assert not fused(rows, 384, 160) and not fused(rows, 512, 512)
+    assert fused(4 * rows, 64, 64, grad=False) and not fused(rows, 128, 128, grad=False)
