@@ -209,7 +209,8 @@ int fgc_knn_search(int64_t n_vert, int32_t n_coords, int64_t n_rs, int32_t K,
  * more than about 70 million points).
  * fgc_knn_tree_preferred: 1 where the tree fits and was measured to be the faster search (long lists in three
  * coordinates, five and more coordinates; with long_tails != 0 -- the points are expected to have sparse tails, as learned
- * coordinates do -- also four coordinates).  No counterparts in the reference.
+ * coordinates do -- also four coordinates).  For searches without direction flags: with them the grid holds candidates
+ * only and is the faster one.  No counterparts in the reference.
  */
 int fgc_knn_tree_preferred(int64_t n_vert, int32_t n_coords, int64_t n_rs, int32_t K, int32_t long_tails);
 int fgc_knn_build_tree(const float *coords, int64_t n_vert, int32_t n_coords, const int64_t *row_splits, int64_t n_rs,

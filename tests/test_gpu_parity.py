@@ -945,3 +945,35 @@ def test_knn_tree_refuses_bad_input():
         status = ctypes.c_int32(0)
         assert _cabi.lib.fgc_read_status(_cabi.ptr(ws), ctypes.byref(status), st) == 0
         assert status.value & _cabi.STATUS_INTERNAL
+
+
+@pytest.fixture
+def forward_flags(monkeypatch):
+    """Flags of every forward call into the library."""
+    import importlib
+    km = importlib.import_module("fastgraphcompute_b200.extensions.binned_select_knn")
+    call, seen = km._cabi.lib.fgc_knn_forward, []
+
+    def recorded(*args):
+        seen.append(args[9])
+        return call(*args)
+    monkeypatch.setattr(km._cabi.lib, "fgc_knn_forward", recorded)
+    return seen
+
+
+@pytest.mark.parametrize("n,D,K", [(70000, 3, 96), (20000, 5, 96), (20000, 8, 20)])
+def test_direction_flags_are_searched_on_the_grid(forward_flags, n, D, K):
+    """The tree's leaves hold points that may not be neighbours; with few candidates a search on it looks at all of them."""
+    g = torch.Generator().manual_seed(n + D)
+    pts = torch.rand((n, D), generator=g).to(DEV)
+    rs = torch.tensor([0, n], device=DEV)
+    direction = torch.where(torch.rand((n,), generator=g) < 0.001, 0, 1).to(DEV)
+    fgc.binned_select_knn(K, pts, rs)
+    idx, dist = fgc.binned_select_knn(K, pts, rs, direction=direction)
+    assert [f & 64 for f in forward_flags] == [64, 0]
+    ids = torch.nonzero(direction == 0).squeeze(1)
+    d = torch.cdist(pts.double(), pts[ids].double()).square().sort(dim=1).values
+    d = torch.where((direction == 1)[:, None], d, torch.zeros_like(d))           # (the candidates search nothing)
+    m = min(K - 1, ids.numel())
+    torch.testing.assert_close(dist[:, 1:1 + m].sort(dim=1).values.double(), d[:, :m], rtol=1e-5, atol=1e-6)
+    assert bool((idx[:, 1 + m:] == -1).all())
