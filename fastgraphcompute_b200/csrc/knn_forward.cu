@@ -53,10 +53,12 @@ static int knn_forward_launch(const float *coords, int64_t n_vert, int32_t n_coo
         FGC_RETURN_IF_CUDA(cudaMemcpyAsync(out_order, fgc_knn_cell_order(ws, n_vert, n_coords, n_rs, K),
                                            sizeof(int32_t) * (size_t)n_vert, cudaMemcpyDeviceToDevice, (cudaStream_t)stream));
     if (ties && n_vert > 0) {
-        // Which of several points at exactly the K-th distance is kept is open, but it should not hang on the
-        // choice of the search: the few such rows are searched again on a grid.
-        rc = fgc_knn_build_grid_dims(coords, n_vert, n_coords, row_splits, n_rs, K, direction, target_occupancy, 0, ws,
-                                     ws_bytes, stream);
+        // Which of several points at exactly the K-th distance is kept is open, but for coordinates without order it should
+        // not hang on the choice of the search: the few such rows are searched again on a grid.  On a lattice, where
+        // nearly every row has such a choice, that would be the whole search twice: beyond a sixteenth of the rows the
+        // tree's choice stands.
+        rc = knn_build_grid_for_ties(coords, n_vert, n_coords, row_splits, n_rs, K, direction, target_occupancy, ws, ws_bytes,
+                                     stream);
         if (rc != FGC_OK) return rc;
         return knn_search_grid(n_vert, n_coords, n_rs, K, direction != nullptr, tf_compat, FGC_SEARCH_FRESH, true, out_idx,
                                out_distsq, ws, ws_bytes, stream);

@@ -34,6 +34,7 @@
 // grid and the stopping rule are this library's own; they never change which
 // points are nearest, only which of several equidistant points is kept.
 #include "knn_grid.cuh"
+#include "knn_tree.cuh"
 #include "shell_table.cuh"
 
 namespace fgc {
@@ -48,13 +49,31 @@ __device__ void grid_setup(KnnGrid *g, const int64_t *__restrict__ row_splits, i
 // Fused finite check + min/max of the binned coordinates; clears the cell table (all of its
 // capacity: the grid that decides how much of it is used does not exist yet); the CTA that
 // finishes last (a ticket counter, no waiting) checks the row splits and chooses the grid.
+// Before the grid of a second look: an empty header and tickets where there are rows to search again, else a
+// status word that ends the kernels of the grid at once.
 __global__ void __launch_bounds__(256)
-k_minmax_setup(const float *__restrict__ coords, int n_vert, int n_coords, int n_bin_dims, KnnGrid *g,
-               int *__restrict__ counts, long long n_counts, const int64_t *__restrict__ row_splits, int n_rs,
-               int bins_target, int bins_cap_first, int bins_cap, int mirror)
+k_tie_gate(KnnGrid *__restrict__ g, const KnnTree *__restrict__ t, int limit)
 {
     chain_wait();
     chain_release();
+    const int status = g->status, tied = t->n_tied;
+    __syncthreads();
+    if (status != 0) return;
+    if (tied == 0 || tied > limit) {
+        if (threadIdx.x == 0) g->status = kStatusNoGrid;
+        return;
+    }
+    for (int i = threadIdx.x; i < (int)((kGridHeaderBytes + kHardTicketBytes) / sizeof(int)); i += 256) ((int *)g)[i] = 0;
+}
+
+__global__ void __launch_bounds__(256)
+k_minmax_setup(const float *__restrict__ coords, int n_vert, int n_coords, int n_bin_dims, KnnGrid *g,
+               int *__restrict__ counts, long long n_counts, const int64_t *__restrict__ row_splits, int n_rs,
+               int bins_target, int bins_cap_first, int bins_cap, int mirror, int gated)
+{
+    chain_wait();
+    chain_release();
+    if (gated && g->status != 0) return;           // (else zero until the last CTA sets it)
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n_counts;
          i += (long long)gridDim.x * blockDim.x)
         counts[i] = 0;
@@ -571,14 +590,12 @@ extern "C" int fgc_knn_build_grid(const float *coords, int64_t n_vert, int32_t n
                                    target_occupancy, 0, workspace, workspace_bytes, stream);
 }
 
-extern "C" int fgc_knn_build_grid_dims(const float *coords, int64_t n_vert, int32_t n_coords,
-                                       const int64_t *row_splits, int64_t n_rs, int32_t K,
-                                       const int64_t *direction_or_null, float target_occupancy,
-                                       int32_t grid_dims, void *workspace, size_t workspace_bytes,
-                                       fgc_stream_t stream)
+namespace fgc {
+
+static int knn_build_grid(const float *coords, int64_t n_vert, int32_t n_coords, const int64_t *row_splits, int64_t n_rs,
+                          int32_t K, const int64_t *direction_or_null, float target_occupancy, int32_t grid_dims,
+                          bool only_for_ties, void *workspace, size_t workspace_bytes, fgc_stream_t stream)
 {
-    FGC_NVTX("fgc_knn_build_grid_dims");
-    using namespace fgc;
     if (grid_dims != 0 && grid_dims != 3 && grid_dims != 4) return FGC_ERR_BAD_ARGUMENT;
     KnnWorkspace L;
     if (!row_splits) return FGC_ERR_BAD_ARGUMENT;
@@ -587,7 +604,11 @@ extern "C" int fgc_knn_build_grid_dims(const float *coords, int64_t n_vert, int3
     cudaStream_t s = (cudaStream_t)stream;
     char *ws = (char *)workspace;
     KnnGrid *grid = (KnnGrid *)(ws + L.header);
-    FGC_RETURN_IF_CUDA(cudaMemsetAsync(grid, 0, kGridHeaderBytes + kHardTicketBytes, s));   // header and k_knn_hard's tickets
+    if (only_for_ties)
+        FGC_RETURN_IF_CUDA(launch_chained(k_tie_gate, 1, 256, 0, s, grid, (const KnnTree *)(ws + L.tickets),
+                                          (int)(n_vert / kTieShare)));
+    else
+        FGC_RETURN_IF_CUDA(cudaMemsetAsync(grid, 0, kGridHeaderBytes + kHardTicketBytes, s));   // header and k_knn_hard's tickets
     if (n_vert == 0) return FGC_OK;
     if (!coords || n_rs < 2) return FGC_ERR_BAD_ARGUMENT;
 
@@ -650,7 +671,7 @@ extern "C" int fgc_knn_build_grid_dims(const float *coords, int64_t n_vert, int3
     if (!adaptive) bins_cap_first = bins_cap;
     k_minmax_setup<<<red_blocks, 256, 0, s>>>(coords, n, n_coords, n_bin_dims, grid, counts,
                                               (long long)bins_cap_first * n_events * mirror + 1, row_splits, (int)n_rs,
-                                              bins_target, bins_cap_first, bins_cap, mirror);
+                                              bins_target, bins_cap_first, bins_cap, mirror, only_for_ties);
     FGC_CHECK_LAUNCH();
     const int allow_fallback = adaptive && n_coords == 4 && forced == 0;
     FGC_RETURN_IF_CUDA(launch_chained(k_histogram, pt_blocks, 256, 0, s, coords, n, n_coords, row_splits, (int)n_rs, direction_or_null,
@@ -681,6 +702,28 @@ extern "C" int fgc_knn_build_grid_dims(const float *coords, int64_t n_vert, int3
                                       n_coords, L.nv, direction_or_null, grid, counts, biglist, hugelist, n_warp_blocks,
                                       sorig, scoords, sbin, sflag));
     return FGC_OK;
+}
+
+}  // namespace fgc
+
+extern "C" int fgc_knn_build_grid_dims(const float *coords, int64_t n_vert, int32_t n_coords,
+                                       const int64_t *row_splits, int64_t n_rs, int32_t K,
+                                       const int64_t *direction_or_null, float target_occupancy,
+                                       int32_t grid_dims, void *workspace, size_t workspace_bytes,
+                                       fgc_stream_t stream)
+{
+    FGC_NVTX("fgc_knn_build_grid_dims");
+    return fgc::knn_build_grid(coords, n_vert, n_coords, row_splits, n_rs, K, direction_or_null, target_occupancy, grid_dims,
+                               false, workspace, workspace_bytes, stream);
+}
+
+int fgc::knn_build_grid_for_ties(const float *coords, int64_t n_vert, int32_t n_coords, const int64_t *row_splits,
+                                 int64_t n_rs, int32_t K, const int64_t *direction_or_null, float target_occupancy,
+                                 void *workspace, size_t workspace_bytes, fgc_stream_t stream)
+{
+    FGC_NVTX("fgc_knn_build_grid_for_ties");
+    return knn_build_grid(coords, n_vert, n_coords, row_splits, n_rs, K, direction_or_null, target_occupancy, 0, true,
+                          workspace, workspace_bytes, stream);
 }
 
 extern "C" const int32_t *fgc_knn_cell_order(const void *workspace, int64_t n_vert, int32_t n_coords,

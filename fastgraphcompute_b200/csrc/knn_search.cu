@@ -132,16 +132,15 @@ struct NeighbourList {
 // a whole (about 150 instructions whatever the count); fewer go in one by one (about 16 each).
 // Measured on B200: 8 is best, 5 and 12 are 0.5 to 2 % slower.
 constexpr int kBulkMin = 8;
-// The search of one query by one warp.  G4: the grid spans four coordinates, else three.
-template <int NV, int R, bool COUNT, bool MARKED, bool G4>
-__device__ __forceinline__ void knn_query(const KnnArgs &a)
+// The search of one query (position qi in cell order) by one warp.  G4: the grid spans four coordinates, else three.
+template <int NV, int R, bool COUNT, bool G4>
+__device__ __forceinline__ void knn_query(const KnnArgs &a, const int qi)
 {
     __shared__ int s_delta[kKnnWarps][32];
     __shared__ float s_bd[kKnnWarps][32];
     __shared__ int s_bj[kKnnWarps][32];
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
-    const int qi = blockIdx.x * kKnnWarps + wib;   // position in cell order
     KnnGrid *__restrict__ g = a.grid;
     if (qi >= a.n_vert) return;
     if (g->status != 0) {
@@ -168,7 +167,6 @@ __device__ __forceinline__ void knn_query(const KnnArgs &a)
     if (!FGC_DBG_OK(orig_q >= 0 && orig_q < a.n_vert, &g->status)) return;
     int64_t *__restrict__ out_i = a.out_idx + (size_t)orig_q * K;
     float *__restrict__ out_d = a.out_dist + (size_t)orig_q * K;
-    if (MARKED && out_i[0] != kTieRow) return;
 
     // queries that may not have neighbours keep the default row
     const bool q_inactive = sflag && (sflag[qi] == 0 || sflag[qi] == 2);
@@ -495,7 +493,11 @@ k_knn_hard(const KnnArgs a)
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
     KnnGrid *__restrict__ g = a.grid;
-    if (g->status != 0) return;
+    if (g->status != 0) {
+        // the end of a second look that searched nothing (a CTA that reads the cleared word finds no queries listed)
+        if (g->status == kStatusNoGrid && blockIdx.x == 0 && threadIdx.x == 0) g->status = 0;
+        return;
+    }
     const int n_hard = min(g->n_hard, a.n_vert);
     if (n_hard == 0) return;
     const int K = a.K, kn = K - 1, nc = a.n_coords;
@@ -615,16 +617,56 @@ k_knn_hard(const KnnArgs a)
 // MODE 0: grid over three coordinates (D <= 3); 1: over four (D >= 5); 2: D = 4, where the grid
 // build decides on the device between the two -- one launch, one uniform branch (two launches
 // of which one returns at once cost the same; out-of-line bodies were slower).
-template <int NV, int R, bool COUNT, bool MARKED, int MODE>
+template <int NV, int R, bool COUNT, int MODE>
 __global__ void __launch_bounds__(kKnnWarps * 32, (R == 1 ? 8 : (R == 2 ? (NV == 1 ? 7 : 6) : (R == 4 ? 6 : 4))))
 k_knn(const KnnArgs a)
 {
     chain_wait();
     chain_release();
-    if (MODE == 0) knn_query<NV, R, COUNT, MARKED, false>(a);
-    else if (MODE == 1) knn_query<NV, R, COUNT, MARKED, true>(a);
-    else if (a.grid->gdims == 4) knn_query<NV, R, COUNT, MARKED, true>(a);
-    else knn_query<NV, R, COUNT, MARKED, false>(a);
+    const int qi = blockIdx.x * kKnnWarps + (threadIdx.x >> 5);
+    if (MODE == 0) knn_query<NV, R, COUNT, false>(a, qi);
+    else if (MODE == 1) knn_query<NV, R, COUNT, true>(a, qi);
+    else if (a.grid->gdims == 4) knn_query<NV, R, COUNT, true>(a, qi);
+    else knn_query<NV, R, COUNT, false>(a, qi);
+}
+
+// The rows that the tree search has marked kTieRow.  A warp looks at 32 rows at once, one per lane and far
+// apart (marked rows come in clusters), and searches the marked ones.  Without a grid the marks are taken off and the
+// tree's choice stands.
+template <int NV, int R, int MODE>
+__global__ void __launch_bounds__(kKnnWarps * 32)
+k_knn_marked(const KnnArgs a)
+{
+    chain_wait();
+    chain_release();
+    const int lane = threadIdx.x & 31;
+    const int n_groups = (int)(((long long)a.n_vert + 31) / 32);
+    const bool search = a.grid->status == 0;
+    if (!search && ((const KnnTree *)a.hard_tickets)->n_tied == 0) return;
+    for (int i = blockIdx.x * kKnnWarps + (threadIdx.x >> 5); i < n_groups; i += gridDim.x * kKnnWarps) {
+        const long long mine = i + (long long)lane * n_groups;
+        int64_t *row = nullptr;
+        int id = 0;
+        if (mine < a.n_vert) {
+            id = search ? __ldg(a.sorig + mine) : (int)mine;
+            row = a.out_idx + (size_t)id * a.K;
+        }
+        const bool marked = row && *row == kTieRow;
+        if (!search) {
+            if (marked) *row = id;
+            continue;
+        }
+        unsigned m = __ballot_sync(FGC_FULL_MASK, marked);
+        while (m) {
+            const int qi = i + (__ffs(m) - 1) * n_groups;
+            m &= m - 1;
+            if (MODE == 0) knn_query<NV, R, false, false>(a, qi);
+            else if (MODE == 1) knn_query<NV, R, false, true>(a, qi);
+            else if (a.grid->gdims == 4) knn_query<NV, R, false, true>(a, qi);
+            else knn_query<NV, R, false, false>(a, qi);
+            __syncwarp();
+        }
+    }
 }
 
 template <int NV, int G4>
@@ -635,21 +677,22 @@ static int launch_knn_nv(const KnnArgs &a, bool only_marked, cudaStream_t s)
     const int R = (kn + 31) / 32;
     const int T = kKnnWarps * 32;
     if (only_marked) {
-        // rows marked kTieRow only (a template: the check cost 0.3 % of a full search, 18.11 -> 18.16 ms)
-        if (R <= 1) FGC_RETURN_IF_CUDA(launch_chained(k_knn<NV, 1, false, true, G4>, blocks, T, 0, s, a));
-        else if (R <= 2) FGC_RETURN_IF_CUDA(launch_chained(k_knn<NV, 2, false, true, G4>, blocks, T, 0, s, a));
-        else if (R <= 4) FGC_RETURN_IF_CUDA(launch_chained(k_knn<NV, 4, false, true, G4>, blocks, T, 0, s, a));
-        else FGC_RETURN_IF_CUDA(launch_chained(k_knn<NV, 8, false, true, G4>, blocks, T, 0, s, a));
+        const unsigned groups = (unsigned)(((a.n_vert + 31LL) / 32 + kKnnWarps - 1) / kKnnWarps);
+        const unsigned few = groups < (unsigned)sm_count() * 8 ? groups : (unsigned)sm_count() * 8;
+        if (R <= 1) FGC_RETURN_IF_CUDA(launch_chained(k_knn_marked<NV, 1, G4>, few, T, 0, s, a));
+        else if (R <= 2) FGC_RETURN_IF_CUDA(launch_chained(k_knn_marked<NV, 2, G4>, few, T, 0, s, a));
+        else if (R <= 4) FGC_RETURN_IF_CUDA(launch_chained(k_knn_marked<NV, 4, G4>, few, T, 0, s, a));
+        else FGC_RETURN_IF_CUDA(launch_chained(k_knn_marked<NV, 8, G4>, few, T, 0, s, a));
     } else if (a.count_evals) {
-        if (R <= 1) FGC_RETURN_IF_CUDA(launch_chained(k_knn<NV, 1, true, false, G4>, blocks, T, 0, s, a));
-        else if (R <= 2) FGC_RETURN_IF_CUDA(launch_chained(k_knn<NV, 2, true, false, G4>, blocks, T, 0, s, a));
-        else if (R <= 4) FGC_RETURN_IF_CUDA(launch_chained(k_knn<NV, 4, true, false, G4>, blocks, T, 0, s, a));
-        else FGC_RETURN_IF_CUDA(launch_chained(k_knn<NV, 8, true, false, G4>, blocks, T, 0, s, a));
+        if (R <= 1) FGC_RETURN_IF_CUDA(launch_chained(k_knn<NV, 1, true, G4>, blocks, T, 0, s, a));
+        else if (R <= 2) FGC_RETURN_IF_CUDA(launch_chained(k_knn<NV, 2, true, G4>, blocks, T, 0, s, a));
+        else if (R <= 4) FGC_RETURN_IF_CUDA(launch_chained(k_knn<NV, 4, true, G4>, blocks, T, 0, s, a));
+        else FGC_RETURN_IF_CUDA(launch_chained(k_knn<NV, 8, true, G4>, blocks, T, 0, s, a));
     } else {
-        if (R <= 1) FGC_RETURN_IF_CUDA(launch_chained(k_knn<NV, 1, false, false, G4>, blocks, T, 0, s, a));
-        else if (R <= 2) FGC_RETURN_IF_CUDA(launch_chained(k_knn<NV, 2, false, false, G4>, blocks, T, 0, s, a));
-        else if (R <= 4) FGC_RETURN_IF_CUDA(launch_chained(k_knn<NV, 4, false, false, G4>, blocks, T, 0, s, a));
-        else FGC_RETURN_IF_CUDA(launch_chained(k_knn<NV, 8, false, false, G4>, blocks, T, 0, s, a));
+        if (R <= 1) FGC_RETURN_IF_CUDA(launch_chained(k_knn<NV, 1, false, G4>, blocks, T, 0, s, a));
+        else if (R <= 2) FGC_RETURN_IF_CUDA(launch_chained(k_knn<NV, 2, false, G4>, blocks, T, 0, s, a));
+        else if (R <= 4) FGC_RETURN_IF_CUDA(launch_chained(k_knn<NV, 4, false, G4>, blocks, T, 0, s, a));
+        else FGC_RETURN_IF_CUDA(launch_chained(k_knn<NV, 8, false, G4>, blocks, T, 0, s, a));
     }
     FGC_CHECK_LAUNCH();
     // the queries that gave up their walk (usually none: the CTAs return at once)

@@ -26,6 +26,7 @@ struct KnnTree {
     uint32_t max_key[kTreeKeyDims];     // ordered(max)
     float origin[kTreeKeyDims];
     float scale;                        // cells of the Hilbert curve per unit length
+    int32_t n_tied;                     // rows marked kTieRow by the search
 };
 static_assert(sizeof(KnnTree) <= kHardTicketBytes, "tree record too large");
 
@@ -83,12 +84,22 @@ inline TreeLayout tree_layout(const KnnWorkspace &w, int64_t n_vert, int n_coord
 
 // Mark in slot 0 of a row whose K-th distance several points share, of which some are left out.
 constexpr int64_t kTieRow = INT64_MIN;
+// Rows that may be marked and searched again, as a share of all rows: see knn_forward_launch.
+constexpr int kTieShare = 16;
+// Status word between the tree search and the end of the second look when there is nothing to search again:
+// the kernels of the grid return at once.
+constexpr int32_t kStatusNoGrid = 1 << 30;
 
 // fgc_knn_search_tree; mark_ties: such rows are marked (and have to be searched again on a grid).
 int knn_search_tree(int64_t n_vert, int32_t n_coords, const int64_t *row_splits, int64_t n_rs, int32_t K,
                     int32_t has_direction, int32_t tf_compat, bool mark_ties, int64_t *out_idx, float *out_distsq,
                     void *workspace, size_t workspace_bytes, fgc_stream_t stream);
-// fgc_knn_search; only_marked: rows marked by knn_search_tree only.
+// fgc_knn_build_grid_dims behind a search with mark_ties: builds nothing (kStatusNoGrid) where no row is marked,
+// or more than a kTieShare-th of them are.
+int knn_build_grid_for_ties(const float *coords, int64_t n_vert, int32_t n_coords, const int64_t *row_splits, int64_t n_rs,
+                            int32_t K, const int64_t *direction_or_null, float target_occupancy, void *workspace,
+                            size_t workspace_bytes, fgc_stream_t stream);
+// fgc_knn_search; only_marked: rows marked by knn_search_tree only (without a grid the marks are taken off).
 int knn_search_grid(int64_t n_vert, int32_t n_coords, int64_t n_rs, int32_t K, int32_t has_direction, int32_t tf_compat,
                     int32_t flags, bool only_marked, int64_t *out_idx, float *out_distsq, void *workspace,
                     size_t workspace_bytes, fgc_stream_t stream);

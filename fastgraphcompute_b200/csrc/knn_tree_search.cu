@@ -55,7 +55,7 @@ struct TreeArgs {
     const float4 *box[3];      // leaves, nodes, top nodes
     const int64_t *row_splits;
     KnnGrid *grid;
-    const KnnTree *tree;
+    KnnTree *tree;
     int64_t *out_idx;
     float *out_dist;
     int n_vert;
@@ -391,7 +391,12 @@ __device__ __forceinline__ void tree_query(const TreeArgs &a, int qi)
         if (sel.n < kn) last = 0;
     }
     tie = tie || (kn > 0 && sel.n >= kn && last == sel.left_out);
-    if (lane == 0) { out_i[0] = a.mark_ties && tie ? kTieRow : (int64_t)orig_q; out_d[0] = 0.f; }
+    const bool marked = a.mark_ties && tie;
+    if (lane == 0) {
+        out_i[0] = marked ? kTieRow : (int64_t)orig_q;
+        out_d[0] = 0.f;
+        if (marked) atomicAdd(&a.tree->n_tied, 1);
+    }
 }
 
 template <int NV, int R>
@@ -453,7 +458,7 @@ int fgc::knn_search_tree(int64_t n_vert, int32_t n_coords, const int64_t *row_sp
     for (int l = 0; l < 3; l++) a.box[l] = (const float4 *)(ws + T.box[l]);
     a.row_splits = row_splits;
     a.grid = (KnnGrid *)(ws + L.header);
-    a.tree = (const KnnTree *)(ws + L.tickets);
+    a.tree = (KnnTree *)(ws + L.tickets);
     a.out_idx = out_idx;
     a.out_dist = out_distsq;
     a.n_vert = (int)n_vert;

@@ -229,7 +229,8 @@ int fgc_knn_search_tree(int64_t n_vert, int32_t n_coords, const int64_t *row_spl
  * it keeps 64 bytes of page-locked memory per calling thread.  Without it nothing waits.
  */
 #define FGC_FORWARD_TREE 64    /* flags: search on a tree instead of a grid */
-#define FGC_FORWARD_GRID_TIES 128 /* with it: rows with a choice among equal K-th distances are searched again on a grid */
+#define FGC_FORWARD_GRID_TIES 128 /* with it: rows with a choice among equal K-th distances are searched again on a grid,
+                                    unless more than a sixteenth of all rows are such (lattice coordinates) */
 int fgc_knn_forward(const float *coords, int64_t n_vert, int32_t n_coords, const int64_t *row_splits,
                     int64_t n_rs, int32_t K, const int64_t *direction_or_null, int32_t tf_compat,
                     float target_occupancy, int32_t flags, int64_t *out_idx, float *out_distsq,

@@ -977,3 +977,51 @@ def test_direction_flags_are_searched_on_the_grid(forward_flags, n, D, K):
     m = min(K - 1, ids.numel())
     torch.testing.assert_close(dist[:, 1:1 + m].sort(dim=1).values.double(), d[:, :m], rtol=1e-5, atol=1e-6)
     assert bool((idx[:, 1 + m:] == -1).all())
+
+
+@pytest.mark.parametrize("n,D,K", [(30000, 3, 66), (20000, 3, 140), (20000, 5, 34), (20000, 6, 12), (20000, 9, 65)])
+def test_rows_with_equal_kth_distances_take_the_grids_choice(n, D, K):
+    """Among several points at exactly the K-th distance the tree keeps those that the grid keeps, while a sixteenth of the
+    rows or fewer have such a choice; on its own it keeps others."""
+    import importlib
+    km = importlib.import_module("fastgraphcompute_b200.extensions.binned_select_knn")
+    g = torch.Generator().manual_seed(D * K)
+    pts = torch.rand((n, D), generator=g)
+    pts[: n // 20] = torch.randint(0, 5, (n // 20, D), generator=g) * 0.25 + 3.0          # a patch of lattice, away from the rest
+    pts = pts[torch.randperm(n, generator=g)].to(DEV)
+    # (row splits small enough for a warp to scan: the whole-CTA scan's choice depends on how many rows share it)
+    rs = torch.cat([torch.arange(0, n, 4000), torch.tensor([n])]).to(DEV)
+    found = []
+    for tree, long_tails in ((False, False), (True, False), (True, True)):       # (the hint leaves the second look out)
+        old = km.search_tree
+        try:
+            km.search_tree = tree
+            idx, dist, _ = km.knn_forward_with_order(pts, rs, K, None, False, long_tails)
+        finally:
+            km.search_tree = old
+        assert torch.equal(idx[:, 0], torch.arange(n, device=DEV))
+        found.append((idx.sort(dim=1).values, dist.sort(dim=1).values))
+    grid, tree, alone = found
+    assert torch.equal(tree[0], grid[0]) and torch.equal(tree[1], grid[1]) and torch.equal(alone[1], grid[1])
+    assert 0 < int((alone[0] != grid[0]).any(dim=1).sum()) <= n // 16
+
+
+@pytest.mark.parametrize("D,K", [(3, 66), (5, 33), (6, 20), (8, 140)])
+def test_tree_search_on_a_lattice(D, K):
+    """Nearly every row has a choice at the K-th distance: the tree's stands, and no row is left marked."""
+    import importlib
+    km = importlib.import_module("fastgraphcompute_b200.extensions.binned_select_knn")
+    g = torch.Generator().manual_seed(D)
+    n = 3000
+    pts = torch.randint(0, 9 if D == 3 else 4, (n, D), generator=g).float()
+    rs = torch.tensor([0, 1000, n])
+    oi, od = oracle.binned_select_knn(K, pts.numpy(), rs.numpy())
+    old = km.search_tree
+    try:
+        km.search_tree = True
+        idx, dist, ws = km.knn_forward_raw(pts.to(DEV), rs.to(DEV), K, None, False)
+    finally:
+        km.search_tree = old
+    parity.assert_knn_parity(idx.cpu().numpy(), dist.cpu().numpy(), oi, od, what="lattice D=%d" % D)
+    assert torch.equal(idx[:, 0], torch.arange(n, device=DEV)) and int(idx.min()) >= -1
+    assert int(ws[:4].view(torch.int32)) == 0                                     # status of the workspace
