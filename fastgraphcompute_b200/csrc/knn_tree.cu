@@ -389,16 +389,18 @@ static cudaError_t launch_boxes(const float *coords, int n, int n_coords, const 
 
 }  // namespace fgc
 
-// Where the tree is the better search (B200, whole forward with the second look at tied rows, ms grid / tree).
-// Three coordinates, K > 65: the grid's list of four slots a lane is slow, and a dense cluster fits into one of
-// its cells: two row splits of 200 k, K = 96 / 200, skewed clusters 6.15 / 2.39 and 12.2 / 4.7, normal 3.26 / 2.48 and
-// 8.74 / 5.63, uniform 2.20 / 2.21 and 4.96 / 4.98; five of 20 k uniform, K = 96: 0.59 / 0.61.  One of 20 k uniform:
-// 0.164 / 0.204, hence the 65536 points.  Four: normal 5.28 / 4.04 (K = 96), but uniform 2.83 / 3.21 and one of 20 k
-// 0.21 / 0.26: the grid.  Six or more: the grid bins four of them (60 k uniform in eight, K = 20: 3.40 / 1.50; 60 k
-// normal in six, K = 40: 1.54 / 1.29).  Five, from K = 32 on: uniform 1.06 / 0.90 (five of 20 k, K = 40), 6.17 /
-// 5.16 (two of 200 k, K = 65), one row split of a million normal points, K = 40: 22 / 18.5, two of 200 k 6.45 / 7.03;
-// K = 16 uniform: 0.35 / 0.45.  Below 16384 points the sort's launches outweigh the search (10 k, K = 100: 0.110 /
-// 0.112 without the second look).
+// Where the tree is the better search.  Neither search is ahead for all data: the figures are the time of the tree over that of
+// the grid, whole forward, B200, for uniform points in a cube / normal ones / 50 clusters of width 0.02 ("mixture").
+// Below 16384 points the sort's launches outweigh the search (10 k in three coordinates, K = 100: 0.110 / 0.112 ms).
+//
+// D = 3: the grid's list of four slots a lane (K > 65) is slow, and a dense cluster fits into one of its cells.  400 k points
+// in two row splits, K = 96: 0.98 / 0.74 / 0.74, skewed clusters 0.41; from 65536 points on.
+// D = 4: K = 96 uniform 1.13, one row split of 20 k 1.2: the grid (but see long_tails).
+// D = 5, K > 65: 800 k in eight row splits, K = 66: 0.69 / 0.87 / 0.69; 17 k: 0.85 / 0.53 / 0.86.  From K = 40 on only with one or
+// two row splits, where the grid's last warps run on alone over sparse tails: 100 k, K = 40: 0.86 / 0.72 / 0.97, but in twenty
+// row splits 0.79 / 1.06 / 1.47 and 400 k in twenty 0.78 / 1.14 / 1.00.  K = 32: 100 k 0.92 / 1.05 / 1.25.
+// D >= 6: the grid bins four of the coordinates (60 k uniform in eight, K = 20: 3.40 / 1.50 ms; 60 k normal in six,
+// K = 40: 1.54 / 1.29).
 //
 // long_tails: the caller expects coordinates with sparse tails, as the learned ones of a GravNet layer have
 // (linear maps of many features).  In four dimensions the grid's last warps then walk empty cells long after all
@@ -415,7 +417,8 @@ extern "C" int fgc_knn_tree_preferred(int64_t n_vert, int32_t n_coords, int64_t 
         return 0;
     const bool tails = long_tails && n_coords == 4 && K >= 32 && n_vert <= 500000;
     const bool long_lists = n_coords == 3 && K > 65 && n_vert >= 65536;
-    if (!(long_lists || n_coords >= 6 || (n_coords == 5 && K >= 32) || tails)) return 0;
+    const bool five = n_coords == 5 && K >= (n_rs <= 3 ? 40 : 66);
+    if (!(long_lists || n_coords >= 6 || five || tails)) return 0;
     return tree_layout(knn_workspace_layout(n_vert, n_coords, n_rs, K), n_vert, n_coords, n_rs).fits ? 1 : 0;
 }
 

@@ -4,6 +4,8 @@ import ctypes
 import os
 import re
 
+import pytest
+
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
@@ -47,7 +49,6 @@ def test_bin_params_mirror_matches_header():
 
 
 def test_cpu_tensors_are_rejected_loudly():
-    import pytest
     import torch
     import fastgraphcompute_b200 as fgc
     with pytest.raises(RuntimeError, match="CUDA tensors only"):
@@ -81,3 +82,12 @@ def test_row_splits_batch_round_trip():
     assert torch.equal(strict_batch_from_row_splits(rs), batch)
     assert strict_batch_from_row_splits(torch.tensor([0, 2, 2, 5], dtype=torch.int32)).tolist() == [0, 0, 2, 2, 2]
     assert row_splits_from_strict_batch(torch.tensor([4, 4, 7])).tolist() == [0, 2, 3]
+
+
+@pytest.mark.parametrize("n,D,row_splits,K,long_tails,tree", [
+    (400000, 5, 1, 40, 0, 1), (400000, 5, 2, 65, 0, 1), (400000, 5, 3, 65, 0, 0), (400000, 5, 20, 40, 0, 0),
+    (400000, 5, 1, 39, 0, 0), (400000, 5, 20, 66, 0, 1), (16384, 5, 20, 66, 0, 1), (16383, 5, 20, 66, 0, 0)])
+def test_search_by_size(n, D, row_splits, K, long_tails, tree):
+    """The tree at the edges of the ranges where it was measured ahead of the grid."""
+    from fastgraphcompute_b200 import _cabi
+    assert _cabi.lib.fgc_knn_tree_preferred(n, D, row_splits + 1, K, long_tails) == tree
