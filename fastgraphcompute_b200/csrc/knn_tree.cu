@@ -393,32 +393,49 @@ static cudaError_t launch_boxes(const float *coords, int n, int n_coords, const 
 // the grid, whole forward, B200, for uniform points in a cube / normal ones / 50 clusters of width 0.02 ("mixture").
 // Below 16384 points the sort's launches outweigh the search (10 k in three coordinates, K = 100: 0.110 / 0.112 ms).
 //
-// D = 3: the grid's list of four slots a lane (K > 65) is slow, and a dense cluster fits into one of its cells.  400 k points
-// in two row splits, K = 96: 0.98 / 0.74 / 0.74, skewed clusters 0.41; from 65536 points on.
-// D = 4: K = 96 uniform 1.13, one row split of 20 k 1.2: the grid (but see long_tails).
-// D = 5, K > 65: 800 k in eight row splits, K = 66: 0.69 / 0.87 / 0.69; 17 k: 0.85 / 0.53 / 0.86.  From K = 40 on only with one or
-// two row splits, where the grid's last warps run on alone over sparse tails: 100 k, K = 40: 0.86 / 0.72 / 0.97, but in twenty
-// row splits 0.79 / 1.06 / 1.47 and 400 k in twenty 0.78 / 1.14 / 1.00.  K = 32: 100 k 0.92 / 1.05 / 1.25.
-// D >= 6: the grid bins four of the coordinates (60 k uniform in eight, K = 20: 3.40 / 1.50 ms; 60 k normal in six,
-// K = 40: 1.54 / 1.29).
+// D = 3, K >= 96: the grid's list of four slots a lane (K > 65) is slow, and a dense cluster fits into one of its cells.  400 k
+// points in two row splits, K = 96: 0.98 / 0.74 / 0.74, skewed clusters 0.41; K = 80: 1.06 / 0.70 / 0.67, K = 66: 1.20 / 0.78 /
+// 0.69.  From 65536 points on (one of 20 k uniform, K = 96: 0.164 / 0.204 ms).
+// D = 4: K = 100 uniform 1.08, one row split of 20 k 1.2: the grid (but see long_tails).
+// D = 5 and more: the grid bins four of the coordinates, the tree's boxes have them all.  K > 65: D = 5, 800 k in eight row
+// splits, K = 66: 0.69 / 0.87 / 0.69; D = 6, 400 k in twenty 0.57 / 0.91 / 0.60.  Shorter lists need the more coordinates the
+// shorter they are; with one or two row splits the grid's last warps run on alone over sparse tails, and the tree is ahead earlier:
+//   D = 5   100 k, K = 40: 0.86 / 0.72 / 0.97;  in twenty row splits 0.79 / 1.06 / 1.47;  K = 32: 0.92 / 1.05 / 1.25
+//   D = 6   400 k, K = 24: 0.56 / 0.78 / 1.19;  in twenty 0.72 / 1.30 / 1.19, K = 48: 0.63 / 1.08 / 0.86
+//   D = 7   400 k, K = 16: 0.51 / 0.89 / 1.30;  in twenty 0.62 / 1.24 / 1.21, K = 40: 0.51 / 1.06 / 0.93
+//   D = 8   400 k, K = 16: 0.46 / 0.86 / 1.25;  in twenty 0.53 / 1.15 / 1.15, K = 24: 0.44 / 1.04 / 1.06
+//   D = 9   100 k, K = 8: 0.50 / 0.85 / 0.87;  in five 0.55 / 0.91 / 0.94;  K = 2: 0.94 / 1.37 / 1.05
+//   D = 12  100 k, K = 2: 0.50 / 0.99 / 0.88;  in five 0.49 / 0.95 / 0.93
+// The tree's worst are small row splits of clusters with hardly more points than K: 5000 in 50 clusters, K = 65, D = 9: 1.55 (0.09
+// uniform, 0.62 normal).
 //
-// long_tails: the caller expects coordinates with sparse tails, as the learned ones of a GravNet layer have
-// (linear maps of many features).  In four dimensions the grid's last warps then walk empty cells long after all
-// others are done: normal points, K = 40 / 64, one row split of 20 k 0.41 / 0.19 and 0.47 / 0.22, of 100 k 1.04 /
-// 0.67 and 1.11 / 0.79, of 400 k 3.20 / 2.45 and 3.49 / 2.91, four of 50 k 1.38 / 1.24 and 1.68 / 1.48.  Batches of a
-// million points hide those warps (16 of 100 k: 8.28 / 9.18 and 10.7 / 11.0); so do K = 16 (four of 50 k:
-// 0.92 / 0.95) and three dimensions (four of 50 k, K = 40: 0.67 / 0.78); uniform points in a cube have no
-// tails (100 k, K = 40: 0.41 / 0.53).
+// long_tails: the caller expects coordinates with sparse tails, as the learned ones of a GravNet layer have (linear
+// maps of many features; "learned" are normal points mapped from 64 to 4).  In four dimensions the grid's last warps then walk
+// empty cells long after all others are done, unless many row splits hide them.  Learned, K = 32 / 40 / 64: one row split of 20 k
+// to 400 k 0.64 to 0.88, four of 25 k 0.93 / 0.78 / 0.74, ten of 20 k 1.10 / 0.96 / 0.89, fifty of 8 k 1.27 / 1.10 / 1.00, K = 66
+// there 0.75.  16 of 100 k: 8.28 / 9.18 (K = 40) and 10.7 / 11.0 ms (K = 64).  K = 16 has less to gain (four of 50 k:
+// 0.92 / 0.95 ms), so have three dimensions (four of 50 k, K = 40: 0.67 / 0.78 ms); uniform points in a cube have no tails
+// (100 k, K = 40: 0.41 / 0.53 ms).
 extern "C" int fgc_knn_tree_preferred(int64_t n_vert, int32_t n_coords, int64_t n_rs, int32_t K, int32_t long_tails)
 {
     using namespace fgc;
     if (n_vert < 16384 || n_vert > 0x7fffffff || n_coords < 2 || n_coords > FGC_MAX_KNN_DIMS || n_rs < 2 ||
         n_rs > 0x7fffffff || K < 1 || K > FGC_MAX_K)
         return 0;
-    const bool tails = long_tails && n_coords == 4 && K >= 32 && n_vert <= 500000;
-    const bool long_lists = n_coords == 3 && K > 65 && n_vert >= 65536;
-    const bool five = n_coords == 5 && K >= (n_rs <= 3 ? 40 : 66);
-    if (!(long_lists || n_coords >= 6 || five || tails)) return 0;
+    const int64_t n_events = n_rs - 1;
+    int least = FGC_MAX_K + 1;                   // shortest list for the tree
+    switch (n_coords) {
+    case 2: break;
+    case 3: if (n_vert >= 65536) least = 96; break;
+    case 4: if (long_tails && n_vert <= 500000) least = n_events <= 4 ? 32 : (n_events <= 16 ? 40 : 66); break;
+    case 5: least = n_events <= 2 ? 40 : 66; break;
+    case 6: least = n_events <= 2 ? 24 : 48; break;
+    case 7: least = n_events <= 2 ? 16 : 40; break;
+    case 8: least = n_events <= 2 ? 16 : 24; break;
+    case 9: case 10: case 11: least = 8; break;
+    default: least = 1;
+    }
+    if (K < least) return 0;
     return tree_layout(knn_workspace_layout(n_vert, n_coords, n_rs, K), n_vert, n_coords, n_rs).fits ? 1 : 0;
 }
 

@@ -86,7 +86,13 @@ def test_row_splits_batch_round_trip():
 
 @pytest.mark.parametrize("n,D,row_splits,K,long_tails,tree", [
     (400000, 5, 1, 40, 0, 1), (400000, 5, 2, 65, 0, 1), (400000, 5, 3, 65, 0, 0), (400000, 5, 20, 40, 0, 0),
-    (400000, 5, 1, 39, 0, 0), (400000, 5, 20, 66, 0, 1), (16384, 5, 20, 66, 0, 1), (16383, 5, 20, 66, 0, 0)])
+    (400000, 5, 1, 39, 0, 0), (400000, 5, 20, 66, 0, 1), (16384, 5, 20, 66, 0, 1), (16383, 5, 20, 66, 0, 0),
+    (65536, 3, 1, 96, 0, 1), (65535, 3, 1, 96, 0, 0), (400000, 3, 2, 95, 0, 0), (400000, 2, 1, 200, 0, 0),
+    (400000, 4, 1, 200, 0, 0), (400000, 4, 4, 32, 1, 1), (400000, 4, 4, 31, 1, 0), (400000, 4, 5, 39, 1, 0),
+    (400000, 4, 16, 40, 1, 1), (400000, 4, 17, 65, 1, 0), (400000, 4, 200, 66, 1, 1), (500001, 4, 1, 40, 1, 0),
+    (400000, 6, 2, 24, 0, 1), (400000, 6, 3, 47, 0, 0), (400000, 6, 3, 48, 0, 1), (400000, 7, 2, 15, 0, 0),
+    (400000, 7, 3, 40, 0, 1), (400000, 8, 2, 16, 0, 1), (400000, 8, 3, 23, 0, 0), (400000, 9, 50, 8, 0, 1),
+    (400000, 11, 1, 7, 0, 0), (400000, 12, 50, 1, 0, 1), (400000, 16, 1, 257, 0, 1)])
 def test_search_by_size(n, D, row_splits, K, long_tails, tree):
     """The tree at the edges of the ranges where it was measured ahead of the grid."""
     from fastgraphcompute_b200 import _cabi
