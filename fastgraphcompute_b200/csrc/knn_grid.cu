@@ -46,9 +46,6 @@ namespace fgc {
 __device__ void grid_setup(KnnGrid *g, const int64_t *__restrict__ row_splits, int n_rs, int n_vert,
                            int n_bin_dims, int bins_target, int bins_cap_first, int bins_cap, int bad_rs, int mirror);
 
-// Fused finite check + min/max of the binned coordinates; clears the cell table (all of its
-// capacity: the grid that decides how much of it is used does not exist yet); the CTA that
-// finishes last (a ticket counter, no waiting) checks the row splits and chooses the grid.
 // Before the grid of a second look: an empty header and tickets where there are rows to search again, else a
 // status word that ends the kernels of the grid at once.
 __global__ void __launch_bounds__(256)
@@ -66,10 +63,15 @@ k_tie_gate(KnnGrid *__restrict__ g, const KnnTree *__restrict__ t, int limit)
     for (int i = threadIdx.x; i < (int)((kGridHeaderBytes + kHardTicketBytes) / sizeof(int)); i += 256) ((int *)g)[i] = 0;
 }
 
+// Fused finite check + min/max of the binned coordinates; clears the cell table (all of its
+// capacity: the grid that decides how much of it is used does not exist yet); counts the points that may
+// be neighbours (mirror > 1); the CTA that finishes last (a ticket counter, no waiting) checks the row splits and
+// chooses the grid.
 __global__ void __launch_bounds__(256)
-k_minmax_setup(const float *__restrict__ coords, int n_vert, int n_coords, int n_bin_dims, KnnGrid *g,
-               int *__restrict__ counts, long long n_counts, const int64_t *__restrict__ row_splits, int n_rs,
-               int bins_target, int bins_cap_first, int bins_cap, int mirror, int gated)
+k_minmax_setup(const float *__restrict__ coords, int n_vert, int n_coords, int n_bin_dims,
+               const int64_t *__restrict__ direction, KnnGrid *g, int *__restrict__ counts, long long n_counts,
+               const int64_t *__restrict__ row_splits, int n_rs, int bins_target, int bins_cap_first, int bins_cap,
+               int mirror, int adaptive, int gated)
 {
     chain_wait();
     chain_release();
@@ -78,9 +80,13 @@ k_minmax_setup(const float *__restrict__ coords, int n_vert, int n_coords, int n
          i += (long long)gridDim.x * blockDim.x)
         counts[i] = 0;
     uint32_t lmin[4] = {0, 0, 0, 0}, lmax[4] = {0, 0, 0, 0};
-    uint32_t bad = 0;
+    uint32_t bad = 0, n_cand = 0;
     for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n_vert; v += gridDim.x * blockDim.x) {
         const float *row = coords + (size_t)v * n_coords;
+        if (mirror > 1) {
+            const int64_t d = direction[v];
+            n_cand += d != 1 && d != 2;
+        }
         for (int c = 0; c < n_coords; c++) {
             const float x = __ldg(row + c);
             if (!is_finite_bits(x)) bad = 1;
@@ -92,10 +98,14 @@ k_minmax_setup(const float *__restrict__ coords, int n_vert, int n_coords, int n
             }
         }
     }
-    __shared__ uint32_t s_min[4], s_max[4], s_bad;
+    __shared__ uint32_t s_min[4], s_max[4], s_bad, s_cand;
     if (threadIdx.x < 4) { s_min[threadIdx.x] = 0; s_max[threadIdx.x] = 0; }
-    if (threadIdx.x == 0) s_bad = 0;
+    if (threadIdx.x == 0) { s_bad = 0; s_cand = 0; }
     __syncthreads();
+    if (mirror > 1) {
+        n_cand = __reduce_add_sync(FGC_FULL_MASK, n_cand);
+        if ((threadIdx.x & 31) == 0) atomicAdd(&s_cand, n_cand);
+    }
 #pragma unroll
     for (int c = 0; c < 4; c++) {
         const uint32_t a = __reduce_max_sync(FGC_FULL_MASK, lmin[c]);
@@ -109,6 +119,7 @@ k_minmax_setup(const float *__restrict__ coords, int n_vert, int n_coords, int n
         atomicMax(&g->max_key[threadIdx.x], s_max[threadIdx.x]);
     }
     if (threadIdx.x == 0 && s_bad) atomicOr(&g->nonfinite, 1u);
+    if (threadIdx.x == 0 && mirror > 1) atomicAdd(&g->sum_sq, (unsigned long long)s_cand);   // (free until the density pass)
     // the last CTA to arrive sees every CTA's extrema and sets the grid up
     __shared__ int s_last;
     __threadfence();
@@ -124,6 +135,18 @@ k_minmax_setup(const float *__restrict__ coords, int n_vert, int n_coords, int n
     bad_rs = __syncthreads_or(bad_rs);
     if (threadIdx.x == 0) {
         g->stat_blocks_done = 0;       // the density pass counts its CTAs with the same ticket
+        if (mirror > 1) {
+            const unsigned long long n_may = atomicExch(&g->sum_sq, 0ull);
+            if (8 * n_may >= 7 * (unsigned long long)n_vert) {
+                // (nearly) all points: one set, which may have twice the cells
+                mirror = 1;
+                bins_cap *= 2;
+            } else if (adaptive) {
+                // cells sized for the points that are met in a walk; not below a third of the points, so that the cells of
+                // the others stay small enough to be put in order
+                bins_target = (int)(bins_target * fmax((double)n_may / (double)n_vert, 1.0 / 3.0) + 0.5);
+            }
+        }
         grid_setup(g, row_splits, n_rs, n_vert, n_bin_dims, bins_target, bins_cap_first, bins_cap, bad_rs, mirror);
     }
 }
@@ -637,16 +660,15 @@ static int knn_build_grid(const float *coords, int64_t n_vert, int32_t n_coords,
     // points in its own cell.
     // With direction flags the points that may not be neighbours go to a second set of cells behind the
     // first: a walk then meets candidates only (B200, a third of the points candidates: ten row splits of
-    // 100 k, K = 64: 2.32 -> 1.33 ms, 64 of 2900, K = 16: 0.220 -> 0.165; no point restricted: 2.98 -> 3.01 and
-    // 0.291 -> 0.269).  One set where the table could not hold two.
+    // 100 k, K = 64: 2.34 -> 1.33 ms, 64 of 2900, K = 16: 0.250 -> 0.193; half of them: 4.56 -> 3.01, 0.386 -> 0.319).
+    // One set where nearly all points are candidates (nine tenths: 3.2 -> 3.0 ms with two, but 1 M clustered points in four
+    // coordinates, K = 20, 2.8 -> 4.1, for want of cells), and where the table could not hold two.
     const int mirror = direction_or_null && 2 * (int64_t)n_events <= L.cap_bins ? 2 : 1;
     const bool adaptive = !(target_occupancy > 0.f);
     if (adaptive) {
         target_occupancy = (float)K / 21.0f;
         if (target_occupancy < 1.5f) target_occupancy = 1.5f;
         if (target_occupancy > 3.0f) target_occupancy = 3.0f;
-        // how many points are candidates is not known here: between all of them and a third
-        if (mirror > 1) target_occupancy *= 2.0f;
     }
     float seen_target = (float)K / 6.0f;
     if (seen_target < 4.f) seen_target = 4.f;
@@ -669,9 +691,9 @@ static int knn_build_grid(const float *coords, int64_t n_vert, int32_t n_coords,
     const int scan_blocks = (int)ceil_div64(max_entries, kScanTile);
     int bins_cap_first = bins_target > (bins_cap - 64) / 4 ? bins_cap : 4 * bins_target + 64;
     if (!adaptive) bins_cap_first = bins_cap;
-    k_minmax_setup<<<red_blocks, 256, 0, s>>>(coords, n, n_coords, n_bin_dims, grid, counts,
+    k_minmax_setup<<<red_blocks, 256, 0, s>>>(coords, n, n_coords, n_bin_dims, direction_or_null, grid, counts,
                                               (long long)bins_cap_first * n_events * mirror + 1, row_splits, (int)n_rs,
-                                              bins_target, bins_cap_first, bins_cap, mirror, only_for_ties);
+                                              bins_target, bins_cap_first, bins_cap, mirror, adaptive, only_for_ties);
     FGC_CHECK_LAUNCH();
     const int allow_fallback = adaptive && n_coords == 4 && forced == 0;
     FGC_RETURN_IF_CUDA(launch_chained(k_histogram, pt_blocks, 256, 0, s, coords, n, n_coords, row_splits, (int)n_rs, direction_or_null,

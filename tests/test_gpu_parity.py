@@ -1025,3 +1025,26 @@ def test_tree_search_on_a_lattice(D, K):
     parity.assert_knn_parity(idx.cpu().numpy(), dist.cpu().numpy(), oi, od, what="lattice D=%d" % D)
     assert torch.equal(idx[:, 0], torch.arange(n, device=DEV)) and int(idx.min()) >= -1
     assert int(ws[:4].view(torch.int32)) == 0                                     # status of the workspace
+
+
+def test_cells_follow_the_points_that_may_be_neighbours():
+    """Direction flags that restrict nothing leave the cells as they are without flags; with a third of the points as
+    candidates there are about a third of the cells."""
+    import importlib
+    km = importlib.import_module("fastgraphcompute_b200.extensions.binned_select_knn")
+    g = torch.Generator().manual_seed(2)
+    n = 60000
+    rs = torch.tensor([0, n], device=DEV)
+
+    def cells(pts, direction):
+        _, _, ws = km.knn_forward_raw(pts, rs, 32, direction, False, count_evals=True)
+        counters, shape, width = km.read_counters(ws)
+        return shape[0] * shape[1] * shape[2], width
+    every = torch.full((n,), 3, device=DEV)
+    third = (torch.rand((n,), generator=g) < 1 / 3).to(DEV)
+    pts = torch.rand((n, 3), generator=g).to(DEV)
+    centres = torch.rand((50, 3), generator=g)
+    clustered = (centres[torch.randint(0, 50, (n,), generator=g)] + 0.02 * torch.randn((n, 3), generator=g)).to(DEV)
+    for x in (pts, clustered):
+        assert cells(x, every) == cells(x, None)
+    assert 0.2 < cells(pts, torch.where(third, 3, 1))[0] / cells(pts, None)[0] < 0.5
