@@ -4,29 +4,91 @@
 // library and for the event and the pinned word of the status check; here they cost one call, and the
 // wait for the status word happens without the interpreter (two row splits of 5000 points, K = 16, forward and
 // backward, B200: 202 -> 157 us; a GravNet layer on ten small events: 308 -> 285 us).
+#include <mutex>
+
 #include "knn_tree.cuh"
 
 namespace fgc {
 
-// Two page-locked words per host thread, mapped on every device, given back when the thread ends.  A call
-// that uses them waits for them, so one slot per thread is enough for any number of streams.
+// Two page-locked words, mapped on every device, and an event of one device.  A call that waits takes a slot of its own
+// for the time of the wait and gives it back, so any number of threads and streams may call at once.  Slots are shared
+// by all threads: a thread that ends frees nothing (freeing page-locked memory may wait for the device, and breaks another
+// thread's graph capture).  At most kKeptSlots stay for later calls, i.e. 4 KB.
 struct StatusSlot {
     int32_t *words = nullptr;
-    ~StatusSlot() { if (words) cudaFreeHost(words); }
+    cudaEvent_t ready = nullptr;
+    int device = -1;
+};
+constexpr size_t kKeptSlots = 64;
+
+struct StatusPool {
+    std::mutex lock;
+    StatusSlot kept[kKeptSlots];
+    size_t n = 0;
 };
 
-static int32_t *status_slot()
+static StatusPool &status_pool()
 {
-    static thread_local StatusSlot slot;
-    if (!slot.words && cudaHostAlloc((void **)&slot.words, 64, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess)
-        slot.words = nullptr;
-    return slot.words;
+    static StatusPool *pool = new StatusPool;      // never destroyed: threads may outlive static objects
+    return *pool;
+}
+
+// Allocations that are harmless to a graph capture of another thread.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+static void free_slot(StatusSlot &s)
+{
+    const RelaxedCapture relaxed;
+    if (s.ready) cudaEventDestroy(s.ready);
+    if (s.words) cudaFreeHost(s.words);
+    s = StatusSlot();
+}
+
+static cudaError_t take_slot(StatusSlot &s)
+{
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    {
+        StatusPool &pool = status_pool();
+        const std::lock_guard<std::mutex> hold(pool.lock);
+        for (size_t i = pool.n; i-- > 0;)
+            if (pool.kept[i].device == device) {
+                s = pool.kept[i];
+                pool.kept[i] = pool.kept[--pool.n];
+                return cudaSuccess;
+            }
+    }
+    const RelaxedCapture relaxed;
+    s.device = device;
+    e = cudaHostAlloc((void **)&s.words, 64, cudaHostAllocPortable | cudaHostAllocMapped);
+    if (e != cudaSuccess) s.words = nullptr;
+    else e = cudaEventCreateWithFlags(&s.ready, cudaEventDisableTiming);
+    if (e != cudaSuccess) free_slot(s);
+    return e;
+}
+
+static void give_back(StatusSlot &s)
+{
+    {
+        StatusPool &pool = status_pool();
+        const std::lock_guard<std::mutex> hold(pool.lock);
+        if (pool.n < kKeptSlots) {
+            pool.kept[pool.n++] = s;
+            return;
+        }
+    }
+    free_slot(s);
 }
 
 static int knn_forward_launch(const float *coords, int64_t n_vert, int32_t n_coords, const int64_t *row_splits, int64_t n_rs,
                               int32_t K, const int64_t *direction, int32_t tf_compat, float target_occupancy, int32_t flags,
                               int64_t *out_idx, float *out_distsq, int32_t *out_order, void *ws, size_t ws_bytes,
-                              int32_t *words, cudaEvent_t ready, fgc_stream_t stream)
+                              const StatusSlot *status, bool *published, fgc_stream_t stream)
 {
     const bool tree = (flags & FGC_FORWARD_TREE) != 0;
     int rc;
@@ -37,10 +99,11 @@ static int knn_forward_launch(const float *coords, int64_t n_vert, int32_t n_coo
                                      ws_bytes, stream);
     }
     if (rc != FGC_OK) return rc;
-    if (ready) {
-        rc = fgc_knn_publish_grid_info(ws, words, stream);
+    if (status) {
+        rc = fgc_knn_publish_grid_info(ws, status->words, stream);
         if (rc != FGC_OK) return rc;
-        FGC_RETURN_IF_CUDA(cudaEventRecord(ready, (cudaStream_t)stream));
+        *published = true;
+        FGC_RETURN_IF_CUDA(cudaEventRecord(status->ready, (cudaStream_t)stream));
     }
     const bool ties = tree && (flags & FGC_FORWARD_GRID_TIES) != 0;
     if (tree) rc = knn_search_tree(n_vert, n_coords, row_splits, n_rs, K, direction != nullptr, tf_compat, ties, out_idx,
@@ -75,25 +138,28 @@ extern "C" int fgc_knn_forward(const float *coords, int64_t n_vert, int32_t n_co
                                int32_t *info_host_or_null, fgc_stream_t stream)
 {
     using namespace fgc;
-    int32_t *words = nullptr;
-    cudaEvent_t ready = nullptr;
-    if (info_host_or_null) {
-        words = status_slot();
-        if (!words) return (int)cudaErrorMemoryAllocation;
-        FGC_RETURN_IF_CUDA(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming));
-    }
+    if (!info_host_or_null)
+        return knn_forward_launch(coords, n_vert, n_coords, row_splits, n_rs, K, direction_or_null, tf_compat, target_occupancy,
+                                  flags, out_idx, out_distsq, out_order_or_null, workspace, workspace_bytes, nullptr, nullptr,
+                                  stream);
+    StatusSlot slot;
+    FGC_RETURN_IF_CUDA(take_slot(slot));
+    bool published = false;
     int rc = knn_forward_launch(coords, n_vert, n_coords, row_splits, n_rs, K, direction_or_null, tf_compat, target_occupancy,
-                                flags, out_idx, out_distsq, out_order_or_null, workspace, workspace_bytes, words, ready,
+                                flags, out_idx, out_distsq, out_order_or_null, workspace, workspace_bytes, &slot, &published,
                                 stream);
-    if (ready) {
-        // (an event that was never recorded is complete: no wait after an early error)
-        const cudaError_t e = cudaEventSynchronize(ready);
-        cudaEventDestroy(ready);
-        if (rc == FGC_OK) rc = (int)e;
-        if (rc == FGC_OK) {
-            info_host_or_null[0] = ((volatile int32_t *)words)[0];
-            info_host_or_null[1] = ((volatile int32_t *)words)[1];
-        }
+    if (!published) {
+        give_back(slot);
+        return rc;
     }
+    // (also after an error of a later launch: the words are on their way)
+    const cudaError_t e = cudaEventSynchronize(slot.ready);
+    if (rc == FGC_OK) rc = (int)e;
+    if (rc == FGC_OK) {
+        info_host_or_null[0] = ((volatile int32_t *)slot.words)[0];
+        info_host_or_null[1] = ((volatile int32_t *)slot.words)[1];
+    }
+    // after an error the event may not stand for these words: the slot is not used again
+    if (rc == FGC_OK) give_back(slot);
     return rc;
 }

@@ -226,7 +226,8 @@ int fgc_knn_search_tree(int64_t n_vert, int32_t n_coords, const int64_t *row_spl
  * flags: FGC_SEARCH_COUNT, FGC_SEARCH_GRID3, FGC_SEARCH_GRID4 as for fgc_knn_search.
  * info_host_or_null [2], host memory: receives what fgc_knn_publish_grid_info stores.  The call then WAITS
  * until the build is done (not for the search, which is enqueued by then) and must not be captured into a graph;
- * it keeps 64 bytes of page-locked memory per calling thread.  Without it nothing waits.
+ * it takes two page-locked words and an event from a pool that all threads share (64 of them are kept).  Without it
+ * nothing waits.
  */
 #define FGC_FORWARD_TREE 64    /* flags: search on a tree instead of a grid */
 #define FGC_FORWARD_GRID_TIES 128 /* with it: rows with a choice among equal K-th distances are searched again on a grid,

@@ -1048,3 +1048,49 @@ def test_cells_follow_the_points_that_may_be_neighbours():
     for x in (pts, clustered):
         assert cells(x, every) == cells(x, None)
     assert 0.2 < cells(pts, torch.where(third, 3, 1))[0] / cells(pts, None)[0] < 0.5
+
+
+def test_forward_from_threads_that_come_and_go():
+    """Calls from many threads at once give the results of a single one, on streams of their own; and a thread that ends
+    while another one captures a graph leaves the capture alone (nothing is freed with a thread)."""
+    import threading
+    g = torch.Generator().manual_seed(7)
+    inputs = [torch.rand((500 + 100 * i, 3), generator=g).to(DEV) for i in range(12)]
+    splits = [torch.tensor([0, x.shape[0]], device=DEV) for x in inputs]
+    expected = [fgc.binned_select_knn(9, x, rs) for x, rs in zip(inputs, splits)]
+    torch.cuda.synchronize()
+    wrong = []
+
+    def work(i):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(5):
+                idx, dist = fgc.binned_select_knn(9, inputs[i], splits[i])
+                torch.cuda.current_stream().synchronize()
+                if not (torch.equal(idx, expected[i][0]) and torch.equal(dist, expected[i][1])):
+                    wrong.append(i)
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(12)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
+
+    called, leave = threading.Event(), threading.Event()
+
+    def one_call():
+        fgc.binned_select_knn(9, inputs[0], splits[0])
+        torch.cuda.synchronize()
+        called.set()
+        leave.wait(60)
+    thread = threading.Thread(target=one_call)
+    thread.start()
+    assert called.wait(60)
+    x = torch.zeros(1000, device=DEV)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        x.add_(1.0)
+        leave.set()
+        thread.join()
+        x.add_(1.0)
+    graph.replay()
+    assert bool((x == 2.0).all())
