@@ -51,7 +51,7 @@ grid_probe_every = 64
 # Search on a tree of boxes instead of a grid: None lets the library choose (fgc_knn_tree_preferred).
 search_tree = None
 pad_min_pairs = 1 << 19    # backward for D = 3, 5, 6, 7: pad to four / eight coordinates from this many (row, slot) pairs on
-_grid_memory = {}        # (device, N, row splits, K) -> [form, calls since the last automatic choice]
+_grid_memory = {}        # (device, N, row splits, K, with direction flags) -> [form, calls since the last automatic choice]
 # forward calls may come from several host threads (one per stream or device) and the backward runs
 # on autograd's own threads: the two module-level tables are only touched under this lock
 _tables_lock = threading.Lock()
@@ -93,12 +93,13 @@ def _forward(coords, row_splits, K, direction, tf_compat, count_evals, order, lo
         if search_tree is None else search_tree)
     check = check_status
     form = 0
+    key = (dev.index, n_vert, n_rs, K, direction is not None)       # (flags change the cells, and with them the form)
     if n_coords == 4 and not tree:
         if grid_dims in (3, 4):
             form = grid_dims
         elif grid_dims == 0 and check:
             with _tables_lock:
-                mem = _grid_memory.get((dev.index, n_vert, n_rs, K))
+                mem = _grid_memory.get(key)
                 if mem is not None and mem[1] < grid_probe_every:
                     form = mem[0]
                     mem[1] += 1
@@ -124,7 +125,7 @@ def _forward(coords, row_splits, K, direction, tf_compat, count_evals, order, lo
             with _tables_lock:
                 if len(_grid_memory) > 256:
                     _grid_memory.clear()
-                _grid_memory[(dev.index, n_vert, n_rs, K)] = [info[1] & 15, 0]      # what the device chose
+                _grid_memory[key] = [info[1] & 15, 0]      # what the device chose
     return idx, dist, ws
 
 

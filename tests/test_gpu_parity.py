@@ -1094,3 +1094,17 @@ def test_forward_from_threads_that_come_and_go():
         x.add_(1.0)
     graph.replay()
     assert bool((x == 2.0).all())
+
+
+def test_grid_form_is_remembered_with_and_without_flags_apart(forward_flags):
+    """Four coordinates: the form that a call with direction flags chose says nothing about one without."""
+    import importlib
+    km = importlib.import_module("fastgraphcompute_b200.extensions.binned_select_knn")
+    n = 5003
+    pts = torch.rand((n, 4), generator=torch.Generator().manual_seed(1)).to(DEV)
+    rs = torch.tensor([0, n], device=DEV)
+    direction = (torch.arange(n, device=DEV) % 3)
+    km._grid_memory.clear()
+    for d in (direction, None, direction, None):
+        fgc.binned_select_knn(12, pts, rs, direction=d)
+    assert [bool(f & 24) for f in forward_flags] == [False, False, True, True]
