@@ -255,7 +255,9 @@ def binned_select_knn_with_order(K: int, coords: torch.Tensor, row_splits: torch
     order) with order int32 [N], a permutation of the points that keeps spatial neighbours
     together.  Kernels that walk the neighbour rows (GravNet aggregation) use it as their
     processing order for cache locality.  long_tails: the points are expected to have sparse tails (learned
-    coordinates); the choice of the search takes it into account, the result does not depend on it.
+    coordinates); the choice of the search takes it into account.  The distances do not depend on it, but which of
+    several points at exactly the K-th distance is kept may: with long_tails the tree's own choice stands, without it
+    the grid's (while a sixteenth of the rows or fewer have one).  A traced or compiled call has no such hint.
 
     Written in the TorchScript subset (the reference's wrapper is ``@torch.jit.script``,
     extensions/binned_select_knn.py:11): modules that call it can be scripted, traced, saved and
