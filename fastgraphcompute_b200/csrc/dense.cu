@@ -15,9 +15,9 @@
 //                   every run.
 //
 // Bound by the fp32 multiply-add rate (2 N O C operations).  Forward and backward of one layer with ReLU,
-// library only -> with these kernels (B200, ms): 200 k rows, 128 to 128: 0.994 -> 0.593; 64 to 128: 0.856 ->
-// 0.394; 128 to 10: 0.355 -> 0.218; 1.6 M rows, 128 to 64: 3.11 -> 2.33; 10 k rows, 128 to 64: 0.153 -> 0.169
-// (launches; the caller keeps the modules there).  Relative error of dW against 64 bits at 200 k rows,
+// library only -> with these kernels (B200, ms): 200 k rows, 128 to 128: 1.02 -> 0.64; 64 to 128: 0.88 ->
+// 0.44; 128 to 10: 0.385 -> 0.281; 800 k rows, 128 to 64: 1.70 -> 1.20; where they lose (launches, narrow and wide
+// weights) the caller keeps the modules.  Relative error of dW against 64 bits at 200 k rows,
 // 128 to 128: 1.1e-6 (library) -> 3.5e-7.
 #include "fgc_common.cuh"
 

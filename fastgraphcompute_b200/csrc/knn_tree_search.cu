@@ -17,7 +17,7 @@
 // What bounds it: issue slots (0.80 of them used; compares, minima and logic run at half rate).  A
 // query of 500 k uniform points in three coordinates with K = 64 takes 3090 warp instructions: 15
 // leaves, 6 nodes, 2.5 selections and the final sort.  Against the grid search (build and
-// search, B200): 800 k points in skewed clusters, K = 128: 16.4 -> 4.3 ms; 400 k uniform, K = 128: 2.82 ->
+// search, B200; the second look at tied rows, which knn_forward.cu adds, takes about 0.03 ms without such rows): 800 k points in skewed clusters, K = 128: 16.4 -> 4.3 ms; 400 k uniform, K = 128: 2.82 ->
 // 2.20; 500 k normal in five coordinates, K = 40: 9.84 -> 8.8; 60 k uniform in eight, K = 20: 3.40 -> 1.5;
 // but 1.6 M uniform in three, K = 64: 4.6 -> 5.3, so the grid stays for few coordinates and short lists.
 //
