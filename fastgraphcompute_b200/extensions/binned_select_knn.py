@@ -51,7 +51,7 @@ grid_probe_every = 64
 # Search on a tree of boxes instead of a grid: None lets the library choose (fgc_knn_tree_preferred).
 search_tree = None
 pad_min_pairs = 1 << 19    # backward for D = 3, 5, 6, 7: pad to four / eight coordinates from this many (row, slot) pairs on
-_grid_memory = {}        # (device, N, row splits, K, with direction flags) -> [form, calls since the last automatic choice]
+_grid_memory = {}        # (device, N, row splits, K[, "direction"]) -> [form, calls since the last automatic choice]
 # forward calls may come from several host threads (one per stream or device) and the backward runs
 # on autograd's own threads: the two module-level tables are only touched under this lock
 _tables_lock = threading.Lock()
@@ -93,7 +93,8 @@ def _forward(coords, row_splits, K, direction, tf_compat, count_evals, order, lo
         if search_tree is None else search_tree)
     check = check_status
     form = 0
-    key = (dev.index, n_vert, n_rs, K, direction is not None)       # (flags change the cells, and with them the form)
+    # (direction flags change the cells, and with them the form: remembered apart)
+    key = (dev.index, n_vert, n_rs, K) if direction is None else (dev.index, n_vert, n_rs, K, "direction")
     if n_coords == 4 and not tree:
         if grid_dims in (3, 4):
             form = grid_dims
