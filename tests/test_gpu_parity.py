@@ -1108,3 +1108,30 @@ def test_grid_form_is_remembered_with_and_without_flags_apart(forward_flags):
     for d in (direction, None, direction, None):
         fgc.binned_select_knn(12, pts, rs, direction=d)
     assert [bool(f & 24) for f in forward_flags] == [False, False, True, True]
+
+
+def test_tree_search_in_a_cuda_graph(forward_flags, monkeypatch):
+    """The tree, with its second look at tied rows, captured without the status check and replayed on other points."""
+    import importlib
+    km = importlib.import_module("fastgraphcompute_b200.extensions.binned_select_knn")
+    n, D, K = 20000, 6, 30
+    g = torch.Generator().manual_seed(11)
+    points = [torch.rand((n, D), generator=g).to(DEV) for _ in range(2)]
+    points.append(torch.randint(0, 6, (n, D), generator=g).float().to(DEV))          # a lattice: marks taken off again
+    rs = torch.tensor([0, 9000, n], device=DEV)
+    expected = [km.knn_forward_raw(p, rs, K, None, False)[:2] for p in points]
+    monkeypatch.setattr(km, "check_status", False)
+    static = points[0].clone()
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        km.knn_forward_raw(static, rs, K, None, False)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        idx, dist, _ = km.knn_forward_raw(static, rs, K, None, False)
+    assert all(f & 64 for f in forward_flags)
+    for p, (ei, ed) in zip(points, expected):
+        static.copy_(p)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(idx, ei) and torch.equal(dist, ed)
