@@ -14,10 +14,11 @@
 // the result is exactly the K-1 smallest computed distances, whatever the tree.  Boxes at exactly the bound
 // are visited, so that a candidate equal to the K-th distance that is left out is always noticed.
 //
-// What bounds it: issue slots (0.80 of them used; compares, minima and logic run at half rate).  A
-// query of 500 k uniform points in three coordinates with K = 64 takes 3090 warp instructions: 15
-// leaves, 6 nodes, 2.5 selections and the final sort.  Against the grid search (build and
-// search, B200; the second look at tied rows, which knn_forward.cu adds, takes about 0.03 ms without such rows): 800 k points in skewed clusters, K = 128: 16.4 -> 4.3 ms; 400 k uniform, K = 128: 2.82 ->
+// What bounds it: issue slots (0.88 of them used; compares, minima and logic run at half rate).  A
+// query of 500 k uniform points in three coordinates with K = 64 takes 3390 warp instructions, the 500 k of them 1.69 ms; one of
+// 200 k normal points in five with K = 40 takes 11 600, at 0.63 of the issue slots (the last warps run on alone).  Against
+// the grid search (build and search, B200; the second look at tied rows, which knn_forward.cu adds, takes 0.02 ms at 20 k
+// points, with a few such rows 0.8 at 800 k): 800 k points in skewed clusters, K = 128: 16.4 -> 4.3 ms; 400 k uniform, K = 128: 2.82 ->
 // 2.20; 500 k normal in five coordinates, K = 40: 9.84 -> 8.8; 60 k uniform in eight, K = 20: 3.40 -> 1.5;
 // but 1.6 M uniform in three, K = 64: 4.6 -> 5.3, so the grid stays for few coordinates and short lists.
 //
