@@ -27,6 +27,7 @@ struct KnnTree {
     float origin[kTreeKeyDims];
     float scale;                        // cells of the Hilbert curve per unit length
     int32_t n_tied;                     // rows marked kTieRow by the search
+    int32_t n_listed;                   // queries that the search by groups leaves to the search one by one
 };
 static_assert(sizeof(KnnTree) <= kHardTicketBytes, "tree record too large");
 
@@ -82,6 +83,42 @@ inline TreeLayout tree_layout(const KnnWorkspace &w, int64_t n_vert, int n_coord
     return t;
 }
 
+// List length class of a search: K - 1 <= 32 R.
+inline int tree_list_rows(int K) { return K <= 33 ? 1 : (K <= 65 ? 2 : (K <= 129 ? 4 : 8)); }
+
+// Scratch of a search by groups: what k_tree_groups leaves for the queries of `slots` leaf slots.
+struct TreeScratch {
+    int slots, list_cap;
+    int *list, *list_n;
+    float *bound;
+};
+constexpr int kGroupDims = 5;                                 // searches by groups take up to so many coordinates
+// Leaves that a leaf's queries may need (mean over uniform, normal and clustered points, K = 16 to 200: 36 to 110 in three
+// coordinates, 140 to 350 in four, 1000 in five); with more they are searched one by one.
+inline int tree_list_cap(int n_coords) { return n_coords <= 3 ? 512 : (n_coords == 4 ? 1024 : 3072); }
+constexpr size_t kTreeScratchBytes = (size_t)256 << 20;       // larger searches take several rounds
+inline size_t tree_slot_bytes(int n_coords) { return 4 * ((size_t)tree_list_cap(n_coords) + 1 + 32); }
+// What a workspace for searches by groups holds behind the sections of the grid.
+inline size_t tree_extra_bytes(int64_t n_vert, int n_coords, int64_t n_rs)
+{
+    if (n_coords > kGroupDims) return 0;
+    const size_t most = kTreeScratchBytes / tree_slot_bytes(n_coords), slots = (size_t)(n_vert / 32 + n_rs + 1);
+    return (slots < most ? slots : most) * tree_slot_bytes(n_coords);
+}
+inline bool tree_scratch(const KnnWorkspace &w, int n_coords, char *ws, size_t bytes, TreeScratch *out)
+{
+    if (n_coords > kGroupDims || bytes < w.total + tree_slot_bytes(n_coords)) return false;
+    size_t slots = (bytes - w.total) / tree_slot_bytes(n_coords);
+    const size_t most = kTreeScratchBytes / tree_slot_bytes(n_coords);
+    if (slots > most) slots = most;
+    out->slots = (int)slots;
+    out->list_cap = tree_list_cap(n_coords);
+    out->list = (int *)(ws + w.total);
+    out->list_n = out->list + slots * out->list_cap;
+    out->bound = (float *)(out->list_n + slots);
+    return true;
+}
+
 // Mark in slot 0 of a row whose K-th distance several points share, of which some are left out.
 constexpr int64_t kTieRow = INT64_MIN;
 // Rows that may be marked and searched again, as a share of all rows: see knn_forward_launch.
@@ -94,6 +131,11 @@ constexpr int32_t kStatusNoGrid = 1 << 30;
 int knn_search_tree(int64_t n_vert, int32_t n_coords, const int64_t *row_splits, int64_t n_rs, int32_t K,
                     int32_t has_direction, int32_t tf_compat, bool mark_ties, int64_t *out_idx, float *out_distsq,
                     void *workspace, size_t workspace_bytes, fgc_stream_t stream);
+// The same for all queries of a leaf at once, directly behind fgc_knn_build_tree, in a workspace with the scratch that
+// fgc_knn_workspace_bytes counts in (tree_scratch).
+int knn_search_tree_groups(int64_t n_vert, int32_t n_coords, const int64_t *row_splits, int64_t n_rs, int32_t K,
+                           int32_t has_direction, int32_t tf_compat, bool mark_ties, int64_t *out_idx, float *out_distsq,
+                           void *workspace, size_t workspace_bytes, fgc_stream_t stream);
 // fgc_knn_build_grid_dims behind a search with mark_ties: builds nothing (kStatusNoGrid) where no row is marked,
 // or more than a kTieShare-th of them are.
 int knn_build_grid_for_ties(const float *coords, int64_t n_vert, int32_t n_coords, const int64_t *row_splits, int64_t n_rs,

@@ -1,0 +1,48 @@
+// Parts shared by the kernels that search the tree: one query at a time (knn_tree_search.cu) and all queries of a leaf
+// (knn_tree_group.cu).
+#pragma once
+#include "knn_tree.cuh"
+
+namespace fgc {
+
+struct TreeArgs {
+    const float4 *scoords;
+    const int *sorig;
+    const uint8_t *sflag;      // nullptr: no direction restriction
+    const float4 *box[3];      // leaves, nodes, top nodes
+    const int64_t *row_splits;
+    KnnGrid *grid;
+    KnnTree *tree;
+    int64_t *out_idx;
+    float *out_dist;
+    int n_vert;
+    int n_rs;
+    int K;
+    int tf_compat;
+    int mark_ties;             // rows with a choice at the K-th distance get kTieRow in slot 0
+    // the search by groups only
+    int slot0, n_slots;        // leaf slots of this launch: from the one up to the other
+    int list_cap;
+    int *listed;               // queries that are searched one by one instead (places in curve order)
+    int *list, *list_n;        // leaves [slots of this launch][list_cap] that a leaf's queries may need; their number (-1: no points)
+    float *bound;              // per query of this launch: at least K - 1 candidates are this near (kNoQuery, kListedQuery)
+};
+
+constexpr uint32_t kNoBox = 0xffffffffu;
+constexpr float kNoQuery = -1.f;         // bound of a query that may not have neighbours
+constexpr float kListedQuery = -2.f;     // bound of a listed query
+
+// Checks of the arguments of a search, and what every kernel needs of them.
+int tree_args(int64_t n_vert, int32_t n_coords, const int64_t *row_splits, int64_t n_rs, int32_t K, int32_t has_direction,
+              int32_t tf_compat, bool mark_ties, int64_t *out_idx, float *out_distsq, void *workspace, size_t workspace_bytes,
+              TreeArgs *a, KnnWorkspace *L, TreeLayout *T);
+// One query per warp, for the listed ones.
+int launch_tree_listed(const TreeArgs &a, int nv, cudaStream_t s);
+
+#define FGC_TRY(expr)                                    \
+    do {                                                 \
+        const cudaError_t rc_ = (expr);                  \
+        if (rc_ != cudaSuccess) return rc_;              \
+    } while (0)
+
+}  // namespace fgc

@@ -29,7 +29,7 @@
 #include <type_traits>
 
 #include "knn_list.cuh"
-#include "knn_tree.cuh"
+#include "knn_tree_args.cuh"
 
 namespace fgc {
 
@@ -48,23 +48,6 @@ constexpr int kFirstExtra = 64, kMoreExtra = 64, kSpare = 8, kMaxList = 32;
 // resident CTAs per SM asked of the compiler (1: 5.7 / 10.2 / 11.0; 5 and 6 within 3 %; 6 spills with
 // more than four coordinates or K > 129: 1.14 against 0.90 ms for 100 k points, K = 200)
 constexpr int tree_ctas(int nv, int r) { return nv > 1 || r > 4 ? 5 : 6; }
-
-struct TreeArgs {
-    const float4 *scoords;
-    const int *sorig;
-    const uint8_t *sflag;      // nullptr: no direction restriction
-    const float4 *box[3];      // leaves, nodes, top nodes
-    const int64_t *row_splits;
-    KnnGrid *grid;
-    KnnTree *tree;
-    int64_t *out_idx;
-    float *out_dist;
-    int n_vert;
-    int n_rs;
-    int K;
-    int tf_compat;
-    int mark_ties;             // rows with a choice at the K-th distance get kTieRow in slot 0
-};
 
 // Row split of a position in curve order (positions of a row split are its original range): 32 pivots
 // at a time.
@@ -103,8 +86,6 @@ __device__ __forceinline__ float box_sq(const float4 (&q)[NV], const float4 *__r
     }
     return acc;
 }
-
-constexpr uint32_t kNoBox = 0xffffffffu;
 
 // Sort key of box `lane` among 32: its distance with the lane in the low bits (cleared first, so the
 // key never exceeds the distance).
@@ -416,6 +397,40 @@ k_knn_tree(const TreeArgs a)
     else tree_query<NV, R>(a, (int)qi);
 }
 
+// The listed queries, usually few.
+template <int NV, int R>
+__global__ void __launch_bounds__(kTreeWarps * 32, tree_ctas(NV, R))
+k_knn_tree_listed(const TreeArgs a)
+{
+    chain_wait();
+    chain_release();
+    if (a.grid->status != 0) return;
+    const int n = min(a.tree->n_listed, a.n_vert);
+    for (int i = blockIdx.x * kTreeWarps + (threadIdx.x >> 5); i < n; i += gridDim.x * kTreeWarps) {
+        const int qi = a.listed[i];
+        if (FGC_DBG_OK(qi >= 0 && qi < a.n_vert, &a.grid->status)) tree_query<NV, R>(a, qi);
+        __syncwarp();
+    }
+}
+
+template <int NV>
+static cudaError_t launch_listed(const TreeArgs &a, cudaStream_t s)
+{
+    const unsigned blocks = (unsigned)sm_count() * 5;
+    const int T = kTreeWarps * 32;
+    switch (tree_list_rows(a.K)) {
+    case 1: return launch_chained(k_knn_tree_listed<NV, 1>, blocks, T, 0, s, a);
+    case 2: return launch_chained(k_knn_tree_listed<NV, 2>, blocks, T, 0, s, a);
+    case 4: return launch_chained(k_knn_tree_listed<NV, 4>, blocks, T, 0, s, a);
+    default: return launch_chained(k_knn_tree_listed<NV, 8>, blocks, T, 0, s, a);
+    }
+}
+
+int launch_tree_listed(const TreeArgs &a, int nv, cudaStream_t s)
+{
+    return (int)(nv == 1 ? launch_listed<1>(a, s) : launch_listed<2>(a, s));
+}
+
 template <int NV>
 static cudaError_t launch_tree(const TreeArgs &a, cudaStream_t s)
 {
@@ -425,6 +440,35 @@ static cudaError_t launch_tree(const TreeArgs &a, cudaStream_t s)
     if (kn <= 64) return launch_chained(k_knn_tree<NV, 2>, blocks, T, 0, s, a);
     if (kn <= 128) return launch_chained(k_knn_tree<NV, 4>, blocks, T, 0, s, a);
     return launch_chained(k_knn_tree<NV, 8>, blocks, T, 0, s, a);
+}
+
+int tree_args(int64_t n_vert, int32_t n_coords, const int64_t *row_splits, int64_t n_rs, int32_t K, int32_t has_direction,
+              int32_t tf_compat, bool mark_ties, int64_t *out_idx, float *out_distsq, void *workspace, size_t workspace_bytes,
+              TreeArgs *a, KnnWorkspace *L, TreeLayout *T)
+{
+    const int rc = check_knn_args(n_vert, n_coords, n_rs, K, workspace, workspace_bytes, L);
+    if (rc != FGC_OK) return rc;
+    if (n_vert == 0) return FGC_OK;
+    if (!row_splits || n_rs < 2 || !out_idx || !out_distsq) return FGC_ERR_BAD_ARGUMENT;
+    *T = tree_layout(*L, n_vert, n_coords, n_rs);
+    if (!T->fits) return FGC_ERR_TOO_LARGE;
+    char *ws = (char *)workspace;
+    *a = TreeArgs();
+    a->scoords = (const float4 *)(ws + L->scoords);
+    a->sorig = (const int *)(ws + L->sorig);
+    a->sflag = has_direction ? (const uint8_t *)(ws + L->sflag) : nullptr;
+    for (int l = 0; l < 3; l++) a->box[l] = (const float4 *)(ws + T->box[l]);
+    a->row_splits = row_splits;
+    a->grid = (KnnGrid *)(ws + L->header);
+    a->tree = (KnnTree *)(ws + L->tickets);
+    a->out_idx = out_idx;
+    a->out_dist = out_distsq;
+    a->n_vert = (int)n_vert;
+    a->n_rs = (int)n_rs;
+    a->K = K;
+    a->tf_compat = tf_compat;
+    a->mark_ties = mark_ties;
+    return FGC_OK;
 }
 
 }  // namespace fgc
@@ -443,30 +487,13 @@ int fgc::knn_search_tree(int64_t n_vert, int32_t n_coords, const int64_t *row_sp
 {
     FGC_NVTX("fgc_knn_search_tree");
     using namespace fgc;
-    KnnWorkspace L;
-    const int rc = check_knn_args(n_vert, n_coords, n_rs, K, workspace, workspace_bytes, &L);
-    if (rc != FGC_OK) return rc;
-    if (n_vert == 0) return FGC_OK;
-    if (!row_splits || n_rs < 2 || !out_idx || !out_distsq) return FGC_ERR_BAD_ARGUMENT;
-    const TreeLayout T = tree_layout(L, n_vert, n_coords, n_rs);
-    if (!T.fits) return FGC_ERR_TOO_LARGE;
-    cudaStream_t s = (cudaStream_t)stream;
-    char *ws = (char *)workspace;
     TreeArgs a;
-    a.scoords = (const float4 *)(ws + L.scoords);
-    a.sorig = (const int *)(ws + L.sorig);
-    a.sflag = has_direction ? (const uint8_t *)(ws + L.sflag) : nullptr;
-    for (int l = 0; l < 3; l++) a.box[l] = (const float4 *)(ws + T.box[l]);
-    a.row_splits = row_splits;
-    a.grid = (KnnGrid *)(ws + L.header);
-    a.tree = (KnnTree *)(ws + L.tickets);
-    a.out_idx = out_idx;
-    a.out_dist = out_distsq;
-    a.n_vert = (int)n_vert;
-    a.n_rs = (int)n_rs;
-    a.K = K;
-    a.tf_compat = tf_compat;
-    a.mark_ties = mark_ties;
+    KnnWorkspace L;
+    TreeLayout T;
+    const int rc = tree_args(n_vert, n_coords, row_splits, n_rs, K, has_direction, tf_compat, mark_ties, out_idx, out_distsq, workspace,
+                             workspace_bytes, &a, &L, &T);
+    if (rc != FGC_OK || n_vert == 0) return rc;
+    cudaStream_t s = (cudaStream_t)stream;
     if (L.nv == 1) FGC_RETURN_IF_CUDA(launch_tree<1>(a, s));
     else if (L.nv == 2) FGC_RETURN_IF_CUDA(launch_tree<2>(a, s));
     else if (L.nv == 3) FGC_RETURN_IF_CUDA(launch_tree<3>(a, s));
