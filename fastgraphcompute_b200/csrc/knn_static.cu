@@ -56,9 +56,9 @@ extern "C" int fgc_binned_knn_fwd_static(const float *coords, int64_t n_vert, in
 {
     using namespace fgc;
     if (!out_status) return FGC_ERR_BAD_ARGUMENT;
-    if (fgc_knn_workspace_bytes(n_vert, n_coords, n_rs, K) == 0) return FGC_ERR_BAD_ARGUMENT;
-    // (a search on the grid needs none of what one on a tree would)
-    if (knn_workspace_layout(n_vert, n_coords, n_rs, K).total > (size_t)FGC_STATIC_WORKSPACE_BYTES) return FGC_ERR_STATIC_TOO_LARGE;
+    const size_t need = fgc_knn_workspace_bytes(n_vert, n_coords, n_rs, K);
+    if (need == 0) return FGC_ERR_BAD_ARGUMENT;
+    if (need > (size_t)FGC_STATIC_WORKSPACE_BYTES) return FGC_ERR_STATIC_TOO_LARGE;
     void *scratch = nullptr;
     int rc = static_scratch_address(&scratch);
     if (rc != FGC_OK) return rc;
