@@ -573,7 +573,13 @@ __global__ void k_publish_status(const int32_t *__restrict__ status_dev, volatil
 extern "C" size_t fgc_knn_workspace_bytes(int64_t n_vert, int32_t n_coords, int64_t n_rs, int32_t K)
 {
     if (n_vert < 0 || n_vert > 0x7fffffff || n_coords < 1 || n_rs < 1 || K < 1) return 0;
-    return fgc::knn_workspace_layout(n_vert, n_coords, n_rs, K).total + fgc::tree_extra_bytes(n_vert, n_coords, n_rs);
+    return fgc::knn_workspace_layout(n_vert, n_coords, n_rs, K).total;
+}
+
+extern "C" size_t fgc_knn_forward_workspace_bytes(int64_t n_vert, int32_t n_coords, int64_t n_rs, int32_t K, int32_t flags)
+{
+    const size_t grid = fgc_knn_workspace_bytes(n_vert, n_coords, n_rs, K);
+    return grid == 0 || !(flags & FGC_FORWARD_TREE) ? grid : grid + fgc::tree_extra_bytes(n_vert, n_coords, n_rs);
 }
 
 extern "C" int fgc_read_status(const void *workspace_or_params, int32_t *status_host,

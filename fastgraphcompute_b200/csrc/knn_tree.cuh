@@ -132,7 +132,7 @@ int knn_search_tree(int64_t n_vert, int32_t n_coords, const int64_t *row_splits,
                     int32_t has_direction, int32_t tf_compat, bool mark_ties, int64_t *out_idx, float *out_distsq,
                     void *workspace, size_t workspace_bytes, fgc_stream_t stream);
 // The same for all queries of a leaf at once, directly behind fgc_knn_build_tree, in a workspace with the scratch that
-// fgc_knn_workspace_bytes counts in (tree_scratch).
+// fgc_knn_forward_workspace_bytes counts in (tree_scratch).
 int knn_search_tree_groups(int64_t n_vert, int32_t n_coords, const int64_t *row_splits, int64_t n_rs, int32_t K,
                            int32_t has_direction, int32_t tf_compat, bool mark_ties, int64_t *out_idx, float *out_distsq,
                            void *workspace, size_t workspace_bytes, fgc_stream_t stream);

@@ -1,0 +1,87 @@
+"""The search on a tree for all queries of a leaf at once (csrc/knn_tree_group.cu), where it can go wrong beyond what
+test_knn_tree_search_matches_oracle covers: bounds in low precision at extreme coordinates, leaves that list too many others, more
+leaves than the scratch holds, a workspace without scratch."""
+import importlib
+
+import pytest
+import torch
+
+DEV = "cuda:0"
+
+
+def _points(kind, n, D, g):
+    x = torch.rand((n, D), generator=g)
+    if kind == "far":            # squares at the end of the range: some distances overflow
+        return torch.randn((n, D), generator=g) * 1e19
+    if kind == "near":           # squares that underflow
+        return x * 1e-20
+    if kind == "offset":         # large against their distances
+        return x + 1000.0
+    if kind == "mixed":          # a dense cloud among points far apart: leaves across both
+        return torch.where(torch.rand((n, 1), generator=g) < 0.5, 0.5 + 1e-4 * x, x * 100)
+    return x
+
+
+def _forward(km, x, rs, K, tree, direction=None):
+    old = km.search_tree
+    try:
+        km.search_tree = tree
+        # (with the hint no second look follows: the record of the search stays in the workspace)
+        return km._forward(x, rs, K, direction, False, False, None, True)
+    finally:
+        km.search_tree = old
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind,sizes,D,K,listed", [
+    ("far", [3000], 3, 17, None), ("far", [2000, 40], 5, 66, None), ("near", [4000], 4, 40, None), ("near", [900, 900], 3, 130, None),
+    ("offset", [5000, 33, 1], 3, 65, None), ("offset", [5000], 5, 33, None), ("mixed", [60000], 3, 9, True), ("mixed", [60000], 4, 100, True),
+    ("uniform", [800000], 5, 9, None)])
+def test_groups_find_what_the_grid_finds(kind, sizes, D, K, listed):
+    """Distances are equal bit for bit, ids up to the choice among equal K-th distances; 800 000 points in five coordinates take
+    two rounds of the scratch."""
+    km = importlib.import_module("fastgraphcompute_b200.extensions.binned_select_knn")
+    g = torch.Generator().manual_seed(D * K)
+    n = sum(sizes)
+    x = _points(kind, n, D, g).to(DEV)
+    rs = torch.tensor([0] + sizes).cumsum(0).to(DEV)
+    direction = torch.randint(0, 4, (n,), generator=g).to(DEV) if kind == "offset" else None
+    gi, gd, _ = _forward(km, x, rs, K, False, direction)
+    ti, td, ws = _forward(km, x, rs, K, True, direction)
+    again = _forward(km, x, rs, K, True, direction)
+    assert torch.equal(ti, again[0]) and torch.equal(td, again[1])
+    assert torch.equal(gd.sort(dim=1).values, td.sort(dim=1).values)
+    edge = gd.amax(dim=1, keepdim=True)
+    inside = [torch.where((i >= 0) & (d < edge), i, torch.full_like(i, -1)).sort(dim=1).values for i, d in ((gi, gd), (ti, td))]
+    assert torch.equal(*inside)
+    if listed:
+        assert int(ws[256:].view(torch.int32)[24]) > 0           # queries that were searched one by one
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("D,K", [(3, 20), (5, 70)])
+def test_a_workspace_without_scratch_is_searched_one_query_at_a_time(D, K, monkeypatch):
+    km = importlib.import_module("fastgraphcompute_b200.extensions.binned_select_knn")
+    x = torch.rand((5000, D), generator=torch.Generator().manual_seed(K)).to(DEV)
+    rs = torch.tensor([0, 2000, 5000], device=DEV)
+    _, expected, ws = _forward(km, x, rs, K, True)
+    lib = km._cabi.lib
+    small = lib.fgc_knn_workspace_bytes(5000, D, 3, K)
+    assert small < ws.numel()
+    monkeypatch.setattr(lib, "fgc_knn_forward_workspace_bytes", lambda *args: small)
+    _, dist, ws = _forward(km, x, rs, K, True)
+    assert ws.numel() == small and torch.equal(dist.sort(dim=1).values, expected.sort(dim=1).values)
+
+
+@pytest.mark.parametrize("n,D,row_splits,K,long_tails,in_order,groups", [
+    (16383, 4, 1, 40, 1, 0, 0), (16384, 4, 1, 8, 1, 1, 1), (16384, 4, 1, 7, 1, 1, 0), (20000, 4, 2, 24, 1, 1, 1), (20000, 4, 2, 23, 1, 1, 0),
+    (20000, 4, 10, 40, 1, 1, 1), (20000, 4, 14, 40, 1, 1, 0), (20000, 3, 1, 16, 1, 1, 1), (20000, 3, 10, 48, 1, 1, 1),
+    (60000, 5, 4, 40, 0, 0, 1), (60000, 5, 5, 40, 0, 0, 0), (60000, 5, 4, 40, 0, 1, 0), (60000, 5, 4, 66, 0, 1, 1),
+    (50000, 4, 1, 72, 0, 1, 1), (50000, 4, 1, 71, 0, 0, 0), (200000, 4, 8, 40, 0, 0, 1), (200000, 4, 7, 40, 0, 0, 0),
+    (800000, 4, 1, 16, 0, 0, 1), (800000, 4, 1, 16, 0, 1, 0), (200000, 3, 1, 64, 0, 0, 1), (200000, 3, 1, 64, 0, 1, 0),
+    (800000, 3, 9, 36, 0, 0, 1), (800000, 3, 9, 35, 0, 0, 0), (150000, 3, 1, 66, 0, 1, 1), (50000, 3, 1, 80, 0, 1, 1),
+    (20000, 3, 1, 128, 0, 1, 1), (400000, 2, 1, 200, 0, 0, 0), (400000, 6, 1, 40, 0, 0, 0)])
+def test_groups_by_size(n, D, row_splits, K, long_tails, in_order, groups):
+    """The edges of the ranges where the search by groups was measured ahead of the grid."""
+    from fastgraphcompute_b200 import _cabi
+    assert _cabi.lib.fgc_knn_groups_preferred(n, D, row_splits + 1, K, long_tails, in_order) == groups
