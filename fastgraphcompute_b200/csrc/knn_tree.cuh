@@ -6,6 +6,9 @@
 // the cells of a grid the boxes follow the density: every leaf holds 32 points whether the data is
 // uniform, normally distributed or clustered.
 //
+// Two searches: one query at a time (knn_tree_search.cu), and in up to five coordinates all queries of a leaf at once
+// (knn_tree_group.cu).
+//
 // The tree lives in the workspace of the grid (knn_grid.cuh): sorted coordinates, original ids and
 // flags in the same sections, everything else in the space of the cell table.  Its record lies
 // in the section behind the grid's header, of which it uses only the status word.

@@ -18,6 +18,17 @@
 // the result is exactly the K-1 smallest computed distances, whatever the tree.  Boxes and points at exactly the bound
 // are taken, so that a candidate equal to the K-th distance that is left out is always noticed.
 //
+// What bounds them (a million uniform points in three coordinates, K = 64, ncu): k_tree_rows issue slots (0.80 of them used, 1510
+// warp instructions a query, arithmetic pipe 0.71), k_tree_groups the shared-memory pipe (0.93; the counting's atomics meet in banks; 185
+// instructions a query).  Whole forward against the search one query at a time / the grid, ms: 6.4 M uniform points in three
+// coordinates, K = 64 13.9 against 21.9 / 18.3; 1.6 M learned ones in four, K = 40 6.9 against 9.6 / 8.4; 800 k skewed in three, K = 128
+// 3.2 against 4.7 / 18.9; a million normal ones in five, K = 40 15.6 against 18.2 / 26.3.
+//
+// Other splits of the work, measured on the first and the third of these: one kernel, a lane per query, the points of a leaf read from
+// shared memory by all 32 lanes (15.5; broadcast 16-byte loads write 512 bytes back each, four cycles an SM); candidates of all
+// 32 queries filtered by the matrix product and kept in the workspace, a second kernel for the rows (15.7 and 7.8: leaves that
+// visit thousands of others run on alone).
+//
 // A leaf far larger than the distances of its neighbours (points far apart that happen to follow one another on the curve)
 // would list too many leaves: its queries are searched one by one (knn_tree_search.cu).
 #include "knn_list.cuh"
@@ -554,7 +565,8 @@ k_tree_rows(const TreeArgs a)
     const int64_t leaf0 = tree_base(ev_begin, e, 5);
     const int rel_q = (int)(slot - leaf0) * 32 + (int)(row & 31);
     const bool writes = rel_q < n_e && t != kListedQuery;
-    if (!writes) t = kNoQuery;
+    // (an open bound as the largest number: distances that overflow are no candidates)
+    t = writes ? fminf(t, 3.402823466e38f) : kNoQuery;
     const int qi = ev_begin + min(rel_q, n_e - 1);
     const float4 *__restrict__ leaf_box = a.box[0] + (size_t)leaf0 * (2 * NV);
     const int *__restrict__ list = a.list + (size_t)(row >> 5) * a.list_cap;
@@ -574,7 +586,7 @@ k_tree_rows(const TreeArgs a)
     };
     auto keep = [&](const float4 (&c)[NV], int j) {
         const float d = dist_sq<NV>(x, c, 0);
-        bool in = d <= t && __float_as_uint(d) < kInfBits && j >= 0 && j != qi;
+        bool in = d <= t && j >= 0 && j != qi;
         if (sflag && in) { const uint8_t f = sflag[j]; in = f != 1 && f != 2; }
         const unsigned mask = __ballot_sync(FGC_FULL_MASK, in);
         if (in) pairs[m + __popc(mask & lanemask_lt())] = make_float2(d, __int_as_float(j));

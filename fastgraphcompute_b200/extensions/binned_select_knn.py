@@ -89,7 +89,7 @@ def _forward(coords, row_splits, K, direction, tf_compat, count_evals, order, lo
     # coordinates, K = 128, grid / tree in ms: a third of them candidates 3.8 / 5.8, one in twenty 6.6 / 24, one in two
     # thousand -- fewer than K - 1 in places -- 4.0 / 938)
     tree = n_vert > 0 and not count_evals and target_occupancy <= 0 and grid_dims == 0 and (
-        (direction is None and (
+        (direction is None and n_vert >= 16384 and (        # (below, both rules say no: two calls less, 3 us)
             _cabi.lib.fgc_knn_tree_preferred(n_vert, n_coords, n_rs, K, int(long_tails)) == 1 or
             _cabi.lib.fgc_knn_groups_preferred(n_vert, n_coords, n_rs, K, int(long_tails), int(in_order)) == 1))
         if search_tree is None else search_tree)

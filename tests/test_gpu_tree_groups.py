@@ -73,6 +73,30 @@ def test_a_workspace_without_scratch_is_searched_one_query_at_a_time(D, K, monke
     assert ws.numel() == small and torch.equal(dist.sort(dim=1).values, expected.sort(dim=1).values)
 
 
+@pytest.mark.gpu
+def test_groups_in_a_cuda_graph(monkeypatch):
+    """Captured without the status check and replayed on other points."""
+    km = importlib.import_module("fastgraphcompute_b200.extensions.binned_select_knn")
+    g = torch.Generator().manual_seed(3)
+    points = [torch.rand((20000, 4), generator=g).to(DEV), torch.randn((20000, 4), generator=g).to(DEV)]
+    rs = torch.tensor([0, 9000, 20000], device=DEV)
+    expected = [_forward(km, p, rs, 40, True)[:2] for p in points]
+    monkeypatch.setattr(km, "check_status", False)
+    static = points[0].clone()
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        _forward(km, static, rs, 40, True)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        idx, dist, _ = _forward(km, static, rs, 40, True)
+    for p, (ei, ed) in zip(points, expected):
+        static.copy_(p)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(idx, ei) and torch.equal(dist, ed)
+
+
 @pytest.mark.parametrize("n,D,row_splits,K,long_tails,in_order,groups", [
     (16383, 4, 1, 40, 1, 0, 0), (16384, 4, 1, 8, 1, 1, 1), (16384, 4, 1, 7, 1, 1, 0), (20000, 4, 2, 24, 1, 1, 1), (20000, 4, 2, 23, 1, 1, 0),
     (20000, 4, 10, 40, 1, 1, 1), (20000, 4, 14, 40, 1, 1, 0), (20000, 3, 1, 16, 1, 1, 1), (20000, 3, 10, 48, 1, 1, 1),
