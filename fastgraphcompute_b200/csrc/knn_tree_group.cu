@@ -97,6 +97,9 @@ __device__ __forceinline__ float widened(float t, float q2)
     return t + 0.0032f * q * c + 6e-6f * s * s + 1e-36f;
 }
 
+// |c|^2 of what is no candidate; with cross terms of up to 2e36 (coordinates up to 1e18) still above 0x7e900000 = 9.6e37.
+constexpr float kNotThere = 1e38f;
+
 // d = a * b + d for a tile of 16 x 8 over 8 places, tf32
 __device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
 {
@@ -188,9 +191,10 @@ __device__ __forceinline__ void bound_leaf(const TreeArgs &a, const int slot)
         for (int i = lane; i < 32 * (kHistClasses + 1); i += 32) s_hist[i] = 0;
         // Classes are the upper bits of a distance: eight to a factor of two, the last one and what is beyond it without an
         // end.  The K-th distance of a point in a leaf of 32 is a tenth to a half of the leaf's squared diagonal at K =
-        // 16 to 128 and more at a border: four factors of two up to twice it, less for short lists.
+        // 16 to 128 and more at a border: four factors of two up to twice it, less for short lists.  The last class begins below
+        // kNotThere, so that what is no candidate is never counted below it, however large the leaf.
         const float share = kn >= 63 ? 2.f : 2.f * powf((float)(kn + 1) * (1.f / 64.f), 2.f / DC);
-        const int last = (int)min(__float_as_uint(share * diag), 0x7f000000u) >> 20;
+        const int last = (int)min(__float_as_uint(share * diag), 0x7e800000u) >> 20;
         const int first = max(last - (kHistClasses - 1), 0);
         // the nearest leaves of the nearest nodes
         const int own_node = own_leaf >> 5, node0 = own_node & ~31;
@@ -268,7 +272,7 @@ __device__ __forceinline__ void bound_leaf(const TreeArgs &a, const int slot)
                 c2 += __shfl_xor_sync(FGC_FULL_MASK, c2, 1);
                 c2 += __shfl_xor_sync(FGC_FULL_MASK, c2, 2);
                 wide = wide || !(c2 <= 1e36f);
-                if (!(there >> (8 * j + g4) & 1)) c2 = 1e38f;
+                if (!(there >> (8 * j + g4) & 1)) c2 = kNotThere;
                 const float c2_high = __uint_as_float(__float_as_uint(c2) & 0xffffe000u), c2_low = c2 - c2_high;
                 uint32_t b[2];
 #pragma unroll

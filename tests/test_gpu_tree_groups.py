@@ -2,6 +2,7 @@
 test_knn_tree_search_matches_oracle covers: bounds in low precision at extreme coordinates, leaves that list too many others, more
 leaves than the scratch holds, a workspace without scratch."""
 import importlib
+import math
 
 import pytest
 import torch
@@ -56,6 +57,26 @@ def test_groups_find_what_the_grid_finds(kind, sizes, D, K, listed):
     assert torch.equal(*inside)
     if listed:
         assert int(ws[256:].view(torch.int32)[24]) > 0           # queries that were searched one by one
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("D,K", [(2, 11), (3, 20)])
+def test_missing_points_of_a_leaf_give_no_bound(D, K):
+    """Row splits of 33 points: one leaf across 2.6e19 with its last point near its middle, another with a single point beside
+    that.  The 31 places behind the single one are nearer than 1e38 to nothing, though the neighbours are 1.7e38 away."""
+    km = importlib.import_module("fastgraphcompute_b200.extensions.binned_select_knn")
+    angle = torch.linspace(0.02, 1.5 * math.pi - 0.02, 31, dtype=torch.float64)          # the quadrants that the curve sees first
+    x = torch.zeros((33, D), dtype=torch.float64)
+    x[:31, 0], x[:31, 1] = 1.3e19 * angle.cos(), 1.3e19 * angle.sin()
+    x[31, :2], x[32, :2] = torch.tensor([1e17, -1e17]), torch.tensor([2e17, -1.5e17])
+    x = x.float()
+    d = (x[:, None] - x[None]).square().sum(dim=2)
+    d = torch.where(torch.isfinite(d), d, torch.full_like(d, float("inf"))).fill_diagonal_(-1.0).sort(dim=1).values[:, 1:K]
+    rs = torch.arange(0, 33 * 100 + 1, 33, device=DEV)
+    idx, dist, _ = _forward(km, x.repeat(100, 1).to(DEV), rs, K, True)
+    assert bool((idx[31::33] >= 0).all()) and bool((idx[32::33] >= 0).all())
+    found = torch.where(idx >= 0, dist, torch.full_like(dist, float("inf"))).cpu()[:, 1:].sort(dim=1).values
+    torch.testing.assert_close(found, d.repeat(100, 1), rtol=1e-6, atol=0.0)
 
 
 @pytest.mark.gpu
