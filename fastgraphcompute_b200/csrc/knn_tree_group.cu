@@ -16,7 +16,7 @@
 // The distance of two boxes, or of a point and a box, is computed with the operations of dist_sq in the same order.  Rounding is
 // monotone, so it never exceeds the computed distance of two points inside: pruning needs no margin and
 // the result is exactly the K-1 smallest computed distances, whatever the tree.  Boxes and points at exactly the bound
-// are taken, so that a candidate equal to the K-th distance that is left out is always noticed.
+// are taken until a candidate equal to it has been left out, so that one that equals the K-th distance is always noticed.
 //
 // What bounds them (a million uniform points in three coordinates, K = 64, ncu): k_tree_rows issue slots (0.80 of them used, 1510
 // warp instructions a query, arithmetic pipe 0.71), k_tree_groups the shared-memory pipe (0.93; the counting's atomics meet in banks; 185
@@ -603,7 +603,8 @@ k_tree_rows(const TreeArgs a)
         __syncwarp();
 #pragma unroll
         for (int r = 0; r < ROWS; r++) v[r] = r * 32 + lane < m ? __float_as_uint(pairs[r * 32 + lane].x) : kNoBox;
-        if (bisect<ROWS>(v, kn, 8, at_most, hi, equal)) left_out = hi;
+        const bool left = bisect<ROWS>(v, kn, 8, at_most, hi, equal);
+        if (left) left_out = hi;
 #pragma unroll
         for (int r = 0; r < ROWS; r++) {
             const unsigned kept = staying(v[r], hi, MOST, equal);
@@ -614,7 +615,10 @@ k_tree_rows(const TreeArgs a)
         }
         __syncwarp();
         m = to;
-        t = __uint_as_float(hi);
+        // Once one that equals the bound has been left out, others there change nothing: only what is nearer is wanted (nothing
+        // if the bound is 0), or many equal points force a cut every two leaves.  Half of the points equal, ms: 20 k in three
+        // coordinates, K = 64 0.70 -> 0.17 (grid 1.06), 100 k in five, K = 40 12.6 -> 0.82 (21.8).
+        t = !left ? __uint_as_float(hi) : (hi > 0 ? __uint_as_float(hi - 1) : kNoQuery);
     };
     // the leaves of `todo`, two at a time
     auto visit = [&](unsigned todo, auto leaf_at) {
