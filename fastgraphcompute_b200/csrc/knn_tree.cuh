@@ -13,6 +13,8 @@
 // flags in the same sections, everything else in the space of the cell table.  Its record lies
 // in the section behind the grid's header, of which it uses only the status word.
 #pragma once
+#include <cstddef>
+
 #include "knn_grid.cuh"
 
 namespace fgc {
@@ -31,8 +33,10 @@ struct KnnTree {
     float scale;                        // cells of the Hilbert curve per unit length
     int32_t n_tied;                     // rows marked kTieRow by the search
     int32_t n_listed;                   // queries that the search by groups leaves to the search one by one
+    int32_t next_listed;                // of those, taken so far
 };
 static_assert(sizeof(KnnTree) <= kHardTicketBytes, "tree record too large");
+static_assert(offsetof(KnnTree, n_listed) == 96, "read there by tests/test_gpu_tree_groups.py");
 
 constexpr int kRadixBits = 11;
 constexpr int kRadixBins = 1 << kRadixBits;

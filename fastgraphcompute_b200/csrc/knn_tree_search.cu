@@ -405,7 +405,9 @@ k_knn_tree(const TreeArgs a)
     else tree_query<NV, R>(a, (int)qi);
 }
 
-// The listed queries, usually few.
+// The listed queries, usually few.  A warp takes the next one when it has finished its last: they differ by orders of
+// magnitude (half of 400 k points in a cloud a millionth as wide as the rest, three coordinates, K = 64: 157 -> 95 ms, the search one
+// query at a time for all of them 104).
 template <int NV, int R>
 __global__ void __launch_bounds__(kTreeWarps * 32, tree_ctas(NV, R))
 k_knn_tree_listed(const TreeArgs a)
@@ -414,7 +416,12 @@ k_knn_tree_listed(const TreeArgs a)
     chain_release();
     if (a.grid->status != 0) return;
     const int n = min(a.tree->n_listed, a.n_vert);
-    for (int i = blockIdx.x * kTreeWarps + (threadIdx.x >> 5); i < n; i += gridDim.x * kTreeWarps) {
+    if (n == 0) return;
+    for (;;) {
+        int i = 0;
+        if ((threadIdx.x & 31) == 0) i = atomicAdd(&a.tree->next_listed, 1);
+        i = __shfl_sync(FGC_FULL_MASK, i, 0);
+        if (i >= n) return;
         const int qi = a.listed[i];
         if (FGC_DBG_OK(qi >= 0 && qi < a.n_vert, &a.grid->status)) tree_query<NV, R>(a, qi);
         __syncwarp();
@@ -424,9 +431,9 @@ k_knn_tree_listed(const TreeArgs a)
 template <int NV>
 static cudaError_t launch_listed(const TreeArgs &a, cudaStream_t s)
 {
-    const unsigned blocks = (unsigned)sm_count() * 5;
-    const int T = kTreeWarps * 32;
-    switch (tree_list_rows(a.K)) {
+    const int rows = tree_list_rows(a.K), T = kTreeWarps * 32;
+    const unsigned blocks = (unsigned)(sm_count() * tree_ctas(NV, rows));
+    switch (rows) {
     case 1: return launch_chained(k_knn_tree_listed<NV, 1>, blocks, T, 0, s, a);
     case 2: return launch_chained(k_knn_tree_listed<NV, 2>, blocks, T, 0, s, a);
     case 4: return launch_chained(k_knn_tree_listed<NV, 4>, blocks, T, 0, s, a);
