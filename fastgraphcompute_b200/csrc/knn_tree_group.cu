@@ -604,7 +604,6 @@ k_tree_rows(const TreeArgs a)
 #pragma unroll
         for (int r = 0; r < ROWS; r++) v[r] = r * 32 + lane < m ? __float_as_uint(pairs[r * 32 + lane].x) : kNoBox;
         const bool left = bisect<ROWS>(v, kn, 8, at_most, hi, equal);
-        if (left) left_out = hi;
 #pragma unroll
         for (int r = 0; r < ROWS; r++) {
             const unsigned kept = staying(v[r], hi, MOST, equal);
@@ -615,10 +614,11 @@ k_tree_rows(const TreeArgs a)
         }
         __syncwarp();
         m = to;
-        // Once one that equals the bound has been left out, others there change nothing: only what is nearer is wanted (nothing
-        // if the bound is 0), or many equal points force a cut every two leaves.  Half of the points equal, ms: 20 k in three
+        // Once one that equals the bound has been left out, others there change nothing: only what is nearer is wanted (0 gives
+        // not a number: nothing is within that), or many equal points force a cut every two leaves.  Half of the points equal, ms: 20 k in three
         // coordinates, K = 64 0.70 -> 0.17 (grid 1.06), 100 k in five, K = 40 12.6 -> 0.82 (21.8).
-        t = !left ? __uint_as_float(hi) : (hi > 0 ? __uint_as_float(hi - 1) : kNoQuery);
+        if (left) left_out = hi;
+        t = __uint_as_float(hi - (left ? 1u : 0u));
     };
     // the leaves of `todo`, two at a time
     auto visit = [&](unsigned todo, auto leaf_at) {
