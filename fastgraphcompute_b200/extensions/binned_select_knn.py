@@ -93,6 +93,17 @@ def _forward(coords, row_splits, K, direction, tf_compat, count_evals, order, lo
             _cabi.lib.fgc_knn_tree_preferred(n_vert, n_coords, n_rs, K, int(long_tails)) == 1 or
             _cabi.lib.fgc_knn_groups_preferred(n_vert, n_coords, n_rs, K, int(long_tails), int(in_order)) == 1))
         if search_tree is None else search_tree)
+    ws = None
+    if tree:
+        forward_bytes = _cabi.lib.fgc_knn_forward_workspace_bytes(n_vert, n_coords, n_rs, K, 64)
+        try:
+            ws = torch.empty(forward_bytes, dtype=torch.uint8, device=dev)
+            nbytes = forward_bytes
+        except torch.cuda.OutOfMemoryError:
+            # no room for the scratch of the search by groups (up to 256 MB): the search without it, or the grid
+            tree = bool(search_tree) or _cabi.lib.fgc_knn_tree_preferred(n_vert, n_coords, n_rs, K, int(long_tails)) == 1
+    if ws is None:
+        ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
     check = check_status
     form = 0
     # (direction flags change the cells, and with them the form: remembered apart)
@@ -109,9 +120,6 @@ def _forward(coords, row_splits, K, direction, tf_compat, count_evals, order, lo
     flags = (1 if count_evals else 0) | (8 if form == 3 else 16 if form == 4 else 0) | (64 if tree else 0)
     if tree and not long_tails:
         flags |= 128        # equal K-th distances: the grid's choice, whichever search ran
-    if tree:
-        nbytes = _cabi.lib.fgc_knn_forward_workspace_bytes(n_vert, n_coords, n_rs, K, flags)
-    ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
     # The status word is final once the grid is built (non-finite input and malformed row_splits are
     # detected by its first two kernels).  A one-thread kernel stores it into page-locked memory and
     # the library looks at it after the search has been launched: the host waits for the short

@@ -205,6 +205,34 @@ def test_a_workspace_without_scratch_is_searched_one_query_at_a_time(D, K, monke
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n,D,K,tree", [(20000, 3, 130, 0), (20000, 5, 96, 64)])
+def test_no_room_for_the_scratch(n, D, K, tree, monkeypatch):
+    """An allocation that fails with the scratch is made without it: the grid, or the search one query at a time where that is
+    ahead of the grid."""
+    km = importlib.import_module("fastgraphcompute_b200.extensions.binned_select_knn")
+    x = torch.rand((n, D), generator=torch.Generator().manual_seed(K)).to(DEV)
+    rs = torch.tensor([0, n], device=DEV)
+    expected = km.knn_forward_with_order(x, rs, K, None, False)[1]
+    lib, empty = km._cabi.lib, torch.empty
+    plain, full = lib.fgc_knn_workspace_bytes(n, D, 2, K), lib.fgc_knn_forward_workspace_bytes(n, D, 2, K, 64)
+    call, seen = lib.fgc_knn_forward, []
+
+    def tight(*args, **kwargs):
+        if args and args[0] == full:
+            raise torch.cuda.OutOfMemoryError("no room")
+        return empty(*args, **kwargs)
+
+    def recorded(*args):
+        seen.append((args[9] & 64, args[14]))
+        return call(*args)
+    monkeypatch.setattr(torch, "empty", tight)
+    monkeypatch.setattr(lib, "fgc_knn_forward", recorded)
+    dist = km.knn_forward_with_order(x, rs, K, None, False)[1]
+    assert seen == [(tree, plain)] and plain < full
+    assert torch.equal(dist.sort(dim=1).values, expected.sort(dim=1).values)
+
+
+@pytest.mark.gpu
 def test_groups_in_a_cuda_graph(monkeypatch):
     """Captured without the status check and replayed on other points."""
     km = importlib.import_module("fastgraphcompute_b200.extensions.binned_select_knn")
