@@ -109,9 +109,10 @@ static int knn_forward_launch(const float *coords, int64_t n_vert, int32_t n_coo
     const bool groups = tree && n_vert > 0 && n_coords <= kGroupDims &&
                         ws_bytes >= knn_workspace_layout(n_vert, n_coords, n_rs, K).total + tree_extra_bytes(n_vert, n_coords, n_rs);
     const bool ties = tree && (flags & FGC_FORWARD_GRID_TIES) != 0;
-    if (groups) rc = knn_search_tree_groups(n_vert, n_coords, row_splits, n_rs, K, direction != nullptr, tf_compat, ties, out_idx,
+    const TieMarks marks = !ties ? TieMarks::kNone : (flags & FGC_FORWARD_GRID_ORDER ? TieMarks::kAny : TieMarks::kKth);
+    if (groups) rc = knn_search_tree_groups(n_vert, n_coords, row_splits, n_rs, K, direction != nullptr, tf_compat, marks, out_idx,
                                             out_distsq, ws, ws_bytes, stream);
-    else if (tree) rc = knn_search_tree(n_vert, n_coords, row_splits, n_rs, K, direction != nullptr, tf_compat, ties, out_idx,
+    else if (tree) rc = knn_search_tree(n_vert, n_coords, row_splits, n_rs, K, direction != nullptr, tf_compat, marks, out_idx,
                                    out_distsq, ws, ws_bytes, stream);
     else rc = fgc_knn_search(n_vert, n_coords, n_rs, K, direction != nullptr, tf_compat,
                              (flags & (FGC_SEARCH_COUNT | FGC_SEARCH_GRID3 | FGC_SEARCH_GRID4)) | FGC_SEARCH_FRESH, out_idx,

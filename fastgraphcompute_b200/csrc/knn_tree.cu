@@ -440,20 +440,25 @@ extern "C" int fgc_knn_tree_preferred(int64_t n_vert, int32_t n_coords, int64_t 
 }
 
 // Where the search by groups (knn_tree_group.cu) is ahead of the grid, beyond where the tree is taken anyway.  The figures are
-// its time over that of the grid, whole forward with the second look at tied rows, B200, uniform / normal / mixture points:
-//   three coordinates  K = 66: 60 k 1.04 / 0.63 / 0.73, 200 k 0.90 / 0.55 / 0.67;  K = 96: 20 k 1.04 / 0.83 / 1.02, 60 k 0.75 / 0.46 / 0.67
-//                      K = 200: 20 k 0.75 / 0.58 / 0.99;  K = 64: 200 k 0.96 / 0.67 / 0.96, 60 k 1.02 / 0.64 / 0.93
-//                      K = 40: a million 0.93 / 0.81 / 0.86, 200 k 1.16 / 0.78 / 1.07;  K = 24: a million 1.04 / 0.85 / 1.04
-//   four               K = 66: 60 k 0.84 / 0.55 / 0.84, 200 k in fifty row splits 0.72 / 0.60 / 1.02;  K = 96: 20 k 1.18 / 0.52 / 0.83
-//                      K = 200: 20 k 0.66 / 0.46 / 0.60;  K = 40: 200 k in twenty row splits or more 0.97 / 0.96 / 0.91, in one 1.04 / 0.60 / 0.65
-//                      K = 16: a million 0.97 / 0.90 / 0.76, K = 8: 1.30 / 1.03 / 0.75
-//   five               K = 40: 60 k in four row splits 0.73 / 0.78 / 1.02, 600 k in five 0.68 / 0.98 / 0.79, 20 k 0.83 / 0.72 / 1.20
-// in_order: which slot a neighbour has among others at the same distance matters (gradients by slot): the grid for sorted lists.
+// its time over that of the grid, whole forward with the second look at rows with equal distances (FGC_FORWARD_GRID_ORDER), B200,
+// uniform / normal / mixture points, and in three coordinates skewed clusters:
+//   three coordinates  K = 128: 20 k in four row splits 0.96 / 0.47 / 0.63 / 0.38;  K = 80: 50 k 0.83 / 0.60 / 0.66 / 0.64, K = 64: 1.21 /
+//                      0.95 / 1.23 / 0.87;  K = 66: 150 k 0.89 / 0.46 / 0.68 / 0.46, K = 64: 1.11 / 0.62 / 0.97 / 0.60, 200 k 1.05 / 0.67 /
+//                      0.89 / 0.49, 300 k in six 0.96 / 0.75 / 0.88 / 0.57, K = 48: 400 k in eight 1.00 / 0.80 / 0.91 / 0.56;  K = 36: 800 k
+//                      0.95 / 0.50 / 0.83 / 0.33, K = 32: 1.03 / 0.52 / 0.97 / 0.37
+//   four               K = 128: 20 k in four 0.49 / 0.46 / 0.58;  K = 72: 50 k 0.94 / 0.44 / 0.71, K = 40: 1.26 / 0.60 / 1.04, 200 k in
+//                      eight 1.04 / 0.82 / 0.91, 13 1.00 / 0.91 / 0.98, K = 24: 1.09 / 0.96 / 1.13;  800 k, K = 24: 1.09 / 0.51 / 0.62, in 16 0.99 / 0.94 /
+//                      0.80, K = 16: 1.13 / 0.49 / 0.67, in 16 1.04 / 1.00 / 0.84, K = 8 1.30 / 1.03 / 0.75
+//   five               K = 40: 60 k in four 0.87 / 0.89 / 1.22, 200 k in four 0.69 / 0.98 / 0.96, 600 k in five 0.67 / 0.98 / 0.84, 20 k 0.83 /
+//                      0.72 / 1.20;  K = 66: in three or more 0.60 / 0.77 / 0.53
+// The worst are row splits of 5000 points in 50 clusters, for which the grid's cells are right (1.05 to 1.3 with K <= 65), and lattices
+// (1.0 to 1.2: a million points, K = 64, on 40 x 40 x 40 places).
+// Whether distances get gradients plays no part: the same call takes the same search with and without, and gives the
+// same neighbours in the same slots.
 // long_tails: learned coordinates as in fgc_knn_tree_preferred, no second look: three coordinates, row splits of 15 k or more 0.60
 // to 0.80 at K = 16, of 10 k 0.95 at K = 24, of 2000 0.99 at K = 40 and 0.86 at 64; four, 0.56 to 0.95 at K = 8, 0.91 to 0.94 at K = 24, 0.81
 // to 0.85 at K = 40.
-extern "C" int fgc_knn_groups_preferred(int64_t n_vert, int32_t n_coords, int64_t n_rs, int32_t K, int32_t long_tails,
-                                        int32_t in_order)
+extern "C" int fgc_knn_groups_preferred(int64_t n_vert, int32_t n_coords, int64_t n_rs, int32_t K, int32_t long_tails)
 {
     using namespace fgc;
     if (n_vert < 16384 || n_vert > 0x7fffffff || n_coords < 3 || n_coords > kGroupDims || n_rs < 2 || n_rs > 0x7fffffff || K < 1 ||
@@ -467,14 +472,13 @@ extern "C" int fgc_knn_groups_preferred(int64_t n_vert, int32_t n_coords, int64_
         else if (mean >= 8000) least = 24;
         else if (mean >= 1500) least = four ? 40 : 48;
     } else if (n_coords == 5) {
-        if (n_vert >= 60000 && mean >= 15000) least = in_order ? 66 : 40;
+        if (n_vert >= 60000 && mean >= 15000) least = 40;
     } else if (n_coords == 4) {
         least = n_vert >= 50000 ? 72 : 128;
-        if (!in_order && n_vert >= 200000 && n_events >= 8) least = 40;
-        if (!in_order && n_vert >= 800000) least = 16;
+        if (n_vert >= 200000 && n_events >= 8) least = 40;
+        if (n_vert >= 800000) least = 16;
     } else {
-        least = n_vert >= 150000 ? 66 : (n_vert >= 50000 ? 80 : 128);
-        if (!in_order && n_vert >= 200000) least = n_vert >= 800000 ? 36 : 64;
+        least = n_vert >= 800000 ? 36 : (n_vert >= 200000 ? 64 : (n_vert >= 150000 ? 66 : (n_vert >= 50000 ? 80 : 128)));
     }
     if (K < least) return 0;
     return tree_layout(knn_workspace_layout(n_vert, n_coords, n_rs, K), n_vert, n_coords, n_rs).fits ? 1 : 0;

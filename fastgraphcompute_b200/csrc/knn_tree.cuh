@@ -126,8 +126,11 @@ inline bool tree_scratch(const KnnWorkspace &w, int n_coords, char *ws, size_t b
     return true;
 }
 
-// Mark in slot 0 of a row whose K-th distance several points share, of which some are left out.
+// Mark in slot 0 of a row that is to be searched again on a grid.
 constexpr int64_t kTieRow = INT64_MIN;
+// Which rows are: none; those whose K-th distance several points share, of which some are left out; with sorted lists (K <= 65)
+// also those that hold equal distances, whose order would be another one.
+enum class TieMarks : int { kNone, kKth, kAny };
 // Rows that may be marked and searched again, as a share of all rows: see knn_forward_launch.
 constexpr int kTieShare = 16;
 // Status word between the tree search and the end of the second look when there is nothing to search again:
@@ -136,12 +139,12 @@ constexpr int32_t kStatusNoGrid = 1 << 30;
 
 // fgc_knn_search_tree; mark_ties: such rows are marked (and have to be searched again on a grid).
 int knn_search_tree(int64_t n_vert, int32_t n_coords, const int64_t *row_splits, int64_t n_rs, int32_t K,
-                    int32_t has_direction, int32_t tf_compat, bool mark_ties, int64_t *out_idx, float *out_distsq,
+                    int32_t has_direction, int32_t tf_compat, TieMarks mark_ties, int64_t *out_idx, float *out_distsq,
                     void *workspace, size_t workspace_bytes, fgc_stream_t stream);
 // The same for all queries of a leaf at once, directly behind fgc_knn_build_tree, in a workspace with the scratch that
 // fgc_knn_forward_workspace_bytes counts in (tree_scratch).
 int knn_search_tree_groups(int64_t n_vert, int32_t n_coords, const int64_t *row_splits, int64_t n_rs, int32_t K,
-                           int32_t has_direction, int32_t tf_compat, bool mark_ties, int64_t *out_idx, float *out_distsq,
+                           int32_t has_direction, int32_t tf_compat, TieMarks mark_ties, int64_t *out_idx, float *out_distsq,
                            void *workspace, size_t workspace_bytes, fgc_stream_t stream);
 // fgc_knn_build_grid_dims behind a search with mark_ties: builds nothing (kStatusNoGrid) where no row is marked,
 // or more than a kTieShare-th of them are.

@@ -19,7 +19,7 @@ struct TreeArgs {
     int n_rs;
     int K;
     int tf_compat;
-    int mark_ties;             // rows with a choice at the K-th distance get kTieRow in slot 0
+    TieMarks mark_ties;        // which rows get kTieRow in slot 0
     // the search by groups only
     int slot0, n_slots;        // leaf slots of this launch: from the one up to the other
     int list_cap;
@@ -32,9 +32,26 @@ constexpr uint32_t kNoBox = 0xffffffffu;
 constexpr float kNoQuery = -1.f;         // bound of a query that may not have neighbours
 constexpr float kListedQuery = -2.f;     // bound of a listed query
 
+// Whether two of the kn nearest in an ascending list (entry r * 32 + lane, id -1: empty) have the same distance.
+template <int R>
+__device__ __forceinline__ bool equal_in_list(const float (&d)[R], const int (&id)[R], int kn, int lane)
+{
+    bool same = false;
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        float next = __shfl_down_sync(FGC_FULL_MASK, d[r], 1);
+        if (r + 1 < R) {
+            const float first = __shfl_sync(FGC_FULL_MASK, d[r + 1 < R ? r + 1 : r], 0);
+            if (lane == 31) next = first;
+        }
+        same = same || (r * 32 + lane + 1 < kn && id[r] >= 0 && d[r] == next);
+    }
+    return __any_sync(FGC_FULL_MASK, same);
+}
+
 // Checks of the arguments of a search, and what every kernel needs of them.
 int tree_args(int64_t n_vert, int32_t n_coords, const int64_t *row_splits, int64_t n_rs, int32_t K, int32_t has_direction,
-              int32_t tf_compat, bool mark_ties, int64_t *out_idx, float *out_distsq, void *workspace, size_t workspace_bytes,
+              int32_t tf_compat, TieMarks mark_ties, int64_t *out_idx, float *out_distsq, void *workspace, size_t workspace_bytes,
               TreeArgs *a, KnnWorkspace *L, TreeLayout *T);
 // One query per warp, for the listed ones.
 int launch_tree_listed(const TreeArgs &a, int nv, cudaStream_t s);

@@ -738,7 +738,7 @@ k_tree_rows(const TreeArgs a)
     int64_t *row_i = a.out_idx + (size_t)orig_q * K;
     float *row_d = a.out_dist + (size_t)orig_q * K;
     const int64_t pad = a.tf_compat ? (int64_t)orig_q : (int64_t)-1;
-    bool tie = false, full;
+    bool tie = false, same = false, full;
     uint32_t kth = 0;
     if constexpr (R <= 2) {
         constexpr int SLOT_BITS = RowShape<R>::SLOT_BITS;
@@ -752,33 +752,43 @@ k_tree_rows(const TreeArgs a)
         int j[R];
         const uint32_t edge = __shfl_sync(FGC_FULL_MASK, kn > 32 ? key[R - 1] : key[0], (kn - 1) & 31);
         full = kn > 0 && edge != kNoBox;
-        bool unclear = full && drop >> SLOT_BITS == edge >> SLOT_BITS;
+        bool unclear = full && drop >> SLOT_BITS == edge >> SLOT_BITS, look = false;
 #pragma unroll
         for (int r = 0; r < R; r++) {
-            float2 p = make_float2(__uint_as_float(kInfBits), __int_as_float(-1));
+            float2 p = make_float2(__uint_as_float(0x7fffffffu), __int_as_float(-1));      // (empty: compares as false)
             if (key[r] != kNoBox) p = pairs[key[r] & ((1u << SLOT_BITS) - 1)];
             d[r] = p.x;
             j[r] = __float_as_int(p.y);
             unclear = unclear || (full && r * 32 + lane >= kn && key[r] >> SLOT_BITS == edge >> SLOT_BITS);
             const float nd = __shfl_down_sync(FGC_FULL_MASK, d[r], 1);
-            unclear = unclear || (lane < 31 && d[r] > nd);
+            look = look || (lane < 31 && d[r] >= nd);
         }
         if (R == 2) {
             const float nd = __shfl_sync(FGC_FULL_MASK, d[R - 1], 0);
-            unclear = unclear || (lane == 31 && d[0] > nd);
+            look = look || (lane == 31 && d[0] >= nd);
         }
-        const bool again = __any_sync(FGC_FULL_MASK, unclear);
-        if (again) {
-            // distances that differ by less than the keys tell: sorted as they are
-            SortedList<R> near;
-            near.init(lane, kn);
-#pragma unroll 1
-            for (int i = lane; i - lane < m; i += 32) near.merge32(lane, kn, i < m ? pairs[i].x : __uint_as_float(kInfBits), i);
+        bool again = false;
+        if (__any_sync(FGC_FULL_MASK, unclear || look)) {
+            // few rows come here: some are equal or in the wrong order
 #pragma unroll
             for (int r = 0; r < R; r++) {
-                d[r] = near.d[r];
-                j[r] = __float_as_uint(near.d[r]) < kInfBits ? __float_as_int(pairs[near.id[r]].y) : -1;
+                const float nd = __shfl_down_sync(FGC_FULL_MASK, d[r], 1), next = __shfl_sync(FGC_FULL_MASK, d[R - 1], 0);
+                unclear = unclear || (lane < 31 ? d[r] > nd : (r + 1 < R && d[r] > next));
             }
+            again = __any_sync(FGC_FULL_MASK, unclear);
+            if (again) {
+                // distances that differ by less than the keys tell: sorted as they are
+                SortedList<R> near;
+                near.init(lane, kn);
+#pragma unroll 1
+                for (int i = lane; i - lane < m; i += 32) near.merge32(lane, kn, i < m ? pairs[i].x : __uint_as_float(kInfBits), i);
+#pragma unroll
+                for (int r = 0; r < R; r++) {
+                    d[r] = near.d[r];
+                    j[r] = __float_as_uint(near.d[r]) < kInfBits ? __float_as_int(pairs[near.id[r]].y) : -1;
+                }
+            }
+            if (a.mark_ties == TieMarks::kAny) same = equal_in_list<R>(d, j, kn, lane);
         }
         kth = __float_as_uint(__shfl_sync(FGC_FULL_MASK, kn > 32 ? d[R - 1] : d[0], (kn - 1) & 31));
         if (again) {
@@ -821,7 +831,7 @@ k_tree_rows(const TreeArgs a)
         }
         kth = __reduce_max_sync(FGC_FULL_MASK, kth);
     }
-    const bool marked = a.mark_ties && full && (tie || kth == left_out);
+    const bool marked = a.mark_ties != TieMarks::kNone && (same || (full && (tie || kth == left_out)));
     if (lane == 0) {
         row_i[0] = marked ? kTieRow : (int64_t)orig_q;
         row_d[0] = 0.f;
@@ -855,7 +865,7 @@ static cudaError_t launch_tree(TreeArgs a, const TreeScratch &scratch, cudaStrea
 }  // namespace fgc
 
 int fgc::knn_search_tree_groups(int64_t n_vert, int32_t n_coords, const int64_t *row_splits, int64_t n_rs, int32_t K,
-                                int32_t has_direction, int32_t tf_compat, bool mark_ties, int64_t *out_idx, float *out_distsq,
+                                int32_t has_direction, int32_t tf_compat, TieMarks mark_ties, int64_t *out_idx, float *out_distsq,
                                 void *workspace, size_t workspace_bytes, fgc_stream_t stream)
 {
     FGC_NVTX("fgc_knn_search_tree_groups");

@@ -341,7 +341,7 @@ __device__ __forceinline__ void tree_query(const TreeArgs &a, int qi)
     int64_t *__restrict__ out_i = a.out_idx + (size_t)orig_q * K;
     float *__restrict__ out_d = a.out_dist + (size_t)orig_q * K;
     uint32_t last = 0;                       // the K-th distance (0: the list is not full)
-    bool tie = false;
+    bool tie = false, same = false;
     const int64_t pad = a.tf_compat ? (int64_t)orig_q : (int64_t)-1;
     if constexpr (R <= 2) {
         // ascending distances
@@ -361,6 +361,7 @@ __device__ __forceinline__ void tree_query(const TreeArgs &a, int qi)
             for (int r = 0; r < R; r++)
                 tie = tie || __any_sync(FGC_FULL_MASK, r * 32 + lane >= kn && __float_as_uint(list.d[r]) == last && list.id[r] >= 0);
         }
+        if (a.mark_ties == TieMarks::kAny) same = equal_in_list<R>(list.d, list.id, kn, lane);
 #pragma unroll
         for (int r = 0; r < R; r++) {
             const int s = r * 32 + lane;
@@ -381,7 +382,7 @@ __device__ __forceinline__ void tree_query(const TreeArgs &a, int qi)
         if (sel.n < kn) last = 0;
     }
     tie = tie || (kn > 0 && sel.n >= kn && last == sel.left_out);
-    const bool marked = a.mark_ties && tie;
+    const bool marked = a.mark_ties != TieMarks::kNone && (tie || same);
     if (lane == 0) {
         out_i[0] = marked ? kTieRow : (int64_t)orig_q;
         out_d[0] = 0.f;
@@ -458,7 +459,7 @@ static cudaError_t launch_tree(const TreeArgs &a, cudaStream_t s)
 }
 
 int tree_args(int64_t n_vert, int32_t n_coords, const int64_t *row_splits, int64_t n_rs, int32_t K, int32_t has_direction,
-              int32_t tf_compat, bool mark_ties, int64_t *out_idx, float *out_distsq, void *workspace, size_t workspace_bytes,
+              int32_t tf_compat, TieMarks mark_ties, int64_t *out_idx, float *out_distsq, void *workspace, size_t workspace_bytes,
               TreeArgs *a, KnnWorkspace *L, TreeLayout *T)
 {
     const int rc = check_knn_args(n_vert, n_coords, n_rs, K, workspace, workspace_bytes, L);
@@ -492,12 +493,12 @@ extern "C" int fgc_knn_search_tree(int64_t n_vert, int32_t n_coords, const int64
                                    int32_t has_direction, int32_t tf_compat, int64_t *out_idx, float *out_distsq,
                                    void *workspace, size_t workspace_bytes, fgc_stream_t stream)
 {
-    return fgc::knn_search_tree(n_vert, n_coords, row_splits, n_rs, K, has_direction, tf_compat, false, out_idx, out_distsq,
+    return fgc::knn_search_tree(n_vert, n_coords, row_splits, n_rs, K, has_direction, tf_compat, fgc::TieMarks::kNone, out_idx, out_distsq,
                                 workspace, workspace_bytes, stream);
 }
 
 int fgc::knn_search_tree(int64_t n_vert, int32_t n_coords, const int64_t *row_splits, int64_t n_rs, int32_t K,
-                         int32_t has_direction, int32_t tf_compat, bool mark_ties, int64_t *out_idx, float *out_distsq,
+                         int32_t has_direction, int32_t tf_compat, TieMarks mark_ties, int64_t *out_idx, float *out_distsq,
                          void *workspace, size_t workspace_bytes, fgc_stream_t stream)
 {
     FGC_NVTX("fgc_knn_search_tree");

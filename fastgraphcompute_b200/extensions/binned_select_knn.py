@@ -62,15 +62,14 @@ def knn_forward_raw(coords, row_splits, K, direction, tf_compat, count_evals=Fal
     return _forward(coords, row_splits, K, direction, tf_compat, count_evals, None, False)
 
 
-def knn_forward_with_order(coords, row_splits, K, direction, tf_compat, long_tails=False, in_order=True):
-    """Launch the forward on prepared tensors; returns (idx, distsq, order).  in_order: distances get gradients slot by slot, so
-    the order of neighbours at equal distances matters (it is the grid's)."""
+def knn_forward_with_order(coords, row_splits, K, direction, tf_compat, long_tails=False):
+    """Launch the forward on prepared tensors; returns (idx, distsq, order)."""
     order = torch.empty((coords.shape[0],), dtype=torch.int32, device=coords.device)
-    idx, dist, _ = _forward(coords, row_splits, K, direction, tf_compat, False, order, long_tails, in_order)
+    idx, dist, _ = _forward(coords, row_splits, K, direction, tf_compat, False, order, long_tails)
     return idx, dist, order
 
 
-def _forward(coords, row_splits, K, direction, tf_compat, count_evals, order, long_tails, in_order=True):
+def _forward(coords, row_splits, K, direction, tf_compat, count_evals, order, long_tails):
     dev = coords.device
     n_vert, n_coords = coords.shape
     n_rs = row_splits.numel()
@@ -81,18 +80,21 @@ def _forward(coords, row_splits, K, direction, tf_compat, count_evals, order, lo
         raise ValueError("binned_select_knn: unsupported problem size")
     if torch.cuda.current_device() != dev.index:
         with torch.cuda.device(dev):
-            return _forward(coords, row_splits, K, direction, tf_compat, count_evals, order, long_tails, in_order)
+            return _forward(coords, row_splits, K, direction, tf_compat, count_evals, order, long_tails)
     idx = torch.empty((n_vert, K), dtype=torch.int64, device=dev)
     dist = torch.empty((n_vert, K), dtype=torch.float32, device=dev)
     # what asks for a grid of a certain kind, or for its counters, gets the grid; so do direction flags: the cells of the
     # grid hold candidates only, the leaves of the tree all points (two row splits of 400 k uniform points in three
     # coordinates, K = 128, grid / tree in ms: a third of them candidates 3.8 / 5.8, one in twenty 6.6 / 24, one in two
     # thousand -- fewer than K - 1 in places -- 4.0 / 938)
-    tree = n_vert > 0 and not count_evals and target_occupancy <= 0 and grid_dims == 0 and (
-        (direction is None and n_vert >= 16384 and (        # (below, both rules say no: two calls less, 3 us)
-            _cabi.lib.fgc_knn_tree_preferred(n_vert, n_coords, n_rs, K, int(long_tails)) == 1 or
-            _cabi.lib.fgc_knn_groups_preferred(n_vert, n_coords, n_rs, K, int(long_tails), int(in_order)) == 1))
-        if search_tree is None else search_tree)
+    tree = n_vert > 0 and not count_evals and target_occupancy <= 0 and grid_dims == 0 and search_tree is not False
+    grid_order = False
+    if tree and search_tree is None:
+        tree = False
+        if direction is None and n_vert >= 16384:           # (below, both rules say no: two calls less, 3 us)
+            tree = _cabi.lib.fgc_knn_tree_preferred(n_vert, n_coords, n_rs, K, int(long_tails)) == 1
+            if not tree and _cabi.lib.fgc_knn_groups_preferred(n_vert, n_coords, n_rs, K, int(long_tails)) == 1:
+                tree, grid_order = True, not long_tails     # (sizes that the grid is otherwise taken for)
     ws = None
     if tree:
         forward_bytes = _cabi.lib.fgc_knn_forward_workspace_bytes(n_vert, n_coords, n_rs, K, 64)
@@ -120,6 +122,8 @@ def _forward(coords, row_splits, K, direction, tf_compat, count_evals, order, lo
     flags = (1 if count_evals else 0) | (8 if form == 3 else 16 if form == 4 else 0) | (64 if tree else 0)
     if tree and not long_tails:
         flags |= 128        # equal K-th distances: the grid's choice, whichever search ran
+        if grid_order:
+            flags |= 256    # equal distances anywhere: the grid's order
     # The status word is final once the grid is built (non-finite input and malformed row_splits are
     # detected by its first two kernels).  A one-thread kernel stores it into page-locked memory and
     # the library looks at it after the search has been launched: the host waits for the short
@@ -242,8 +246,7 @@ class _BinnedKNN(torch.autograd.Function):
     @staticmethod
     def forward(ctx, coords, row_splits, K, direction, tf_compat, long_tails):
         _cabi.require_cuda(coords, "coords")
-        idx, dist, order = knn_forward_with_order(coords, row_splits, K, direction, tf_compat, long_tails,
-                                                  ctx.needs_input_grad[0])
+        idx, dist, order = knn_forward_with_order(coords, row_splits, K, direction, tf_compat, long_tails)
         ctx.save_for_backward(idx, coords, order)
         ctx.mark_non_differentiable(idx, order)
         # no zero tensors for the gradients of idx and order (an int64 [N, K] fill per backward)

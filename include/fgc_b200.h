@@ -216,10 +216,9 @@ int fgc_knn_tree_preferred(int64_t n_vert, int32_t n_coords, int64_t n_rs, int32
 /*
  * 1 where fgc_knn_forward with FGC_FORWARD_TREE was measured to be ahead of the grid although
  * fgc_knn_tree_preferred, which stands for fgc_knn_search_tree, is 0: in up to five coordinates it takes all
- * queries of a leaf at once.  in_order != 0: the order of neighbours at equal distances has to be the grid's.
+ * queries of a leaf at once.
  */
-int fgc_knn_groups_preferred(int64_t n_vert, int32_t n_coords, int64_t n_rs, int32_t K, int32_t long_tails,
-                             int32_t in_order);
+int fgc_knn_groups_preferred(int64_t n_vert, int32_t n_coords, int64_t n_rs, int32_t K, int32_t long_tails);
 int fgc_knn_build_tree(const float *coords, int64_t n_vert, int32_t n_coords, const int64_t *row_splits, int64_t n_rs,
                        int32_t K, const int64_t *direction_or_null, void *workspace, size_t workspace_bytes,
                        fgc_stream_t stream);
@@ -239,6 +238,8 @@ int fgc_knn_search_tree(int64_t n_vert, int32_t n_coords, const int64_t *row_spl
 #define FGC_FORWARD_TREE 64    /* flags: search on a tree instead of a grid */
 #define FGC_FORWARD_GRID_TIES 128 /* with it: rows with a choice among equal K-th distances are searched again on a grid,
                                     unless more than a sixteenth of all rows are such (lattice coordinates) */
+#define FGC_FORWARD_GRID_ORDER 256 /* with both: K <= 65: so are rows that hold equal distances, whose slots the grid may
+                                     give in another order */
 /*
  * Workspace with which fgc_knn_forward is fastest: with FGC_FORWARD_TREE and up to five coordinates up to 256 MB more than
  * fgc_knn_workspace_bytes, for the search of all queries of a leaf at once.  With fgc_knn_workspace_bytes it takes one

@@ -256,15 +256,81 @@ def test_groups_in_a_cuda_graph(monkeypatch):
         assert torch.equal(idx, ei) and torch.equal(dist, ed)
 
 
-@pytest.mark.parametrize("n,D,row_splits,K,long_tails,in_order,groups", [
-    (16383, 4, 1, 40, 1, 0, 0), (16384, 4, 1, 8, 1, 1, 1), (16384, 4, 1, 7, 1, 1, 0), (20000, 4, 2, 24, 1, 1, 1), (20000, 4, 2, 23, 1, 1, 0),
-    (20000, 4, 10, 40, 1, 1, 1), (20000, 4, 14, 40, 1, 1, 0), (20000, 3, 1, 16, 1, 1, 1), (20000, 3, 10, 48, 1, 1, 1),
-    (60000, 5, 4, 40, 0, 0, 1), (60000, 5, 5, 40, 0, 0, 0), (60000, 5, 4, 40, 0, 1, 0), (60000, 5, 4, 66, 0, 1, 1),
-    (50000, 4, 1, 72, 0, 1, 1), (50000, 4, 1, 71, 0, 0, 0), (200000, 4, 8, 40, 0, 0, 1), (200000, 4, 7, 40, 0, 0, 0),
-    (800000, 4, 1, 16, 0, 0, 1), (800000, 4, 1, 16, 0, 1, 0), (200000, 3, 1, 64, 0, 0, 1), (200000, 3, 1, 64, 0, 1, 0),
-    (800000, 3, 9, 36, 0, 0, 1), (800000, 3, 9, 35, 0, 0, 0), (150000, 3, 1, 66, 0, 1, 1), (50000, 3, 1, 80, 0, 1, 1),
-    (20000, 3, 1, 128, 0, 1, 1), (400000, 2, 1, 200, 0, 0, 0), (400000, 6, 1, 40, 0, 0, 0)])
-def test_groups_by_size(n, D, row_splits, K, long_tails, in_order, groups):
+@pytest.mark.gpu
+@pytest.mark.parametrize("D,K", [(3, 9), (3, 33), (4, 34), (4, 65), (5, 20), (5, 65)])
+@pytest.mark.parametrize("scratch", [True, False])
+def test_equal_distances_take_the_grids_slots(D, K, scratch, monkeypatch):
+    """Where the search by groups is taken instead of the grid, neighbours at equal distances have the slots that the grid gives
+    them (while a sixteenth of the rows or fewer hold such)."""
+    km = importlib.import_module("fastgraphcompute_b200.extensions.binned_select_knn")
+    g = torch.Generator().manual_seed(D * K)
+    n = 20000
+    x = torch.rand((n, D), generator=g)
+    x[: n // 25] = torch.randint(0, 5, (n // 25, D), generator=g) * 0.25 + 3.0          # a patch of lattice, away from the rest
+    x = x[torch.randperm(n, generator=g)].to(DEV)
+    # (row splits small enough for a warp of the grid search to scan: its whole-CTA scan leaves rows unsorted)
+    rs = torch.cat([torch.arange(0, n, 4000), torch.tensor([n])]).to(DEV)
+    grid = km._forward(x, rs, K, None, False, False, None, False)
+    lib = km._cabi.lib
+    call, seen = lib.fgc_knn_forward, []
+
+    def recorded(*args):
+        seen.append(args[9])
+        return call(*args)
+    if not scratch:
+        _without_scratch(km, monkeypatch)
+    monkeypatch.setattr(lib, "fgc_knn_forward", recorded)
+    monkeypatch.setattr(lib, "fgc_knn_groups_preferred", lambda *args: 1)
+    groups = km._forward(x, rs, K, None, False, False, None, False)
+    monkeypatch.setattr(km, "search_tree", True)
+    alone = km._forward(x, rs, K, None, False, False, None, True)
+    assert [f & 448 for f in seen] == [448, 64]
+    assert torch.equal(groups[0], grid[0]) and torch.equal(groups[1], grid[1]) and torch.equal(alone[1], grid[1])
+    assert 0 < int((alone[0] != grid[0]).any(dim=1).sum()) <= n // 16
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,D,row_splits,K", [(200000, 3, 1, 64), (200000, 4, 10, 40), (60000, 5, 4, 40), (800000, 4, 2, 16)])
+def test_gradients_change_no_search(n, D, row_splits, K, monkeypatch):
+    """The rule chooses the search by groups at these sizes, with and without gradients: same neighbours, same slots; the
+    distances are the grid's, and so are the sets."""
+    from fastgraphcompute_b200 import binned_select_knn
+    km = importlib.import_module("fastgraphcompute_b200.extensions.binned_select_knn")
+    g = torch.Generator().manual_seed(K)
+    x = torch.randn((n, D), generator=g)
+    x[: n // 50] = torch.round(x[: n // 50] * 4) / 4
+    x = x[torch.randperm(n, generator=g)].to(DEV)
+    rs = torch.linspace(0, n, row_splits + 1).long().to(DEV)
+    lib = km._cabi.lib
+    call, seen = lib.fgc_knn_forward, []
+
+    def recorded(*args):
+        seen.append(args[9] & 64)
+        return call(*args)
+    monkeypatch.setattr(lib, "fgc_knn_forward", recorded)
+    idx, dist = binned_select_knn(K, x, rs)
+    idx_g, dist_g = binned_select_knn(K, x.clone().requires_grad_(True), rs)
+    traced = torch.ops.fgc_b200.knn_forward(x, rs, K, None, False)
+    assert seen == [64, 64, 64]
+    assert torch.equal(idx, idx_g) and torch.equal(dist, dist_g.detach())
+    assert torch.equal(idx, traced[0]) and torch.equal(dist, traced[1])
+    monkeypatch.setattr(km, "search_tree", False)
+    gi, gd = binned_select_knn(K, x, rs)
+    assert torch.equal(dist.sort(dim=1).values, gd.sort(dim=1).values)
+    edge = gd.amax(dim=1, keepdim=True)
+    inside = [torch.where(d < edge, i, torch.full_like(i, -1)).sort(dim=1).values for i, d in ((gi, gd), (idx, dist))]
+    assert torch.equal(*inside)
+
+
+@pytest.mark.parametrize("n,D,row_splits,K,long_tails,groups", [
+    (16383, 4, 1, 40, 1, 0), (16384, 4, 1, 8, 1, 1), (16384, 4, 1, 7, 1, 0), (20000, 4, 2, 24, 1, 1), (20000, 4, 2, 23, 1, 0),
+    (20000, 4, 10, 40, 1, 1), (20000, 4, 14, 40, 1, 0), (20000, 3, 1, 16, 1, 1), (20000, 3, 10, 48, 1, 1),
+    (60000, 5, 4, 40, 0, 1), (60000, 5, 5, 40, 0, 0), (60000, 5, 4, 39, 0, 0), (60000, 5, 4, 66, 0, 1),
+    (50000, 4, 1, 72, 0, 1), (50000, 4, 1, 71, 0, 0), (200000, 4, 8, 40, 0, 1), (200000, 4, 7, 40, 0, 0),
+    (800000, 4, 1, 16, 0, 1), (800000, 4, 1, 15, 0, 0), (200000, 3, 1, 64, 0, 1), (199999, 3, 1, 64, 0, 0),
+    (800000, 3, 9, 36, 0, 1), (800000, 3, 9, 35, 0, 0), (150000, 3, 1, 66, 0, 1), (50000, 3, 1, 80, 0, 1),
+    (20000, 3, 1, 128, 0, 1), (400000, 2, 1, 200, 0, 0), (400000, 6, 1, 40, 0, 0)])
+def test_groups_by_size(n, D, row_splits, K, long_tails, groups):
     """The edges of the ranges where the search by groups was measured ahead of the grid."""
     from fastgraphcompute_b200 import _cabi
-    assert _cabi.lib.fgc_knn_groups_preferred(n, D, row_splits + 1, K, long_tails, in_order) == groups
+    assert _cabi.lib.fgc_knn_groups_preferred(n, D, row_splits + 1, K, long_tails) == groups
