@@ -453,6 +453,11 @@ extern "C" int fgc_knn_tree_preferred(int64_t n_vert, int32_t n_coords, int64_t 
 //                      0.72 / 1.20;  K = 66: in three or more 0.60 / 0.77 / 0.53
 // The worst are row splits of 5000 points in 50 clusters, for which the grid's cells are right (1.05 to 1.3 with K <= 65), and lattices
 // (1.0 to 1.2: a million points, K = 64, on 40 x 40 x 40 places).
+// Small row splits: a leaf warp has few queries, and the grid takes whole ones (least_mean).  Uniform points, splits of 100 / 200 / 256 /
+// 300 / 400 points: three coordinates, K = 36 800 k 1.43 / 0.89 / 0.76 / 0.68 / 0.57, K = 64 200 k 1.76 / 1.19 / 1.05 / 0.95 / 0.76, K = 66 1.24 / 0.57 /
+// 0.46, K = 128 1.78 / 0.73 / 0.52, K = 200 1.32 / 1.28 / 0.62, K = 257 20 k - / - / 1.32 / - / 0.65; four, K = 40 200 k - / 1.20 / 1.04 / 0.96 / 0.79.
+// Short lists in four coordinates: K = 16 in splits of 1500 0.90 / 1.12 / 1.47, of 5000 0.89 / 1.08 / 1.09, K = 24 of 1500 0.82 / 1.03 / 1.24,
+// K = 32 0.79 / 0.99 / 0.77.
 // Whether distances get gradients plays no part: the same call takes the same search with and without, and gives the
 // same neighbours in the same slots.
 // long_tails: learned coordinates as in fgc_knn_tree_preferred, no second look: three coordinates, row splits of 15 k or more 0.60
@@ -476,11 +481,12 @@ extern "C" int fgc_knn_groups_preferred(int64_t n_vert, int32_t n_coords, int64_
     } else if (n_coords == 4) {
         least = n_vert >= 50000 ? 72 : 128;
         if (n_vert >= 200000 && n_events >= 8) least = 40;
-        if (n_vert >= 800000) least = 16;
+        if (n_vert >= 800000) least = mean >= 5000 ? 16 : 32;
     } else {
         least = n_vert >= 800000 ? 36 : (n_vert >= 200000 ? 64 : (n_vert >= 150000 ? 66 : (n_vert >= 50000 ? 80 : 128)));
     }
-    if (K < least) return 0;
+    const int64_t least_mean = K <= 65 ? (n_vert >= 800000 ? 256 : 300) : (K < 160 ? 200 : K + K / 4);
+    if (K < least || (!long_tails && mean < least_mean)) return 0;
     return tree_layout(knn_workspace_layout(n_vert, n_coords, n_rs, K), n_vert, n_coords, n_rs).fits ? 1 : 0;
 }
 

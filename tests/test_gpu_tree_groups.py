@@ -329,6 +329,9 @@ def test_gradients_change_no_search(n, D, row_splits, K, monkeypatch):
     (50000, 4, 1, 72, 0, 1), (50000, 4, 1, 71, 0, 0), (200000, 4, 8, 40, 0, 1), (200000, 4, 7, 40, 0, 0),
     (800000, 4, 1, 16, 0, 1), (800000, 4, 1, 15, 0, 0), (200000, 3, 1, 64, 0, 1), (199999, 3, 1, 64, 0, 0),
     (800000, 3, 9, 36, 0, 1), (800000, 3, 9, 35, 0, 0), (150000, 3, 1, 66, 0, 1), (50000, 3, 1, 80, 0, 1),
+    (800000, 4, 160, 31, 0, 1), (800000, 4, 161, 31, 0, 0), (800000, 4, 161, 32, 0, 1), (800000, 4, 16000, 40, 0, 0),
+    (800000, 3, 3125, 36, 0, 1), (800000, 3, 3126, 36, 0, 0), (200000, 3, 666, 64, 0, 1), (200000, 3, 667, 64, 0, 0),
+    (200000, 4, 1000, 159, 0, 1), (200000, 4, 1001, 72, 0, 0), (20000, 3, 80, 200, 0, 1), (20000, 3, 81, 200, 0, 0),
     (20000, 3, 1, 128, 0, 1), (400000, 2, 1, 200, 0, 0), (400000, 6, 1, 40, 0, 0)])
 def test_groups_by_size(n, D, row_splits, K, long_tails, groups):
     """The edges of the ranges where the search by groups was measured ahead of the grid."""
