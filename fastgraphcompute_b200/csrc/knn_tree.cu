@@ -389,9 +389,19 @@ static cudaError_t launch_boxes(const float *coords, int n, int n_coords, const 
 
 }  // namespace fgc
 
+// Points per row split that the search by groups needs: with fewer a leaf's warp has few queries, and the grid takes whole
+// row splits.  Time over the grid's, uniform points, splits of 100 / 200 / 256 / 300 / 400 points: three coordinates, K = 36, 800 k 1.43 / 0.89 / 0.76 /
+// 0.68 / 0.57, K = 64, 200 k 1.76 / 1.19 / 1.05 / 0.95 / 0.76, K = 66 1.24 / 0.57 / 0.46, K = 128 1.78 / 0.73 / 0.52, K = 200 1.32 / 1.28 / 0.62, 20 k,
+// K = 257 in splits of 256 1.32, 400 0.65; four, 200 k, K = 40 - / 1.20 / 1.04 / 0.96 / 0.79; five, 800 k, K = 66 1.07 / 0.54, in splits of 50 2.2.
+static int64_t least_row_split(int64_t n_vert, int K)
+{
+    return K <= 65 ? (n_vert >= 800000 ? 256 : 300) : (K < 160 ? 200 : K + K / 4);
+}
+
 // Where the tree is the better search.  Neither search is ahead for all data: the figures are the time of the tree over that of
 // the grid, whole forward, B200, for uniform points in a cube / normal ones / 50 clusters of width 0.02 ("mixture").
-// Below 16384 points the sort's launches outweigh the search (10 k in three coordinates, K = 100: 0.110 / 0.112 ms).
+// Below 16384 points the sort's launches outweigh the search (10 k in three coordinates, K = 100: 0.110 / 0.112 ms); in up to
+// five coordinates, where the forward searches by groups, so they do for tiny row splits (least_row_split).
 //
 // D = 3, K >= 96: the grid's list of four slots a lane (K > 65) is slow, and a dense cluster fits into one of its cells.  400 k
 // points in two row splits, K = 96: 0.98 / 0.74 / 0.74, skewed clusters 0.41; K = 80: 1.06 / 0.70 / 0.67, K = 66: 1.20 / 0.78 /
@@ -435,7 +445,7 @@ extern "C" int fgc_knn_tree_preferred(int64_t n_vert, int32_t n_coords, int64_t 
     case 9: case 10: case 11: least = 8; break;
     default: least = 1;
     }
-    if (K < least) return 0;
+    if (K < least || (K > 65 && n_coords <= kGroupDims && n_vert / n_events < least_row_split(n_vert, K))) return 0;
     return tree_layout(knn_workspace_layout(n_vert, n_coords, n_rs, K), n_vert, n_coords, n_rs).fits ? 1 : 0;
 }
 
@@ -453,9 +463,6 @@ extern "C" int fgc_knn_tree_preferred(int64_t n_vert, int32_t n_coords, int64_t 
 //                      0.72 / 1.20;  K = 66: in three or more 0.60 / 0.77 / 0.53
 // The worst are row splits of 5000 points in 50 clusters, for which the grid's cells are right (1.05 to 1.3 with K <= 65), and lattices
 // (1.0 to 1.2: a million points, K = 64, on 40 x 40 x 40 places).
-// Small row splits: a leaf warp has few queries, and the grid takes whole ones (least_mean).  Uniform points, splits of 100 / 200 / 256 /
-// 300 / 400 points: three coordinates, K = 36 800 k 1.43 / 0.89 / 0.76 / 0.68 / 0.57, K = 64 200 k 1.76 / 1.19 / 1.05 / 0.95 / 0.76, K = 66 1.24 / 0.57 /
-// 0.46, K = 128 1.78 / 0.73 / 0.52, K = 200 1.32 / 1.28 / 0.62, K = 257 20 k - / - / 1.32 / - / 0.65; four, K = 40 200 k - / 1.20 / 1.04 / 0.96 / 0.79.
 // Short lists in four coordinates: K = 16 in splits of 1500 0.90 / 1.12 / 1.47, of 5000 0.89 / 1.08 / 1.09, K = 24 of 1500 0.82 / 1.03 / 1.24,
 // K = 32 0.79 / 0.99 / 0.77.
 // Whether distances get gradients plays no part: the same call takes the same search with and without, and gives the
@@ -485,8 +492,7 @@ extern "C" int fgc_knn_groups_preferred(int64_t n_vert, int32_t n_coords, int64_
     } else {
         least = n_vert >= 800000 ? 36 : (n_vert >= 200000 ? 64 : (n_vert >= 150000 ? 66 : (n_vert >= 50000 ? 80 : 128)));
     }
-    const int64_t least_mean = K <= 65 ? (n_vert >= 800000 ? 256 : 300) : (K < 160 ? 200 : K + K / 4);
-    if (K < least || (!long_tails && mean < least_mean)) return 0;
+    if (K < least || mean < least_row_split(n_vert, K)) return 0;
     return tree_layout(knn_workspace_layout(n_vert, n_coords, n_rs, K), n_vert, n_coords, n_rs).fits ? 1 : 0;
 }
 

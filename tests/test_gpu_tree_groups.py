@@ -337,3 +337,14 @@ def test_groups_by_size(n, D, row_splits, K, long_tails, groups):
     """The edges of the ranges where the search by groups was measured ahead of the grid."""
     from fastgraphcompute_b200 import _cabi
     assert _cabi.lib.fgc_knn_groups_preferred(n, D, row_splits + 1, K, long_tails) == groups
+
+
+@pytest.mark.parametrize("n,D,row_splits,K,long_tails,tree", [
+    (800000, 3, 16000, 100, 0, 0), (800000, 3, 4000, 100, 0, 1), (800000, 3, 4001, 100, 0, 0), (800000, 3, 3200, 200, 0, 1), (800000, 3, 3201, 200, 0, 0),
+    (800000, 4, 16000, 36, 0, 0), (200000, 4, 4000, 66, 1, 0), (200000, 4, 1000, 66, 1, 1), (800000, 5, 16000, 66, 0, 0), (800000, 5, 4000, 66, 0, 1),
+    (60000, 5, 1, 40, 0, 1), (60000, 6, 1200, 66, 0, 1)])
+def test_tiny_row_splits_are_searched_on_the_grid(n, D, row_splits, K, long_tails, tree):
+    """Both rules together: which calls leave the grid."""
+    from fastgraphcompute_b200 import _cabi
+    lib = _cabi.lib
+    assert tree == max(rule(n, D, row_splits + 1, K, long_tails) for rule in (lib.fgc_knn_tree_preferred, lib.fgc_knn_groups_preferred))
