@@ -86,11 +86,12 @@ __device__ __forceinline__ int seed_leaves(int kn, int dims)
     return min(4 + kn / 6, 28) + (dims >= 4 ? 6 : 0) + (dims >= 5 ? 6 : 0);
 }
 
-// A squared distance t with what rounding can add to |c|^2 - 2 c.q + |q|^2 for a point c within t of q (coordinates
-// relative to some centre, |q|^2 = q2, so that |c| <= |q| + sqrt(t)).  In tf32 the coordinates of q are off by 2^-11 of their
-// size (rounded) and those of c by 2^-10 (cut off): 3 * 2^-10 * |q| |c| on 2 c.q, taken as 0.0032.  Everything else is
-// in single precision or split in two: at most 50 operations that are off by 2^-23 of (|q| + |c|)^2.  The last term
-// is for squares that underflow.
+// An upper bound on the distance d of a point c from q whose |c|^2 - 2 c.q + |q|^2 comes out as t or less (coordinates relative to
+// some centre, |q|^2 = q2).  |c| is at most |q| + sqrt(d).  Both operands are rounded to tf32, 2^-11 of their size: e(d) = 2^-9 |q| (|q| +
+// sqrt(d)) on 2 c.q.  Everything else is in single precision or split in two: at most 50 operations that are off by 2^-23 of
+// (|q| + |c|)^2.  So d <= t + e(d).  The sum T below has sqrt(t) in the place of sqrt(d): |q| + sqrt(T) is at most 1.057 (|q| + sqrt(t)),
+// since T - t is 0.0032 |q| (|q| + sqrt(t)) and a little, so e(T) <= 0.0021 |q| (|q| + sqrt(t)) is less than T - t, and beyond T e grows
+// by less than a fiftieth of d: no larger d fits.  The last term is for squares that underflow.
 __device__ __forceinline__ float widened(float t, float q2)
 {
     const float q = sqrtf(q2), c = q + sqrtf(t), s = q + c;
@@ -279,7 +280,7 @@ __device__ __forceinline__ void bound_leaf(const TreeArgs &a, const int slot)
                 for (int i4 = 0; i4 < 2; i4++) {
                     float z = 4 * i4 + p4 == DC ? c2_high : (4 * i4 + p4 == DC + 1 ? c2_low : 0.f);
                     if (i4 < CHUNKS && 4 * i4 + p4 < DC) z = y[i4 < CHUNKS ? i4 : 0];
-                    b[i4] = __float_as_uint(z);
+                    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(b[i4]) : "f"(z));
                 }
 #pragma unroll
                 for (int m = 0; m < 2; m++) {

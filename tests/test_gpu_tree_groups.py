@@ -83,6 +83,32 @@ def test_groups_find_what_the_grid_finds(kind, sizes, D, K, listed):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("kind,D,K", [("uniform", 3, 17), ("offset", 4, 40), ("pairs", 3, 2), ("pairs", 5, 8), ("mixed", 3, 9), ("uniform", 5, 100),
+                                      ("near", 4, 30)])
+def test_bounds_hold(kind, D, K):
+    """No query's bound, taken from distances in low precision, is below its K-th distance; "pairs" are clouds of eight points whose
+    distances are a millionth of those between them, several to a leaf."""
+    km = importlib.import_module("fastgraphcompute_b200.extensions.binned_select_knn")
+    g = torch.Generator().manual_seed(K)
+    n = 20000
+    x = _points(kind, n, D, g)
+    if kind == "pairs":
+        x = torch.rand((n // 8, D), generator=g).repeat_interleave(8, dim=0) + 1e-3 * torch.rand((n, D), generator=g)
+    x = x.to(DEV)
+    rs = torch.tensor([0, n], device=DEV)
+    _, dist, ws = _forward(km, x, rs, K, True)
+    plain = km._cabi.lib.fgc_knn_workspace_bytes(n, D, 2, K)
+    cap = {3: 512, 4: 1024, 5: 3072}[D]                    # leaves of a list; then their number and 32 bounds a leaf
+    slots = (ws.numel() - plain) // (4 * (cap + 33))
+    bound = ws[plain:].view(torch.float32)[slots * (cap + 1):][:n]
+    kth = torch.where(dist > 0, dist, torch.zeros_like(dist)).amax(dim=1)[km.cell_order(ws, n, D, 2, K).long()]
+    taken = bound >= 0                                      # (negative: searched one query at a time)
+    assert bool(taken.any()) and bool((bound[taken] >= kth[taken]).all())
+    if kind == "uniform":
+        assert float((bound / kth).median()) < 2.0
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("D,K", [(2, 11), (3, 20)])
 def test_missing_points_of_a_leaf_give_no_bound(D, K):
     """Row splits of 33 points: one leaf across 2.6e19 with its last point near its middle, another with a single point beside
