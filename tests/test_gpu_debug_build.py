@@ -23,8 +23,8 @@ def test_golden_cases_under_the_bounds_check_build():
     env["FGC_B200_LIB"] = DEBUG_LIB
     env["PYTHONPATH"] = ROOT + os.pathsep + env.get("PYTHONPATH", "")
     r = subprocess.run([sys.executable, "-m", "pytest", "-q", "-x", "-m", "gpu", "-p", "no:cacheprovider",
-                        os.path.join(ROOT, "tests", "test_gpu_parity.py"),
-                        "-k", "golden or repeated_search or random_configurations or tree_search"],
+                        os.path.join(ROOT, "tests", "test_gpu_parity.py"), os.path.join(ROOT, "tests", "test_gpu_tree_groups.py"),
+                        "-k", "golden or repeated_search or random_configurations or tree_search or (tree_groups and not no_longer)"],
                        env=env, cwd=ROOT, capture_output=True, text=True, timeout=1500)
     tail = r.stdout[-3000:] + r.stderr[-2000:]
     assert r.returncode == 0 and " passed" in r.stdout, tail

@@ -7,6 +7,9 @@ import math
 import pytest
 import torch
 
+import parity
+from oracle import oracle
+
 DEV = "cuda:0"
 
 
@@ -228,6 +231,66 @@ def test_a_workspace_without_scratch_is_searched_one_query_at_a_time(D, K, monke
     monkeypatch.setattr(lib, "fgc_knn_forward_workspace_bytes", lambda *args: small)
     _, dist, ws = _forward(km, x, rs, K, True)
     assert ws.numel() == small and torch.equal(dist.sort(dim=1).values, expected.sort(dim=1).values)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sizes,D,K", [
+    ([1, 31, 32, 33, 0, 65], 2, 34), ([1023, 1024, 1025, 2], 3, 2), ([900, 40], 3, 1), ([3000], 3, 66), ([0, 2100, 0], 4, 129), ([700, 1300], 4, 130),
+    ([900], 4, 257), ([1100], 3, 200), ([40, 90, 1100], 5, 65), ([700], 5, 20), ([800, 300], 5, 129), ([600], 5, 257), ([33000], 5, 9)])
+@pytest.mark.parametrize("entry", ["forward", "search_tree"])
+def test_one_query_at_a_time_matches_oracle(sizes, D, K, entry, monkeypatch):
+    """The search one query at a time in up to five coordinates, which a workspace without scratch and fgc_knn_search_tree reach: the
+    list forms (K = 33, 65, 129, 257) and float4 counts, empty and tiny row splits, equal distances, direction flags, own-id
+    padding; several searches on one tree."""
+    km = importlib.import_module("fastgraphcompute_b200.extensions.binned_select_knn")
+    cabi, lib = km._cabi, km._cabi.lib
+    g = torch.Generator().manual_seed(100 * D + K)
+    n = sum(sizes)
+    pts = torch.randn((n, D), generator=g)
+    pts[: n // 4] = torch.round(pts[: n // 4] * 2) / 2          # equal distances, equal points
+    rs = torch.tensor([0] + sizes, dtype=torch.int64).cumsum(0)
+    x, splits = pts.to(DEV), rs.to(DEV)
+    _without_scratch(km, monkeypatch)
+    monkeypatch.setattr(km, "search_tree", True)
+    for direction in (None, torch.randint(0, 4, (n,), generator=g)):
+        compat = direction is not None
+        oi, od = oracle.binned_select_knn(K, pts.numpy(), rs.numpy(), torch_compatible_indices=compat,
+                                          direction=None if direction is None else direction.numpy())
+        flags = None if direction is None else direction.to(DEV)
+        if entry == "forward":
+            found = [km.knn_forward_raw(x, splits, K, flags, compat)[:2] for _ in range(2)]
+        else:
+            nb, st = lib.fgc_knn_workspace_bytes(n, D, splits.numel(), K), cabi.current_stream(x.device)
+            ws = torch.empty(nb, dtype=torch.uint8, device=DEV)
+            assert lib.fgc_knn_build_tree(cabi.ptr(x), n, D, cabi.ptr(splits), splits.numel(), K, cabi.ptr(flags), cabi.ptr(ws), nb, st) == 0
+            found = []
+            for _ in range(2):
+                idx, dist = torch.empty((n, K), dtype=torch.int64, device=DEV), torch.empty((n, K), device=DEV)
+                assert lib.fgc_knn_search_tree(n, D, cabi.ptr(splits), splits.numel(), K, int(compat), int(compat), cabi.ptr(idx),
+                                               cabi.ptr(dist), cabi.ptr(ws), nb, st) == 0
+                found.append((idx, dist))
+        assert torch.equal(found[0][0], found[1][0]) and torch.equal(found[0][1], found[1][1])
+        parity.assert_knn_parity(found[0][0].cpu().numpy(), found[0][1].cpu().numpy(), oi, od, what="one query D=%d K=%d" % (D, K))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("flags", [False, True])
+def test_two_rounds_with_the_second_look(flags, monkeypatch):
+    """800 000 points in five coordinates take two rounds of the scratch; tied rows of both are searched again."""
+    km = importlib.import_module("fastgraphcompute_b200.extensions.binned_select_knn")
+    g = torch.Generator().manual_seed(4)
+    n, K = 800000, 7
+    x = torch.rand((n, 5), generator=g)
+    x[: n // 40] = torch.randint(0, 9, (n // 40, 5), generator=g) * 0.25 + 3.0          # lattices, away from the rest
+    x[n - n // 80:] = torch.randint(0, 7, (n // 80, 5), generator=g) * 0.25 - 3.0
+    x = x[torch.randperm(n, generator=g)].to(DEV)
+    rs = torch.cat([torch.arange(0, n, 4000), torch.tensor([n])]).to(DEV)
+    direction = torch.randint(0, 4, (n,), generator=g).to(DEV) if flags else None
+    grid = km._forward(x, rs, K, direction, False, False, None, False)
+    monkeypatch.setattr(km, "search_tree", True)
+    tree = km._forward(x, rs, K, direction, False, False, None, False)
+    assert torch.equal(tree[0].sort(dim=1).values, grid[0].sort(dim=1).values)
+    assert torch.equal(tree[1].sort(dim=1).values, grid[1].sort(dim=1).values)
 
 
 @pytest.mark.gpu
