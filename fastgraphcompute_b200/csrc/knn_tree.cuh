@@ -101,9 +101,12 @@ struct TreeScratch {
 };
 constexpr int kGroupDims = 5;                                 // searches by groups take up to so many coordinates
 // Leaves that a leaf's queries may need (mean over uniform, normal and clustered points, K = 16 to 200: 36 to 110 in three
-// coordinates, 140 to 350 in four, 1000 in five); with more they are searched one by one.
-inline int tree_list_cap(int n_coords) { return n_coords <= 3 ? 512 : (n_coords == 4 ? 1024 : 3072); }
-constexpr size_t kTreeScratchBytes = (size_t)256 << 20;       // larger searches take several rounds
+// coordinates, 140 to 350 in four, 1000 in five); with more they are searched one by one.  A million normal points in five
+// coordinates, K = 40, with 768 / 1536 / 2304 / 3072 of them: 17.2 / 15.0 / 15.2 / 15.3 ms (77 / 16 / 7 / 4 % listed); 600 k uniform ones, K =
+// 200: 12.0 / 11.0 / 11.0 / 10.9.  A leaf of 32 points takes 2180 / 4228 / 6276 bytes in three / four / five.
+inline int tree_list_cap(int n_coords) { return n_coords <= 3 ? 512 : (n_coords == 4 ? 1024 : 1536); }
+// Larger searches take several rounds (6.4 M points in three coordinates 13.54 ms, with half of it 13.59; 3 M in five 43.4 and 43.6).
+constexpr size_t kTreeScratchBytes = (size_t)256 << 20;
 inline size_t tree_slot_bytes(int n_coords) { return 4 * ((size_t)tree_list_cap(n_coords) + 1 + 32); }
 // What a workspace for searches by groups holds behind the sections of the grid.
 inline size_t tree_extra_bytes(int64_t n_vert, int n_coords, int64_t n_rs)

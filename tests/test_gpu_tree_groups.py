@@ -63,10 +63,10 @@ def _forward(km, x, rs, K, tree, direction=None):
 @pytest.mark.parametrize("kind,sizes,D,K,listed", [
     ("far", [3000], 3, 17, None), ("far", [2000, 40], 5, 66, None), ("near", [4000], 4, 40, None), ("near", [900, 900], 3, 130, None),
     ("offset", [5000, 33, 1], 3, 65, None), ("offset", [5000], 5, 33, None), ("mixed", [60000], 3, 9, True), ("mixed", [60000], 4, 100, True),
-    ("uniform", [800000], 5, 9, None)])
+    ("uniform", [1500000], 5, 9, None)])
 def test_groups_find_what_the_grid_finds(kind, sizes, D, K, listed):
-    """Distances are equal bit for bit, ids up to the choice among equal K-th distances; 800 000 points in five coordinates take
-    two rounds of the scratch."""
+    """Distances are equal bit for bit, ids up to the choice among equal K-th distances; 1 500 000 points in five coordinates
+    take two rounds of the scratch."""
     km = importlib.import_module("fastgraphcompute_b200.extensions.binned_select_knn")
     g = torch.Generator().manual_seed(D * K)
     n = sum(sizes)
@@ -101,7 +101,7 @@ def test_bounds_hold(kind, D, K):
     rs = torch.tensor([0, n], device=DEV)
     _, dist, ws = _forward(km, x, rs, K, True)
     plain = km._cabi.lib.fgc_knn_workspace_bytes(n, D, 2, K)
-    cap = {3: 512, 4: 1024, 5: 3072}[D]                    # leaves of a list; then their number and 32 bounds a leaf
+    cap = {3: 512, 4: 1024, 5: 1536}[D]                    # leaves of a list; then their number and 32 bounds a leaf
     slots = (ws.numel() - plain) // (4 * (cap + 33))
     bound = ws[plain:].view(torch.float32)[slots * (cap + 1):][:n]
     kth = torch.where(dist > 0, dist, torch.zeros_like(dist)).amax(dim=1)[km.cell_order(ws, n, D, 2, K).long()]
@@ -276,10 +276,10 @@ def test_one_query_at_a_time_matches_oracle(sizes, D, K, entry, monkeypatch):
 @pytest.mark.gpu
 @pytest.mark.parametrize("flags", [False, True])
 def test_two_rounds_with_the_second_look(flags, monkeypatch):
-    """800 000 points in five coordinates take two rounds of the scratch; tied rows of both are searched again."""
+    """1 500 000 points in five coordinates take two rounds of the scratch; tied rows of both are searched again."""
     km = importlib.import_module("fastgraphcompute_b200.extensions.binned_select_knn")
     g = torch.Generator().manual_seed(4)
-    n, K = 800000, 7
+    n, K = 1500000, 7
     x = torch.rand((n, 5), generator=g)
     x[: n // 40] = torch.randint(0, 9, (n // 40, 5), generator=g) * 0.25 + 3.0          # lattices, away from the rest
     x[n - n // 80:] = torch.randint(0, 7, (n // 80, 5), generator=g) * 0.25 - 3.0
