@@ -91,19 +91,11 @@ __device__ __forceinline__ float box_sq(const float4 (&q)[NV], const float4 *__r
 // key never exceeds the distance).
 __device__ __forceinline__ uint32_t box_key(float d, int lane) { return (__float_as_uint(d) & ~31u) | (uint32_t)lane; }
 
-// Whether a box at distance d has to be visited: within the bound tau, and at exactly it only until a candidate there has been
-// left out.  Afterwards others change nothing, and where many points are equal they would be all that is visited (half of 100 k
-// in three coordinates, K = 64, listed by the search by groups: 10.3 -> 0.38 ms, grid 13.7).
-__device__ __forceinline__ bool box_wanted(uint32_t d, uint32_t tau, uint32_t left_out)
-{
-    return d < tau || (d == tau && left_out != tau);
-}
-
-// The nearest of the 32 boxes that have not been taken yet, or -1 when none is wanted.
-__device__ __forceinline__ int next_box(uint32_t &key, uint32_t tau, uint32_t left_out, int lane)
+// The nearest of the 32 boxes that have not been taken yet, or -1 when none is nearer than `beyond`.
+__device__ __forceinline__ int next_box(uint32_t &key, uint32_t beyond, int lane)
 {
     const uint32_t m = __reduce_min_sync(FGC_FULL_MASK, key);
-    if (!box_wanted(m & ~31u, tau, left_out)) return -1;
+    if ((m & ~31u) >= beyond) return -1;
     const int src = (int)(m & 31u);
     if (lane == src) key = kNoBox;
     return src;
@@ -117,8 +109,11 @@ struct BisectSelect {
     static constexpr int CAP = R <= 2 ? 32 * (R + 3) : 64 * R;
     // a leaf is appended as a whole: what may be there before it, plus 32, has to fit
     static_assert(32 * R + kFirstExtra + 31 <= CAP, "array too short for the first bound");
-    uint32_t tau;              // nothing at or above this distance is wanted
     uint32_t left_out;         // the last distance at which a candidate was left out that equals the bound
+    // Points and boxes nearer than this are wanted: everything up to the bound, and once a candidate at the bound has been left
+    // out only what is nearer.  Others at it change nothing then, and where many points are equal they would be all that
+    // is visited (half of 100 k in three coordinates, K = 64, listed by the search by groups: 10.3 -> 0.34 ms, grid 13.7).
+    uint32_t beyond;
     int n;
     // At least kn of the smallest entries stay, at most kn + spare.
     __device__ __forceinline__ void select(float *bd, int *bj, int lane, int kn, int spare)
@@ -155,6 +150,7 @@ struct BisectSelect {
             equal = kn - __reduce_add_sync(FGC_FULL_MASK, below);
             left_out = hi;
         }
+        beyond = hi + (equal < CAP ? 0u : 1u);
         int to = 0;
         __syncwarp();
 #pragma unroll
@@ -174,7 +170,6 @@ struct BisectSelect {
             to += __popc(m);
         }
         n = to;
-        tau = hi;
         __syncwarp();
     }
     __device__ __forceinline__ void add(float *bd, int *bj, int lane, unsigned m, float d, int j)
@@ -243,7 +238,7 @@ __device__ __forceinline__ void tree_query(const TreeArgs &a, int qi)
     int *lleaf = s_leaf[w];
     uint32_t *lkey = s_key[w];
     Select sel;
-    sel.tau = kInfBits;
+    sel.beyond = kInfBits;
     sel.left_out = kNoBox;
     sel.n = 0;
     if (kn > 0 && !(sflag && (sflag[qi] == 0 || sflag[qi] == 2))) {
@@ -267,8 +262,7 @@ __device__ __forceinline__ void tree_query(const TreeArgs &a, int qi)
                 dc = dist_sq<NV>(q, c, 0);
                 if (sflag) { const uint8_t f = sflag[j]; if (f == 1 || f == 2) dc = __uint_as_float(kInfBits); }
             }
-            const unsigned m = __ballot_sync(FGC_FULL_MASK, __float_as_uint(dc) < sel.tau);
-            if (__any_sync(FGC_FULL_MASK, __float_as_uint(dc) == sel.tau)) sel.left_out = sel.tau;
+            const unsigned m = __ballot_sync(FGC_FULL_MASK, __float_as_uint(dc) < sel.beyond);
             if (m) sel.add(bd, bj, lane, m, dc, j);
         };
         // First bound: the nearest leaves of the query's own node, until there are kFirstExtra
@@ -279,7 +273,7 @@ __device__ __forceinline__ void tree_query(const TreeArgs &a, int qi)
             uint32_t key0 = kNoBox;
             const int mine = own * 32 + lane;
             if (mine < n_leaf) key0 = box_key(box_sq<NV>(q, leaf_box + (size_t)mine * (2 * NV)), lane);
-            for (int c0; sel.n < kn + kFirstExtra && (c0 = next_box(key0, kInfBits, kNoBox, lane)) >= 0;) {
+            for (int c0; sel.n < kn + kFirstExtra && (c0 = next_box(key0, kInfBits, lane)) >= 0;) {
                 seen |= 1u << c0;
                 visit(own * 32 + c0);
             }
@@ -298,7 +292,7 @@ __device__ __forceinline__ void tree_query(const TreeArgs &a, int qi)
             }
             for (int i = 0; i < n_list; i++) {
                 const uint32_t k = __shfl_sync(FGC_FULL_MASK, i < 32 ? k0 : k1, i & 31);
-                if (!box_wanted(k & ~63u, sel.tau, sel.left_out)) break;
+                if ((k & ~63u) >= sel.beyond) break;
                 visit(lleaf[k & 63u]);
                 if (sel.n > Select::CAP - 32 || sel.n > kn + kMoreExtra) sel.select(bd, bj, lane, kn, kSpare);
             }
@@ -312,17 +306,17 @@ __device__ __forceinline__ void tree_query(const TreeArgs &a, int qi)
             uint32_t key2 = kNoBox;
             const int mine2 = group * 32 + lane;
             if (mine2 < n_top) key2 = n_top == 1 ? (uint32_t)lane : box_key(box_sq<NV>(q, top_box + (size_t)mine2 * (2 * NV)), lane);
-            for (int c2; (c2 = next_box(key2, sel.tau, sel.left_out, lane)) >= 0;) {
+            for (int c2; (c2 = next_box(key2, sel.beyond, lane)) >= 0;) {
                 const int mine1 = (group * 32 + c2) * 32 + lane;
                 uint32_t key1 = kNoBox;
                 if (mine1 < n_node) key1 = n_node == 1 ? (uint32_t)lane : box_key(box_sq<NV>(q, node_box + (size_t)mine1 * (2 * NV)), lane);
-                for (int c1; (c1 = next_box(key1, sel.tau, sel.left_out, lane)) >= 0;) {
+                for (int c1; (c1 = next_box(key1, sel.beyond, lane)) >= 0;) {
                     const int node = (group * 32 + c2) * 32 + c1;
                     const int leaf = node * 32 + lane;
                     uint32_t d0 = kNoBox;
                     if (leaf < n_leaf && !(node == own && (seen >> lane & 1)))
                         d0 = __float_as_uint(box_sq<NV>(q, leaf_box + (size_t)leaf * (2 * NV)));
-                    const bool want = d0 != kNoBox && box_wanted(d0, sel.tau, sel.left_out);
+                    const bool want = d0 < sel.beyond;
                     const unsigned m = __ballot_sync(FGC_FULL_MASK, want);
                     if (want) {
                         const int at = n_list + __popc(m & lanemask_lt());
