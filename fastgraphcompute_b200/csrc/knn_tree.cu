@@ -399,7 +399,8 @@ static int64_t least_row_split(int64_t n_vert, int K)
 }
 
 // Where the tree is the better search.  Neither search is ahead for all data: the figures are the time of the tree over that of
-// the grid, whole forward, B200, for uniform points in a cube / normal ones / 50 clusters of width 0.02 ("mixture").
+// the grid, whole forward, B200, for uniform points in a cube / normal ones / 50 clusters of width 0.02 ("mixture"); up to five
+// coordinates they are of the search one query at a time (the forward's search by groups takes 0.6 to 0.9 of its time).
 // Below 16384 points the sort's launches outweigh the search (10 k in three coordinates, K = 100: 0.110 / 0.112 ms); in up to
 // five coordinates, where the forward searches by groups, so they do for tiny row splits (least_row_split).
 //

@@ -18,13 +18,14 @@
 // the result is exactly the K-1 smallest computed distances, whatever the tree.  Boxes and points at exactly the bound
 // are taken until a candidate equal to it has been left out, so that one that equals the K-th distance is always noticed.
 //
-// What bounds them (a million uniform points in three coordinates, K = 64, ncu): k_tree_rows issue slots (0.80 of them used, 1510
-// warp instructions a query, arithmetic pipe 0.71), k_tree_groups the shared-memory pipe (0.93; the counting's atomics meet in banks; 185
-// instructions a query).  Whole forward against the search one query at a time / the grid, ms: 6.4 M uniform points in three
-// coordinates, K = 64 13.9 against 21.9 / 18.3; 1.6 M learned ones in four, K = 40 6.9 against 9.6 / 8.4; 800 k skewed in three, K = 128
-// 3.2 against 4.7 / 18.9; a million normal ones in five, K = 40 15.6 against 18.2 / 26.3.
+// What bounds them (a million uniform points in ten row splits, three coordinates, K = 64, ncu): k_tree_rows issue slots (0.79 of them
+// used, 1490 warp instructions a query, arithmetic pipe 0.70; 46 registers, 57 % of the warps resident), k_tree_groups the shared-memory
+// pipe (0.93; the counting's atomics meet in banks; 190 instructions a query; 72 registers and 60 bytes of them spilled, 28 one-warp CTAs
+// an SM).  Whole forward / one query at a time / the grid, ms, without a second look in the first two: 6.4 M uniform points in three
+// coordinates, K = 64 13.5 / 21.5 / 18.3; 1.6 M learned ones in four, K = 40 6.6 / 9.4 / 8.4; 800 k skewed in three, K = 128 3.0 / 4.6 / 18.8; a
+// million normal ones in five, K = 40 15.0 / 18.2 / 26.4.  The second look adds 0.85, 0.4, 1.5 and 0.4.
 //
-// Other splits of the work, measured on the first and the third of these: one kernel, a lane per query, the points of a leaf read from
+// Other splits of the work, measured on the first and the third of these (then 13.9 and 3.2): one kernel, a lane per query, the points of a leaf read from
 // shared memory by all 32 lanes (15.5; broadcast 16-byte loads write 512 bytes back each, four cycles an SM); candidates of all
 // 32 queries filtered by the matrix product and kept in the workspace, a second kernel for the rows (15.7 and 7.8: leaves that
 // visit thousands of others run on alone).
@@ -650,8 +651,8 @@ k_tree_rows(const TreeArgs a)
         }
     } else {
         // In five coordinates the boxes of a list are 64 KB, which every warp would read for itself: the eight of a CTA read them
-        // once, and leave those near enough to some of their queries in shared memory (a million normal points, K = 40: 18.4 ->
-        // 15.6 ms).  With up to four, where a list is one or two steps long, waiting for one another costs more
+        // once, and leave those near enough to some of their queries in shared memory (a million normal points, K = 40, lists of up to
+        // 3072: 18.4 -> 15.6 ms).  With up to four, where a list is one or two steps long, waiting for one another costs more
         // than it saves (6.4 M uniform points in three, K = 64: 13.9 -> 15.2 ms).
         constexpr int NC = kGroupDims;
         __shared__ float s_box[2 * NC][kRowWarps * 32];

@@ -11,16 +11,17 @@
 //
 // The distance of a box is computed with the operations of dist_sq in the same order.  Rounding is
 // monotone, so it never exceeds the computed distance of a point inside: pruning needs no margin and
-// the result is exactly the K-1 smallest computed distances, whatever the tree.  Boxes at exactly the bound
-// are visited until a candidate there has been left out, so that one that equals the K-th distance is always noticed.
+// the result is exactly the K-1 smallest computed distances, whatever the tree.  Boxes and points at exactly the
+// bound are taken until a candidate there has been left out, so that one that equals the K-th distance is always noticed.
+//
+// In up to five coordinates the forward takes it only for what the search by groups (knn_tree_group.cu) leaves, and in workspaces
+// without its scratch; from six on, and in fgc_knn_search_tree, for every query.
 //
 // What bounds it: issue slots (0.88 of them used; compares, minima and logic run at half rate).  A
-// query of 500 k uniform points in three coordinates with K = 64 takes 3390 warp instructions, the 500 k of them 1.69 ms; one of
-// 200 k normal points in five with K = 40 takes 11 600, at 0.63 of the issue slots (the last warps run on alone).  Against
-// the grid search (build and search, B200; the second look at tied rows, which knn_forward.cu adds, takes 0.02 ms at 20 k
-// points, with a few such rows 0.8 at 800 k): 800 k points in skewed clusters, K = 128: 16.4 -> 4.3 ms; 400 k uniform, K = 128: 2.82 ->
-// 2.20; 500 k normal in five coordinates, K = 40: 9.84 -> 8.8; 60 k uniform in eight, K = 20: 3.40 -> 1.5;
-// but 1.6 M uniform in three, K = 64: 4.6 -> 5.3, so the grid stays for few coordinates and short lists.
+// query of 500 k uniform points in three coordinates with K = 64 takes 3350 warp instructions, the 500 k of them 1.67 ms; one of
+// 200 k normal points in five with K = 40 takes 11 500, at 0.61 of the issue slots (the last warps run on alone).  Against
+// the grid (whole forward without the second look at tied rows): a million normal points in five coordinates, K = 40 26.4 ->
+// 18.2 ms; 60 k uniform in eight, K = 20: 3.40 -> 1.5; 400 k normal in six, K = 24 0.78 of its time; 6.4 M uniform in three, K = 64: 18.3 -> 21.5.
 //
 // Other forms measured: candidates merged into a sorted list 32 at a time instead of selected by
 // bisection (28.8 against 22.3 ms, 6.4 M uniform points, K = 64); one query per lane with a column of

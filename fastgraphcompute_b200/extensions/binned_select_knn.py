@@ -48,7 +48,7 @@ def _raise_for_status(status):
 # Needs check_status (that is where the choice comes back to the host).
 grid_dims = 0
 grid_probe_every = 64
-# Search on a tree of boxes instead of a grid: None lets the library choose (fgc_knn_tree_preferred).
+# Search on a tree of boxes instead of a grid: None lets the library choose (fgc_knn_tree_preferred, fgc_knn_groups_preferred).
 search_tree = None
 pad_min_pairs = 1 << 19    # backward for D = 3, 5, 6, 7: pad to four / eight coordinates from this many (row, slot) pairs on
 _grid_memory = {}        # (device, N, row splits, K[, "direction"]) -> [form, calls since the last automatic choice]
@@ -275,7 +275,8 @@ def binned_select_knn_with_order(K: int, coords: torch.Tensor, row_splits: torch
     processing order for cache locality.  long_tails: the points are expected to have sparse tails (learned
     coordinates); the choice of the search takes it into account.  The distances do not depend on it, but which of
     several points at exactly the K-th distance is kept may: with long_tails the tree's own choice stands, without it
-    the grid's (while a sixteenth of the rows or fewer have one).  A traced or compiled call has no such hint.
+    the grid's (while a sixteenth of the rows or fewer have one).  A traced or compiled call has no such hint.  Whether
+    coords requires gradients changes nothing in idx and distsq.
 
     Written in the TorchScript subset (the reference's wrapper is ``@torch.jit.script``,
     extensions/binned_select_knn.py:11): modules that call it can be scripted, traced, saved and
@@ -336,7 +337,7 @@ def binned_select_knn(K: int, coords: torch.Tensor, row_splits: torch.Tensor,
     Returns:
         (indices int64 [N,K], squared distances float32 [N,K]).  Slot 0 is the point
         itself; the order of the other slots is unspecified, as in the reference (it is
-        the same on every run, though).  Differentiable w.r.t. coords through the distances.
+        the same on every run, though, with and without gradients).  Differentiable w.r.t. coords through the distances.
     """
     if not torch.jit.is_scripting():
         # conveniences outside TorchScript: python numbers / lists where the reference takes tensors

@@ -207,16 +207,16 @@ int fgc_knn_search(int64_t n_vert, int32_t n_coords, int64_t n_rs, int32_t K,
  * of one workspace may overlap in time).  fgc_knn_cell_order gives the curve order.
  * FGC_ERR_TOO_LARGE when the tree does not fit into the workspace (far more row splits than points, or
  * more than about 70 million points).
- * fgc_knn_tree_preferred: 1 where the tree fits and was measured to be the faster search (long lists in three
+ * fgc_knn_tree_preferred: 1 where the tree fits and was measured to be the faster search of fgc_knn_forward (long lists in three
  * coordinates, five and more coordinates; with long_tails != 0 -- the points are expected to have sparse tails, as learned
  * coordinates do -- also four coordinates).  For searches without direction flags: with them the grid holds candidates
  * only and is the faster one.  No counterparts in the reference.
  */
 int fgc_knn_tree_preferred(int64_t n_vert, int32_t n_coords, int64_t n_rs, int32_t K, int32_t long_tails);
 /*
- * 1 where fgc_knn_forward with FGC_FORWARD_TREE was measured to be ahead of the grid although
- * fgc_knn_tree_preferred, which stands for fgc_knn_search_tree, is 0: in up to five coordinates it takes all
- * queries of a leaf at once.
+ * 1 where fgc_knn_forward with FGC_FORWARD_TREE and the workspace of fgc_knn_forward_workspace_bytes was measured to be ahead
+ * of the grid although fgc_knn_tree_preferred is 0: in three to five coordinates, where it takes all queries of a leaf at
+ * once (fgc_knn_search_tree, and a smaller workspace, do not).
  */
 int fgc_knn_groups_preferred(int64_t n_vert, int32_t n_coords, int64_t n_rs, int32_t K, int32_t long_tails);
 int fgc_knn_build_tree(const float *coords, int64_t n_vert, int32_t n_coords, const int64_t *row_splits, int64_t n_rs,
