@@ -125,7 +125,8 @@ static int knn_forward_launch(const float *coords, int64_t n_vert, int32_t n_coo
         // Which of several points at exactly the K-th distance is kept is open, but for coordinates without order it should
         // not hang on the choice of the search: the few such rows are searched again on a grid.  On a lattice, where
         // nearly every row has such a choice, that would be the whole search twice: beyond a sixteenth of the rows the
-        // tree's choice stands.  With FGC_FORWARD_GRID_ORDER rows with equal distances inside the list are among them.
+        // tree's choice stands.  With FGC_FORWARD_GRID_ORDER rows with equal distances inside the list are among them, or left out where they make
+        // the rows too many (4 % of the points twice, K = 65: three rows in four).
         rc = knn_build_grid_for_ties(coords, n_vert, n_coords, row_splits, n_rs, K, direction, target_occupancy, ws, ws_bytes,
                                      stream);
         if (rc != FGC_OK) return rc;

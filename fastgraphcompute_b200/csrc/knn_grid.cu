@@ -53,14 +53,17 @@ k_tie_gate(KnnGrid *__restrict__ g, const KnnTree *__restrict__ t, int limit)
 {
     chain_wait();
     chain_release();
-    const int status = g->status, tied = t->n_tied;
+    const int status = g->status;
+    const long long tied = t->n_tied, both = tied + t->n_equal;
     __syncthreads();
     if (status != 0) return;
-    if (tied == 0 || tied > limit) {
+    if (both == 0 || tied > limit || (tied == 0 && both > limit)) {
         if (threadIdx.x == 0) g->status = kStatusNoGrid;
         return;
     }
     for (int i = threadIdx.x; i < (int)((kGridHeaderBytes + kHardTicketBytes) / sizeof(int)); i += 256) ((int *)g)[i] = 0;
+    __syncthreads();
+    if (threadIdx.x == 0) g->leave_equal = both > limit;
 }
 
 // Fused finite check + min/max of the binned coordinates; clears the cell table (all of its

@@ -50,7 +50,10 @@ struct KnnGrid {
     // optional debug counters (filled when a search is launched with count_evals):
     // [0] distance evaluations, [1] 32-candidate steps, [2] list insertions,
     // [3] 32-item metadata batches, [4] shells, [5] queries that scanned their whole row split
-    unsigned long long counters[6];
+    union {
+        unsigned long long counters[6];
+        int32_t leave_equal;   // in a second look behind a search on a tree, which counts nothing: rows marked kEqualRow stay
+    };
     // division of a cell id by B, n1*n2*n3, n2*n3 and n3 as multiply + shift (grid_set_divisors)
     uint32_t div_m[4];
     uint32_t div_s[4];

@@ -630,7 +630,7 @@ k_knn(const KnnArgs a)
     else knn_query<NV, R, COUNT, false>(a, qi);
 }
 
-// The rows that the tree search has marked kTieRow.  A warp looks at 32 rows at once, one per lane and far
+// The rows that the tree search has marked kTieRow or, unless they are too many, kEqualRow.  A warp looks at 32 rows at once, one per lane and far
 // apart (marked rows come in clusters), and searches the marked ones.  Without a grid the marks are taken off and the
 // tree's choice stands.
 template <int NV, int R, int MODE>
@@ -641,8 +641,9 @@ k_knn_marked(const KnnArgs a)
     chain_release();
     const int lane = threadIdx.x & 31;
     const int n_groups = (int)(((long long)a.n_vert + 31) / 32);
-    const bool search = a.grid->status == 0;
-    if (!search && ((const KnnTree *)a.hard_tickets)->n_tied == 0) return;
+    const bool search = a.grid->status == 0, leave_equal = a.grid->leave_equal != 0;
+    const KnnTree *tree = (const KnnTree *)a.hard_tickets;
+    if (!search && tree->n_tied == 0 && tree->n_equal == 0) return;
     for (int i = blockIdx.x * kKnnWarps + (threadIdx.x >> 5); i < n_groups; i += gridDim.x * kKnnWarps) {
         const long long mine = i + (long long)lane * n_groups;
         int64_t *row = nullptr;
@@ -651,12 +652,11 @@ k_knn_marked(const KnnArgs a)
             id = search ? __ldg(a.sorig + mine) : (int)mine;
             row = a.out_idx + (size_t)id * a.K;
         }
-        const bool marked = row && *row == kTieRow;
-        if (!search) {
-            if (marked) *row = id;
-            continue;
-        }
-        unsigned m = __ballot_sync(FGC_FULL_MASK, marked);
+        const int64_t mark = row ? *row : 0;
+        const bool equal = mark == kEqualRow, marked = mark == kTieRow || equal;
+        if (marked && (!search || (equal && leave_equal))) *row = id;
+        if (!search) continue;
+        unsigned m = __ballot_sync(FGC_FULL_MASK, marked && !(equal && leave_equal));
         while (m) {
             const int qi = i + (__ffs(m) - 1) * n_groups;
             m &= m - 1;

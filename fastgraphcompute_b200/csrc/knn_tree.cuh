@@ -32,11 +32,12 @@ struct KnnTree {
     float origin[kTreeKeyDims];
     float scale;                        // cells of the Hilbert curve per unit length
     int32_t n_tied;                     // rows marked kTieRow by the search
+    int32_t n_equal;                    // rows marked kEqualRow
     int32_t n_listed;                   // queries that the search by groups leaves to the search one by one
     int32_t next_listed;                // of those, taken so far
 };
 static_assert(sizeof(KnnTree) <= kHardTicketBytes, "tree record too large");
-static_assert(offsetof(KnnTree, n_listed) == 96, "read there by tests/test_gpu_tree_groups.py");
+static_assert(offsetof(KnnTree, n_listed) == 100, "read there by tests/test_gpu_tree_groups.py");
 
 constexpr int kRadixBits = 11;
 constexpr int kRadixBins = 1 << kRadixBits;
@@ -129,12 +130,13 @@ inline bool tree_scratch(const KnnWorkspace &w, int n_coords, char *ws, size_t b
     return true;
 }
 
-// Mark in slot 0 of a row that is to be searched again on a grid.
-constexpr int64_t kTieRow = INT64_MIN;
-// Which rows are: none; those whose K-th distance several points share, of which some are left out; with sorted lists (K <= 65)
-// also those that hold equal distances, whose order would be another one.
+// Marks in slot 0 of a row that is to be searched again on a grid: several points share its K-th distance and some are left out;
+// or only its order would be another one, since it holds equal distances.
+constexpr int64_t kTieRow = INT64_MIN, kEqualRow = INT64_MIN + 1;
+// Which rows are marked: none; kTieRow only; both, with sorted lists (K <= 65).
 enum class TieMarks : int { kNone, kKth, kAny };
-// Rows that may be marked and searched again, as a share of all rows: see knn_forward_launch.
+// Rows that may be marked and searched again, as a share of all rows (if both kinds together are more, those marked kTieRow): see
+// knn_forward_launch.
 constexpr int kTieShare = 16;
 // Status word between the tree search and the end of the second look when there is nothing to search again:
 // the kernels of the grid return at once.
@@ -150,7 +152,7 @@ int knn_search_tree_groups(int64_t n_vert, int32_t n_coords, const int64_t *row_
                            int32_t has_direction, int32_t tf_compat, TieMarks mark_ties, int64_t *out_idx, float *out_distsq,
                            void *workspace, size_t workspace_bytes, fgc_stream_t stream);
 // fgc_knn_build_grid_dims behind a search with mark_ties: builds nothing (kStatusNoGrid) where no row is marked,
-// or more than a kTieShare-th of them are.
+// or more than a kTieShare-th of them are (see k_tie_gate).
 int knn_build_grid_for_ties(const float *coords, int64_t n_vert, int32_t n_coords, const int64_t *row_splits, int64_t n_rs,
                             int32_t K, const int64_t *direction_or_null, float target_occupancy, void *workspace,
                             size_t workspace_bytes, fgc_stream_t stream);

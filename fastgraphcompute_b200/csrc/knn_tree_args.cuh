@@ -49,6 +49,14 @@ __device__ __forceinline__ bool equal_in_list(const float (&d)[R], const int (&i
     return __any_sync(FGC_FULL_MASK, same);
 }
 
+// Slot 0 of a row: the point itself, or the mark.  tie: a choice at the K-th distance; same: equal distances in the list.
+__device__ __forceinline__ int64_t mark_row(const TreeArgs &a, bool tie, bool same, int orig_q)
+{
+    if (a.mark_ties == TieMarks::kNone || !(tie || same)) return orig_q;
+    atomicAdd(tie ? &a.tree->n_tied : &a.tree->n_equal, 1);
+    return tie ? kTieRow : kEqualRow;
+}
+
 // Checks of the arguments of a search, and what every kernel needs of them.
 int tree_args(int64_t n_vert, int32_t n_coords, const int64_t *row_splits, int64_t n_rs, int32_t K, int32_t has_direction,
               int32_t tf_compat, TieMarks mark_ties, int64_t *out_idx, float *out_distsq, void *workspace, size_t workspace_bytes,

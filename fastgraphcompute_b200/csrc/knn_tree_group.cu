@@ -833,11 +833,9 @@ k_tree_rows(const TreeArgs a)
         }
         kth = __reduce_max_sync(FGC_FULL_MASK, kth);
     }
-    const bool marked = a.mark_ties != TieMarks::kNone && (same || (full && (tie || kth == left_out)));
     if (lane == 0) {
-        row_i[0] = marked ? kTieRow : (int64_t)orig_q;
+        row_i[0] = mark_row(a, full && (tie || kth == left_out), same, orig_q);
         row_d[0] = 0.f;
-        if (marked) atomicAdd(&a.tree->n_tied, 1);
     }
 }
 

@@ -377,11 +377,9 @@ __device__ __forceinline__ void tree_query(const TreeArgs &a, int qi)
         if (sel.n < kn) last = 0;
     }
     tie = tie || (kn > 0 && sel.n >= kn && last == sel.left_out);
-    const bool marked = a.mark_ties != TieMarks::kNone && (tie || same);
     if (lane == 0) {
-        out_i[0] = marked ? kTieRow : (int64_t)orig_q;
+        out_i[0] = mark_row(a, tie, same, orig_q);
         out_d[0] = 0.f;
-        if (marked) atomicAdd(&a.tree->n_tied, 1);
     }
 }
 

@@ -239,7 +239,8 @@ int fgc_knn_search_tree(int64_t n_vert, int32_t n_coords, const int64_t *row_spl
 #define FGC_FORWARD_GRID_TIES 128 /* with it: rows with a choice among equal K-th distances are searched again on a grid,
                                     unless more than a sixteenth of all rows are such (lattice coordinates) */
 #define FGC_FORWARD_GRID_ORDER 256 /* with both: K <= 65: so are rows that hold equal distances, whose slots the grid may
-                                     give in another order */
+                                     give in another order; if both kinds are more than a sixteenth, only
+                                     those of FGC_FORWARD_GRID_TIES are */
 /*
  * Workspace with which fgc_knn_forward is fastest: with FGC_FORWARD_TREE and up to five coordinates up to 256 MB more than
  * fgc_knn_workspace_bytes, for the search of all queries of a leaf at once.  With fgc_knn_workspace_bytes it takes one

@@ -28,7 +28,7 @@ def _points(kind, n, D, g):
 
 def _listed(ws):
     """Queries that were searched one by one (KnnTree::n_listed, behind the grid's header)."""
-    return int(ws[256:].view(torch.int32)[24])
+    return int(ws[256:].view(torch.int32)[25])
 
 
 def _without_scratch(km, monkeypatch):
@@ -376,6 +376,36 @@ def test_equal_distances_take_the_grids_slots(D, K, scratch, monkeypatch):
     assert [f & 448 for f in seen] == [448, 64]
     assert torch.equal(groups[0], grid[0]) and torch.equal(groups[1], grid[1]) and torch.equal(alone[1], grid[1])
     assert 0 < int((alone[0] != grid[0]).any(dim=1).sum()) <= n // 16
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("pairs,same_slots", [(0.0005, True), (0.04, False), (1.0, False)])
+@pytest.mark.parametrize("scratch", [True, False])
+def test_pairs_of_equal_points(pairs, same_slots, scratch, monkeypatch):
+    """Points that occur twice: with a few the slots are the grid's; with 4 % of them three rows in four hold equal distances and only
+    those with a choice at the K-th place are searched again, so that the sets are the grid's; with all of them the tree's choice
+    stands.  No mark stays in a row."""
+    km = importlib.import_module("fastgraphcompute_b200.extensions.binned_select_knn")
+    g = torch.Generator().manual_seed(9)
+    n, D, K = 20000, 3, 65
+    x = torch.rand((n, D), generator=g)
+    m = int(n * pairs / 2)
+    x[:m] = x[m:2 * m]
+    x = x[torch.randperm(n, generator=g)].to(DEV)
+    rs = torch.cat([torch.arange(0, n, 4000), torch.tensor([n])]).to(DEV)
+    grid = km._forward(x, rs, K, None, False, False, None, False)
+    if not scratch:
+        _without_scratch(km, monkeypatch)
+    monkeypatch.setattr(km._cabi.lib, "fgc_knn_groups_preferred", lambda *args: 1)
+    groups = km._forward(x, rs, K, None, False, False, None, False)
+    assert torch.equal(groups[0][:, 0], torch.arange(n, device=DEV)) and int(groups[0].min()) >= 0
+    assert torch.equal(groups[1].sort(dim=1).values, grid[1].sort(dim=1).values)
+    sets = torch.equal(groups[0].sort(dim=1).values, grid[0].sort(dim=1).values)
+    assert sets == (pairs < 1.0)
+    if same_slots:
+        assert torch.equal(groups[0], grid[0])
+    elif pairs < 1.0:
+        assert not torch.equal(groups[0], grid[0])
 
 
 @pytest.mark.gpu
