@@ -106,8 +106,11 @@ static int knn_forward_launch(const float *coords, int64_t n_vert, int32_t n_coo
         FGC_RETURN_IF_CUDA(cudaEventRecord(status->ready, (cudaStream_t)stream));
     }
     // all queries of a leaf at once, in workspaces with room for its scratch
-    const bool groups = tree && n_vert > 0 && n_coords <= kGroupDims &&
-                        ws_bytes >= knn_workspace_layout(n_vert, n_coords, n_rs, K).total + tree_extra_bytes(n_vert, n_coords, n_rs);
+    bool groups = false;
+    if (tree && n_vert > 0 && n_coords <= kGroupDims) {
+        const KnnWorkspace L = knn_workspace_layout(n_vert, n_coords, n_rs, K);
+        groups = ws_bytes >= L.total + tree_extra_bytes(n_vert, n_coords, n_rs) && tree_layout(L, n_vert, n_coords, n_rs).groups;
+    }
     const bool ties = tree && (flags & FGC_FORWARD_GRID_TIES) != 0;
     const TieMarks marks = !ties ? TieMarks::kNone : (flags & FGC_FORWARD_GRID_ORDER ? TieMarks::kAny : TieMarks::kKth);
     if (groups) rc = knn_search_tree_groups(n_vert, n_coords, row_splits, n_rs, K, direction != nullptr, tf_compat, marks, out_idx,

@@ -254,7 +254,7 @@ __global__ void __launch_bounds__(256)
 k_tree_leaves(const float *__restrict__ coords, int n_vert, int n_coords, const int64_t *__restrict__ direction,
               const int64_t *__restrict__ row_splits, int n_rs, KnnGrid *__restrict__ g, const int *__restrict__ ids,
               int *__restrict__ sorig, float4 *__restrict__ scoords, uint8_t *__restrict__ sflag,
-              float4 *__restrict__ leaf_box, float4 *__restrict__ node_box)
+              float4 *__restrict__ leaf_box, float4 *__restrict__ node_box, float4 *__restrict__ half_box)
 {
     chain_wait();
     chain_release();
@@ -288,14 +288,30 @@ k_tree_leaves(const float *__restrict__ coords, int n_vert, int n_coords, const 
             }
         }
         float lo[4 * NV], hi[4 * NV];
+        float half_lo[4 * NV], half_hi[4 * NV];                // of the lane's half
 #pragma unroll
         for (int c = 0; c < 4 * NV; c++) {
             const uint32_t k = float_to_ordered(x[c]);
-            const uint32_t a = __reduce_min_sync(FGC_FULL_MASK, act ? k : 0xffffffffu);
-            const uint32_t b = __reduce_max_sync(FGC_FULL_MASK, act ? k : 0u);
+            const bool low = lane < 16;
+            const uint32_t a0 = __reduce_min_sync(FGC_FULL_MASK, act && low ? k : 0xffffffffu);
+            const uint32_t b0 = __reduce_max_sync(FGC_FULL_MASK, act && low ? k : 0u);
+            const uint32_t a1 = __reduce_min_sync(FGC_FULL_MASK, act && !low ? k : 0xffffffffu);
+            const uint32_t b1 = __reduce_max_sync(FGC_FULL_MASK, act && !low ? k : 0u);
+            const uint32_t a = min(a0, a1), b = max(b0, b1);
             lo[c] = ordered_to_float(a);
             hi[c] = ordered_to_float(b);
+            // (a half without points is infinitely far from everything)
+            half_lo[c] = low ? ordered_to_float(a0) : (a1 <= b1 ? ordered_to_float(a1) : __uint_as_float(0x7f800000u));
+            half_hi[c] = low ? ordered_to_float(b0) : (a1 <= b1 ? ordered_to_float(b1) : __uint_as_float(0xff800000u));
             if (lane == 0) { atomicMin(&s_lo[c], a); atomicMax(&s_hi[c], b); }
+        }
+        if (NV == 2 && half_box && (lane & 15) == 0) {
+            float4 *out = half_box + (size_t)((leaf0 + l) * 2 + (lane >> 4)) * 2 * NV;
+#pragma unroll
+            for (int v = 0; v < NV; v++) {
+                out[v] = make_float4(half_lo[4 * v], half_lo[4 * v + 1], half_lo[4 * v + 2], half_lo[4 * v + 3]);
+                out[NV + v] = make_float4(half_hi[4 * v], half_hi[4 * v + 1], half_hi[4 * v + 2], half_hi[4 * v + 3]);
+            }
         }
         if (lane == 0) {
             float4 *out = leaf_box + (size_t)(leaf0 + l) * 2 * NV;
@@ -381,7 +397,7 @@ static cudaError_t launch_boxes(const float *coords, int n, int n_coords, const 
     FGC_TRY(launch_chained(k_tree_leaves<NV>, (unsigned)T.n_box[1], 256, 0, s, coords, n, n_coords, direction,
                            row_splits, n_rs, g, (const int *)(ws + T.ids[T.passes & 1]), (int *)(ws + L.sorig),
                            (float4 *)(ws + L.scoords), (uint8_t *)(ws + L.sflag), (float4 *)(ws + T.box[0]),
-                           (float4 *)(ws + T.box[1])));
+                           (float4 *)(ws + T.box[1]), n_coords == kHalfDims && T.groups ? (float4 *)(ws + T.half_box) : nullptr));
     if (n <= 32768) return cudaSuccess;                  // no row split has more than one top node: never read
     return launch_chained(k_tree_top<NV>, (unsigned)((T.n_box[2] + 7) / 8), 256, 0, s, row_splits, n_rs, g,
                           (const float4 *)(ws + T.box[1]), (float4 *)(ws + T.box[2]), T.n_box[2]);

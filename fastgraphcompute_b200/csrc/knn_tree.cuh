@@ -47,14 +47,19 @@ constexpr int kRadixBins = 1 << kRadixBits;
 // one unused box per row split.
 __host__ __device__ inline int64_t tree_base(int64_t ev_begin, int64_t e, int shift) { return (ev_begin >> shift) + e; }
 
+constexpr int kGroupDims = 5;          // searches by groups take up to so many coordinates,
+constexpr int kHalfDims = 5;           // and in so many they look at boxes of 16 points
+
 struct TreeLayout {
     size_t keys[2], ids[2], hist, hist_sums, box[3], end;
+    size_t listed, half_box, leaf_info;      // of the search by groups, in the place of the keys when they are sorted
     int64_t n_box[3];      // slots per level: leaves, nodes, top nodes
     int rounds;            // a CTA of a radix pass takes 256 * rounds keys
     int tiles;
     int key_dims, bits;    // Hilbert curve: dimensions and bits per dimension
     int passes;
     bool fits;
+    bool groups;           // room for half_box and leaf_info: row splits of thirty points or more, or few of them
 };
 
 inline TreeLayout tree_layout(const KnnWorkspace &w, int64_t n_vert, int n_coords, int64_t n_rs)
@@ -88,6 +93,10 @@ inline TreeLayout tree_layout(const KnnWorkspace &w, int64_t n_vert, int n_coord
     t.end = off;
     // the sections from the cell table up to the original ids are the tree's to use
     t.fits = t.end <= w.sorig && t.bits >= 1 && entries < ((size_t)1 << 31);
+    t.listed = t.keys[0];
+    t.half_box = align_up(t.listed + 4 * (size_t)n_vert, 256);
+    t.leaf_info = align_up(t.half_box + (n_coords == kHalfDims ? sizeof(float4) * 4 * w.nv * (size_t)t.n_box[0] : 0), 256);
+    t.groups = n_coords <= kGroupDims && t.leaf_info + (sizeof(int4) + 4 * sizeof(int2)) * (size_t)t.n_box[0] <= t.ids[0];
     return t;
 }
 
@@ -96,16 +105,18 @@ inline int tree_list_rows(int K) { return K <= 33 ? 1 : (K <= 65 ? 2 : (K <= 129
 
 // Scratch of a search by groups: what k_tree_groups leaves for the queries of `slots` leaf slots.
 struct TreeScratch {
-    int slots, list_cap;
+    int slots, list_cap, list_room;
     int *list, *list_n;
     float *bound;
 };
-constexpr int kGroupDims = 5;                                 // searches by groups take up to so many coordinates
 // Leaves that a leaf's queries may need (mean over uniform, normal and clustered points, K = 16 to 200: 36 to 110 in three
 // coordinates, 140 to 350 in four, 1000 in five); with more they are searched one by one.  A million normal points in five
 // coordinates, K = 40, with 768 / 1536 / 2304 / 3072 of them: 17.2 / 15.0 / 15.2 / 15.3 ms (77 / 16 / 7 / 4 % listed); 600 k uniform ones, K =
 // 200: 12.0 / 11.0 / 11.0 / 10.9.  A leaf of 32 points takes 2180 / 4228 / 6276 bytes in three / four / five.
-inline int tree_list_cap(int n_coords) { return n_coords <= 3 ? 512 : (n_coords == 4 ? 1024 : 1536); }
+__host__ __device__ constexpr int tree_list_cap(int n_coords) { return n_coords <= 3 ? 512 : (n_coords == 4 ? 1024 : 1536); }
+// The four lists of eight queries each that are made of it (knn_tree_group.cu) may take twice that in five coordinates (a million
+// normal points, K = 40: with as much as the one list 0.24 of all leaves have room for four).
+__host__ __device__ constexpr int tree_list_room(int n_coords) { return n_coords <= 4 ? 1 : 2; }
 // Larger searches take several rounds (6.4 M points in three coordinates 13.54 ms, with half of it 13.59; 3 M in five 43.4 and 43.6).
 constexpr size_t kTreeScratchBytes = (size_t)256 << 20;
 inline size_t tree_slot_bytes(int n_coords) { return 4 * ((size_t)tree_list_cap(n_coords) + 1 + 32); }
@@ -113,17 +124,19 @@ inline size_t tree_slot_bytes(int n_coords) { return 4 * ((size_t)tree_list_cap(
 inline size_t tree_extra_bytes(int64_t n_vert, int n_coords, int64_t n_rs)
 {
     if (n_coords > kGroupDims) return 0;
-    const size_t most = kTreeScratchBytes / tree_slot_bytes(n_coords), slots = (size_t)(n_vert / 32 + n_rs + 1);
+    const size_t most = kTreeScratchBytes / tree_slot_bytes(n_coords), slots = tree_list_room(n_coords) * (size_t)(n_vert / 32 + n_rs + 1);
     return (slots < most ? slots : most) * tree_slot_bytes(n_coords);
 }
 inline bool tree_scratch(const KnnWorkspace &w, int n_coords, char *ws, size_t bytes, TreeScratch *out)
 {
-    if (n_coords > kGroupDims || bytes < w.total + tree_slot_bytes(n_coords)) return false;
+    const int room = tree_list_room(n_coords);
+    if (n_coords > kGroupDims || bytes < w.total + room * tree_slot_bytes(n_coords)) return false;
     size_t slots = (bytes - w.total) / tree_slot_bytes(n_coords);
     const size_t most = kTreeScratchBytes / tree_slot_bytes(n_coords);
     if (slots > most) slots = most;
-    out->slots = (int)slots;
+    out->slots = (int)(slots / room);
     out->list_cap = tree_list_cap(n_coords);
+    out->list_room = room * out->list_cap;
     out->list = (int *)(ws + w.total);
     out->list_n = out->list + slots * out->list_cap;
     out->bound = (float *)(out->list_n + slots);

@@ -10,6 +10,7 @@ struct TreeArgs {
     const int *sorig;
     const uint8_t *sflag;      // nullptr: no direction restriction
     const float4 *box[3];      // leaves, nodes, top nodes
+    const float4 *half_box;    // halves of leaves (16 points)
     const int64_t *row_splits;
     KnnGrid *grid;
     KnnTree *tree;
@@ -22,9 +23,11 @@ struct TreeArgs {
     TieMarks mark_ties;        // which rows get kTieRow in slot 0
     // the search by groups only
     int slot0, n_slots;        // leaf slots of this launch: from the one up to the other
-    int list_cap;
+    int list_cap, list_room;
     int *listed;               // queries that are searched one by one instead (places in curve order)
-    int *list, *list_n;        // leaves [slots of this launch][list_cap] that a leaf's queries may need; their number (-1: no points)
+    int *list, *list_n;        // leaves [slots of this launch][list_room] that a leaf's queries may need; their number (-1: no points)
+    int4 *leaf_info;           // per leaf slot: first point of the leaf in its row split, begin and size of the row split
+    int2 *leaf_part;           // per eight queries of a leaf slot: begin and length of their part of the list
     float *bound;              // per query of this launch: at least K - 1 candidates are this near (kNoQuery, kListedQuery)
 };
 

@@ -8,8 +8,8 @@
 //                 distance.  |c|^2 - 2 c.q + |q|^2, with coordinates relative to the leaf, is a product of 32 queries x 32 points
 //                 over two more places than there are coordinates: a few matrix instructions in tf32, |c|^2 in two parts.
 //                 The bound is widened by what rounding can add, so it stays an upper bound.  Then the leaves whose box is
-//                 within the largest of the bounds are listed.
-//  k_tree_rows    One warp per query.  It compares its own bound with the boxes of the list, visits those within it, keeps
+//                 within the largest of the bounds are listed, and of those again, for every eight of the queries, the leaves within theirs.
+//  k_tree_rows    One warp per query.  It compares its own bound with the boxes of its list, visits those within it, keeps
 //                 the points within it -- distances by dist_sq, which is what is returned -- and sorts them (K <= 65)
 //                 or selects the K - 1 smallest.  On uniform data a quarter more points than K pass.
 //
@@ -18,14 +18,16 @@
 // the result is exactly the K-1 smallest computed distances, whatever the tree.  Boxes and points at exactly the bound
 // are taken until a candidate equal to it has been left out, so that one that equals the K-th distance is always noticed.
 //
-// What bounds them (a million uniform points in ten row splits, three coordinates, K = 64, ncu): k_tree_rows issue slots (0.79 of them
-// used, 1490 warp instructions a query, arithmetic pipe 0.70; 46 registers, 57 % of the warps resident), k_tree_groups the shared-memory
-// pipe (0.93; the counting's atomics meet in banks; 190 instructions a query; 72 registers and 60 bytes of them spilled, 28 one-warp CTAs
-// an SM).  Whole forward / one query at a time / the grid, ms, without a second look in the first two: 6.4 M uniform points in three
-// coordinates, K = 64 13.5 / 21.5 / 18.3; 1.6 M learned ones in four, K = 40 6.6 / 9.4 / 8.4; 800 k skewed in three, K = 128 3.0 / 4.6 / 18.8; a
-// million normal ones in five, K = 40 15.0 / 18.2 / 26.4.  The second look adds 0.85, 0.4, 1.5 and 0.4.
+// What bounds them (a million uniform points in ten row splits, three coordinates, K = 64, ncu): k_tree_rows issue slots (1000 warp
+// instructions a query: some 250 for its list and its boxes, 350 for 16 leaves, 400 for the sort and the row) and the latency of list, box and
+// point one after the other, hence the many warps; k_tree_groups the shared-memory pipe (0.83; the counting's atomics) and issue slots
+// (0.71; 240 instructions a query; 72 registers, some of them spilled, 28 one-warp CTAs an SM).
+// Whole forward in ms, before this split of the lists and of the visits / now / one query at a time / the grid, without a second look in the
+// first three: 6.4 M uniform points in three coordinates, K = 64 13.5 / 10.1 / 21.5 / 18.3; 1.6 M learned ones in four, K = 40 6.6 / 4.8 / 9.4 /
+// 8.4; 800 k skewed in three, K = 128 3.0 / 2.3 / 4.6 / 18.8; a million normal ones in five, K = 40 15.0 / 13.4 / 18.2 / 26.4.  The second look adds
+// 0.85, 0.4, 1.5 and 0.4.
 //
-// Other splits of the work, measured on the first and the third of these (then 13.9 and 3.2): one kernel, a lane per query, the points of a leaf read from
+// Other splits of the work, measured on the first and the third of these when they took 13.9 and 3.2: one kernel, a lane per query, the points of a leaf read from
 // shared memory by all 32 lanes (15.5; broadcast 16-byte loads write 512 bytes back each, four cycles an SM); candidates of all
 // 32 queries filtered by the matrix product and kept in the workspace, a second kernel for the rows (15.7 and 7.8: leaves that
 // visit thousands of others run on alone).
@@ -84,7 +86,7 @@ constexpr int kHistClasses = 32;
 constexpr int kSeedNodes = 4;
 __device__ __forceinline__ int seed_leaves(int kn, int dims)
 {
-    return min(4 + kn / 6, 28) + (dims >= 4 ? 6 : 0) + (dims >= 5 ? 6 : 0);
+    return min(6 + kn / 6, 26) + (dims >= 4 ? 6 : 0) + (dims >= 5 ? 6 : 0);
 }
 
 // An upper bound on the distance d of a point c from q whose |c|^2 - 2 c.q + |q|^2 comes out as t or less (coordinates relative to
@@ -115,7 +117,9 @@ __device__ __forceinline__ void bound_leaf(const TreeArgs &a, const int slot)
 {
     static_assert(DC + 2 <= 8, "one matrix product over coordinates and |c|^2 twice");
     constexpr int CHUNKS = (DC + 3) / 4;
-    __shared__ __align__(16) int s_hist[32 * (kHistClasses + 1)];
+    // classes of the counting, then the list of leaves
+    __shared__ __align__(16) int s_hist[tree_list_cap(DC) > 32 * (kHistClasses + 1) ? tree_list_cap(DC) : 32 * (kHistClasses + 1)];
+    __shared__ float s_part[4][2 * 4 * NV + 1];                 // boxes of eight queries, the largest bound among them
     const int lane = threadIdx.x & 31;
     const int kn = a.K - 1;
     const uint8_t *__restrict__ sflag = a.sflag;
@@ -139,7 +143,8 @@ __device__ __forceinline__ void bound_leaf(const TreeArgs &a, const int slot)
     if (sflag && (sflag[qi] == 0 || sflag[qi] == 2)) active = false;
     if (!__any_sync(FGC_FULL_MASK, active)) {            // no query of the leaf may have neighbours
         a.bound[place * 32 + lane] = kNoQuery;
-        if (lane == 0) a.list_n[place] = 0;
+        if (lane == 0) { a.list_n[place] = 0; a.leaf_info[slot] = make_int4(own_leaf * 32, ev_begin, n_e, 0); }
+        if (lane < 4) a.leaf_part[slot * 4 + lane] = make_int2(0, 0);
         return;
     }
 
@@ -252,6 +257,21 @@ __device__ __forceinline__ void bound_leaf(const TreeArgs &a, const int slot)
         int *mine = s_hist + g4 * (kHistClasses + 1) - first;
         const int lo_bits = first << 20, hi_bits = (first + kHistClasses - 1) << 20;
         const int n_seed = seed_leaves(kn, DC);
+        // Once K points are below the end of some class, what is beyond it is counted in the next class: it changes nothing there, and
+        // the counts of a row that all go to one place do not meet those of other rows in a bank.
+        auto classes_below = [&]() {             // classes whose end has fewer than K + 1 points before it (the query itself is counted)
+            __syncwarp();
+            int below = 0, classes = 0;
+#pragma unroll 16
+            for (int b = 0; b < kHistClasses; b++) {
+                below += s_hist[lane * (kHistClasses + 1) + b];
+                classes += below <= kn ? 1 : 0;
+            }
+            return classes;
+        };
+        int next_look = kn / 32 + 4, end[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) end[k] = hi_bits;
         int leaf = next_seed();
         if (leaf >= 0) load(leaf, c);
         for (int i = 0; i < n_seed && leaf >= 0; i++) {
@@ -293,6 +313,13 @@ __device__ __forceinline__ void bound_leaf(const TreeArgs &a, const int slot)
             const bool usable = !__any_sync(FGC_FULL_MASK, wide);
             leaf = next_seed();
             if (leaf >= 0) load(leaf, c);
+            if (i == next_look) {
+                const int classes = classes_below();
+                const int open = min((first + classes + 1) << 20, hi_bits);
+#pragma unroll
+                for (int k = 0; k < 4; k++) end[k] = __shfl_sync(FGC_FULL_MASK, open, g4 + 8 * k);
+                next_look += 8;
+            }
             if (!usable) continue;
 #pragma unroll
             for (int m = 0; m < 2; m++)
@@ -300,18 +327,11 @@ __device__ __forceinline__ void bound_leaf(const TreeArgs &a, const int slot)
                 for (int j = 0; j < 4; j++)
 #pragma unroll
                     for (int k = 0; k < 4; k++) {
-                        const int b = min(max(__float_as_int(f[m][j][k]), lo_bits), hi_bits) >> 20;
+                        const int b = min(max(__float_as_int(f[m][j][k]), lo_bits), end[2 * m + (k >> 1)]) >> 20;
                         atomicAdd(mine + (16 * m + 8 * (k >> 1)) * (kHistClasses + 1) + b, 1);
                     }
         }
-        __syncwarp();
-        // the query itself is among those counted, or the bound is a place too far
-        int below = 0, classes = 0;
-#pragma unroll 16
-        for (int b = 0; b < kHistClasses; b++) {
-            below += s_hist[lane * (kHistClasses + 1) + b];
-            classes += below <= kn ? 1 : 0;
-        }
+        const int classes = classes_below();
         if (classes < kHistClasses - 1 && q2 <= 1e36f) {
             t = widened(__uint_as_float((uint32_t)(first + classes + 1) << 20), q2);
             if (!is_finite_bits(t)) t = __uint_as_float(kInfBits);
@@ -322,7 +342,8 @@ __device__ __forceinline__ void bound_leaf(const TreeArgs &a, const int slot)
     if (!active) t = kNoQuery;
     a.bound[place * 32 + lane] = t;
     const float tmax = __uint_as_float(__reduce_max_sync(FGC_FULL_MASK, __float_as_uint(fmaxf(t, 0.f))));
-    int *__restrict__ list = a.list + (size_t)place * a.list_cap;
+    int *list = s_hist;
+    __syncwarp();
     const int own_node = own_leaf >> 5;
     int n = 0;
     auto take_node = [&](int node) {
@@ -362,7 +383,75 @@ __device__ __forceinline__ void bound_leaf(const TreeArgs &a, const int slot)
         if (active) a.bound[place * 32 + lane] = kListedQuery;       // (the others still get their default rows)
         n = 0;
     }
-    if (lane == 0) a.list_n[place] = n;
+    // The same for eight queries at a time: what a query has to look through is a third (four coordinates) to two thirds (three) of
+    // the list for 32.  A leaf is kept with four bits, one for each eight; then the four lists are written one behind the other.
+    if (n > 0) {
+        float lo[4 * NV], hi[4 * NV], most = t;
+        const float inf = __uint_as_float(kInfBits);
+#pragma unroll
+        for (int v = 0; v < NV; v++) {
+            const float4 q = __ldg(a.scoords + (size_t)qi * NV + v);
+            lo[4 * v] = hi[4 * v] = q.x; lo[4 * v + 1] = hi[4 * v + 1] = q.y;
+            lo[4 * v + 2] = hi[4 * v + 2] = q.z; lo[4 * v + 3] = hi[4 * v + 3] = q.w;
+        }
+#pragma unroll
+        for (int c = 0; c < DC; c++) {
+            if (!active) { lo[c] = inf; hi[c] = -inf; }
+#pragma unroll
+            for (int x = 4; x > 0; x >>= 1) {
+                lo[c] = fminf(lo[c], __shfl_xor_sync(FGC_FULL_MASK, lo[c], x));
+                hi[c] = fmaxf(hi[c], __shfl_xor_sync(FGC_FULL_MASK, hi[c], x));
+            }
+            if ((lane & 7) == 0) { s_part[lane >> 3][c] = lo[c]; s_part[lane >> 3][DC + c] = hi[c]; }
+        }
+#pragma unroll
+        for (int x = 4; x > 0; x >>= 1) most = fmaxf(most, __shfl_xor_sync(FGC_FULL_MASK, most, x));
+        if ((lane & 7) == 0) s_part[lane >> 3][2 * DC] = most;
+        __syncwarp();
+        int count[4] = {0, 0, 0, 0};
+        for (int i0 = 0; i0 < n; i0 += 32) {
+            const bool in = i0 + lane < n;
+            const int leaf = in ? list[i0 + lane] : 0;
+            float box[8 * NV];
+#pragma unroll
+            for (int v = 0; v < 2 * NV; v++) {
+                const float4 b = __ldg(leaf_box + (size_t)leaf * (2 * NV) + v);
+                box[4 * v] = b.x; box[4 * v + 1] = b.y; box[4 * v + 2] = b.z; box[4 * v + 3] = b.w;
+            }
+            int bits = 0;
+#pragma unroll
+            for (int p = 0; p < 4; p++) {
+                float acc = 0.f;
+#pragma unroll
+                for (int c = 0; c < DC; c++) {
+                    const float g = fmaxf(fmaxf(__fsub_rn(box[c], s_part[p][DC + c]), __fsub_rn(s_part[p][c], box[4 * NV + c])), 0.f);
+                    acc = c == 0 ? __fmul_rn(g, g) : __fadd_rn(acc, __fmul_rn(g, g));
+                }
+                const bool want = in && acc <= s_part[p][2 * DC];
+                bits |= want ? 1 << p : 0;
+                count[p] += __popc(__ballot_sync(FGC_FULL_MASK, want));
+            }
+            if (in) list[i0 + lane] = leaf | bits << 28;
+        }
+        __syncwarp();
+        const bool apart = count[0] + count[1] + count[2] + count[3] <= a.list_room;      // (else all have the one list)
+        int *__restrict__ out = a.list + (size_t)place * a.list_room;
+        int at = 0;
+        for (int p = 0; p < (apart ? 4 : 1); p++) {
+            if (lane == p) a.leaf_part[slot * 4 + p] = make_int2(at, count[p]);
+            for (int i0 = 0; i0 < n; i0 += 32) {
+                const int leaf = i0 + lane < n ? list[i0 + lane] : 0;
+                const bool want = i0 + lane < n && (!apart || (leaf >> 28 & 1 << p));
+                const unsigned m = __ballot_sync(FGC_FULL_MASK, want);
+                if (want) out[at + __popc(m & lanemask_lt())] = leaf & 0xfffffff;
+                at += __popc(m);
+            }
+        }
+        if (!apart && lane < 4) a.leaf_part[slot * 4 + lane] = make_int2(0, n);
+    } else if (lane < 4) {
+        a.leaf_part[slot * 4 + lane] = make_int2(0, 0);
+    }
+    if (lane == 0) { a.list_n[place] = n; a.leaf_info[slot] = make_int4(own_leaf * 32, ev_begin, n_e, 0); }
 }
 
 template <int NV, int DC>
@@ -536,15 +625,99 @@ __device__ __forceinline__ unsigned staying(uint32_t v, uint32_t hi, int most, i
     return __ballot_sync(FGC_FULL_MASK, keep);
 }
 
-template <int NV, int R>
-__global__ void __launch_bounds__(kRowWarps * 32, R == 8 ? 3 : (R == 4 || NV == 2 ? 4 : 5))
+// 16 bytes of coordinates in one read, used or not (left to itself the compiler reads three of four in two pieces).
+__device__ __forceinline__ float4 read_four(const float4 *p)
+{
+    float4 v;
+    asm("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+// Coordinates of a point, and its squared distance: the operations of dist_sq in the same order without the coordinates that
+// are 0 on both sides.
+template <int DC>
+struct RowPoint {
+    float4 a;
+    float e;              // the fifth
+};
+template <int DC>
+__device__ __forceinline__ RowPoint<DC> row_point(const float4 *__restrict__ scoords, int j)
+{
+    RowPoint<DC> p;
+    p.e = 0.f;
+    if constexpr (DC <= 4) {
+        p.a = read_four(scoords + j);
+    } else {
+        p.a = read_four(scoords + 2 * (size_t)j);
+        p.e = __ldg(reinterpret_cast<const float *>(scoords + 2 * (size_t)j + 1));
+    }
+    return p;
+}
+template <int DC>
+__device__ __forceinline__ float row_dist(const RowPoint<DC> &q, const RowPoint<DC> &c)
+{
+    float s0, s1, s2, s3 = 0.f;
+    sq_diff_f32x2(q.a.x, q.a.y, c.a.x, c.a.y, s0, s1);
+    if constexpr (DC == 3) {
+        const float z = __fsub_rn(q.a.z, c.a.z);
+        s2 = __fmul_rn(z, z);
+    } else {
+        sq_diff_f32x2(q.a.z, q.a.w, c.a.z, c.a.w, s2, s3);
+    }
+    float acc = __fadd_rn(__fadd_rn(s0, s1), s2);
+    if constexpr (DC >= 4) acc = __fadd_rn(acc, s3);
+    if constexpr (DC >= 5) {
+        const float e = __fsub_rn(q.e, c.e);
+        acc = __fadd_rn(acc, __fmul_rn(e, e));
+    }
+    return acc;
+}
+// The squared distance to a box, likewise.
+__device__ __forceinline__ float gap_sq(float lo, float hi, float x)
+{
+    const float g = fmaxf(fmaxf(__fsub_rn(lo, x), __fsub_rn(x, hi)), 0.f);
+    return __fmul_rn(g, g);
+}
+template <int DC>
+__device__ __forceinline__ float row_box(const RowPoint<DC> &q, const float4 *__restrict__ box)
+{
+    constexpr int NV = DC <= 4 ? 1 : 2;
+    const float4 lo = read_four(box), hi = read_four(box + NV);
+    float acc = __fadd_rn(__fadd_rn(gap_sq(lo.x, hi.x, q.a.x), gap_sq(lo.y, hi.y, q.a.y)), gap_sq(lo.z, hi.z, q.a.z));
+    if constexpr (DC >= 4) acc = __fadd_rn(acc, gap_sq(lo.w, hi.w, q.a.w));
+    if constexpr (DC >= 5) acc = __fadd_rn(acc, gap_sq(__ldg(&box[1].x), __ldg(&box[3].x), q.e));
+    return acc;
+}
+
+// A store, or a count, in shared memory under a predicate (as a branch it takes three instructions more).
+__device__ __forceinline__ void store_if(bool p, uint32_t at, float d, int j)
+{
+    asm volatile("{ .reg .pred q; setp.ne.u32 q, %0, 0; @q st.shared.v2.b32 [%1], {%2, %3}; }"
+                 :: "r"((uint32_t)p), "r"(at), "r"(__float_as_uint(d)), "r"(j) : "memory");
+}
+
+// Leaves (halves of them, even ones and then odd ones) wanted by a query and not yet visited: what one step of boxes finds behind
+// what is left of the steps before, and up to three (seven) behind the last one that fill four steps.
+constexpr int kWanted = 32 + 32 + 8;
+// Resident CTAs an SM asked of the compiler: the chain from a list to its boxes to the points is hidden by other warps, and a few
+// spilled registers cost less than warps that are not there.  Time of the rows in ms with 4 / 5 / 6 / 7 CTAs: 6.4 M uniform points in three
+// coordinates, K = 64 8.8 / 7.7 / 7.2 / 8.1, 800 k, K = 16 0.73 / 0.64 / 0.57 / 0.53; 1.6 M learned ones in four, K = 40 4.1 / 3.8 / 3.6 / 3.6; 800 k
+// skewed in three, K = 128 1.74 / 1.61 / 1.50 / 1.53; 400 k uniform in four, K = 200 1.81 / 1.66 / 1.74 / -.
+constexpr int row_ctas(int r) { return r == 1 ? 7 : (r == 8 ? 5 : 6); }
+
+template <int DC, int R, bool FLAGS>
+__global__ void __launch_bounds__(kRowWarps * 32, row_ctas(R))
 k_tree_rows(const TreeArgs a)
 {
     chain_wait();
     chain_release();
+    constexpr int NV = DC <= 4 ? 1 : 2;
     constexpr int ROWS = RowShape<R>::ROWS, MOST = ROWS * 32;
+    constexpr bool HALVES = DC >= kHalfDims;
+    constexpr int STEP = HALVES ? 8 : 4;
     __shared__ float2 s_pairs[kRowWarps][MOST];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    __shared__ __align__(16) int s_wanted[kRowWarps][kWanted];
+    __shared__ int s_near[HALVES ? kRowWarps : 1][64];
+    const int lane = threadIdx.x & 31, w = __shfl_sync(FGC_FULL_MASK, (int)threadIdx.x >> 5, 0);      // (known to be the same in a warp)
     const int K = a.K, kn = K - 1;
     if (a.grid->status != 0) {
         // rows of points without neighbours: bad input, no tree was built
@@ -558,44 +731,35 @@ k_tree_rows(const TreeArgs a)
         }
         return;
     }
-    // queries of this launch, in curve order: the eight of a CTA are of one leaf
-    const int64_t row = (int64_t)blockIdx.x * kRowWarps + w;
-    const int64_t slot = a.slot0 + (row >> 5);
+    // queries of this launch, in curve order: the eight of a CTA are those of one list
+    const int row = (int)blockIdx.x * kRowWarps + w;
+    const int slot = a.slot0 + (row >> 5);
     if (slot >= a.n_slots) return;
-    const int n_list = __ldg(a.list_n + (row >> 5));
-    if (n_list < 0) return;
+    if (__ldg(a.list_n + (row >> 5)) < 0) return;
+    const int4 info = __ldg(a.leaf_info + slot);
+    const int2 part = __ldg(a.leaf_part + slot * 4 + (row >> 3 & 3));
     float t = __ldg(a.bound + row);
-    const int e = warp_event_of_leaf(a.row_splits, a.n_rs, slot, lane);
-    const int ev_begin = (int)__ldg(a.row_splits + e);
-    const int n_e = (int)__ldg(a.row_splits + e + 1) - ev_begin;
-    const int64_t leaf0 = tree_base(ev_begin, e, 5);
-    const int rel_q = (int)(slot - leaf0) * 32 + (int)(row & 31);
+    const int ev_begin = info.y, n_e = info.z, ev_end = ev_begin + n_e, n_list = part.y;
+    const int rel_q = info.x + (row & 31);
     const bool writes = rel_q < n_e && t != kListedQuery;
     // (an open bound as the largest number: distances that overflow are no candidates)
     t = writes ? fminf(t, 3.402823466e38f) : kNoQuery;
     const int qi = ev_begin + min(rel_q, n_e - 1);
-    const float4 *__restrict__ leaf_box = a.box[0] + (size_t)leaf0 * (2 * NV);
-    const int *__restrict__ list = a.list + (size_t)(row >> 5) * a.list_cap;
-    const uint8_t *__restrict__ sflag = a.sflag;
+    const int *__restrict__ list = a.list + (size_t)(row >> 5) * a.list_room + part.x;
+    const float4 *__restrict__ leaf_box = a.box[0] + (size_t)(slot - (info.x >> 5)) * (2 * NV);
+    const float4 *__restrict__ half_box = a.half_box + (size_t)(slot - (info.x >> 5)) * (4 * NV);
+    const float4 *__restrict__ scoords = a.scoords;
     float2 *pairs = s_pairs[w];
-    float4 x[NV];
-#pragma unroll
-    for (int v = 0; v < NV; v++) x[v] = __ldg(a.scoords + (size_t)qi * NV + v);
+    const uint32_t pairs_at = (uint32_t)__cvta_generic_to_shared(pairs);
+    int *wanted = s_wanted[w], *near = s_near[HALVES ? w : 0];
+    const RowPoint<DC> x = row_point<DC>(scoords, qi);
     int m = 0;                               // points kept
     uint32_t left_out = kNoBox;              // the last distance at which a point was left out that equals the bound
-    auto load = [&](int leaf, float4 (&c)[NV], int &j) {
-        const int rel = leaf * 32 + lane;
-        j = rel < n_e ? ev_begin + rel : -1;
-        if (!FGC_DBG_OK(j < a.n_vert, &a.grid->status)) j = -1;
-#pragma unroll
-        for (int v = 0; v < NV; v++) c[v] = __ldg(a.scoords + (size_t)(j < 0 ? qi : j) * NV + v);
-    };
-    auto keep = [&](const float4 (&c)[NV], int j) {
-        const float d = dist_sq<NV>(x, c, 0);
-        bool in = d <= t && j >= 0 && j != qi;
-        if (sflag && in) { const uint8_t f = sflag[j]; in = f != 1 && f != 2; }
+    auto keep = [&](const RowPoint<DC> &c, int j) {
+        const float d = row_dist<DC>(x, c);
+        const bool in = (d <= t) & (j != qi);
         const unsigned mask = __ballot_sync(FGC_FULL_MASK, in);
-        if (in) pairs[m + __popc(mask & lanemask_lt())] = make_float2(d, __int_as_float(j));
+        store_if(in, pairs_at + 8 * (m + __popc(mask & lanemask_lt())), d, j);
         m += __popc(mask);
     };
     // down to the kn nearest or a few more, and the bound with them
@@ -622,117 +786,82 @@ k_tree_rows(const TreeArgs a)
         if (left) left_out = hi;
         t = __uint_as_float(hi - (left ? 1u : 0u));
     };
-    // the leaves of `todo`, two at a time
-    auto visit = [&](unsigned todo, auto leaf_at) {
-        while (todo) {
-            const int b0 = __ffs(todo) - 1;
-            todo &= todo - 1;
-            const int b1 = todo ? __ffs(todo) - 1 : -1;
-            todo &= todo - 1;
-            float4 c0[NV], c1[NV];
-            int j0, j1;
-            load(leaf_at(b0), c0, j0);
-            load(leaf_at(b1 < 0 ? b0 : b1), c1, j1);
-            if (b1 < 0) j1 = -1;
+    // Visits.  Lanes whose leaf is wanted write its first point down; then four leaves a step, whose points are on their way
+    // together: one 16-byte read gives the four, where picking them out of a ballot took five instructions each.  In five
+    // coordinates only the halves within the bound are visited, two side by side (a million normal points, K = 40: 9.5 -> 8.8 ms; with
+    // fewer coordinates the boxes of the halves cost more than they save: 6.4 M uniform points in three, K = 64 8.6 against 7.7).
+    int n_wanted = 0, n_near = 0, near0 = 0;
+    const int *mine = HALVES ? wanted + (lane >> 4) * (kWanted / 2) : wanted;
+    auto fetch = [&](int first, int &j, RowPoint<DC> &c) {
+        j = first + (HALVES ? lane & 15 : lane);
+        j = j < ev_end ? j : qi;
+        if (!FGC_DBG_OK(j >= ev_begin && j < a.n_vert, &a.grid->status)) j = qi;
+        c = row_point<DC>(scoords, j);
+        if constexpr (FLAGS) { const uint8_t f = a.sflag[j]; if (f == 1 || f == 2) j = qi; }
+    };
+    auto visit_wanted = [&]() {
+        if (lane < STEP - 1)                     // (no points there)
+            wanted[HALVES ? ((n_wanted + lane) & 1) * (kWanted / 2) + ((n_wanted + lane) >> 1) : n_wanted + lane] = ev_end;
+        __syncwarp();
+        for (int i = 0; i < n_wanted && t >= 0.f; i += STEP) {
+            const int4 first = *reinterpret_cast<const int4 *>(mine + (HALVES ? i >> 1 : i));
+            int j0, j1, j2, j3;
+            RowPoint<DC> c0, c1, c2, c3;
+            fetch(first.x, j0, c0);
+            fetch(first.y, j1, c1);
+            fetch(first.z, j2, c2);
+            fetch(first.w, j3, c3);
             keep(c0, j0);
             keep(c1, j1);
             if (m > MOST - 64) cut();
+            if (i + STEP / 2 < n_wanted) {
+                keep(c2, j2);
+                keep(c3, j3);
+                if (m > MOST - 64) cut();
+            }
         }
+        n_wanted = 0;
+        __syncwarp();
     };
-    if constexpr (NV == 1) {
-        for (int base = 0; base < n_list && t >= 0.f; base += 32) {
-            int leaf = 0;
-            bool want = false;
-            if (base + lane < n_list) {
-                leaf = __ldg(list + base + lane);
-                want = box_box_sq<NV>(x, x, leaf_box + (size_t)leaf * (2 * NV)) <= t;
-            }
-            visit(__ballot_sync(FGC_FULL_MASK, want), [&](int b) { return __shfl_sync(FGC_FULL_MASK, leaf, b); });
+    // the halves of the next up to 16 near leaves
+    auto halves = [&]() {
+        __syncwarp();
+        const int i = lane >> 1;
+        int first = 0;
+        bool want = false;
+        if (i < n_near) {
+            const int half = near[(near0 + i) & 63] * 2 + (lane & 1);
+            first = ev_begin + half * 16;
+            want = row_box<DC>(x, half_box + (size_t)half * (2 * NV)) <= t;
         }
-    } else {
-        // In five coordinates the boxes of a list are 64 KB, which every warp would read for itself: the eight of a CTA read them
-        // once, and leave those near enough to some of their queries in shared memory (a million normal points, K = 40, lists of up to
-        // 3072: 18.4 -> 15.6 ms).  With up to four, where a list is one or two steps long, waiting for one another costs more
-        // than it saves (6.4 M uniform points in three, K = 64: 13.9 -> 15.2 ms).
-        constexpr int NC = kGroupDims;
-        __shared__ float s_box[2 * NC][kRowWarps * 32];
-        __shared__ int s_leaf[kRowWarps * 32];
-        __shared__ float s_query[kRowWarps][4 * NV], s_eight[2][NC], s_bound[kRowWarps];
-        __shared__ int s_count[kRowWarps];
-        float xc[4 * NV];
-#pragma unroll
-        for (int v = 0; v < NV; v++) { xc[4 * v] = x[v].x; xc[4 * v + 1] = x[v].y; xc[4 * v + 2] = x[v].z; xc[4 * v + 3] = x[v].w; }
-        if (lane == 0) {
-            s_bound[w] = t;
-#pragma unroll
-            for (int v = 0; v < NV; v++) {
-                s_query[w][4 * v] = x[v].x; s_query[w][4 * v + 1] = x[v].y;
-                s_query[w][4 * v + 2] = x[v].z; s_query[w][4 * v + 3] = x[v].w;
-            }
+        const unsigned mask = __ballot_sync(FGC_FULL_MASK, want);
+        const int at = n_wanted + __popc(mask & lanemask_lt());
+        if (want) wanted[(at & 1) * (kWanted / 2) + (at >> 1)] = first;
+        n_wanted += __popc(mask);
+        near0 += 16;
+        n_near -= 16;
+        if (n_wanted > 32) visit_wanted();
+    };
+    for (int base = 0; base < n_list && t >= 0.f; base += 32) {
+        int leaf = 0;
+        bool want = false;
+        if (base + lane < n_list) {
+            leaf = __ldg(list + base + lane);
+            want = row_box<DC>(x, leaf_box + (size_t)leaf * (2 * NV)) <= t;
         }
-        __syncthreads();
-        if (threadIdx.x < NC) {
-            float lo = __uint_as_float(kInfBits), hi = -__uint_as_float(kInfBits);
-#pragma unroll
-            for (int k = 0; k < kRowWarps; k++)
-                if (s_bound[k] >= 0.f) { lo = fminf(lo, s_query[k][threadIdx.x]); hi = fmaxf(hi, s_query[k][threadIdx.x]); }
-            s_eight[0][threadIdx.x] = lo;
-            s_eight[1][threadIdx.x] = hi;
-        }
-        float tmax = s_bound[0];
-#pragma unroll
-        for (int k = 1; k < kRowWarps; k++) tmax = fmaxf(tmax, s_bound[k]);
-        __syncthreads();
-        for (int base = 0; base < n_list && tmax >= 0.f; base += kRowWarps * 32) {
-            int leaf = 0;
-            bool want = false;
-            float box[8 * NV];
-            if (base + (int)threadIdx.x < n_list) {
-                leaf = __ldg(list + base + threadIdx.x);
-#pragma unroll
-                for (int v = 0; v < 2 * NV; v++) {
-                    const float4 b = __ldg(leaf_box + (size_t)leaf * (2 * NV) + v);
-                    box[4 * v] = b.x; box[4 * v + 1] = b.y; box[4 * v + 2] = b.z; box[4 * v + 3] = b.w;
-                }
-                float acc = 0.f;
-#pragma unroll
-                for (int c = 0; c < NC; c++) {
-                    const float g = fmaxf(fmaxf(__fsub_rn(box[c], s_eight[1][c]), __fsub_rn(s_eight[0][c], box[4 * NV + c])), 0.f);
-                    acc = c == 0 ? __fmul_rn(g, g) : __fadd_rn(acc, __fmul_rn(g, g));
-                }
-                want = acc <= tmax;
-            }
-            const unsigned mine = __ballot_sync(FGC_FULL_MASK, want);
-            if (lane == 0) s_count[w] = __popc(mine);
-            __syncthreads();
-            int at = __popc(mine & lanemask_lt()), total = 0;
-#pragma unroll
-            for (int k = 0; k < kRowWarps; k++) {
-                if (k == w) at += total;
-                total += s_count[k];
-            }
-            if (want) {
-                s_leaf[at] = leaf;
-#pragma unroll
-                for (int c = 0; c < NC; c++) {
-                    s_box[c][at] = box[c];
-                    s_box[NC + c][at] = box[4 * NV + c];
-                }
-            }
-            __syncthreads();
-            for (int i0 = 0; i0 < total && t >= 0.f; i0 += 32) {
-                const int i = i0 + lane;
-                float acc = 0.f;
-#pragma unroll
-                for (int c = 0; c < NC; c++) {
-                    const float g = fmaxf(fmaxf(__fsub_rn(s_box[c][i], xc[c]), __fsub_rn(xc[c], s_box[NC + c][i])), 0.f);
-                    acc = c == 0 ? __fmul_rn(g, g) : __fadd_rn(acc, __fmul_rn(g, g));
-                }
-                visit(__ballot_sync(FGC_FULL_MASK, i < total && acc <= t), [&](int b) { return s_leaf[i0 + b]; });
-            }
-            __syncthreads();
+        const unsigned mask = __ballot_sync(FGC_FULL_MASK, want);
+        if constexpr (HALVES) {
+            if (want) near[(near0 + n_near + __popc(mask & lanemask_lt())) & 63] = leaf;
+            n_near += __popc(mask);
+            while (n_near >= 16 && t >= 0.f) halves();
+        } else {
+            if (want) wanted[n_wanted + __popc(mask & lanemask_lt())] = ev_begin + leaf * 32;
+            n_wanted += __popc(mask);
+            if (n_wanted > 32) visit_wanted();
         }
     }
+    while (n_near > 0 && t >= 0.f) halves();
+    if (n_wanted > 0) visit_wanted();
     if (!writes) return;
     __syncwarp();
     const int orig_q = __ldg(a.sorig + qi);
@@ -839,12 +968,20 @@ k_tree_rows(const TreeArgs a)
     }
 }
 
+template <int DC, int R>
+static cudaError_t launch_rows(const TreeArgs &a, unsigned blocks, cudaStream_t s)
+{
+    return a.sflag ? launch_chained(k_tree_rows<DC, R, true>, blocks, kRowWarps * 32, 0, s, a)
+                   : launch_chained(k_tree_rows<DC, R, false>, blocks, kRowWarps * 32, 0, s, a);
+}
+
 template <int NV, int DC>
 static cudaError_t launch_tree(TreeArgs a, const TreeScratch &scratch, cudaStream_t s)
 {
     a.list = scratch.list;
     a.list_n = scratch.list_n;
     a.list_cap = scratch.list_cap;
+    a.list_room = scratch.list_room;
     a.bound = scratch.bound;
     const int n_slots = a.n_slots;
     for (int slot = 0; slot < n_slots; slot = a.n_slots) {
@@ -853,10 +990,10 @@ static cudaError_t launch_tree(TreeArgs a, const TreeScratch &scratch, cudaStrea
         const unsigned count = (unsigned)(a.n_slots - slot), rows = count * (32 / kRowWarps);
         FGC_TRY(launch_chained(k_tree_groups<NV, DC>, count, 32, 0, s, a));
         switch (tree_list_rows(a.K)) {
-        case 1: FGC_TRY(launch_chained(k_tree_rows<NV, 1>, rows, kRowWarps * 32, 0, s, a)); break;
-        case 2: FGC_TRY(launch_chained(k_tree_rows<NV, 2>, rows, kRowWarps * 32, 0, s, a)); break;
-        case 4: FGC_TRY(launch_chained(k_tree_rows<NV, 4>, rows, kRowWarps * 32, 0, s, a)); break;
-        default: FGC_TRY(launch_chained(k_tree_rows<NV, 8>, rows, kRowWarps * 32, 0, s, a));
+        case 1: FGC_TRY((launch_rows<DC, 1>(a, rows, s))); break;
+        case 2: FGC_TRY((launch_rows<DC, 2>(a, rows, s))); break;
+        case 4: FGC_TRY((launch_rows<DC, 4>(a, rows, s))); break;
+        default: FGC_TRY((launch_rows<DC, 8>(a, rows, s)));
         }
     }
     return cudaSuccess;
@@ -880,7 +1017,11 @@ int fgc::knn_search_tree_groups(int64_t n_vert, int32_t n_coords, const int64_t 
     if (!tree_scratch(L, n_coords, (char *)workspace, workspace_bytes, &scratch)) return FGC_ERR_WORKSPACE;
     cudaStream_t s = (cudaStream_t)stream;
     a.n_slots = (int)T.n_box[0];
-    a.listed = (int *)((char *)workspace + T.keys[0]);           // free since the build
+    if (!T.groups) return FGC_ERR_WORKSPACE;
+    a.listed = (int *)((char *)workspace + T.listed);
+    a.half_box = (const float4 *)((char *)workspace + T.half_box);
+    a.leaf_info = (int4 *)((char *)workspace + T.leaf_info);
+    a.leaf_part = (int2 *)(a.leaf_info + T.n_box[0]);
     if (n_coords <= 3) FGC_RETURN_IF_CUDA((launch_tree<1, 3>(a, scratch, s)));
     else if (n_coords == 4) FGC_RETURN_IF_CUDA((launch_tree<1, 4>(a, scratch, s)));
     else FGC_RETURN_IF_CUDA((launch_tree<2, 5>(a, scratch, s)));

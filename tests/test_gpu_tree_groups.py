@@ -467,3 +467,26 @@ def test_tiny_row_splits_are_searched_on_the_grid(n, D, row_splits, K, long_tail
     from fastgraphcompute_b200 import _cabi
     lib = _cabi.lib
     assert tree == max(rule(n, D, row_splits + 1, K, long_tails) for rule in (lib.fgc_knn_tree_preferred, lib.fgc_knn_groups_preferred))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind,sizes,D,K", [
+    ("uniform", [1, 15, 16, 17, 31, 33, 47, 49, 1000, 8], 5, 9),        # halves of leaves without points, or with a few
+    ("uniform", [9] * 150, 5, 6),                                       # no room for what the search by groups keeps per leaf
+    ("uniform", [7, 8, 9, 24, 25, 39, 41, 700], 3, 6),                  # eights of a leaf without queries, or with a few
+    ("normal", [40000], 4, 257), ("normal", [60000], 5, 100)])          # four lists longer together than the room for them
+@pytest.mark.parametrize("flags", [False, True])
+def test_lists_of_eight_queries(kind, sizes, D, K, flags):
+    """Bit-equal distances and the same ids as the grid finds."""
+    km = importlib.import_module("fastgraphcompute_b200.extensions.binned_select_knn")
+    g = torch.Generator().manual_seed(D * K)
+    n = sum(sizes)
+    x = (torch.randn((n, D), generator=g) if kind == "normal" else torch.rand((n, D), generator=g)).to(DEV)
+    rs = torch.tensor([0] + sizes).cumsum(0).to(DEV)
+    direction = torch.randint(0, 4, (n,), generator=g).to(DEV) if flags else None
+    gi, gd, _ = _forward(km, x, rs, K, False, direction)
+    ti, td, _ = _forward(km, x, rs, K, True, direction)
+    assert torch.equal(gd.sort(dim=1).values, td.sort(dim=1).values)
+    edge = gd.amax(dim=1, keepdim=True)
+    inside = [torch.where((i >= 0) & (d < edge), i, torch.full_like(i, -1)).sort(dim=1).values for i, d in ((gi, gd), (ti, td))]
+    assert torch.equal(*inside)
