@@ -152,6 +152,8 @@ SIGNATURES = {
     "fgc_gravnet_project_bwd": (ctypes.c_int, [c_void_p, c_i64, c_i32, c_i32, c_i32, c_void_p, c_void_p, c_void_p,
                                                c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                                c_void_p]),
+    "fgc_dense_forward": (ctypes.c_int, [c_void_p, c_void_p, c_void_p, c_i64, c_i32, c_i32, c_i32, c_void_p, c_void_p]),
+    "fgc_dense_input_gradient": (ctypes.c_int, [c_void_p, c_void_p, c_void_p, c_i64, c_i32, c_i32, c_void_p, c_void_p]),
     "fgc_bias_act": (ctypes.c_int, [c_void_p, c_void_p, c_i64, c_i32, c_i32, c_void_p]),
     "fgc_dense_backward_bytes": (c_size, [c_i64, c_i32, c_i32]),
     "fgc_dense_backward": (ctypes.c_int, [c_void_p, c_void_p, c_void_p, c_i64, c_i32, c_i32, c_void_p, c_void_p, c_void_p,

@@ -1,31 +1,30 @@
-// Dense layers around the message passing for sm_100a: bias and ReLU of a layer's output in one pass,
-// and the backward of bias, weight and ReLU in one pass over the incoming gradient.
+// Dense layers around the message passing for sm_100a, on the tensor cores at fp32 accuracy (tensor_core.cuh).
 //
-// The products with the weight matrix itself (forward and input gradient) stay with the library GEMMs.
-// The weight gradient dW[o, c] = sum over rows of dY[row, o] * x[row, c] is the shape a general GEMM
-// is worst at -- hundreds of thousands of rows summed into a 128 x 128 result -- and the ReLU mask and the
-// bias gradient read the same dY again:
+// Tall matrices against a small weight: hundreds of thousands of rows, up to a few hundred columns.  The scalar fp32
+// products of a library take several times what it takes to read the rows, and bias, ReLU and its mask cost passes of their own.
 //
-//   k_dense_bwd     a CTA owns one tile of dW (up to 128 x 128) and a range of rows.  Rows are natural
-//                   outer-product operands (both sides are contiguous in a row), so tiles go to shared
-//                   memory as they are, 16 rows at a time, double-buffered through registers; on the way dY is
-//                   masked by the layer's output, written out for the input-gradient GEMM and summed
-//                   for the bias.  Scalar fp32 multiply-adds, 8 x 8 per thread.
+//   k_dense_rows    out = act(A W + b) for 128 rows at a time: a forward, or an input gradient with A the incoming gradient, masked
+//                   by the layer's output on the way.  A CTA keeps the weight, split into three parts, in shared memory and
+//                   goes through tiles of rows, 64 columns a step: sixteen warps load two steps ahead into registers, split and write
+//                   to one of three buffers, one thread issues the products of a step, four warps write the results of a tile
+//                   while the next one is formed (two sets of accumulators in TMEM).
+//   k_dense_weight  dW = dY^T x and db: a CTA goes through a range of rows, 64 at a time, which are M- and N-major operands as
+//                   they are.  The accumulators of every 64 rows are added to fp32 registers, so that no sum is
+//                   rounded by the tensor core more than a few times.
 //   k_dense_reduce  adds the CTAs' partial results in a fixed order: the result is the same on
 //                   every run.
 //
-// Bound by latency between the fp32 multiply-adds: two CTAs of eight warps on an SM fill 0.56 of the issue slots, 400 k rows,
-// 128 to 128, 0.46 ms, i.e. 28 of 72 TFLOP/s and 1.7 TB/s.  Forward and backward of one layer with ReLU,
-// library only -> with these kernels (B200, ms): 200 k rows, 128 to 128: 1.02 -> 0.64; 64 to 128: 0.88 ->
-// 0.44; 128 to 10: 0.385 -> 0.281; 800 k rows, 128 to 64: 1.70 -> 1.20; where they lose (launches, narrow and wide
-// weights) the caller keeps the modules.  Relative error of dW against 64 bits at 200 k rows,
-// 128 to 128: 1.1e-6 (library) -> 3.5e-7.
-#include "fgc_common.cuh"
+// Tiles with numbers that cannot be split (infinities, NaN, 2^60 and more) are computed by scalar operations.
+//
+// Forward and backward with ReLU, us, modules / library products with passes of our own for bias, mask and dW / now: 200 k rows, 128 to 128
+// 1018 / 640 / 318; 64 to 128 884 / 440 / 287; 1.6 M rows, 128 to 64 3156 / 2300 / 1577.  Relative error against 64 bits, library / now:
+// forward 2.0e-7 / 1.2e-7, input gradient 1.4e-7 / 0.8e-7, dW 1.1e-6 (3.5e-7 summed in fp32 by 148 CTAs) / 1.4e-7.
+//
+// k_dense_rows (200 k rows, 128 to 128: 80 us; read and written once it would be 31): latency between splitting warps and the loads two
+// steps ahead, tensor pipe 0.26.  k_dense_weight (126 us; 47): one step of loads ahead, 3 M instructions an SM to split and add up.
+#include "tensor_core.cuh"
 
 namespace fgc {
-
-constexpr int kDenseThreads = 256;
-constexpr int kDenseRows = 16;       // rows per step
 
 // y = act(y + b), in place.  VEC: four columns at a time (n_out % 4 == 0, 16-byte aligned).
 template <bool VEC>
@@ -56,143 +55,492 @@ k_bias_act(float *__restrict__ y, const float *__restrict__ b, long long n_rows,
     }
 }
 
-// Four consecutive columns of a row, zero beyond the matrix.
+
+// Eight columns from `at` on, zero where fewer are left; `at` is 16-byte aligned if VEC.
 template <bool VEC>
-__device__ __forceinline__ float4 dense_load4(const float *__restrict__ m, long long row, long long row_end, int col, int n_cols)
+__device__ __forceinline__ void dense_load8_at(const float *__restrict__ at, int left, float4 (&v)[2])
 {
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (row < row_end && col < n_cols) {
-        const float *p = m + (size_t)row * n_cols + col;
-        if constexpr (VEC) v = __ldg((const float4 *)p);
-        else {
-            v.x = __ldg(p);
-            if (col + 1 < n_cols) v.y = __ldg(p + 1);
-            if (col + 2 < n_cols) v.z = __ldg(p + 2);
-            if (col + 3 < n_cols) v.w = __ldg(p + 3);
-        }
+    v[0] = v[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if constexpr (VEC) {
+        if (left > 0) v[0] = __ldg((const float4 *)at);
+        if (left > 4) v[1] = __ldg((const float4 *)at + 1);
+    } else {
+        float *o = reinterpret_cast<float *>(v);
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+            if (i < left) o[i] = __ldg(at + i);
     }
-    return v;
+}
+// The gradient passes unless the output is at or below zero (a NaN lets it pass, as in torch).
+__device__ __forceinline__ void mask8(float4 (&g)[2], const float4 (&y)[2])
+{
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        if (y[i].x <= 0.f) g[i].x = 0.f;
+        if (y[i].y <= 0.f) g[i].y = 0.f;
+        if (y[i].z <= 0.f) g[i].z = 0.f;
+        if (y[i].w <= 0.f) g[i].w = 0.f;
+    }
+}
+__device__ __forceinline__ uint32_t split_to(char *operand, int part_bytes, int row, int unit, const float4 (&v)[2])
+{
+    const float f[8] = {v[0].x, v[0].y, v[0].z, v[0].w, v[1].x, v[1].y, v[1].z, v[1].w};
+    uint4 part[3];
+    const uint32_t most = split8(f, part);
+    char *to = operand + operand_at(row, unit);
+#pragma unroll
+    for (int k = 0; k < 3; k++) *reinterpret_cast<uint4 *>(to + k * part_bytes) = part[k];
+    return most;
 }
 
-// BO x BC: tile of dW.  Thread (ty, tx) owns outputs 4 ty + 64 k + {0..3} and inputs 4 tx + 64 j + {0..3}.
-template <int BO, int BC, bool VEC>
-__global__ void __launch_bounds__(kDenseThreads, 2)
-k_dense_bwd(const float *__restrict__ x, const float *__restrict__ dy, const float *__restrict__ y, long long n_rows,
-            int n_in, int n_out, long long rows_per_cta, float *__restrict__ dy_masked, float *__restrict__ part_w,
-            float *__restrict__ part_b)
+// ----------------------------------------------------------------------------- rows times a weight
+
+struct DenseRows {
+    const float *a, *mask, *w, *bias;      // [n_rows, n_sum], the same or null, weight, [n_cols] or null
+    float *out;                            // [n_rows, n_cols]
+    long long n_rows;
+    int n_sum, n_cols;
+    int w_sum, w_col;                      // steps of the weight along what is summed over, and from column to column
+    int relu;
+    int chunks, tile_cols, buffers;        // 64 numbers of the sum each; columns of a CTA; steps that are split ahead
+};
+// Warps of a CTA: 16 load and split, four write results, one issues products.
+constexpr int kRowsSplit = 16, kRowsWrite = 4, kRowsThreads = 32 * (kRowsSplit + kRowsWrite + 1), kRowsTile = 128;
+constexpr int kRowsBuffer = 3 * kRowsTile * 128, kRowsStage = 32 * 20 * 4;
+constexpr int kRowsBad = 8;                // tiles that splitting may be ahead of writing: five
+inline size_t dense_rows_smem(int buffers, int chunks, int tile_cols)
 {
-    constexpr int MO = BO / 16, MC = BC / 16;
-    constexpr int LO = kDenseRows * BO / 4 / kDenseThreads, LC = kDenseRows * BC / 4 / kDenseThreads;   // float4 loads per thread
-    __shared__ float4 s_y[2][kDenseRows][BO / 4];
-    __shared__ float4 s_x[2][kDenseRows][BC / 4];
-    const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
-    const int o0 = blockIdx.z * BO, c0 = blockIdx.y * BC;
-    const long long first = (long long)blockIdx.x * rows_per_cta;
-    const long long last = min(n_rows, first + rows_per_cta);
-    const int oc = (t % (BO / 4)) * 4, orow = t / (BO / 4);
-    const int xc = (t % (BC / 4)) * 4, xrow = t / (BC / 4);
-    const bool owner = blockIdx.y == 0;          // of the mask and the bias sum
-    float acc[MO][MC];
+    return 1024 + buffers * (size_t)kRowsBuffer + 3 * (size_t)chunks * tile_cols * 128 + kRowsWrite * (size_t)kRowsStage + 256;
+}
+
+template <bool VEC, bool MASK>
+__global__ void __launch_bounds__(kRowsThreads, 1)
+k_dense_rows(const DenseRows g)
+{
+    extern __shared__ char s_raw[];
+    char *s = s_raw + ((1024 - (smem_at(s_raw) & 1023)) & 1023);
+    char *s_a = s, *s_w = s + g.buffers * kRowsBuffer;
+    const int w_part = g.chunks * g.tile_cols * 128;
+    float *s_stage = reinterpret_cast<float *>(s_w + 3 * w_part);
+    uint64_t *s_bar = reinterpret_cast<uint64_t *>(reinterpret_cast<char *>(s_stage) + kRowsWrite * kRowsStage);
+    uint32_t *s_tmem = reinterpret_cast<uint32_t *>(s_bar + 10);
+    volatile int *s_late = reinterpret_cast<int *>(s_tmem + 1), *s_bad = s_late + 1;       // a wait that gave up; tiles not to be split
+    const uint32_t bar = smem_at(s_bar), full = bar, empty = bar + 24, done = bar + 48, read = bar + 64;
+    const int t = threadIdx.x, lane = t & 31, w = __shfl_sync(FGC_FULL_MASK, t >> 5, 0);
+    const int col0 = blockIdx.y * g.tile_cols, NT = g.tile_cols;
+    const uint32_t columns = tmem_columns(4 * NT);
+    if (w == 0) tmem_alloc(smem_at(s_tmem), columns);
+    if (t == 0) {
+        for (int i = 0; i < 3; i++) {
+            mbar_init(full + 8 * i, kRowsSplit);
+            mbar_init(empty + 8 * i, 1);
+        }
+        for (int i = 0; i < 2; i++) {
+            mbar_init(done + 8 * i, 1);
+            mbar_init(read + 8 * i, kRowsWrite);
+        }
+        *s_late = 0;
+        for (int i = 0; i < kRowsBad; i++) s_bad[i] = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    // the weight: row n of the operand is output column col0 + n
+    uint32_t most = 0;
+    for (int i = t; i < g.chunks * NT * 8; i += kRowsThreads) {
+        const int unit = i & 7, n = (i >> 3) % NT, chunk = (i >> 3) / NT;
+        float4 v[2];
+        float *f = reinterpret_cast<float *>(v);
 #pragma unroll
-    for (int i = 0; i < MO; i++)
+        for (int k = 0; k < 8; k++) {
+            const int at = chunk * 64 + unit * 8 + k;
+            f[k] = col0 + n < g.n_cols && at < g.n_sum ? __ldg(g.w + (size_t)at * g.w_sum + (size_t)(col0 + n) * g.w_col) : 0.f;
+        }
+        most = max(most, split_to(s_w + chunk * NT * 128, w_part, n, unit, v));
+    }
+    smem_to_tensor_core();
+    tc_before_sync();
+    const bool plain_all = __syncthreads_or(most >= kUnsplit);
+    tc_after_sync();
+    const uint32_t tmem = *s_tmem;
+    const long long n_tiles = (g.n_rows + kRowsTile - 1) / kRowsTile;
+    const int my_tiles = (int)((n_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x);
+    const int steps = my_tiles * g.chunks;
+
+    if (w < kRowsSplit) {
+        const int row_in = t >> 3, unit = t & 7;               // of the two passes of 64 rows over a tile
+        long long row = (long long)blockIdx.x * kRowsTile + row_in;          // of the next load
+        int col = unit * 8;
+        auto fetch = [&](float4 (&a)[2][2], float4 (&m)[2][2]) {
 #pragma unroll
-        for (int j = 0; j < MC; j++) acc[i][j] = 0.f;
-    // two levels, so that a thread never adds thousands of rows one to another
-    float4 bsum = make_float4(0.f, 0.f, 0.f, 0.f), btotal = bsum;
-    auto fold = [&]() {
-        btotal.x += bsum.x; btotal.y += bsum.y; btotal.z += bsum.z; btotal.w += bsum.w;
-        bsum = make_float4(0.f, 0.f, 0.f, 0.f);
-    };
-    float4 ry[LO], rx[LC];
-    auto fetch = [&](long long row0) {
+            for (int i = 0; i < 2; i++) {
+                const size_t at = (size_t)(row + 64 * i) * g.n_sum + col;
+                const int left = row + 64 * i < g.n_rows ? g.n_sum - col : 0;
+                dense_load8_at<VEC>(g.a + at, left, a[i]);
+                if constexpr (MASK) dense_load8_at<VEC>(g.mask + at, left, m[i]);
+            }
+            col += 64;
+            if (col >= 64 * g.chunks) {
+                col = unit * 8;
+                row += (long long)gridDim.x * kRowsTile;
+            }
+        };
+        int b = 0, round = 0, chunk = 0, tile = 0;
+        auto split_step = [&](float4 (&a)[2][2], float4 (&m)[2][2]) {
+            if (round > 0 && !__all_sync(FGC_FULL_MASK, wait_unless(empty + 8 * b, (round - 1) & 1, s_late))) return;
+            uint32_t top = 0;
 #pragma unroll
-        for (int k = 0; k < LO; k++) {
-            const long long row = row0 + orow + k * (kDenseThreads / (BO / 4));
-            ry[k] = dense_load4<VEC>(dy, row, last, o0 + oc, n_out);
-            if (y) {
-                const float4 a = dense_load4<VEC>(y, row, last, o0 + oc, n_out);
-                // the gradient passes unless the output is at or below zero (a NaN lets it pass, as in torch)
-                if (a.x <= 0.f) ry[k].x = 0.f;
-                if (a.y <= 0.f) ry[k].y = 0.f;
-                if (a.z <= 0.f) ry[k].z = 0.f;
-                if (a.w <= 0.f) ry[k].w = 0.f;
-                if (owner && dy_masked && row < last && o0 + oc < n_out) {
-                    float *p = dy_masked + (size_t)row * n_out + o0 + oc;
-                    if constexpr (VEC) *(float4 *)p = ry[k];
-                    else {
-                        const int left = n_out - o0 - oc;
-                        p[0] = ry[k].x;
-                        if (left > 1) p[1] = ry[k].y;
-                        if (left > 2) p[2] = ry[k].z;
-                        if (left > 3) p[3] = ry[k].w;
+            for (int i = 0; i < 2; i++) {
+                if constexpr (MASK) mask8(a[i], m[i]);
+                top = max(top, split_to(s_a + b * kRowsBuffer, kRowsTile * 128, row_in + 64 * i, unit, a[i]));
+            }
+            if (top >= kUnsplit) s_bad[tile & (kRowsBad - 1)] = 1;
+            smem_to_tensor_core();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(full + 8 * b);
+            fetch(a, m);                         // (two steps ahead; beyond the last row nothing is read)
+            if (++b == g.buffers) { b = 0; round++; }
+            if (++chunk == g.chunks) { chunk = 0; tile++; }
+        };
+        float4 va[2][2][2], vm[2][2][2];
+        fetch(va[0], vm[0]);
+        fetch(va[1], vm[1]);
+        for (int step = 0; step < steps; step += 2) {
+            split_step(va[0], vm[0]);
+            if (step + 1 < steps) split_step(va[1], vm[1]);
+        }
+    } else if (w == kRowsSplit + kRowsWrite) {
+        if (lane == 0) {
+            const uint32_t desc = product_desc(NT, false), a_at = smem_at(s_a), w_at = smem_at(s_w);
+            int b = 0, round = 0, chunk = 0, tile = 0;
+            for (int step = 0; step < steps; step++) {
+                if (chunk == 0 && tile >= 2) {
+                    if (!wait_unless(read + 8 * (tile & 1), ((tile >> 1) - 1) & 1, s_late)) break;
+                    s_bad[(tile - 2) & (kRowsBad - 1)] = 0;
+                }
+                if (!wait_unless(full + 8 * b, round & 1, s_late)) break;
+                tc_after_sync();
+                const uint32_t acc = tmem + (uint32_t)((tile & 1) * 2 * NT);
+                const int left = g.n_sum - chunk * 64, parts = left >= 64 ? 4 : (left + 15) / 16;
+                tc_steps(acc, acc + NT, operand_desc(a_at + b * kRowsBuffer, 16), kRowsTile * 128, operand_desc(w_at + chunk * NT * 128, 16), w_part, 32,
+                         desc, parts, chunk > 0);
+                tc_commit(empty + 8 * b);
+                if (++b == g.buffers) { b = 0; round++; }
+                if (++chunk == g.chunks) {
+                    tc_commit(done + 8 * (tile & 1));
+                    chunk = 0;
+                    tile++;
+                }
+            }
+        }
+    } else {
+        // results: 16 columns at a time of the warp's 32 rows, through shared memory, so that four lanes write 64 bytes of a row
+        const int quarter = w & 3;
+        float *stage = s_stage + quarter * (kRowsStage / 4);
+        for (int tile = 0; tile < my_tiles; tile++) {
+            const long long row0 = ((long long)blockIdx.x + (long long)tile * gridDim.x) * kRowsTile + 32 * quarter;
+            const uint32_t acc = tmem + (uint32_t)((tile & 1) * 2 * NT) + ((uint32_t)(32 * quarter) << 16);
+            bool plain = !__all_sync(FGC_FULL_MASK, wait_unless(done + 8 * (tile & 1), (tile >> 1) & 1, s_late));
+            plain = plain || plain_all || s_bad[tile & (kRowsBad - 1)];
+            plain = __any_sync(FGC_FULL_MASK, plain);
+            tc_after_sync();
+            for (int c = 0; c < NT; c += 16) {
+                float v[16];
+                if (!plain) {
+                    uint32_t big[16], small[16];
+                    tmem_read16(acc + c, big);
+                    tmem_read16(acc + NT + c, small);
+                    tmem_wait_read();
+#pragma unroll
+                    for (int k = 0; k < 16; k++) v[k] = __uint_as_float(big[k]) + __uint_as_float(small[k]);
+                } else {
+                    const long long row = row0 + lane;
+#pragma unroll 1
+                    for (int k = 0; k < 16; k++) {
+                        float sum = 0.f;
+                        if (row < g.n_rows && col0 + c + k < g.n_cols)
+                            for (int i = 0; i < g.n_sum; i++) {
+                                float a = __ldg(g.a + (size_t)row * g.n_sum + i);
+                                if (MASK && __ldg(g.mask + (size_t)row * g.n_sum + i) <= 0.f) a = 0.f;
+                                sum = fmaf(a, __ldg(g.w + (size_t)i * g.w_sum + (size_t)(col0 + c + k) * g.w_col), sum);
+                            }
+                        stage[lane * 20 + k] = sum;
+                    }
+#pragma unroll
+                    for (int k = 0; k < 16; k++) v[k] = stage[lane * 20 + k];
+                }
+                if (g.bias) {
+#pragma unroll
+                    for (int k = 0; k < 16; k++) v[k] += col0 + c + k < g.n_cols ? __ldg(g.bias + col0 + c + k) : 0.f;
+                }
+                if (g.relu) {
+#pragma unroll
+                    for (int k = 0; k < 16; k++) v[k] = v[k] < 0.f ? 0.f : v[k];              // (NaN stays NaN, as in torch.relu)
+                }
+#pragma unroll
+                for (int k = 0; k < 4; k++)
+                    *reinterpret_cast<float4 *>(stage + lane * 20 + 4 * k) = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+                __syncwarp();
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const int r = 8 * i + (lane >> 2), cc = 4 * (lane & 3), col = col0 + c + cc;
+                    const float4 o = *reinterpret_cast<const float4 *>(stage + r * 20 + cc);
+                    if (row0 + r < g.n_rows && col < g.n_cols) {
+                        float *to = g.out + (size_t)(row0 + r) * g.n_cols + col;
+                        if (VEC && (g.n_cols & 3) == 0) *reinterpret_cast<float4 *>(to) = o;
+                        else {
+                            to[0] = o.x;
+                            if (col + 1 < g.n_cols) to[1] = o.y;
+                            if (col + 2 < g.n_cols) to[2] = o.z;
+                            if (col + 3 < g.n_cols) to[3] = o.w;
+                        }
+                    }
+                }
+                __syncwarp();
+            }
+            tc_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(read + 8 * (tile & 1));
+        }
+    }
+    tc_before_sync();
+    __syncthreads();
+    if (w == 0) {
+        tc_after_sync();
+        tmem_free(tmem, columns);
+    }
+}
+
+// Columns of a CTA: as many as fit beside the buffers, in equal shares.
+static int dense_tile_cols(int chunks, int n_cols)
+{
+    int most = (int)((227 * 1024 - dense_rows_smem(2, chunks, 0)) / (3 * chunks * 128)) / 16 * 16;
+    if (most > 128) most = 128;
+    if (most < 16) return 0;
+    const int padded = (n_cols + 15) / 16 * 16, shares = (padded + most - 1) / most;
+    return ((padded + shares - 1) / shares + 15) / 16 * 16;
+}
+
+template <bool VEC, bool MASK>
+static cudaError_t launch_rows(const DenseRows &g, cudaStream_t s)
+{
+    const size_t smem = dense_rows_smem(g.buffers, g.chunks, g.tile_cols);
+    const cudaError_t e = cudaFuncSetAttribute(k_dense_rows<VEC, MASK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    const unsigned shares = (unsigned)((g.n_cols + g.tile_cols - 1) / g.tile_cols);
+    const long long tiles = (g.n_rows + kRowsTile - 1) / kRowsTile;
+    long long ctas = sm_count() / shares;
+    if (ctas < 1) ctas = 1;
+    if (ctas > tiles) ctas = tiles;
+    k_dense_rows<VEC, MASK><<<dim3((unsigned)ctas, shares), kRowsThreads, smem, s>>>(g);
+    return cudaGetLastError();
+}
+
+static int dense_rows(DenseRows g, cudaStream_t s)
+{
+    g.chunks = (g.n_sum + 63) / 64;
+    g.tile_cols = g.chunks <= FGC_DENSE_MAX_SUM / 64 ? dense_tile_cols(g.chunks, g.n_cols) : 0;
+    if (g.tile_cols == 0) return FGC_ERR_TOO_LARGE;
+    g.buffers = dense_rows_smem(3, g.chunks, g.tile_cols) <= 227 * 1024 ? 3 : 2;
+    const bool vec = g.n_sum % 4 == 0 && (((uintptr_t)g.a | (uintptr_t)g.mask | (uintptr_t)g.out) & 15) == 0;
+    if (g.mask) return (int)(vec ? launch_rows<true, true>(g, s) : launch_rows<false, true>(g, s));
+    return (int)(vec ? launch_rows<true, false>(g, s) : launch_rows<false, false>(g, s));
+}
+
+// ----------------------------------------------------------------------------- sums over rows
+
+// Warps of a CTA: 16 load and split, eight add up, one issues products.
+constexpr int kWeightSplit = 16, kWeightAdd = 8, kWeightThreads = 32 * (kWeightSplit + kWeightAdd + 1), kWeightRows = 64;
+constexpr int kWeightChunk = 3 * kWeightRows * 128;                    // the three parts of 64 columns
+constexpr int kWeightBuffer = 4 * kWeightChunk;                        // two of the matrix with 128 columns, two of the other
+constexpr int kWeightBias = 32 * 128 * 4;                              // a thread's sums of dY
+constexpr size_t kWeightSmem = 1024 + 2 * (size_t)kWeightBuffer + kWeightBias + 128;
+static_assert(kWeightSmem <= 227 * 1024, "buffers too large");
+
+struct DenseWeight {
+    const float *x, *dy, *y;               // [n_rows, n_in], [n_rows, n_out], the same as dy or null
+    long long n_rows, rows_per_cta;
+    int n_in, n_out;
+    int tile_in, tile_out;                 // columns of a CTA, of x and of dy
+    int swap;                              // the accumulators' rows are inputs (else outputs)
+    float *dy_masked, *part_w, *part_b;
+};
+
+template <bool VEC>
+__global__ void __launch_bounds__(kWeightThreads, 1)
+k_dense_weight(const DenseWeight g)
+{
+    extern __shared__ char s_raw[];
+    char *s = s_raw + ((1024 - (smem_at(s_raw) & 1023)) & 1023);
+    float *s_bias = reinterpret_cast<float *>(s + 2 * kWeightBuffer);
+    uint64_t *s_bar = reinterpret_cast<uint64_t *>(s + 2 * kWeightBuffer + kWeightBias);
+    uint32_t *s_tmem = reinterpret_cast<uint32_t *>(s_bar + 6);
+    volatile int *s_late = reinterpret_cast<int *>(s_tmem + 1), *s_bad = s_late + 1;       // a wait that gave up; steps not to be split
+    const uint32_t full = smem_at(s_bar), done = full + 16, read = full + 32;              // two each
+    const int t = threadIdx.x, lane = t & 31, w = __shfl_sync(FGC_FULL_MASK, t >> 5, 0);
+    const int c0 = blockIdx.y * g.tile_in, o0 = blockIdx.z * g.tile_out;
+    const long long first = (long long)blockIdx.x * g.rows_per_cta, last = min(g.n_rows, first + g.rows_per_cta);
+    const int steps = first < last ? (int)((last - first + kWeightRows - 1) / kWeightRows) : 0;
+    const bool owner = blockIdx.y == 0;                        // of the mask and the bias sum
+    const int NT = ((g.swap ? g.tile_out : g.tile_in) + 15) / 16 * 16;
+    const uint32_t columns = tmem_columns(4 * NT);
+    const int n_in = min(g.n_in, c0 + g.tile_in), n_out = min(g.n_out, o0 + g.tile_out);
+    if (w == 0) tmem_alloc(smem_at(s_tmem), columns);
+    if (t == 0) {
+        for (int i = 0; i < 2; i++) {
+            mbar_init(full + 8 * i, kWeightSplit);
+            mbar_init(done + 8 * i, 1);
+            mbar_init(read + 8 * i, kWeightAdd);
+        }
+        *s_late = 0;
+        for (int i = 0; i < kRowsBad; i++) s_bad[i] = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    tc_before_sync();
+    __syncthreads();
+    tc_after_sync();
+    const uint32_t tmem = *s_tmem;
+
+    if (w < kWeightSplit) {
+        // The matrix whose columns are rows of the result comes first in a buffer.  Columns beyond a tile are not written: what is
+        // there makes rows and columns of the result that are not read.
+        const int unit = t & 15, row_in = t >> 4;              // 16 units of eight columns, 32 rows at a time
+        char *s_x = s + (g.swap ? 0 : 2 * kWeightChunk) + (unit >> 3) * kWeightChunk;
+        char *s_y = s + (g.swap ? 2 * kWeightChunk : 0) + (unit >> 3) * kWeightChunk;
+        const int x_left = n_in - c0 - unit * 8, y_left = n_out - o0 - unit * 8;
+        const bool has_x = unit * 8 < g.tile_in, has_y = unit * 8 < g.tile_out;
+        const float *px = g.x + (size_t)(first + row_in) * g.n_in + c0 + unit * 8;
+        size_t at_y = (size_t)(first + row_in) * g.n_out + o0 + unit * 8;
+        long long row = first + row_in;                        // of the next load
+        float4 vx[2][2], vy[2][2], vm[2][2];
+        float sum[8] = {};
+        float *total = s_bias + row_in * 128 + unit * 8;       // two levels, so that a thread never adds thousands of rows one to another
+        auto fold = [&]() {
+#pragma unroll
+            for (int k = 0; k < 8; k++) { total[k] += sum[k]; sum[k] = 0.f; }
+        };
+#pragma unroll
+        for (int k = 0; k < 8; k++) total[k] = 0.f;
+        auto fetch = [&]() {
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                const bool in = row + 32 * i < last;
+                if (has_x) dense_load8_at<VEC>(px + (size_t)(32 * i) * g.n_in, in ? x_left : 0, vx[i]);
+                if (has_y) dense_load8_at<VEC>(g.dy + at_y + (size_t)(32 * i) * g.n_out, in ? y_left : 0, vy[i]);
+                if (has_y && g.y) dense_load8_at<VEC>(g.y + at_y + (size_t)(32 * i) * g.n_out, in ? y_left : 0, vm[i]);
+            }
+        };
+        if (steps > 0) fetch();
+        for (int step = 0; step < steps; step++) {
+            const int b = step & 1;
+            uint32_t top = 0;
+            if (step >= 2 && !__all_sync(FGC_FULL_MASK, wait_unless(done + 8 * b, ((step >> 1) - 1) & 1, s_late))) top = kUnsplit;
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                if (has_x) top = max(top, split_to(s_x + b * kWeightBuffer, kWeightRows * 128, row_in + 32 * i, unit & 7, vx[i]));
+                if (has_y) {
+                    if (g.y) mask8(vy[i], vm[i]);
+                    const float *v = reinterpret_cast<const float *>(vy[i]);
+                    if (owner && g.dy_masked && row + 32 * i < last) {
+#pragma unroll
+                        for (int k = 0; k < 8; k++)
+                            if (k < y_left) g.dy_masked[at_y + (size_t)(32 * i) * g.n_out + k] = v[k];
+                    }
+#pragma unroll
+                    for (int k = 0; k < 8; k++) sum[k] += v[k];
+                    top = max(top, split_to(s_y + b * kWeightBuffer, kWeightRows * 128, row_in + 32 * i, unit & 7, vy[i]));
+                }
+            }
+            if (top >= kUnsplit) s_bad[step & (kRowsBad - 1)] = 1;
+            smem_to_tensor_core();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(full + 8 * b);
+            row += kWeightRows;
+            px += (size_t)kWeightRows * g.n_in;
+            at_y += (size_t)kWeightRows * g.n_out;
+            if (step + 1 < steps) fetch();
+            if ((step & 15) == 15) fold();
+        }
+        fold();
+    } else if (w == kWeightSplit + kWeightAdd) {
+        if (lane == 0) {
+            const uint32_t desc = product_desc(NT, true), s_at = smem_at(s);
+            for (int step = 0; step < steps; step++) {
+                const int b = step & 1;
+                if (step >= 2) {
+                    if (!wait_unless(read + 8 * b, ((step >> 1) - 1) & 1, s_late)) break;
+                    s_bad[(step - 2) & (kRowsBad - 1)] = 0;
+                }
+                if (!wait_unless(full + 8 * b, (step >> 1) & 1, s_late)) break;
+                tc_after_sync();
+                const uint32_t acc = tmem + (uint32_t)(b * 2 * NT), at = s_at + b * kWeightBuffer;
+                tc_steps(acc, acc + NT, operand_desc(at, kWeightChunk), kWeightRows * 128, operand_desc(at + 2 * kWeightChunk, kWeightChunk),
+                         kWeightRows * 128, 2048, desc, kWeightRows / 16, false);
+                tc_commit(done + 8 * b);
+            }
+        }
+    } else {
+        // sums of 64 rows into registers: 32 rows of the result a warp, half of the columns, one row a lane
+        float total[64] = {};
+        const int half = (w - kWeightSplit) >> 2, n_half = 64 * half;
+        const int m = 32 * (w & 3) + lane + (g.swap ? c0 : o0), n0 = n_half + (g.swap ? o0 : c0);
+        auto masked_dy = [&](long long row, int o) {
+            const float d = __ldg(g.dy + (size_t)row * g.n_out + o);
+            return g.y && __ldg(g.y + (size_t)row * g.n_out + o) <= 0.f ? 0.f : d;
+        };
+        for (int step = 0; step < steps; step++) {
+            const int b = step & 1;
+            bool plain = !wait_unless(done + 8 * b, (step >> 1) & 1, s_late) || s_bad[step & (kRowsBad - 1)];
+            plain = __any_sync(FGC_FULL_MASK, plain);
+            tc_after_sync();
+            if (!plain) {
+                const uint32_t acc = tmem + (uint32_t)(b * 2 * NT) + ((uint32_t)(32 * (w & 3)) << 16);
+#pragma unroll
+                for (int h = 0; h < 4; h++) {
+                    if (n_half + 16 * h < NT) {
+                        uint32_t big[16], small[16];
+                        tmem_read16(acc + n_half + 16 * h, big);
+                        tmem_read16(acc + NT + n_half + 16 * h, small);
+                        tmem_wait_read();
+#pragma unroll
+                        for (int k = 0; k < 16; k++) total[16 * h + k] += __uint_as_float(big[k]) + __uint_as_float(small[k]);
+                    }
+                }
+            } else {
+                const long long row0 = first + (long long)step * kWeightRows;
+                for (long long row = row0; row < min(last, row0 + kWeightRows); row++) {
+                    const float a = g.swap ? (m < n_in ? __ldg(g.x + (size_t)row * g.n_in + m) : 0.f) : (m < n_out ? masked_dy(row, m) : 0.f);
+#pragma unroll
+                    for (int k = 0; k < 64; k++) {
+                        const int n = n0 + k;
+                        const float v = g.swap ? (n < n_out ? masked_dy(row, n) : 0.f) : (n < n_in ? __ldg(g.x + (size_t)row * g.n_in + n) : 0.f);
+                        total[k] = fmaf(a, v, total[k]);
                     }
                 }
             }
-            bsum.x += ry[k].x; bsum.y += ry[k].y; bsum.z += ry[k].z; bsum.w += ry[k].w;
+            tc_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(read + 8 * b);
         }
+        float *pw = g.part_w + (size_t)blockIdx.x * g.n_out * g.n_in;
 #pragma unroll
-        for (int k = 0; k < LC; k++)
-            rx[k] = dense_load4<VEC>(x, row0 + xrow + k * (kDenseThreads / (BC / 4)), last, c0 + xc, n_in);
-    };
-    auto stage = [&](int b) {
-#pragma unroll
-        for (int k = 0; k < LO; k++) s_y[b][orow + k * (kDenseThreads / (BO / 4))][oc >> 2] = ry[k];
-#pragma unroll
-        for (int k = 0; k < LC; k++) s_x[b][xrow + k * (kDenseThreads / (BC / 4))][xc >> 2] = rx[k];
-    };
-    int b = 0, steps = 0;
-    if (first < last) {
-        fetch(first);
-        stage(0);
+        for (int k = 0; k < 64; k++) {
+            if (g.swap) {
+                if (m < n_in && n0 + k < n_out) pw[(size_t)(n0 + k) * g.n_in + m] = total[k];
+            } else {
+                if (m < n_out && n0 + k < n_in) pw[(size_t)m * g.n_in + n0 + k] = total[k];
+            }
+        }
     }
+    tc_before_sync();
     __syncthreads();
-    for (long long row0 = first; row0 < last; row0 += kDenseRows) {
-        const bool more = row0 + kDenseRows < last;
-        if ((++steps & 15) == 0) fold();
-        if (more) fetch(row0 + kDenseRows);
-#pragma unroll
-        for (int r = 0; r < kDenseRows; r++) {
-            float a[MO], v[MC];
-#pragma unroll
-            for (int k = 0; k < MO / 4; k++) {
-                const float4 f = s_y[b][r][ty + 16 * k];
-                a[4 * k] = f.x; a[4 * k + 1] = f.y; a[4 * k + 2] = f.z; a[4 * k + 3] = f.w;
-            }
-#pragma unroll
-            for (int k = 0; k < MC / 4; k++) {
-                const float4 f = s_x[b][r][tx + 16 * k];
-                v[4 * k] = f.x; v[4 * k + 1] = f.y; v[4 * k + 2] = f.z; v[4 * k + 3] = f.w;
-            }
-#pragma unroll
-            for (int i = 0; i < MO; i++)
-#pragma unroll
-                for (int j = 0; j < MC; j++) acc[i][j] = fmaf(a[i], v[j], acc[i][j]);
-        }
-        if (more) stage(b ^ 1);
-        b ^= 1;
-        __syncthreads();
+    if (w == 0) {
+        tc_after_sync();
+        tmem_free(tmem, columns);
     }
-    float *pw = part_w + (size_t)blockIdx.x * n_out * n_in;
-#pragma unroll
-    for (int i = 0; i < MO; i++) {
-        const int o = o0 + 4 * ty + 64 * (i >> 2) + (i & 3);
-#pragma unroll
-        for (int j = 0; j < MC; j++) {
-            const int c = c0 + 4 * tx + 64 * (j >> 2) + (j & 3);
-            if (o < n_out && c < n_in) pw[(size_t)o * n_in + c] = acc[i][j];
-        }
-    }
-    if (owner) {
-        // threads that loaded the same four columns, added in a fixed order
-        float4 *sb = &s_x[0][0][0];
-        fold();
-        sb[t] = btotal;
-        __syncthreads();
-        if (t < BO) {
-            float s = 0.f;
-            for (int k = 0; k < kDenseThreads / (BO / 4); k++) s += ((const float *)(sb + k * (BO / 4) + (t >> 2)))[t & 3];
-            if (o0 + t < n_out) part_b[(size_t)blockIdx.x * n_out + o0 + t] = s;
-        }
+    // threads that loaded the same columns, added in a fixed order
+    if (owner && t < g.tile_out && o0 + t < n_out) {
+        float sum = 0.f;
+        for (int k = 0; k < 32; k++) sum += s_bias[k * 128 + t];
+        g.part_b[(size_t)blockIdx.x * g.n_out + o0 + t] = sum;
     }
 }
 
@@ -224,25 +572,26 @@ k_dense_reduce(const float *__restrict__ part_w, const float *__restrict__ part_
 }
 
 struct DenseSplit {
-    int bo, bc, tiles_o, tiles_c, parts;
+    int tile_out, tile_in, tiles_out, tiles_in, parts;
     long long rows;
 };
 
-// Tiles of 64 or 128 per dimension, whichever covers it with less padding; as many row ranges as keep
-// two CTAs on every SM, but at least 64 rows each.
+// Tiles of up to 128 columns, in equal shares of whole units; as many row ranges as there are SMs for, at least 64 rows each.
 static DenseSplit dense_split(int64_t n_rows, int n_in, int n_out)
 {
     DenseSplit d;
-    d.bo = n_out <= 64 ? 64 : 128;
-    d.bc = n_in <= 64 || (n_in > 128 && n_in <= 192) ? 64 : 128;
-    d.tiles_o = (n_out + d.bo - 1) / d.bo;
-    d.tiles_c = (n_in + d.bc - 1) / d.bc;
-    const int64_t tiles = (int64_t)d.tiles_o * d.tiles_c;
-    int64_t parts = 296 / tiles;
+    auto share = [](int n, int &tiles) {
+        tiles = (n + 127) / 128;
+        return ((n + tiles - 1) / tiles + 7) / 8 * 8;
+    };
+    d.tile_out = share(n_out, d.tiles_out);
+    d.tile_in = share(n_in, d.tiles_in);
+    const int64_t tiles = (int64_t)d.tiles_out * d.tiles_in;
+    int64_t parts = sm_count() / tiles;
     if (parts < 1) parts = 1;
-    const int64_t most = (n_rows + 63) / 64;
+    const int64_t most = (n_rows + kWeightRows - 1) / kWeightRows;
     if (parts > most) parts = most < 1 ? 1 : most;
-    d.rows = ((n_rows + parts - 1) / parts + kDenseRows - 1) / kDenseRows * kDenseRows;
+    d.rows = ((n_rows + parts - 1) / parts + kWeightRows - 1) / kWeightRows * kWeightRows;
     d.parts = d.rows > 0 ? (int)((n_rows + d.rows - 1) / d.rows) : 0;
     if (d.parts < 1) d.parts = 1;
     return d;
@@ -253,16 +602,37 @@ static bool dense_args_ok(int64_t n_rows, int32_t n_in, int32_t n_out)
     return n_rows >= 0 && n_in >= 1 && n_out >= 1 && n_in <= 65535 && n_out <= 65535;
 }
 
-template <int BO, int BC>
-static void launch_dense_bwd(const DenseSplit &d, bool vec, cudaStream_t s, const float *x, const float *dy, const float *y,
-                             int64_t n_rows, int n_in, int n_out, float *dy_masked, float *part_w, float *part_b)
+}  // namespace fgc
+
+extern "C" int fgc_dense_forward(const float *x, const float *weight, const float *bias_or_null, int64_t n_rows, int32_t n_in,
+                                 int32_t n_out, int32_t relu, float *out, fgc_stream_t stream)
 {
-    const dim3 grid((unsigned)d.parts, (unsigned)d.tiles_c, (unsigned)d.tiles_o);
-    if (vec) k_dense_bwd<BO, BC, true><<<grid, kDenseThreads, 0, s>>>(x, dy, y, n_rows, n_in, n_out, d.rows, dy_masked, part_w, part_b);
-    else k_dense_bwd<BO, BC, false><<<grid, kDenseThreads, 0, s>>>(x, dy, y, n_rows, n_in, n_out, d.rows, dy_masked, part_w, part_b);
+    FGC_NVTX("fgc_dense_forward");
+    using namespace fgc;
+    if (!dense_args_ok(n_rows, n_in, n_out)) return FGC_ERR_BAD_ARGUMENT;
+    if (n_in > FGC_DENSE_MAX_SUM) return FGC_ERR_TOO_LARGE;
+    if (n_rows == 0) return FGC_OK;
+    if (!x || !weight || !out) return FGC_ERR_BAD_ARGUMENT;
+    DenseRows g = {};
+    g.a = x; g.w = weight; g.bias = bias_or_null; g.out = out; g.n_rows = n_rows;
+    g.n_sum = n_in; g.n_cols = n_out; g.w_sum = 1; g.w_col = n_in; g.relu = relu;
+    return dense_rows(g, (cudaStream_t)stream);
 }
 
-}  // namespace fgc
+extern "C" int fgc_dense_input_gradient(const float *dy, const float *y_or_null, const float *weight, int64_t n_rows, int32_t n_in,
+                                        int32_t n_out, float *dx, fgc_stream_t stream)
+{
+    FGC_NVTX("fgc_dense_input_gradient");
+    using namespace fgc;
+    if (!dense_args_ok(n_rows, n_in, n_out)) return FGC_ERR_BAD_ARGUMENT;
+    if (n_out > FGC_DENSE_MAX_SUM) return FGC_ERR_TOO_LARGE;
+    if (n_rows == 0) return FGC_OK;
+    if (!dy || !weight || !dx) return FGC_ERR_BAD_ARGUMENT;
+    DenseRows g = {};
+    g.a = dy; g.mask = y_or_null; g.w = weight; g.out = dx; g.n_rows = n_rows;
+    g.n_sum = n_out; g.n_cols = n_in; g.w_sum = n_in; g.w_col = 1;
+    return dense_rows(g, (cudaStream_t)stream);
+}
 
 extern "C" int fgc_bias_act(float *y, const float *bias, int64_t n_rows, int32_t n_out, int32_t relu, fgc_stream_t stream)
 {
@@ -301,20 +671,16 @@ extern "C" int fgc_dense_backward(const float *x, const float *dy, const float *
         return FGC_ERR_WORKSPACE;
     const DenseSplit d = dense_split(n_rows, n_in, n_out);
     cudaStream_t s = (cudaStream_t)stream;
-    float *part_w = (float *)workspace;
-    float *part_b = part_w + (size_t)d.parts * n_in * n_out;
-    const bool vec = n_in % 4 == 0 && n_out % 4 == 0 &&
-                     (((uintptr_t)x | (uintptr_t)dy | (uintptr_t)y_or_null | (uintptr_t)dy_masked_or_null) & 15) == 0;
-    if (d.bo == 64 && d.bc == 64)
-        launch_dense_bwd<64, 64>(d, vec, s, x, dy, y_or_null, n_rows, n_in, n_out, dy_masked_or_null, part_w, part_b);
-    else if (d.bo == 64)
-        launch_dense_bwd<64, 128>(d, vec, s, x, dy, y_or_null, n_rows, n_in, n_out, dy_masked_or_null, part_w, part_b);
-    else if (d.bc == 64)
-        launch_dense_bwd<128, 64>(d, vec, s, x, dy, y_or_null, n_rows, n_in, n_out, dy_masked_or_null, part_w, part_b);
-    else
-        launch_dense_bwd<128, 128>(d, vec, s, x, dy, y_or_null, n_rows, n_in, n_out, dy_masked_or_null, part_w, part_b);
+    DenseWeight g = {};
+    g.x = x; g.dy = dy; g.y = y_or_null; g.n_rows = n_rows; g.rows_per_cta = d.rows; g.n_in = n_in; g.n_out = n_out;
+    g.tile_in = d.tile_in; g.tile_out = d.tile_out; g.swap = d.tile_out <= 64 && d.tile_in > d.tile_out;
+    g.dy_masked = dy_masked_or_null; g.part_w = (float *)workspace; g.part_b = g.part_w + (size_t)d.parts * n_in * n_out;
+    const bool vec = n_in % 4 == 0 && n_out % 4 == 0 && (((uintptr_t)x | (uintptr_t)dy | (uintptr_t)y_or_null) & 15) == 0;
+    auto *const kernel = vec ? k_dense_weight<true> : k_dense_weight<false>;
+    FGC_RETURN_IF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWeightSmem));
+    kernel<<<dim3((unsigned)d.parts, (unsigned)d.tiles_in, (unsigned)d.tiles_out), kWeightThreads, kWeightSmem, s>>>(g);
     FGC_CHECK_LAUNCH();
     const long long n_w = (long long)n_in * n_out;
-    k_dense_reduce<<<(unsigned)((n_w + n_out + 31) / 32), 256, 0, s>>>(part_w, part_b, d.parts, n_w, n_out, dw, db);
+    k_dense_reduce<<<(unsigned)((n_w + n_out + 31) / 32), 256, 0, s>>>(g.part_w, g.part_b, d.parts, n_w, n_out, dw, db);
     return (int)cudaGetLastError();
 }

@@ -1,4 +1,4 @@
-"""torch.nn.Linear (and a ReLU behind it) with the library's kernels around the GEMMs.
+"""torch.nn.Linear (and a ReLU behind it) with this library's kernels.
 
 The modules stay what they are -- parameters, names, hooks, activation -- and are called as
 usual wherever the plain form is not given: see ``_plain_linear`` and ``fused_ok``.
@@ -14,7 +14,10 @@ from . import _cabi
 # with ReLU take 186 us as modules and 197 fused at 16 384 rows, 247 and 193 at 32 768, 604 and 360 at 200 000.
 min_rows = 32768
 
-# Results of this many entries or more get bias and ReLU in a pass of their own: the library's product with the bias in
+# Sums over more columns (FGC_DENSE_MAX_SUM) stay with the library.
+max_sum = 512
+
+# Products from the library: results of this many entries or more get bias and ReLU in a pass of their own: the library's product with the bias in
 # it is then slower than the plain product and the pass (forward alone, module / pass, us: 200 000 rows, 64 to 128
 # without ReLU 230 / 160, with it 264 / 161; 131 072 rows, 128 to 64 98 / 95 and 106 / 96).  Below, the pass and its
 # launch cost more than they save (200 000 rows, 128 to 10 85 / 91; 32 768 rows, 128 to 128 59 / 64).
@@ -22,12 +25,19 @@ pass_from = 1 << 23
 
 
 class _Linear(torch.autograd.Function):
-    """act(x @ weight^T + bias): GEMMs from the library, bias and ReLU in one pass over a large result, their
-    gradients and the weight's in one pass over the incoming gradient (csrc/dense.cu)."""
+    """act(x @ weight^T + bias) on the tensor cores at fp32 accuracy, forward and gradients (csrc/dense.cu); products that sum over
+    more than max_sum columns from the library, with bias and ReLU in one pass over a large result."""
 
     @staticmethod
     def forward(ctx, x, weight, bias, relu):
-        if x.shape[0] * weight.shape[0] < pass_from:
+        if max_sum >= x.shape[1]:
+            x, weight = x.contiguous(), weight.contiguous()
+            y = torch.empty((x.shape[0], weight.shape[0]), dtype=torch.float32, device=x.device)
+            with _cabi.on_device(x.device):
+                _cabi.check(_cabi.lib.fgc_dense_forward(
+                    _cabi.ptr(x), _cabi.ptr(weight), _cabi.ptr(bias.contiguous()), x.shape[0], x.shape[1], weight.shape[0], int(relu),
+                    _cabi.ptr(y), _cabi.current_stream(x.device)), "fgc_dense_forward")
+        elif x.shape[0] * weight.shape[0] < pass_from:
             y = torch.addmm(bias, x, weight.t())
             if relu:
                 y.relu_()
@@ -51,7 +61,8 @@ class _Linear(torch.autograd.Function):
         x, dy = x.contiguous(), dy.contiguous()
         n, n_in = x.shape
         n_out = dy.shape[1]
-        masked = torch.empty_like(dy) if y is not None and need_x else None
+        own = need_x and n_out <= max_sum                        # (else the library's product, of the masked gradient)
+        masked = torch.empty_like(dy) if y is not None and need_x and not own else None
         dw = torch.empty((n_out, n_in), dtype=torch.float32, device=x.device)
         db = torch.empty((n_out,), dtype=torch.float32, device=x.device)
         nbytes = _cabi.lib.fgc_dense_backward_bytes(n, n_in, n_out)
@@ -61,7 +72,14 @@ class _Linear(torch.autograd.Function):
                 _cabi.ptr(x), _cabi.ptr(dy), _cabi.ptr(y), n, n_in, n_out, _cabi.ptr(masked), _cabi.ptr(dw), _cabi.ptr(db),
                 _cabi.ptr(ws), nbytes, _cabi.current_stream(x.device)), "fgc_dense_backward")
         dx = None
-        if need_x:
+        if own:
+            dx = torch.empty_like(x)
+            weight = weight.contiguous()
+            with _cabi.on_device(x.device):
+                _cabi.check(_cabi.lib.fgc_dense_input_gradient(
+                    _cabi.ptr(dy), _cabi.ptr(y), _cabi.ptr(weight), n, n_in, n_out, _cabi.ptr(dx), _cabi.current_stream(x.device)),
+                    "fgc_dense_input_gradient")
+        elif need_x:
             dx = torch.mm(dy if masked is None else masked, weight)
         return dx, dw if need_w else None, db if need_b else None, None
 

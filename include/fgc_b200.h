@@ -564,15 +564,24 @@ int fgc_strict_batch_from_row_splits(const int64_t *row_splits, int64_t n_rs, in
                                      int64_t *out_batch, fgc_stream_t stream);
 
 /*
- * Dense layers around the message passing (torch.nn.Linear and ReLU in the reference, gnn_ops.py:60-68): the
- * products with the weight matrix stay with the caller's GEMM library.
+ * Dense layers around the message passing (torch.nn.Linear and ReLU in the reference, gnn_ops.py:60-68), fp32 matrices
+ * row by row, on the tensor cores at fp32 accuracy.
  *
+ * fgc_dense_forward: out [n_rows, n_out] = act(x weight^T + bias), weight [n_out, n_in]; act is ReLU when relu != 0.
+ * fgc_dense_input_gradient: dx [n_rows, n_in] = dY weight, with dY the gradient of a layer's output, masked where y_or_null, the
+ * output of its ReLU, is not above zero.
+ * Both sum over FGC_DENSE_MAX_SUM columns at most (n_in of the first, n_out of the second; FGC_ERR_TOO_LARGE beyond).
  * fgc_bias_act: y[row, :] = act(y[row, :] + bias), in place; act is ReLU when relu != 0.
  * fgc_dense_backward: with dY the gradient of a layer's output (masked where y_or_null, the output of
  * its ReLU, is not above zero): dw [n_out, n_in] = dY^T x, db [n_out] = column sums of dY, and the masked
  * dY itself when asked for.  Sums have a fixed order.
  * workspace: fgc_dense_backward_bytes() (0 on bad arguments), 16-byte aligned.
  */
+#define FGC_DENSE_MAX_SUM 512
+int fgc_dense_forward(const float *x, const float *weight, const float *bias_or_null, int64_t n_rows, int32_t n_in, int32_t n_out,
+                      int32_t relu, float *out, fgc_stream_t stream);
+int fgc_dense_input_gradient(const float *dy, const float *y_or_null, const float *weight, int64_t n_rows, int32_t n_in,
+                             int32_t n_out, float *dx, fgc_stream_t stream);
 int fgc_bias_act(float *y, const float *bias, int64_t n_rows, int32_t n_out, int32_t relu, fgc_stream_t stream);
 size_t fgc_dense_backward_bytes(int64_t n_rows, int32_t n_in, int32_t n_out);
 int fgc_dense_backward(const float *x, const float *dy, const float *y_or_null, int64_t n_rows, int32_t n_in,

@@ -130,3 +130,63 @@ def test_dense_layer_is_fused_only_where_it_pays():
     assert not fused(rows, 128, 10) and not fused(4 * rows, 32, 16) and not fused(4 * rows, 64, 4)
     assert not fused(rows, 384, 160) and not fused(rows, 512, 512)
     assert fused(4 * rows, 64, 64, grad=False) and not fused(rows, 128, 128, grad=False)
+
+
+@pytest.mark.parametrize("n,n_in,n_out", [(127, 63, 16), (128, 64, 17), (129, 65, 80), (148 * 128 + 1, 128, 129), (5000, 191, 96), (641, 193, 144),
+                                          (300, 512, 40), (300, 513, 40), (300, 40, 513), (63, 128, 8), (148 * 64 + 1, 8, 128)])
+def test_tensor_core_tiles_against_64_bits(monkeypatch, n, n_in, n_out):
+    """Rows, sums and columns around the tiles of 64 and 128, several shares of the columns, sums too long for the tensor cores.  The
+    three parts of a number hold all its bits and three of nine products are left out, 2^-24 of the result each at most: the bound
+    is that of a sum in fp32 (test_dense_layer_against_64_bits)."""
+    from fastgraphcompute_b200 import dense
+    monkeypatch.setattr(dense, "min_rows", 1)
+    torch.manual_seed(n + n_in)
+    lin = nn.Linear(n_in, n_out).to(DEV)
+    x = torch.randn((n, n_in), device=DEV).requires_grad_(True)
+    g = torch.randn((n, n_out), device=DEV)
+    out = dense._Linear.apply(x, lin.weight, lin.bias, True)
+    grads = torch.autograd.grad(out, [x, lin.weight, lin.bias], g)
+    xd, wd, bd = x.detach().double(), lin.weight.detach().double(), lin.bias.detach().double()
+    gd = torch.where(out.detach() <= 0, 0.0, g.double())
+    eps = 2.0 ** -24
+    for a, ref, mag, m in ((out.detach(), (xd @ wd.T + bd).relu(), xd.abs() @ wd.abs().T + bd.abs(), n_in),
+                           (grads[0], gd @ wd, gd.abs() @ wd.abs(), n_out), (grads[1], gd.T @ xd, gd.abs().T @ xd.abs(), n),
+                           (grads[2], gd.sum(0), gd.abs().sum(0), n)):
+        assert (a.double() - ref).abs().max() <= 4 * eps * (m ** 0.5 + 4) * mag.max() + 1e-30
+
+
+@pytest.mark.parametrize("where", ["x", "weight", "gradient"])
+@pytest.mark.parametrize("value", [2.0 ** 60, 3e38, float("inf"), float("nan"), 1e-30])
+def test_numbers_that_are_not_split(monkeypatch, where, value):
+    """Numbers beyond 2^60, infinities and NaN give what plain products give, in their rows and columns only; tiny ones keep their bits."""
+    from fastgraphcompute_b200 import dense
+    monkeypatch.setattr(dense, "min_rows", 1)
+    torch.manual_seed(3)
+    n, n_in, n_out = 1500, 72, 24
+    lin = nn.Linear(n_in, n_out).to(DEV)
+    x, g = torch.randn((n, n_in), device=DEV), torch.randn((n, n_out), device=DEV)
+    with torch.no_grad():
+        if where == "x":
+            x[700] = 0.0
+            x[700, 5] = value
+        elif where == "weight":
+            lin.weight[3] = 0.0
+            lin.weight[3, 7] = value
+        else:
+            g[900] = 0.0
+            g[900, 2] = value
+    xa, xb = x.clone().requires_grad_(True), x.clone().requires_grad_(True)
+    out, ref = dense._Linear.apply(xa, lin.weight, lin.bias, False), torch.addmm(lin.bias, xb, lin.weight.t())
+    # (sums that cancel are compared against their largest terms: 72 or 24 of them, or 1500, of fp32 rounding)
+    for a, b in zip((out,) + torch.autograd.grad(out, [xa, lin.weight], g), (ref,) + torch.autograd.grad(ref, [xb, lin.weight], g)):
+        a, b = a.detach(), b.detach()
+        odd = ~(torch.isfinite(b) & (b.abs() < 1e15))
+        torch.testing.assert_close(a[odd], b[odd], rtol=1e-5, atol=0.0, equal_nan=True)
+        torch.testing.assert_close(a[~odd], b[~odd], rtol=1e-4, atol=1e-4)
+    if value == 1e-30 and where == "x":
+        bias_free = (x[700].double() @ lin.weight.detach().double().t())
+        own = torch.empty((n, n_out), device=DEV)
+        from fastgraphcompute_b200 import _cabi
+        assert _cabi.lib.fgc_dense_forward(_cabi.ptr(x), _cabi.ptr(lin.weight.detach()), None, n, n_in, n_out, 0, _cabi.ptr(own),
+                                           _cabi.current_stream(x.device)) == 0
+        torch.testing.assert_close(own[700].double(), bias_free, rtol=1e-6, atol=0.0)
