@@ -93,6 +93,7 @@ SIGNATURES = {
                                       c_void_p, c_void_p, c_size, c_void_p]),
     "fgc_knn_tree_preferred": (ctypes.c_int, [c_i64, c_i32, c_i64, c_i32, c_i32]),
     "fgc_knn_groups_preferred": (ctypes.c_int, [c_i64, c_i32, c_i64, c_i32, c_i32]),
+    "fgc_knn_groups_ahead": (ctypes.c_int, [c_i64, c_i32, c_i64, c_i32, c_i32]),
     "fgc_knn_build_tree": (ctypes.c_int, [c_void_p, c_i64, c_i32, c_void_p, c_i64, c_i32, c_void_p, c_void_p, c_size,
                                           c_void_p]),
     "fgc_knn_search_tree": (ctypes.c_int, [c_i64, c_i32, c_void_p, c_i64, c_i32, c_i32, c_i32, c_void_p, c_void_p,

@@ -513,6 +513,54 @@ extern "C" int fgc_knn_groups_preferred(int64_t n_vert, int32_t n_coords, int64_
     return tree_layout(knn_workspace_layout(n_vert, n_coords, n_rs, K), n_vert, n_coords, n_rs).fits ? 1 : 0;
 }
 
+// What the search by groups has won since: with lists for eight queries it takes 0.6 to 0.8 of the time that the figures above are of.
+// Time over that of the grid, as above, in one row split / eight (mean size in brackets where it matters):
+//   three coordinates  K = 12: 1.6 M in 16 0.95 / 0.82 / 0.90 / 0.43, K = 8 1.10;  K = 16: 800 k 0.94 / 0.78 / 0.93 / 0.44, in 160 0.93 / 0.90 / 1.10 /
+//                      0.54;  K = 32: 400 k 0.93 / 0.46 / 0.90 / 0.40 and 0.92 / 0.74 / 0.99 / 0.48, K = 24 1.00; K = 40, in 80 0.82 / 0.76 / 1.05 / 0.18;
+//                      K = 48: 200 k 0.98 / 0.52 / 0.86 / 0.53 and 0.97 / 0.74 / 0.95 / 0.64, K = 40 1.01;  K = 64: 100 k 0.99 / 0.55 / 0.93 / 0.61 and
+//                      0.97 / 0.63 / 1.06 / 0.60;  K = 66: 50 k 0.83 / 0.59 / 0.82 / 0.63
+//   four               K = 12: 1.6 M in 16 0.85 / 0.74 / 0.61, K = 8 1.03;  K = 16: 400 k 0.95 / 0.43 / 0.61 and 0.90 / 0.75 / 0.76;  K = 24: 400 k in 80
+//                      0.74 / 0.78 / 1.12, 200 k 1.00 / 0.51 / 0.72 and 0.97 / 0.78 / 0.96;  K = 32: 200 k in 40 0.85 / 0.84 / 1.30;  K = 40: 100 k 0.94 /
+//                      0.48 / 0.81 and 0.89 / 0.74 / 1.01;  K = 66: 50 k 0.85 / 0.38 / 0.51
+//   five               K = 16: 200 k in one 0.83 / 0.84 / 0.89, 800 k in eight 0.80 / 1.03 / 0.90;  K = 32: 200 k in eight 0.62 / 0.99 / 1.04
+//   learned, three     K = 8: 20 k in one 0.97, 50 k 0.84;  K = 16: 50 k in ten 0.78, 200 k in 40 0.96, 10 k in one 0.82, 3 k 0.82;  K = 24: 20 k in
+//                      ten 0.92, 50 k in 25 0.84
+//   learned, four      K = 8: 50 k in ten 0.87, 200 k in 40 0.97;  K = 10: 10 k in one 0.73, 3 k 0.87;  K = 16: 20 k in ten 0.91, 50 k in 25 0.84
+// In row splits of 5000 points in 50 clusters, a hundred each, the grid is ahead by 0.1 to 0.3 of its time at K = 24 to 40.
+extern "C" int fgc_knn_groups_ahead(int64_t n_vert, int32_t n_coords, int64_t n_rs, int32_t K, int32_t long_tails)
+{
+    using namespace fgc;
+    if (n_vert < 3000 || n_vert > 0x7fffffff || n_coords < 3 || n_coords > kGroupDims || n_rs < 2 || n_rs > 0x7fffffff || K < 1 ||
+        K > FGC_MAX_K)
+        return 0;
+    const int64_t mean = n_vert / (n_rs - 1);
+    const bool large = mean >= 10000;
+    int least = FGC_MAX_K + 1;                   // shortest list
+    if (long_tails && n_coords <= 4) {
+        if (n_vert < 16384) least = mean >= 3000 ? (n_coords == 4 ? 10 : 16) : least;
+        else if (n_coords == 4) least = mean >= 4000 ? 8 : (mean >= 1500 ? 16 : least);
+        else least = mean >= 15000 ? 8 : (mean >= 4000 ? 16 : (mean >= 1500 ? 24 : least));
+    } else if (n_coords == 5) {
+        if (n_vert >= 200000) least = mean >= 100000 ? 16 : (mean >= 15000 ? 32 : least);
+    } else if (n_coords == 4) {
+        if (n_vert >= 50000) least = 66;
+        if (n_vert >= 100000 && large) least = 40;
+        if (n_vert >= 200000 && mean >= 4000) least = mean >= 20000 ? 24 : 32;
+        if (n_vert >= 400000 && mean >= 4000) least = mean >= 20000 ? 16 : 24;
+        if (n_vert >= 800000 && mean >= 4000) least = 16;
+        if (n_vert >= 1500000 && large) least = 12;
+    } else {
+        if (n_vert >= 50000) least = 66;
+        if (n_vert >= 100000 && large) least = 64;
+        if (n_vert >= 200000 && large) least = 48;
+        if (n_vert >= 400000 && mean >= 4000) least = large ? 32 : 40;
+        if (n_vert >= 800000 && mean >= 4000) least = 16;
+        if (n_vert >= 1500000 && large) least = 12;
+    }
+    if (K < least || mean < least_row_split(n_vert, K)) return 0;
+    return tree_layout(knn_workspace_layout(n_vert, n_coords, n_rs, K), n_vert, n_coords, n_rs).groups ? 1 : 0;
+}
+
 extern "C" int fgc_knn_build_tree(const float *coords, int64_t n_vert, int32_t n_coords, const int64_t *row_splits,
                                   int64_t n_rs, int32_t K, const int64_t *direction_or_null, void *workspace,
                                   size_t workspace_bytes, fgc_stream_t stream)

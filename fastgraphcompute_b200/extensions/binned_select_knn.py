@@ -48,7 +48,8 @@ def _raise_for_status(status):
 # Needs check_status (that is where the choice comes back to the host).
 grid_dims = 0
 grid_probe_every = 64
-# Search on a tree of boxes instead of a grid: None lets the library choose (fgc_knn_tree_preferred, fgc_knn_groups_preferred).
+# Search on a tree of boxes instead of a grid: None lets the library choose (fgc_knn_tree_preferred, fgc_knn_groups_preferred,
+# fgc_knn_groups_ahead).
 search_tree = None
 pad_min_pairs = 1 << 19    # backward for D = 3, 5, 6, 7: pad to four / eight coordinates from this many (row, slot) pairs on
 _grid_memory = {}        # (device, N, row splits, K[, "direction"]) -> [form, calls since the last automatic choice]
@@ -91,9 +92,10 @@ def _forward(coords, row_splits, K, direction, tf_compat, count_evals, order, lo
     grid_order = False
     if tree and search_tree is None:
         tree = False
-        if direction is None and n_vert >= 16384:           # (below, both rules say no: two calls less, 3 us)
-            tree = _cabi.lib.fgc_knn_tree_preferred(n_vert, n_coords, n_rs, K, int(long_tails)) == 1
-            if not tree and _cabi.lib.fgc_knn_groups_preferred(n_vert, n_coords, n_rs, K, int(long_tails)) == 1:
+        if direction is None and n_vert >= (3000 if long_tails else 16384):      # (below, the rules say no: calls less, 3 us)
+            size = (n_vert, n_coords, n_rs, K, int(long_tails))
+            tree = _cabi.lib.fgc_knn_tree_preferred(*size) == 1
+            if not tree and (_cabi.lib.fgc_knn_groups_ahead(*size) == 1 or _cabi.lib.fgc_knn_groups_preferred(*size) == 1):
                 tree, grid_order = True, not long_tails     # (sizes that the grid is otherwise taken for)
     ws = None
     if tree:

@@ -216,9 +216,11 @@ int fgc_knn_tree_preferred(int64_t n_vert, int32_t n_coords, int64_t n_rs, int32
 /*
  * 1 where fgc_knn_forward with FGC_FORWARD_TREE and the workspace of fgc_knn_forward_workspace_bytes was measured to be ahead
  * of the grid although fgc_knn_tree_preferred is 0: in three to five coordinates, where it takes all queries of a leaf at
- * once (fgc_knn_search_tree, and a smaller workspace, do not).
+ * once (fgc_knn_search_tree, and a smaller workspace, do not).  fgc_knn_groups_ahead: the same, with the ranges that it won when
+ * its lists were divided among eight queries.
  */
 int fgc_knn_groups_preferred(int64_t n_vert, int32_t n_coords, int64_t n_rs, int32_t K, int32_t long_tails);
+int fgc_knn_groups_ahead(int64_t n_vert, int32_t n_coords, int64_t n_rs, int32_t K, int32_t long_tails);
 int fgc_knn_build_tree(const float *coords, int64_t n_vert, int32_t n_coords, const int64_t *row_splits, int64_t n_rs,
                        int32_t K, const int64_t *direction_or_null, void *workspace, size_t workspace_bytes,
                        fgc_stream_t stream);

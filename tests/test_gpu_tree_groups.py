@@ -490,3 +490,19 @@ def test_lists_of_eight_queries(kind, sizes, D, K, flags):
     edge = gd.amax(dim=1, keepdim=True)
     inside = [torch.where((i >= 0) & (d < edge), i, torch.full_like(i, -1)).sort(dim=1).values for i, d in ((gi, gd), (ti, td))]
     assert torch.equal(*inside)
+
+
+@pytest.mark.parametrize("n,D,row_splits,K,long_tails,ahead", [
+    (49999, 3, 1, 66, 0, 0), (50000, 3, 1, 66, 0, 1), (50000, 3, 1, 65, 0, 0), (100000, 3, 10, 64, 0, 1), (100000, 3, 11, 64, 0, 0),
+    (200000, 3, 20, 48, 0, 1), (200000, 3, 20, 47, 0, 0), (400000, 3, 40, 32, 0, 1), (400000, 3, 100, 32, 0, 0), (400000, 3, 100, 40, 0, 1),
+    (800000, 3, 200, 16, 0, 1), (800000, 3, 201, 16, 0, 0), (1500000, 3, 150, 12, 0, 1), (1500000, 3, 150, 11, 0, 0),
+    (100000, 4, 10, 40, 0, 1), (200000, 4, 10, 24, 0, 1), (200000, 4, 11, 24, 0, 0), (200000, 4, 50, 32, 0, 1), (400000, 4, 20, 16, 0, 1),
+    (400000, 4, 100, 24, 0, 1), (800000, 4, 200, 16, 0, 1), (800000, 4, 200, 15, 0, 0), (50000, 4, 400, 66, 0, 0),
+    (200000, 5, 2, 16, 0, 1), (200000, 5, 3, 16, 0, 0), (200000, 5, 13, 32, 0, 1), (200000, 5, 14, 32, 0, 0),
+    (2999, 4, 1, 16, 1, 0), (3000, 4, 1, 10, 1, 1), (3000, 4, 1, 9, 1, 0), (6001, 3, 2, 16, 1, 1), (5999, 3, 2, 16, 1, 0),
+    (16384, 3, 1, 8, 1, 1), (16384, 3, 4, 15, 1, 0), (20000, 4, 5, 8, 1, 1), (20000, 4, 13, 16, 1, 1), (20000, 4, 14, 16, 1, 0),
+    (400000, 2, 1, 200, 0, 0), (400000, 6, 1, 40, 0, 0), (400000, 3, 1, 0, 0, 0), (400000, 3, 1, 258, 0, 0)])
+def test_groups_ahead_by_size(n, D, row_splits, K, long_tails, ahead):
+    """The edges of the ranges where the search by groups is ahead of the grid with its lists divided among eight queries."""
+    from fastgraphcompute_b200 import _cabi
+    assert _cabi.lib.fgc_knn_groups_ahead(n, D, row_splits + 1, K, long_tails) == ahead
