@@ -479,33 +479,43 @@ k_rank_place(const float *__restrict__ coords, int n_vert, int n_coords, int nv,
     }
 }
 
-// Step 3: the cells of the work lists.  The first n_warp_blocks CTAs take the cells that one
-// warp can sort (in registers / shared memory), the remaining CTAs take the cells beyond
-// kWarpSortMaxShared points, one CTA per cell: bitonic sort in its all-ascending form, in
-// place in global memory (the sequence is treated as padded to a power of two with
-// +infinity; a compare-exchange whose upper partner lies in the padding never swaps, so it
-// is simply skipped).  After the sort the same warp / CTA places the cell's points.
-constexpr int kSortWarps = 4;
+// Step 3: the cells of the work lists.  The first n_warp_blocks CTAs take the cells that one warp can sort (in registers /
+// shared memory), the others those beyond kWarpSortMaxShared points, one CTA per cell.  The ids of a cell are different numbers of
+// one row split: a bit for each in shared memory, and the place of an id is the number of bits before it -- three passes over the
+// cell whatever its size, where a sorting network in global memory took hundreds (a second look at 800 k skewed points whose
+// largest cell holds some 50 k: 1.36 -> 0.1 ms).  Ids that span more than the bits go through them a window at a time.  After the
+// sort the same warp / CTA places the cell's points.
+constexpr int kSortWarps = 16;
+constexpr int kSortShared = kSortWarps * kWarpSortMaxShared * (int)sizeof(int);       // of the warps
+constexpr int kSortMostBits = 96 * 1024 * 8;
+
+// Bytes for the bits of n_vert ids (two CTAs an SM).
+static int sort_shared_bytes(int64_t n_vert)
+{
+    const int64_t bytes = (n_vert < kSortMostBits ? n_vert + 31 : kSortMostBits) / 32 * 4;
+    return bytes > kSortShared ? (int)bytes : kSortShared;
+}
 
 __global__ void __launch_bounds__(kSortWarps * 32)
 k_sort_large_cells(const float *__restrict__ coords, int n_coords, int nv,
                    const int64_t *__restrict__ direction, const KnnGrid *__restrict__ g,
                    const int *__restrict__ bounds, const int *__restrict__ biglist,
-                   const int *__restrict__ hugelist, int n_warp_blocks,
+                   const int *__restrict__ hugelist, int n_warp_blocks, const int *__restrict__ stmp, int n_words,
                    int *__restrict__ sorig, float4 *__restrict__ scoords, int *__restrict__ sbin,
                    uint8_t *__restrict__ sflag)
 {
     chain_wait();
     chain_release();
-    __shared__ int s_keys[kSortWarps][kWarpSortMaxShared];
+    extern __shared__ int s_sort[];
+    __shared__ int s_part[kSortWarps], s_low, s_high;
     if (g->status != 0) return;
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     if ((int)blockIdx.x < n_warp_blocks) {
-        const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
         const int n_big = g->n_big_cells;
         for (int w = blockIdx.x * kSortWarps + wib; w < n_big; w += n_warp_blocks * kSortWarps) {
             const int cell = biglist[w];
             const int beg = bounds[cell], n = bounds[cell + 1] - beg;
-            warp_sort_segment(sorig + beg, n, s_keys[wib], lane);
+            warp_sort_segment(sorig + beg, n, s_sort + wib * kWarpSortMaxShared, lane);
             __syncwarp();
             for (int t = lane; t < n; t += 32)
                 place_point(beg + t, sorig[beg + t], grid_cell(g, cell), coords, n_coords, nv, direction, sorig, scoords,
@@ -519,33 +529,61 @@ k_sort_large_cells(const float *__restrict__ coords, int n_coords, int nv,
     for (int w = blockIdx.x - n_warp_blocks; w < n_huge; w += n_cta) {
         const int cell = hugelist[w];
         const int beg = bounds[cell], n = bounds[cell + 1] - beg;
-        int *seg = sorig + beg;
-        int P = 1;
-        while (P < n) P <<= 1;
-        for (int k = 2; k <= P; k <<= 1) {
-            // flip: element i of a block of k against its mirror image
-            for (int t = threadIdx.x; t < P / 2; t += blockDim.x) {
-                const int half = k >> 1, blk = t / half, off = t - blk * half;
-                const int a = blk * k + off, b = blk * k + (k - 1 - off);
-                if (b < n) {
-                    const int ka = seg[a], kb = seg[b];
-                    if (ka > kb) { seg[a] = kb; seg[b] = ka; }
-                }
+        if (threadIdx.x == 0) { s_low = 0x7fffffff; s_high = 0; }
+        __syncthreads();
+        int low = 0x7fffffff, high = 0;
+        for (int t = threadIdx.x; t < n; t += blockDim.x) {
+            const int v = stmp[beg + t];
+            low = min(low, v);
+            high = max(high, v);
+        }
+        low = __reduce_min_sync(FGC_FULL_MASK, low);
+        high = __reduce_max_sync(FGC_FULL_MASK, high);
+        if (lane == 0) { atomicMin(&s_low, low); atomicMax(&s_high, high); }
+        __syncthreads();
+        low = s_low;
+        high = s_high;
+        int done = 0;                                          // ids of earlier windows
+        for (long long first = low; first <= high; first += 32ll * n_words) {
+            const int words = (int)min((long long)n_words, (high - first) / 32 + 1);
+            for (int i = threadIdx.x; i < words; i += blockDim.x) s_sort[i] = 0;
+            __syncthreads();
+            for (int t = threadIdx.x; t < n; t += blockDim.x) {
+                const long long off = (long long)stmp[beg + t] - first;
+                if (off >= 0 && off < 32ll * words) atomicOr(s_sort + (int)(off >> 5), 1 << (int)(off & 31));
             }
             __syncthreads();
-            for (int j = k >> 2; j > 0; j >>= 1) {
-                for (int t = threadIdx.x; t < P / 2; t += blockDim.x) {
-                    const int a = 2 * j * (t / j) + (t % j), b = a + j;
-                    if (b < n) {
-                        const int ka = seg[a], kb = seg[b];
-                        if (ka > kb) { seg[a] = kb; seg[b] = ka; }
-                    }
-                }
-                __syncthreads();
+            // a run of words per thread, an exclusive scan of their counts, then the ids of the run in order
+            const int run = (words + (int)blockDim.x - 1) / (int)blockDim.x;
+            const int i0 = min(words, (int)threadIdx.x * run), i1 = min(words, i0 + run);
+            int count = 0;
+            for (int i = i0; i < i1; i++) count += __popc(s_sort[i]);
+            int before = count;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int x = __shfl_up_sync(FGC_FULL_MASK, before, o);
+                if (lane >= o) before += x;
             }
+            if (lane == 31) s_part[wib] = before;
+            before -= count;
+            __syncthreads();
+            int total = 0;
+#pragma unroll
+            for (int k = 0; k < kSortWarps; k++) {
+                if (k == wib) before += total;
+                total += s_part[k];
+            }
+            int at = done + before;
+            for (int i = i0; i < i1; i++) {
+                for (uint32_t bits = (uint32_t)s_sort[i]; bits; bits &= bits - 1, at++) {
+                    if (FGC_DBG_OK(at >= 0 && at < n, (int *)&g->status)) sorig[beg + at] = (int)(first + 32ll * i + __ffs(bits) - 1);
+                }
+            }
+            done += total;
+            __syncthreads();
         }
         for (int t = threadIdx.x; t < n; t += blockDim.x)
-            place_point(beg + t, seg[t], grid_cell(g, cell), coords, n_coords, nv, direction, sorig, scoords, sbin, sflag);
+            place_point(beg + t, sorig[beg + t], grid_cell(g, cell), coords, n_coords, nv, direction, sorig, scoords, sbin, sflag);
         __syncthreads();
     }
 }
@@ -728,10 +766,12 @@ static int knn_build_grid(const float *coords, int64_t n_vert, int32_t n_coords,
     FGC_RETURN_IF_CUDA(launch_chained(k_fill_ids, pt_blocks, 256, 0, s, n, grid, counts, pbin, prank, stmp));
     FGC_RETURN_IF_CUDA(launch_chained(k_rank_place, pt_blocks, 256, 0, s, coords, n, n_coords, L.nv, direction_or_null,
                                       grid, counts, pbin, prank, stmp, sorig, scoords, sbin, sflag, biglist, hugelist));
-    const int n_warp_blocks = fgc::sm_count() * 4;
-    FGC_RETURN_IF_CUDA(launch_chained(k_sort_large_cells, n_warp_blocks + fgc::sm_count(), kSortWarps * 32, 0, s, coords,
-                                      n_coords, L.nv, direction_or_null, grid, counts, biglist, hugelist, n_warp_blocks,
-                                      sorig, scoords, sbin, sflag));
+    const int n_warp_blocks = fgc::sm_count(), sort_bytes = sort_shared_bytes(n_vert);
+    if (sort_bytes > 48 * 1024)
+        FGC_RETURN_IF_CUDA(cudaFuncSetAttribute(k_sort_large_cells, cudaFuncAttributeMaxDynamicSharedMemorySize, sort_bytes));
+    FGC_RETURN_IF_CUDA(launch_chained(k_sort_large_cells, n_warp_blocks + fgc::sm_count() / 2, kSortWarps * 32, sort_bytes, s, coords,
+                                      n_coords, L.nv, direction_or_null, grid, counts, biglist, hugelist, n_warp_blocks, stmp,
+                                      sort_bytes / 4, sorig, scoords, sbin, sflag));
     return FGC_OK;
 }
 

@@ -506,3 +506,27 @@ def test_groups_ahead_by_size(n, D, row_splits, K, long_tails, ahead):
     """The edges of the ranges where the search by groups is ahead of the grid with its lists divided among eight queries."""
     from fastgraphcompute_b200 import _cabi
     assert _cabi.lib.fgc_knn_groups_ahead(n, D, row_splits + 1, K, long_tails) == ahead
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,cloud", [(3000, 513), (40000, 2000), (1000000, 70000)])
+def test_large_cells_are_in_order(n, cloud):
+    """The grid's cells beyond 512 points: ids ascending inside a cell (a cloud smaller than a cell lies in eight at most), ids that span
+    more than one window of bits (786 432), and the rows that follow."""
+    km = importlib.import_module("fastgraphcompute_b200.extensions.binned_select_knn")
+    g = torch.Generator().manual_seed(n)
+    x = torch.rand((n, 3), generator=g)
+    inside = torch.randperm(n, generator=g)[:cloud]
+    x[inside] = 0.3 + 1e-7 * torch.randint(0, 64, (cloud, 3), generator=g)
+    x, rs = x.to(DEV), torch.tensor([0, n], device=DEV)
+    runs = [_forward(km, x, rs, 9, False) for _ in range(2)]
+    assert torch.equal(runs[0][0], runs[1][0]) and torch.equal(runs[0][1], runs[1][1])
+    order = km.cell_order(runs[0][2], n, 3, 2, 9).long()
+    assert torch.equal(order.sort().values, torch.arange(n, device=DEV))
+    mark = torch.zeros(n, dtype=torch.bool, device=DEV)
+    mark[inside.to(DEV)] = True
+    ids = order[mark[order]]
+    assert int((ids[1:] < ids[:-1]).sum()) <= 7
+    assert km.read_counters(runs[0][2])[0][7] >= 1
+    _, dist, _ = _forward(km, x, rs, 9, True)
+    assert torch.equal(dist.sort(dim=1).values, runs[0][1].sort(dim=1).values)
