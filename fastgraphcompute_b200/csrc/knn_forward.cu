@@ -5,6 +5,7 @@
 // wait for the status word happens without the interpreter (two row splits of 5000 points, K = 16, forward and
 // backward, B200, timed in turn: 196 -> 168 us; a GravNet layer on ten small events: 303 -> 289 us).
 #include <mutex>
+#include <thread>
 
 #include "knn_tree.cuh"
 
@@ -15,11 +16,12 @@ namespace fgc {
 // by all threads: a thread that ends frees nothing (freeing page-locked memory may wait for the device, and breaks another
 // thread's graph capture).  At most kKeptSlots stay for later calls, i.e. 4 KB.
 struct StatusSlot {
-    int32_t *words = nullptr;
+    int32_t *words = nullptr;          // written as one
     cudaEvent_t ready = nullptr;
     int device = -1;
 };
 constexpr size_t kKeptSlots = 64;
+constexpr int64_t kNoWords = -1;               // (a status has no sign)
 
 struct StatusPool {
     std::mutex lock;
@@ -92,15 +94,16 @@ static int knn_forward_launch(const float *coords, int64_t n_vert, int32_t n_coo
 {
     const bool tree = (flags & FGC_FORWARD_TREE) != 0;
     int rc;
+    bool done = false;                     // status words and cell order are written by the build
     if (tree) rc = fgc_knn_build_tree(coords, n_vert, n_coords, row_splits, n_rs, K, direction, ws, ws_bytes, stream);
     else {
         const int dims = flags & FGC_SEARCH_GRID3 ? 3 : (flags & FGC_SEARCH_GRID4 ? 4 : 0);
-        rc = fgc_knn_build_grid_dims(coords, n_vert, n_coords, row_splits, n_rs, K, direction, target_occupancy, dims, ws,
-                                     ws_bytes, stream);
+        rc = knn_build_grid_forward(coords, n_vert, n_coords, row_splits, n_rs, K, direction, target_occupancy, dims,
+                                    status ? status->words : nullptr, out_order, &done, ws, ws_bytes, stream);
     }
     if (rc != FGC_OK) return rc;
     if (status) {
-        rc = fgc_knn_publish_grid_info(ws, status->words, stream);
+        if (!done) rc = fgc_knn_publish_grid_info(ws, status->words, stream);
         if (rc != FGC_OK) return rc;
         *published = true;
         FGC_RETURN_IF_CUDA(cudaEventRecord(status->ready, (cudaStream_t)stream));
@@ -121,7 +124,7 @@ static int knn_forward_launch(const float *coords, int64_t n_vert, int32_t n_coo
                              (flags & (FGC_SEARCH_COUNT | FGC_SEARCH_GRID3 | FGC_SEARCH_GRID4)) | FGC_SEARCH_FRESH, out_idx,
                              out_distsq, ws, ws_bytes, stream);
     if (rc != FGC_OK) return rc;
-    if (out_order && n_vert > 0)
+    if (out_order && n_vert > 0 && !done)
         FGC_RETURN_IF_CUDA(cudaMemcpyAsync(out_order, fgc_knn_cell_order(ws, n_vert, n_coords, n_rs, K),
                                            sizeof(int32_t) * (size_t)n_vert, cudaMemcpyDeviceToDevice, (cudaStream_t)stream));
     if (ties && n_vert > 0) {
@@ -154,6 +157,7 @@ extern "C" int fgc_knn_forward(const float *coords, int64_t n_vert, int32_t n_co
                                   stream);
     StatusSlot slot;
     FGC_RETURN_IF_CUDA(take_slot(slot));
+    *(volatile int64_t *)slot.words = kNoWords;
     bool published = false;
     int rc = knn_forward_launch(coords, n_vert, n_coords, row_splits, n_rs, K, direction_or_null, tf_compat, target_occupancy,
                                 flags, out_idx, out_distsq, out_order_or_null, workspace, workspace_bytes, &slot, &published,
@@ -162,12 +166,19 @@ extern "C" int fgc_knn_forward(const float *coords, int64_t n_vert, int32_t n_co
         give_back(slot);
         return rc;
     }
-    // (also after an error of a later launch: the words are on their way)
-    const cudaError_t e = cudaEventSynchronize(slot.ready);
-    if (rc == FGC_OK) rc = (int)e;
+    // The words are on their way (also after an error of a later launch), and here long before the build has ended: looked for until the
+    // event behind the build says that it has.
+    volatile int64_t *const words = (volatile int64_t *)slot.words;
+    cudaError_t e = cudaErrorNotReady;
+    for (int i = 1; *words == kNoWords && e == cudaErrorNotReady; i++)
+        if (i % 1024 == 0) {
+            if (i > 1 << 17) std::this_thread::yield();
+            e = cudaEventQuery(slot.ready);
+        }
+    if (*words == kNoWords && rc == FGC_OK) rc = e == cudaSuccess ? (int)cudaErrorUnknown : (int)e;
     if (rc == FGC_OK) {
-        info_host_or_null[0] = ((volatile int32_t *)slot.words)[0];
-        info_host_or_null[1] = ((volatile int32_t *)slot.words)[1];
+        info_host_or_null[0] = (int32_t)*words;
+        info_host_or_null[1] = (int32_t)(*words >> 32);
     }
     // after an error the event may not stand for these words: the slot is not used again
     if (rc == FGC_OK) give_back(slot);

@@ -1,7 +1,8 @@
 // binned_select_knn forward for sm_100a, part 1: the search grid (this file) --
 // part 2, the search itself, is knn_search.cu.
 //
-// Pipeline (all on the caller's stream, no host synchronisation; 9 launches, 11 while the
+// Pipeline (batches of up to kSmallBuild points take the same passes in one launch, knn_grid_small.cu; all on the
+// caller's stream, no host synchronisation; 9 launches, 11 while the
 // device still has to choose the grid's form for D = 4):
 //   k_minmax_setup  fused finite check + min/max of the binned coordinates; clears the cell
 //                 table; its last CTA validates the row splits and chooses cell width / grid
@@ -33,7 +34,7 @@
 // dimensions in order with one rounding per operation.  The visiting order, the
 // grid and the stopping rule are this library's own; they never change which
 // points are nearest, only which of several equidistant points is kept.
-#include "knn_grid.cuh"
+#include "knn_grid_build.cuh"
 #include "knn_tree.cuh"
 #include "shell_table.cuh"
 
@@ -42,9 +43,6 @@ namespace fgc {
 // ---------------------------------------------------------------------------
 // grid construction
 // ---------------------------------------------------------------------------
-
-__device__ void grid_setup(KnnGrid *g, const int64_t *__restrict__ row_splits, int n_rs, int n_vert,
-                           int n_bin_dims, int bins_target, int bins_cap_first, int bins_cap, int bad_rs, int mirror);
 
 // Before the grid of a second look: an empty header and tickets where there are rows to search again, else a
 // status word that ends the kernels of the grid at once.
@@ -138,180 +136,17 @@ k_minmax_setup(const float *__restrict__ coords, int n_vert, int n_coords, int n
     bad_rs = __syncthreads_or(bad_rs);
     if (threadIdx.x == 0) {
         g->stat_blocks_done = 0;       // the density pass counts its CTAs with the same ticket
-        if (mirror > 1) {
-            const unsigned long long n_may = atomicExch(&g->sum_sq, 0ull);
-            if (8 * n_may >= 7 * (unsigned long long)n_vert) {
-                // (nearly) all points: one set, which may have twice the cells
-                mirror = 1;
-                bins_cap *= 2;
-            } else if (adaptive) {
-                // cells sized for the points that are met in a walk; not below a third of the points, so that the cells of
-                // the others stay small enough to be put in order
-                bins_target = (int)(bins_target * fmax((double)n_may / (double)n_vert, 1.0 / 3.0) + 0.5);
-            }
+        if (mirror > 1) choose_sets(atomicExch(&g->sum_sq, 0ull), n_vert, adaptive, mirror, bins_target, bins_cap);
+        uint32_t min_key[4], max_key[4];
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            min_key[c] = atomicMax(&g->min_key[c], 0u);
+            max_key[c] = atomicMax(&g->max_key[c], 0u);
         }
-        grid_setup(g, row_splits, n_rs, n_vert, n_bin_dims, bins_target, bins_cap_first, bins_cap, bad_rs, mirror);
+        if (row_splits[0] != 0 || row_splits[n_rs - 1] != (int64_t)n_vert) bad_rs = 1;
+        grid_setup(g, min_key, max_key, atomicOr(&g->nonfinite, 0u) != 0, n_rs, n_bin_dims, bins_target, bins_cap_first, bins_cap, bad_rs,
+                   mirror);
     }
-}
-
-// Cells per dimension for a wanted cell width; widens the cells until the table fits.
-__device__ inline void fit_shape(const float (&ext)[4], double wd, int bins_cap, int (&n)[4], float &w)
-{
-    for (int iter = 0; iter < 400; iter++) {
-        w = (float)wd;
-        const float inv = __fdiv_rn(1.0f, w);
-        double prod = 1.0;
-        for (int gd = 0; gd < 4; gd++) {
-            n[gd] = ext[gd] > 0.f ? (int)floorf(__fmul_rn(ext[gd], inv)) + 1 : 1;
-            prod *= (double)n[gd];
-        }
-        if (prod <= (double)bins_cap) break;
-        wd *= 1.05;
-    }
-}
-
-// One thread.  Chooses the cell width so that a row split of average size gets
-// about bins_target cells, bounded by bins_cap cells per row split.
-__device__ void grid_setup(KnnGrid *g, const int64_t *__restrict__ row_splits, int n_rs, int n_vert,
-                           int n_bin_dims, int bins_target, int bins_cap_first, int bins_cap, int bad_rs, int mirror)
-{
-    int status = 0;
-    if (atomicOr(&g->nonfinite, 0u)) status |= FGC_STATUS_NONFINITE;
-    if (bad_rs || row_splits[0] != 0 || row_splits[n_rs - 1] != (int64_t)n_vert)
-        status |= FGC_STATUS_BAD_ROW_SPLITS;
-    const int n_events = n_rs - 1;
-    const int G = n_bin_dims >= 4 ? 4 : 3;      // grid dimensions in use
-    const int sh = G - n_bin_dims;
-    float ext[4];
-    double vol = 1.0;
-    int nz = 0;
-    float ext_max = 0.f;
-    for (int gd = 0; gd < 4; gd++) {
-        if (gd >= G) {
-            g->cdim[gd] = -1;
-            g->origin[gd] = 0.f;
-            ext[gd] = 0.f;
-        } else if (gd < sh || (status & FGC_STATUS_NONFINITE)) {
-            g->cdim[gd] = gd < sh ? -1 : gd - sh;
-            g->origin[gd] = 0.f;
-            ext[gd] = 0.f;
-        } else {
-            const int c = gd - sh;
-            const float lo = ordered_to_float(~atomicMax(&g->min_key[c], 0u));
-            const float hi = ordered_to_float(atomicMax(&g->max_key[c], 0u));
-            g->cdim[gd] = c;
-            g->origin[gd] = lo;
-            ext[gd] = __fsub_rn(hi, lo);
-            if (!(ext[gd] >= 0.f) || !is_finite_bits(ext[gd])) ext[gd] = 0.f;
-        }
-        if (ext[gd] > 0.f) { vol *= (double)ext[gd]; nz++; }
-        ext_max = fmaxf(ext_max, ext[gd]);
-    }
-    int n[4] = {1, 1, 1, 1};
-    float w = 1.f;
-    if (nz > 0) {
-        if (bins_target < 1) bins_target = 1;
-        double wd = pow(vol / (double)bins_target, 1.0 / (double)nz);
-        // a degenerate extent ratio can make the width underflow: keep it representable
-        if (!(wd > (double)ext_max * 1e-6)) wd = (double)ext_max * 1e-6;
-        fit_shape(ext, wd, bins_cap_first, n, w);
-    }
-    long long B = (long long)n[0] * n[1] * n[2] * n[3];
-    if (B > bins_cap_first) {  // cannot happen after the loop above unless the extents are absurd
-        n[0] = n[1] = n[2] = n[3] = 1; B = 1; w = fmaxf(ext_max, 1.f) * 2.f;
-        status |= FGC_STATUS_INTERNAL;
-    }
-    g->n[0] = n[0]; g->n[1] = n[1]; g->n[2] = n[2]; g->n[3] = n[3];
-    g->gdims = G;
-    g->B = (int)B;
-    g->n_events = n_events;
-    g->mirror = mirror;
-    g->total_bins = (int)(B * n_events * mirror);
-    grid_set_divisors(g);
-    g->w = w;
-    g->inv_w = __fdiv_rn(1.0f, w);
-    g->slack = 4e-6f * fmaxf(ext_max, w);
-    g->ext[0] = ext[0]; g->ext[1] = ext[1]; g->ext[2] = ext[2]; g->ext[3] = ext[3];
-    g->bins_cap = bins_cap;
-    g->status = status;
-}
-
-// Density pass.  The first grid is sized from the bounding box, i.e. from the MEAN density.
-// Clustered data puts most points into cells far above that mean, and the cost of a query
-// grows with the occupancy of the cells around it.  sum_c c^2 / N is the occupancy a typical
-// point sees in its own cell; when it is well above the wanted value the grid is rebuilt
-// with cells shrunk by the cube root of the ratio (occupancy scales with the cell volume
-// where the density is locally smooth).
-// pass 0: the density pass on the first grid.  pass 1: a second one, only after pass 0 fell
-// back from a grid over four coordinates to one over three (D = 4 only): a dense cell table
-// over the four-dimensional bounding box cannot follow strongly clustered data -- the wanted
-// cell size would need far more cells than the table holds -- so data that asks for cells more
-// than 2.8x finer than the mean density suggests is binned in three coordinates, where the
-// same table reaches the wanted size.
-__device__ void grid_refine(KnnGrid *g, unsigned long long sum_sq, int n_vert, float seen_target,
-                            float seen_target3, int bins_target3, int pass, int allow_fallback)
-{
-    const float target = pass == 0 ? seen_target : seen_target3;
-    const double seen = (double)sum_sq / (double)(n_vert > 0 ? n_vert : 1);
-    if (!(seen > 1.5 * (double)target)) return;
-    int nz = 0;
-    float ext[4], ext_max = 0.f;
-    for (int gd = 0; gd < 4; gd++) {
-        ext[gd] = g->ext[gd];
-        if (ext[gd] > 0.f) nz++;
-        ext_max = fmaxf(ext_max, ext[gd]);
-    }
-    if (nz == 0) return;
-    double shrink = pow((double)target / seen, 1.0 / (double)nz);
-    int n[4] = {1, 1, 1, 1};
-    float w = g->w;
-    if (pass == 0 && allow_fallback && g->gdims == 4 && shrink < 0.36) {
-        g->gdims = 3;
-        g->cdim[3] = -1; g->origin[3] = 0.f; g->ext[3] = 0.f;
-        ext[3] = 0.f;
-        double vol = 1.0;
-        nz = 0; ext_max = 0.f;
-        for (int gd = 0; gd < 3; gd++) {
-            if (ext[gd] > 0.f) { vol *= (double)ext[gd]; nz++; }
-            ext_max = fmaxf(ext_max, ext[gd]);
-        }
-        if (nz > 0) {
-            double wd = pow(vol / (double)(bins_target3 < 1 ? 1 : bins_target3), 1.0 / (double)nz);
-            if (!(wd > (double)ext_max * 1e-6)) wd = (double)ext_max * 1e-6;
-            fit_shape(ext, wd, g->bins_cap, n, w);
-        } else {
-            w = 1.f;
-        }
-        const long long B3 = (long long)n[0] * n[1] * n[2];
-        g->n[0] = n[0]; g->n[1] = n[1]; g->n[2] = n[2]; g->n[3] = 1;
-        g->B = (int)B3;
-        g->total_bins = (int)(B3 * g->n_events * g->mirror);
-        grid_set_divisors(g);
-        g->w = w;
-        g->inv_w = __fdiv_rn(1.0f, w);
-        g->slack = 4e-6f * fmaxf(ext_max, w);
-        g->fallback3 = 1;
-        g->refined = 1;
-        g->sum_sq = 0;              // the second density pass starts from scratch
-        g->stat_blocks_done = 0;
-        return;
-    }
-    // Never more than 2.2x: data that mixes very dense clusters with a thin background
-    // would otherwise pay with long walks through empty cells for the background queries.
-    if (shrink < 1.0 / 2.2) shrink = 1.0 / 2.2;
-    double wd = (double)g->w * shrink;
-    if (!(wd > (double)ext_max * 1e-6)) wd = (double)ext_max * 1e-6;
-    fit_shape(ext, wd, g->bins_cap, n, w);
-    const long long B = (long long)n[0] * n[1] * n[2] * n[3];
-    if (B > g->bins_cap || !(w < g->w)) return;
-    g->n[0] = n[0]; g->n[1] = n[1]; g->n[2] = n[2]; g->n[3] = n[3];
-    g->B = (int)B;
-    g->total_bins = (int)(B * g->n_events * g->mirror);
-    grid_set_divisors(g);
-    g->w = w;
-    g->inv_w = __fdiv_rn(1.0f, w);
-    g->slack = 4e-6f * fmaxf(ext_max, w);
-    g->refined = pass + 1;
 }
 
 __global__ void __launch_bounds__(256)
@@ -323,15 +158,6 @@ k_zero_counts(int *__restrict__ counts, const KnnGrid *g, int stage)
     const int n = g->total_bins + 1;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         counts[i] = 0;
-}
-
-// Cell coordinate of a shifted coordinate; identical in every kernel that needs it.
-__device__ __forceinline__ int cell_of(float x, float origin, float inv_w, int n)
-{
-    const float t = __fsub_rn(x, origin);
-    int b = (int)floorf(__fmul_rn(t, inv_w));
-    b = b < 0 ? 0 : b;
-    return b >= n ? n - 1 : b;
 }
 
 // refine_pass >= 0: the kernel is also the density pass of that number.  A point that arrives
@@ -355,16 +181,7 @@ k_histogram(const float *__restrict__ coords, int n_vert, int n_coords,
     bool candidate = true;
     unsigned long long sq = 0;
     if (live) {
-        const float *row = coords + (size_t)v * n_coords;
-        int b[4];
-#pragma unroll
-        for (int gd = 0; gd < 4; gd++) {
-            const int c = g->cdim[gd];
-            b[gd] = c < 0 ? 0 : cell_of(__ldg(row + c), g->origin[gd], g->inv_w, g->n[gd]);
-        }
-        const int e = row_split_of(row_splits, n_rs, v);
-        // the fourth dimension has one cell (b[3] = 0) in a grid over three coordinates
-        flat = e * g->B + ((b[0] * g->n[1] + b[1]) * g->n[2] + b[2]) * g->n[3] + b[3];
+        flat = point_cell(g, coords + (size_t)v * n_coords, row_split_of(row_splits, n_rs, v));
         if (g->mirror > 1) {
             const int64_t d = direction[v];
             candidate = d != 1 && d != 2;
@@ -419,30 +236,6 @@ k_fill_ids(int n_vert, const KnnGrid *__restrict__ g, const int *__restrict__ bo
     if (FGC_DBG_OK(pos >= 0 && pos < n_vert, &g->status)) stmp[pos] = v;
 }
 
-// Everything that is kept per point in cell order: original id, coordinates padded to
-// float4, cell id, direction flag.
-__device__ __forceinline__ void place_point(int pos, int v, int bin, const float *__restrict__ coords,
-                                            int n_coords, int nv, const int64_t *__restrict__ direction,
-                                            int *__restrict__ sorig, float4 *__restrict__ scoords,
-                                            int *__restrict__ sbin, uint8_t *__restrict__ sflag)
-{
-    const float *row = coords + (size_t)v * n_coords;
-    for (int q = 0; q < nv; q++) {
-        float4 o;
-        o.x = 4 * q + 0 < n_coords ? __ldg(row + 4 * q + 0) : 0.f;
-        o.y = 4 * q + 1 < n_coords ? __ldg(row + 4 * q + 1) : 0.f;
-        o.z = 4 * q + 2 < n_coords ? __ldg(row + 4 * q + 2) : 0.f;
-        o.w = 4 * q + 3 < n_coords ? __ldg(row + 4 * q + 3) : 0.f;
-        scoords[(size_t)pos * nv + q] = o;
-    }
-    sorig[pos] = v;
-    sbin[pos] = bin;
-    if (direction) {
-        const int64_t d = direction[v];
-        sflag[pos] = (d >= 0 && d <= 2) ? (uint8_t)d : (uint8_t)3;
-    }
-}
-
 // Step 2: the ids inside every cell in ascending order, so that the cell-ordered layout --
 // and with it the order in which the search visits candidates, its choice among equidistant
 // candidates and the slot order of its output -- is the same on every run.  One thread per
@@ -479,16 +272,6 @@ k_rank_place(const float *__restrict__ coords, int n_vert, int n_coords, int nv,
     }
 }
 
-// Step 3: the cells of the work lists.  The first n_warp_blocks CTAs take the cells that one warp can sort (in registers /
-// shared memory), the others those beyond kWarpSortMaxShared points, one CTA per cell.  The ids of a cell are different numbers of
-// one row split: a bit for each in shared memory, and the place of an id is the number of bits before it -- three passes over the
-// cell whatever its size, where a sorting network in global memory took hundreds (a second look at 800 k skewed points whose
-// largest cell holds some 50 k: 1.36 -> 0.1 ms).  Ids that span more than the bits go through them a window at a time.  After the
-// sort the same warp / CTA places the cell's points.
-constexpr int kSortWarps = 16;
-constexpr int kSortShared = kSortWarps * kWarpSortMaxShared * (int)sizeof(int);       // of the warps
-constexpr int kSortMostBits = 96 * 1024 * 8;
-
 // Bytes for the bits of n_vert ids (two CTAs an SM).
 static int sort_shared_bytes(int64_t n_vert)
 {
@@ -496,9 +279,12 @@ static int sort_shared_bytes(int64_t n_vert)
     return bytes > kSortShared ? (int)bytes : kSortShared;
 }
 
+// Step 3: the cells of the work lists.  The first n_warp_blocks CTAs take the cells that one warp can sort (in registers /
+// shared memory), the others those beyond kWarpSortMaxShared points, one CTA per cell.  After the sort the same warp / CTA
+// places the cell's points.
 __global__ void __launch_bounds__(kSortWarps * 32)
 k_sort_large_cells(const float *__restrict__ coords, int n_coords, int nv,
-                   const int64_t *__restrict__ direction, const KnnGrid *__restrict__ g,
+                   const int64_t *__restrict__ direction, KnnGrid *__restrict__ g,
                    const int *__restrict__ bounds, const int *__restrict__ biglist,
                    const int *__restrict__ hugelist, int n_warp_blocks, const int *__restrict__ stmp, int n_words,
                    int *__restrict__ sorig, float4 *__restrict__ scoords, int *__restrict__ sbin,
@@ -507,7 +293,6 @@ k_sort_large_cells(const float *__restrict__ coords, int n_coords, int nv,
     chain_wait();
     chain_release();
     extern __shared__ int s_sort[];
-    __shared__ int s_part[kSortWarps], s_low, s_high;
     if (g->status != 0) return;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     if ((int)blockIdx.x < n_warp_blocks) {
@@ -529,59 +314,7 @@ k_sort_large_cells(const float *__restrict__ coords, int n_coords, int nv,
     for (int w = blockIdx.x - n_warp_blocks; w < n_huge; w += n_cta) {
         const int cell = hugelist[w];
         const int beg = bounds[cell], n = bounds[cell + 1] - beg;
-        if (threadIdx.x == 0) { s_low = 0x7fffffff; s_high = 0; }
-        __syncthreads();
-        int low = 0x7fffffff, high = 0;
-        for (int t = threadIdx.x; t < n; t += blockDim.x) {
-            const int v = stmp[beg + t];
-            low = min(low, v);
-            high = max(high, v);
-        }
-        low = __reduce_min_sync(FGC_FULL_MASK, low);
-        high = __reduce_max_sync(FGC_FULL_MASK, high);
-        if (lane == 0) { atomicMin(&s_low, low); atomicMax(&s_high, high); }
-        __syncthreads();
-        low = s_low;
-        high = s_high;
-        int done = 0;                                          // ids of earlier windows
-        for (long long first = low; first <= high; first += 32ll * n_words) {
-            const int words = (int)min((long long)n_words, (high - first) / 32 + 1);
-            for (int i = threadIdx.x; i < words; i += blockDim.x) s_sort[i] = 0;
-            __syncthreads();
-            for (int t = threadIdx.x; t < n; t += blockDim.x) {
-                const long long off = (long long)stmp[beg + t] - first;
-                if (off >= 0 && off < 32ll * words) atomicOr(s_sort + (int)(off >> 5), 1 << (int)(off & 31));
-            }
-            __syncthreads();
-            // a run of words per thread, an exclusive scan of their counts, then the ids of the run in order
-            const int run = (words + (int)blockDim.x - 1) / (int)blockDim.x;
-            const int i0 = min(words, (int)threadIdx.x * run), i1 = min(words, i0 + run);
-            int count = 0;
-            for (int i = i0; i < i1; i++) count += __popc(s_sort[i]);
-            int before = count;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int x = __shfl_up_sync(FGC_FULL_MASK, before, o);
-                if (lane >= o) before += x;
-            }
-            if (lane == 31) s_part[wib] = before;
-            before -= count;
-            __syncthreads();
-            int total = 0;
-#pragma unroll
-            for (int k = 0; k < kSortWarps; k++) {
-                if (k == wib) before += total;
-                total += s_part[k];
-            }
-            int at = done + before;
-            for (int i = i0; i < i1; i++) {
-                for (uint32_t bits = (uint32_t)s_sort[i]; bits; bits &= bits - 1, at++) {
-                    if (FGC_DBG_OK(at >= 0 && at < n, (int *)&g->status)) sorig[beg + at] = (int)(first + 32ll * i + __ffs(bits) - 1);
-                }
-            }
-            done += total;
-            __syncthreads();
-        }
+        sort_cell_by_cta(beg, n, stmp, sorig, s_sort, n_words, &g->status);
         for (int t = threadIdx.x; t < n; t += blockDim.x)
             place_point(beg + t, sorig[beg + t], grid_cell(g, cell), coords, n_coords, nv, direction, sorig, scoords, sbin, sflag);
         __syncthreads();
@@ -594,8 +327,7 @@ __global__ void k_publish_grid_info(const KnnGrid *__restrict__ g, volatile int3
     chain_wait();
     chain_release();
     if (threadIdx.x == 0 && blockIdx.x == 0) {
-        info_mapped[0] = g->status;
-        info_mapped[1] = g->gdims + 16 * g->fallback3;
+        store_info(info_mapped, g->status, g->gdims + 16 * g->fallback3);
         __threadfence_system();
     }
 }
@@ -664,7 +396,8 @@ namespace fgc {
 
 static int knn_build_grid(const float *coords, int64_t n_vert, int32_t n_coords, const int64_t *row_splits, int64_t n_rs,
                           int32_t K, const int64_t *direction_or_null, float target_occupancy, int32_t grid_dims,
-                          bool only_for_ties, void *workspace, size_t workspace_bytes, fgc_stream_t stream)
+                          bool only_for_ties, int32_t *info_mapped, int32_t *out_order, bool *done, void *workspace,
+                          size_t workspace_bytes, fgc_stream_t stream)
 {
     if (grid_dims != 0 && grid_dims != 3 && grid_dims != 4) return FGC_ERR_BAD_ARGUMENT;
     KnnWorkspace L;
@@ -674,10 +407,11 @@ static int knn_build_grid(const float *coords, int64_t n_vert, int32_t n_coords,
     cudaStream_t s = (cudaStream_t)stream;
     char *ws = (char *)workspace;
     KnnGrid *grid = (KnnGrid *)(ws + L.header);
+    const bool small = !only_for_ties && n_vert > 0 && n_vert <= kSmallBuild;
     if (only_for_ties)
         FGC_RETURN_IF_CUDA(launch_chained(k_tie_gate, 1, 256, 0, s, grid, (const KnnTree *)(ws + L.tickets),
                                           (int)(n_vert / kTieShare)));
-    else
+    else if (!small)
         FGC_RETURN_IF_CUDA(cudaMemsetAsync(grid, 0, kGridHeaderBytes + kHardTicketBytes, s));   // header and k_knn_hard's tickets
     if (n_vert == 0) return FGC_OK;
     if (!coords || n_rs < 2) return FGC_ERR_BAD_ARGUMENT;
@@ -738,11 +472,23 @@ static int knn_build_grid(const float *coords, int64_t n_vert, int32_t n_coords,
     const int scan_blocks = (int)ceil_div64(max_entries, kScanTile);
     int bins_cap_first = bins_target > (bins_cap - 64) / 4 ? bins_cap : 4 * bins_target + 64;
     if (!adaptive) bins_cap_first = bins_cap;
+    const int allow_fallback = adaptive && n_coords == 4 && forced == 0;
+    if (small) {
+        GridBuild b = {};
+        b.coords = coords; b.row_splits = row_splits; b.direction = direction_or_null; b.grid = grid;
+        b.counts = counts; b.stmp = stmp; b.sorig = sorig; b.sbin = sbin; b.biglist = biglist; b.hugelist = hugelist;
+        b.sflag = sflag; b.scoords = scoords; b.n_vert = n; b.n_coords = n_coords; b.nv = L.nv; b.n_rs = (int)n_rs; b.n_bin_dims = n_bin_dims;
+        b.mirror = mirror; b.bins_target = bins_target; b.bins_cap_first = bins_cap_first; b.bins_cap = bins_cap; b.adaptive = adaptive;
+        b.allow_fallback = allow_fallback; b.seen_target = seen_target; b.seen_target3 = seen_target3; b.out_order = out_order;
+        b.info_mapped = info_mapped;
+        FGC_RETURN_IF_CUDA(launch_small_build(b, s));
+        if (done) *done = true;
+        return FGC_OK;
+    }
     k_minmax_setup<<<red_blocks, 256, 0, s>>>(coords, n, n_coords, n_bin_dims, direction_or_null, grid, counts,
                                               (long long)bins_cap_first * n_events * mirror + 1, row_splits, (int)n_rs,
                                               bins_target, bins_cap_first, bins_cap, mirror, adaptive, only_for_ties);
     FGC_CHECK_LAUNCH();
-    const int allow_fallback = adaptive && n_coords == 4 && forced == 0;
     FGC_RETURN_IF_CUDA(launch_chained(k_histogram, pt_blocks, 256, 0, s, coords, n, n_coords, row_splits, (int)n_rs, direction_or_null,
                                       grid, counts, pbin, prank, 0, adaptive ? 0 : -1, seen_target, seen_target3,
                                       bins_target, allow_fallback));
@@ -785,7 +531,17 @@ extern "C" int fgc_knn_build_grid_dims(const float *coords, int64_t n_vert, int3
 {
     FGC_NVTX("fgc_knn_build_grid_dims");
     return fgc::knn_build_grid(coords, n_vert, n_coords, row_splits, n_rs, K, direction_or_null, target_occupancy, grid_dims,
-                               false, workspace, workspace_bytes, stream);
+                               false, nullptr, nullptr, nullptr, workspace, workspace_bytes, stream);
+}
+
+int fgc::knn_build_grid_forward(const float *coords, int64_t n_vert, int32_t n_coords, const int64_t *row_splits, int64_t n_rs,
+                                int32_t K, const int64_t *direction_or_null, float target_occupancy, int32_t grid_dims,
+                                int32_t *info_mapped, int32_t *out_order, bool *done, void *workspace, size_t workspace_bytes,
+                                fgc_stream_t stream)
+{
+    FGC_NVTX("fgc_knn_build_grid_dims");
+    return knn_build_grid(coords, n_vert, n_coords, row_splits, n_rs, K, direction_or_null, target_occupancy, grid_dims, false,
+                          info_mapped, out_order, done, workspace, workspace_bytes, stream);
 }
 
 int fgc::knn_build_grid_for_ties(const float *coords, int64_t n_vert, int32_t n_coords, const int64_t *row_splits,
@@ -794,7 +550,7 @@ int fgc::knn_build_grid_for_ties(const float *coords, int64_t n_vert, int32_t n_
 {
     FGC_NVTX("fgc_knn_build_grid_for_ties");
     return knn_build_grid(coords, n_vert, n_coords, row_splits, n_rs, K, direction_or_null, target_occupancy, 0, true,
-                          workspace, workspace_bytes, stream);
+                          nullptr, nullptr, nullptr, workspace, workspace_bytes, stream);
 }
 
 extern "C" const int32_t *fgc_knn_cell_order(const void *workspace, int64_t n_vert, int32_t n_coords,

@@ -197,6 +197,12 @@ inline KnnWorkspace knn_workspace_layout(int64_t n_vert, int n_coords, int64_t n
     return w;
 }
 
+// fgc_knn_build_grid_dims; small batches write the two words of fgc_knn_publish_grid_info and the cell order on the way (*done is set then).
+int knn_build_grid_forward(const float *coords, int64_t n_vert, int32_t n_coords, const int64_t *row_splits, int64_t n_rs,
+                           int32_t K, const int64_t *direction_or_null, float target_occupancy, int32_t grid_dims,
+                           int32_t *info_mapped, int32_t *out_order, bool *done, void *workspace, size_t workspace_bytes,
+                           fgc_stream_t stream);
+
 // Argument checks shared by the kNN entry points.
 inline int check_knn_args(int64_t n_vert, int32_t n_coords, int64_t n_rs, int32_t K,
                           const void *workspace, size_t workspace_bytes, KnnWorkspace *L)

@@ -69,3 +69,54 @@ def test_radius_filter_entry_point_in_place():
     a, b = idx.clone(), dist.clone()          # no radius: untouched
     assert _cabi.lib.fgc_knn_radius_filter(_cabi.ptr(a), _cabi.ptr(b), 3, 5, -1.0, 0, st) == 0
     assert torch.equal(a, idx) and torch.equal(b, dist)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sizes,D,K", [([1], 3, 4), ([0, 2, 0], 2, 3), ([512, 513], 3, 9), ([4096], 4, 17), ([4097, 1], 4, 40), ([16384], 3, 16),
+                                       ([16385], 3, 16), ([7] * 600, 3, 5), ([3000, 2000], 6, 20), ([9000, 0, 7000], 4, 66)])
+@pytest.mark.parametrize("kind", ["uniform", "clusters"])
+@pytest.mark.parametrize("flags", [False, True])
+def test_grid_of_a_small_batch(sizes, D, K, kind, flags):
+    """The build in one launch and the chain beyond 16384 points: tiles of 4096 threads, row splits beyond those kept in shared memory
+    (512), cells of more than 32 and 512 points, four coordinates that fall back to three, direction flags; the same rows twice, and
+    the cell order a permutation that the backward may use."""
+    import importlib
+    import parity
+    from oracle import oracle
+    km = importlib.import_module("fastgraphcompute_b200.extensions.binned_select_knn")
+    g = torch.Generator().manual_seed(sum(sizes) + D)
+    n = sum(sizes)
+    x = torch.rand((n, D), generator=g)
+    if kind == "clusters":
+        x = torch.where(torch.rand((n, 1), generator=g) < 0.9, 0.2 + 0.002 * torch.randn((n, D), generator=g), x)
+        x[: n // 3] = 0.5
+    rs = torch.tensor([0] + sizes).cumsum(0)
+    direction = torch.randint(0, 4, (n,), generator=g) if flags else None
+    old = km.search_tree
+    try:
+        km.search_tree = False
+        found = [km.knn_forward_with_order(x.cuda(), rs.cuda(), K, None if direction is None else direction.cuda(), False) for _ in range(3)]
+    finally:
+        km.search_tree = old
+    oi, od = oracle.binned_select_knn(K, x.numpy(), rs.numpy(), direction=None if direction is None else direction.numpy())
+    for idx, dist, order in found:
+        parity.assert_knn_parity(idx.cpu().numpy(), dist.cpu().numpy(), oi, od, what="small grid")
+        assert torch.equal(order.long().sort().values.cpu(), torch.arange(n))
+    # (D = 4: the first call lets the device choose the form of the grid, the others ask for it)
+    assert torch.equal(found[1][0], found[2][0]) and torch.equal(found[1][1], found[2][1]) and torch.equal(found[1][2], found[2][2])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [300, 16384, 20000])
+def test_bad_input_of_a_small_batch(n):
+    from fastgraphcompute_b200 import binned_select_knn
+    x = torch.rand((n, 3), device="cuda")
+    x[n - 1, 1] = float("nan")
+    with pytest.raises(RuntimeError, match="non-finite"):
+        binned_select_knn(5, x, torch.tensor([0, n], device="cuda"))
+    x[n - 1, 1] = 0.0
+    for bad in ([1, n], [0, n - 1], [0, n, n - 2, n]):
+        with pytest.raises(RuntimeError, match="row_splits"):
+            binned_select_knn(5, x, torch.tensor(bad, device="cuda"))
+    idx, _ = binned_select_knn(5, x, torch.tensor([0, n], device="cuda"))
+    assert int(idx.min()) >= 0
