@@ -4,7 +4,7 @@
 // selection, and walking the levels of the tree) is paid once for 32.
 //
 //  k_tree_groups  One warp per leaf.  The points of the leaves nearest to its own are counted by distance for every query
-//                 (32 classes, eight to a factor of two); the class in which the K-th falls gives an upper bound on its K-th
+//                 (40 classes, eight to a factor of two); the class in which the K-th falls gives an upper bound on its K-th
 //                 distance.  |c|^2 - 2 c.q + |q|^2, with coordinates relative to the leaf, is a product of 32 queries x 32 points
 //                 over two more places than there are coordinates: a few matrix instructions in tf32, |c|^2 in two parts.
 //                 The bound is widened by what rounding can add, so it stays an upper bound.  Then the leaves whose box is
@@ -78,15 +78,17 @@ __device__ __forceinline__ float box_box_sq(const float4 (&lo)[NV], const float4
 
 // ----------------------------------------------------------------------------- bounds and lists
 
-constexpr int kHistClasses = 32;
+constexpr int kHistClasses = 40;
 // Leaves that the bound is taken from: more make it tighter.
 // Measured with 5 / 8 / 12 / 16 / 24 / 36 of them (400 k points, whole forward, ms): uniform in three coordinates, K = 16 0.67 / 0.67 /
 // 0.69 / 0.71 / 0.76 / 0.82, K = 64 1.15 / 1.07 / 1.04 / 1.05 / 1.09 / 1.18, K = 200 6.3 / 2.6 / 2.3 / 2.23 / 2.18 / 2.22; four learned
 // coordinates, K = 40 2.06 / 1.94 / 1.89 / 1.88 / 1.93 / 1.98; five, normal, K = 40 8.4 / 7.8 / 7.3 / 7.2 / 7.1 / 7.1.
-constexpr int kSeedNodes = 4;
+// They are looked for in so many nodes: with eight instead of four 1.6 M learned points in four coordinates, K = 40 take 4.8 instead of 5.0 ms, a million
+// normal ones in five 12.3 instead of 13.2, with twelve leaves more 12.0; in three 6.4 M uniform ones, K = 64 10.6 instead of 10.3.
+__host__ __device__ constexpr int seed_nodes(int dims) { return dims <= 3 ? 4 : 8; }
 __device__ __forceinline__ int seed_leaves(int kn, int dims)
 {
-    return min(6 + kn / 6, 26) + (dims >= 4 ? 6 : 0) + (dims >= 5 ? 6 : 0);
+    return min(6 + kn / 6, 26) + (dims >= 4 ? 8 : 0) + (dims >= 5 ? 12 : 0);
 }
 
 // An upper bound on the distance d of a point c from q whose |c|^2 - 2 c.q + |q|^2 comes out as t or less (coordinates relative to
@@ -116,7 +118,8 @@ template <int NV, int DC>
 __device__ __forceinline__ void bound_leaf(const TreeArgs &a, const int slot)
 {
     static_assert(DC + 2 <= 8, "one matrix product over coordinates and |c|^2 twice");
-    constexpr int CHUNKS = (DC + 3) / 4;
+    constexpr int CHUNKS = (DC + 3) / 4, NODES = seed_nodes(DC);
+    static_assert(NODES <= 8, "three bits of a key");
     // classes of the counting, then the list of leaves
     __shared__ __align__(16) int s_hist[tree_list_cap(DC) > 32 * (kHistClasses + 1) ? tree_list_cap(DC) : 32 * (kHistClasses + 1)];
     __shared__ float s_part[4][2 * 4 * NV + 1];                 // boxes of eight queries, the largest bound among them
@@ -198,20 +201,21 @@ __device__ __forceinline__ void bound_leaf(const TreeArgs &a, const int slot)
         for (int i = lane; i < 32 * (kHistClasses + 1); i += 32) s_hist[i] = 0;
         // Classes are the upper bits of a distance: eight to a factor of two, the last one and what is beyond it without an
         // end.  The K-th distance of a point in a leaf of 32 is a tenth to a half of the leaf's squared diagonal at K =
-        // 16 to 128 and more at a border: four factors of two up to twice it, less for short lists.  The last class begins below
+        // 16 to 128, less in more coordinates and more at a border: five factors of two up to twice it, less for short lists (with four the
+        // first class was the K-th's for most points in five coordinates: a million normal ones, K = 40 13.7 -> 13.2 ms).  The last class begins below
         // kNotThere, so that what is no candidate is never counted below it, however large the leaf.
         const float share = kn >= 63 ? 2.f : 2.f * powf((float)(kn + 1) * (1.f / 64.f), 2.f / DC);
         const int last = (int)min(__float_as_uint(share * diag), 0x7e800000u) >> 20;
         const int first = max(last - (kHistClasses - 1), 0);
         // the nearest leaves of the nearest nodes
         const int own_node = own_leaf >> 5, node0 = own_node & ~31;
-        uint32_t nkey = kNoBox, lkey[kSeedNodes];
-        int node_of[kSeedNodes];
+        uint32_t nkey = kNoBox, lkey[NODES];
+        int node_of[NODES];
         if (node0 + lane < n_node)
             nkey = node0 + lane == own_node ? (uint32_t)lane
                    : ((__float_as_uint(box_box_sq<NV>(mid, mid, node_box + (size_t)(node0 + lane) * (2 * NV))) & ~31u) | (uint32_t)lane);
 #pragma unroll
-        for (int k = 0; k < kSeedNodes; k++) {
+        for (int k = 0; k < NODES; k++) {
             const uint32_t m = __reduce_min_sync(FGC_FULL_MASK, nkey);
             lkey[k] = kNoBox;
             node_of[k] = node0 + (int)(m & 31u);
@@ -219,7 +223,7 @@ __device__ __forceinline__ void bound_leaf(const TreeArgs &a, const int slot)
                 if (lane == (int)(m & 31u)) nkey = kNoBox;
                 const int leaf = node_of[k] * 32 + lane;
                 if (leaf < n_leaf)
-                    lkey[k] = (__float_as_uint(box_box_sq<NV>(mid, mid, leaf_box + (size_t)leaf * (2 * NV))) & ~127u) |
+                    lkey[k] = (__float_as_uint(box_box_sq<NV>(mid, mid, leaf_box + (size_t)leaf * (2 * NV))) & ~255u) |
                               (uint32_t)(k << 5 | lane);
             }
         }
@@ -227,13 +231,13 @@ __device__ __forceinline__ void bound_leaf(const TreeArgs &a, const int slot)
         auto next_seed = [&]() -> int {
             uint32_t m = lkey[0];
 #pragma unroll
-            for (int k = 1; k < kSeedNodes; k++) m = min(m, lkey[k]);
+            for (int k = 1; k < NODES; k++) m = min(m, lkey[k]);
             m = __reduce_min_sync(FGC_FULL_MASK, m);
             if (m == kNoBox) return -1;
-            const int src = (int)(m & 31u), from = (int)(m >> 5 & 3u);
+            const int src = (int)(m & 31u), from = (int)(m >> 5 & 7u);
             int node = node_of[0];
 #pragma unroll
-            for (int k = 0; k < kSeedNodes; k++) {
+            for (int k = 0; k < NODES; k++) {
                 if (k == from) {
                     if (lane == src) lkey[k] = kNoBox;
                     node = node_of[k];
