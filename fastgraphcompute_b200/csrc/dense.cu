@@ -5,8 +5,8 @@
 //
 //   k_dense_rows    out = act(A W + b) for 128 rows at a time: a forward, or an input gradient with A the incoming gradient, masked
 //                   by the layer's output on the way.  A CTA keeps the weight, split into three parts, in shared memory and
-//                   goes through tiles of rows, 64 columns a step: sixteen warps load two steps ahead into registers, split and write
-//                   to one of three buffers, one thread issues the products of a step, four warps write the results of a tile
+//                   goes through tiles of rows, 64 columns a step: sixteen warps load one or two steps ahead into registers, split and write
+//                   to one of three buffers, one thread issues the products of a step, eight warps write the results of a tile
 //                   while the next one is formed (two sets of accumulators in TMEM).
 //   k_dense_weight  dW = dY^T x and db: a CTA goes through a range of rows, 64 at a time, which are M- and N-major operands as
 //                   they are.  The accumulators of every 64 rows are added to fp32 registers, so that no sum is
@@ -16,12 +16,15 @@
 //
 // Tiles with numbers that cannot be split (infinities, NaN, 2^60 and more) are computed by scalar operations.
 //
-// Forward and backward with ReLU, us, modules / library products with passes of our own for bias, mask and dW / now: 200 k rows, 128 to 128
-// 1018 / 640 / 318; 64 to 128 884 / 440 / 287; 1.6 M rows, 128 to 64 3156 / 2300 / 1577.  Relative error against 64 bits, library / now:
-// forward 2.0e-7 / 1.2e-7, input gradient 1.4e-7 / 0.8e-7, dW 1.1e-6 (3.5e-7 summed in fp32 by 148 CTAs) / 1.4e-7.
+// Kernels with ReLU, us (read and written once): 200 k rows, 128 to 128: forward 59 (31), input gradient 71 (47), dW 106 (47); 1.6 M rows, 128 to
+// 64: 270 (188), 391 (250), 476 (250).  Forward and backward of the first, modules / library products with passes of our own for bias,
+// mask and dW / now: 1018 / 640 / 270.  Relative error against 64 bits, library / now: forward 2.0e-7 / 1.2e-7, input gradient 1.4e-7 / 0.8e-7,
+// dW 1.1e-6 (3.5e-7 summed in fp32 by 148 CTAs) / 1.4e-7.
 //
-// k_dense_rows (200 k rows, 128 to 128: 80 us; read and written once it would be 31): latency between splitting warps and the loads two
-// steps ahead, tensor pipe 0.26.  k_dense_weight (126 us; 47): one step of loads ahead, 3 M instructions an SM to split and add up.
+// What bounds them is the latency of the splitting warps between loads and buffers (0.35 of the issue slots, tensor pipe 0.25).  With four warps instead of
+// eight to write results a forward took 80 instead of 59 us (they read, added and wrote one sixteen of columns after the other); with
+// loads of a whole step issued when the last one had been split dW took 126 instead of 106, and 105 instead of 60 for 64 to 64,
+// where half of the threads had no columns.
 #include "tensor_core.cuh"
 
 namespace fgc {
@@ -104,13 +107,13 @@ struct DenseRows {
     int relu;
     int chunks, tile_cols, buffers;        // 64 numbers of the sum each; columns of a CTA; steps that are split ahead
 };
-// Warps of a CTA: 16 load and split, four write results, one issues products.
-constexpr int kRowsSplit = 16, kRowsWrite = 4, kRowsThreads = 32 * (kRowsSplit + kRowsWrite + 1), kRowsTile = 128;
+// Warps of a CTA: 16 load and split, eight write results, one issues products.
+constexpr int kRowsSplit = 16, kRowsWrite = 8, kRowsThreads = 32 * (kRowsSplit + kRowsWrite + 1), kRowsTile = 128;
 constexpr int kRowsBuffer = 3 * kRowsTile * 128, kRowsStage = 32 * 20 * 4;
 constexpr int kRowsBad = 8;                // tiles that splitting may be ahead of writing: five
 inline size_t dense_rows_smem(int buffers, int chunks, int tile_cols)
 {
-    return 1024 + buffers * (size_t)kRowsBuffer + 3 * (size_t)chunks * tile_cols * 128 + kRowsWrite * (size_t)kRowsStage + 256;
+    return 1024 + buffers * (size_t)kRowsBuffer + 3 * (size_t)chunks * tile_cols * 128 + kRowsWrite * (size_t)kRowsStage + 128 * 4 + 256;
 }
 
 template <bool VEC, bool MASK>
@@ -122,7 +125,8 @@ k_dense_rows(const DenseRows g)
     char *s_a = s, *s_w = s + g.buffers * kRowsBuffer;
     const int w_part = g.chunks * g.tile_cols * 128;
     float *s_stage = reinterpret_cast<float *>(s_w + 3 * w_part);
-    uint64_t *s_bar = reinterpret_cast<uint64_t *>(reinterpret_cast<char *>(s_stage) + kRowsWrite * kRowsStage);
+    float *s_bias = s_stage + kRowsWrite * (kRowsStage / 4);                               // of the CTA's columns
+    uint64_t *s_bar = reinterpret_cast<uint64_t *>(s_bias + 128);
     uint32_t *s_tmem = reinterpret_cast<uint32_t *>(s_bar + 10);
     volatile int *s_late = reinterpret_cast<int *>(s_tmem + 1), *s_bad = s_late + 1;       // a wait that gave up; tiles not to be split
     const uint32_t bar = smem_at(s_bar), full = bar, empty = bar + 24, done = bar + 48, read = bar + 64;
@@ -143,6 +147,7 @@ k_dense_rows(const DenseRows g)
         for (int i = 0; i < kRowsBad; i++) s_bad[i] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    if (t < NT) s_bias[t] = g.bias && col0 + t < g.n_cols ? __ldg(g.bias + col0 + t) : 0.f;
     // the weight: row n of the operand is output column col0 + n
     uint32_t most = 0;
     for (int i = t; i < g.chunks * NT * 8; i += kRowsThreads) {
@@ -169,14 +174,13 @@ k_dense_rows(const DenseRows g)
         const int row_in = t >> 3, unit = t & 7;               // of the two passes of 64 rows over a tile
         long long row = (long long)blockIdx.x * kRowsTile + row_in;          // of the next load
         int col = unit * 8;
-        auto fetch = [&](float4 (&a)[2][2], float4 (&m)[2][2]) {
-#pragma unroll
-            for (int i = 0; i < 2; i++) {
-                const size_t at = (size_t)(row + 64 * i) * g.n_sum + col;
-                const int left = row + 64 * i < g.n_rows ? g.n_sum - col : 0;
-                dense_load8_at<VEC>(g.a + at, left, a[i]);
-                if constexpr (MASK) dense_load8_at<VEC>(g.mask + at, left, m[i]);
-            }
+        auto fetch = [&](int i, float4 (&a)[2][2], float4 (&m)[2][2]) {
+            const size_t at = (size_t)(row + 64 * i) * g.n_sum + col;
+            const int left = row + 64 * i < g.n_rows ? g.n_sum - col : 0;
+            dense_load8_at<VEC>(g.a + at, left, a[i]);
+            if constexpr (MASK) dense_load8_at<VEC>(g.mask + at, left, m[i]);
+        };
+        auto advance = [&]() {
             col += 64;
             if (col >= 64 * g.chunks) {
                 col = unit * 8;
@@ -184,6 +188,7 @@ k_dense_rows(const DenseRows g)
             }
         };
         int b = 0, round = 0, chunk = 0, tile = 0;
+        // (a register is loaded again as soon as it has been split; beyond the last row nothing is read)
         auto split_step = [&](float4 (&a)[2][2], float4 (&m)[2][2]) {
             if (round > 0 && !__all_sync(FGC_FULL_MASK, wait_unless(empty + 8 * b, (round - 1) & 1, s_late))) return;
             uint32_t top = 0;
@@ -191,21 +196,29 @@ k_dense_rows(const DenseRows g)
             for (int i = 0; i < 2; i++) {
                 if constexpr (MASK) mask8(a[i], m[i]);
                 top = max(top, split_to(s_a + b * kRowsBuffer, kRowsTile * 128, row_in + 64 * i, unit, a[i]));
+                fetch(i, a, m);
             }
+            advance();
             if (top >= kUnsplit) s_bad[tile & (kRowsBad - 1)] = 1;
             smem_to_tensor_core();
             __syncwarp();
             if (lane == 0) mbar_arrive(full + 8 * b);
-            fetch(a, m);                         // (two steps ahead; beyond the last row nothing is read)
             if (++b == g.buffers) { b = 0; round++; }
             if (++chunk == g.chunks) { chunk = 0; tile++; }
         };
-        float4 va[2][2][2], vm[2][2][2];
-        fetch(va[0], vm[0]);
-        fetch(va[1], vm[1]);
-        for (int step = 0; step < steps; step += 2) {
-            split_step(va[0], vm[0]);
-            if (step + 1 < steps) split_step(va[1], vm[1]);
+        // loads two steps ahead, or one with a mask, for want of registers
+        constexpr int AHEAD = MASK ? 1 : 2;
+        float4 va[AHEAD][2][2], vm[AHEAD][2][2];
+#pragma unroll
+        for (int k = 0; k < AHEAD; k++) {
+            fetch(0, va[k], vm[k]);
+            fetch(1, va[k], vm[k]);
+            advance();
+        }
+        for (int step = 0; step < steps; step += AHEAD) {
+#pragma unroll
+            for (int k = 0; k < AHEAD; k++)
+                if (step + k < steps) split_step(va[k], vm[k]);
         }
     } else if (w == kRowsSplit + kRowsWrite) {
         if (lane == 0) {
@@ -232,9 +245,10 @@ k_dense_rows(const DenseRows g)
             }
         }
     } else {
-        // results: 16 columns at a time of the warp's 32 rows, through shared memory, so that four lanes write 64 bytes of a row
-        const int quarter = w & 3;
-        float *stage = s_stage + quarter * (kRowsStage / 4);
+        // Results of the warp's 32 rows, 16 columns at a time, of two warps one takes the even sixteens and one the odd ones; through
+        // shared memory, so that four lanes write 64 bytes of a row.  The next sixteen are read while these are written.
+        const int quarter = w & 3, odd = (w - kRowsSplit) >> 2;
+        float *stage = s_stage + (w - kRowsSplit) * (kRowsStage / 4);
         for (int tile = 0; tile < my_tiles; tile++) {
             const long long row0 = ((long long)blockIdx.x + (long long)tile * gridDim.x) * kRowsTile + 32 * quarter;
             const uint32_t acc = tmem + (uint32_t)((tile & 1) * 2 * NT) + ((uint32_t)(32 * quarter) << 16);
@@ -242,15 +256,19 @@ k_dense_rows(const DenseRows g)
             plain = plain || plain_all || s_bad[tile & (kRowsBad - 1)];
             plain = __any_sync(FGC_FULL_MASK, plain);
             tc_after_sync();
-            for (int c = 0; c < NT; c += 16) {
+            uint32_t big[16], small[16];
+            auto read16 = [&](int c) {
+                tmem_read16(acc + c, big);
+                tmem_read16(acc + NT + c, small);
+            };
+            if (!plain && 16 * odd < NT) read16(16 * odd);
+            for (int c = 16 * odd; c < NT; c += 32) {
                 float v[16];
                 if (!plain) {
-                    uint32_t big[16], small[16];
-                    tmem_read16(acc + c, big);
-                    tmem_read16(acc + NT + c, small);
                     tmem_wait_read();
 #pragma unroll
                     for (int k = 0; k < 16; k++) v[k] = __uint_as_float(big[k]) + __uint_as_float(small[k]);
+                    if (c + 32 < NT) read16(c + 32);
                 } else {
                     const long long row = row0 + lane;
 #pragma unroll 1
@@ -267,17 +285,18 @@ k_dense_rows(const DenseRows g)
 #pragma unroll
                     for (int k = 0; k < 16; k++) v[k] = stage[lane * 20 + k];
                 }
-                if (g.bias) {
 #pragma unroll
-                    for (int k = 0; k < 16; k++) v[k] += col0 + c + k < g.n_cols ? __ldg(g.bias + col0 + c + k) : 0.f;
+                for (int k = 0; k < 4; k++) {
+                    const float4 bias = *reinterpret_cast<const float4 *>(s_bias + c + 4 * k);
+                    float4 o = make_float4(v[4 * k] + bias.x, v[4 * k + 1] + bias.y, v[4 * k + 2] + bias.z, v[4 * k + 3] + bias.w);
+                    if (g.relu) {                                                         // (NaN stays NaN, as in torch.relu)
+                        o.x = o.x < 0.f ? 0.f : o.x;
+                        o.y = o.y < 0.f ? 0.f : o.y;
+                        o.z = o.z < 0.f ? 0.f : o.z;
+                        o.w = o.w < 0.f ? 0.f : o.w;
+                    }
+                    *reinterpret_cast<float4 *>(stage + lane * 20 + 4 * k) = o;
                 }
-                if (g.relu) {
-#pragma unroll
-                    for (int k = 0; k < 16; k++) v[k] = v[k] < 0.f ? 0.f : v[k];              // (NaN stays NaN, as in torch.relu)
-                }
-#pragma unroll
-                for (int k = 0; k < 4; k++)
-                    *reinterpret_cast<float4 *>(stage + lane * 20 + 4 * k) = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
                 __syncwarp();
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
@@ -402,61 +421,74 @@ k_dense_weight(const DenseWeight g)
     if (w < kWeightSplit) {
         // The matrix whose columns are rows of the result comes first in a buffer.  Columns beyond a tile are not written: what is
         // there makes rows and columns of the result that are not read.
-        const int unit = t & 15, row_in = t >> 4;              // 16 units of eight columns, 32 rows at a time
-        char *s_x = s + (g.swap ? 0 : 2 * kWeightChunk) + (unit >> 3) * kWeightChunk;
-        char *s_y = s + (g.swap ? 2 * kWeightChunk : 0) + (unit >> 3) * kWeightChunk;
-        const int x_left = n_in - c0 - unit * 8, y_left = n_out - o0 - unit * 8;
-        const bool has_x = unit * 8 < g.tile_in, has_y = unit * 8 < g.tile_out;
-        const float *px = g.x + (size_t)(first + row_in) * g.n_in + c0 + unit * 8;
-        size_t at_y = (size_t)(first + row_in) * g.n_out + o0 + unit * 8;
-        long long row = first + row_in;                        // of the next load
+        // Units of eight columns: eight or 16 to a row, so that 64 rows take one pass or two.  A register is loaded again as soon as it
+        // has been split: the loads of a step are on their way during the rest of the one before.
+        const int wide_x = g.tile_in > 64 ? 1 : 0, wide_y = g.tile_out > 64 ? 1 : 0;
+        const int unit_x = t & (7 + 8 * wide_x), row_x = t >> (3 + wide_x), unit_y = t & (7 + 8 * wide_y), row_y = t >> (3 + wide_y);
+        char *s_x = s + (g.swap ? 0 : 2 * kWeightChunk) + (unit_x >> 3) * kWeightChunk;
+        char *s_y = s + (g.swap ? 2 * kWeightChunk : 0) + (unit_y >> 3) * kWeightChunk;
+        const int x_left = n_in - c0 - unit_x * 8, y_left = n_out - o0 - unit_y * 8;
+        const float *px = g.x + (size_t)(first + row_x) * g.n_in + c0 + unit_x * 8;
+        size_t at_y = (size_t)(first + row_y) * g.n_out + o0 + unit_y * 8;
+        long long row0 = first;                                // of the step
         float4 vx[2][2], vy[2][2], vm[2][2];
         float sum[8] = {};
-        float *total = s_bias + row_in * 128 + unit * 8;       // two levels, so that a thread never adds thousands of rows one to another
+        float *total = s_bias + row_y * (64 + 64 * wide_y) + unit_y * 8;         // two levels, so that a thread never adds thousands of rows one to another
         auto fold = [&]() {
 #pragma unroll
             for (int k = 0; k < 8; k++) { total[k] += sum[k]; sum[k] = 0.f; }
         };
 #pragma unroll
         for (int k = 0; k < 8; k++) total[k] = 0.f;
-        auto fetch = [&]() {
-#pragma unroll
-            for (int i = 0; i < 2; i++) {
-                const bool in = row + 32 * i < last;
-                if (has_x) dense_load8_at<VEC>(px + (size_t)(32 * i) * g.n_in, in ? x_left : 0, vx[i]);
-                if (has_y) dense_load8_at<VEC>(g.dy + at_y + (size_t)(32 * i) * g.n_out, in ? y_left : 0, vy[i]);
-                if (has_y && g.y) dense_load8_at<VEC>(g.y + at_y + (size_t)(32 * i) * g.n_out, in ? y_left : 0, vm[i]);
-            }
+        auto fetch_x = [&](int i) { dense_load8_at<VEC>(px + (size_t)(32 * i) * g.n_in, row0 + row_x + 32 * i < last ? x_left : 0, vx[i]); };
+        auto fetch_y = [&](int i) {
+            const int left = row0 + row_y + 32 * i < last ? y_left : 0;
+            dense_load8_at<VEC>(g.dy + at_y + (size_t)(32 * i) * g.n_out, left, vy[i]);
+            if (g.y) dense_load8_at<VEC>(g.y + at_y + (size_t)(32 * i) * g.n_out, left, vm[i]);
         };
-        if (steps > 0) fetch();
+        if (steps > 0) {
+            fetch_x(0);
+            if (wide_x) fetch_x(1);
+            fetch_y(0);
+            if (wide_y) fetch_y(1);
+        }
         for (int step = 0; step < steps; step++) {
             const int b = step & 1;
             uint32_t top = 0;
             if (step >= 2 && !__all_sync(FGC_FULL_MASK, wait_unless(done + 8 * b, ((step >> 1) - 1) & 1, s_late))) top = kUnsplit;
+            // (the rows of the next step from here on; beyond the last nothing is read)
+            const long long row_now = row0;
+            const size_t y_now = at_y;
+            row0 += kWeightRows;
+            px += (size_t)kWeightRows * g.n_in;
+            at_y += (size_t)kWeightRows * g.n_out;
 #pragma unroll
             for (int i = 0; i < 2; i++) {
-                if (has_x) top = max(top, split_to(s_x + b * kWeightBuffer, kWeightRows * 128, row_in + 32 * i, unit & 7, vx[i]));
-                if (has_y) {
+                if (i == 0 || wide_x) {
+                    top = max(top, split_to(s_x + b * kWeightBuffer, kWeightRows * 128, row_x + 32 * i, unit_x & 7, vx[i]));
+                    fetch_x(i);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                if (i == 0 || wide_y) {
                     if (g.y) mask8(vy[i], vm[i]);
                     const float *v = reinterpret_cast<const float *>(vy[i]);
-                    if (owner && g.dy_masked && row + 32 * i < last) {
+                    if (owner && g.dy_masked && row_now + row_y + 32 * i < last) {
 #pragma unroll
                         for (int k = 0; k < 8; k++)
-                            if (k < y_left) g.dy_masked[at_y + (size_t)(32 * i) * g.n_out + k] = v[k];
+                            if (k < y_left) g.dy_masked[y_now + (size_t)(32 * i) * g.n_out + k] = v[k];
                     }
 #pragma unroll
                     for (int k = 0; k < 8; k++) sum[k] += v[k];
-                    top = max(top, split_to(s_y + b * kWeightBuffer, kWeightRows * 128, row_in + 32 * i, unit & 7, vy[i]));
+                    top = max(top, split_to(s_y + b * kWeightBuffer, kWeightRows * 128, row_y + 32 * i, unit_y & 7, vy[i]));
+                    fetch_y(i);
                 }
             }
             if (top >= kUnsplit) s_bad[step & (kRowsBad - 1)] = 1;
             smem_to_tensor_core();
             __syncwarp();
             if (lane == 0) mbar_arrive(full + 8 * b);
-            row += kWeightRows;
-            px += (size_t)kWeightRows * g.n_in;
-            at_y += (size_t)kWeightRows * g.n_out;
-            if (step + 1 < steps) fetch();
             if ((step & 15) == 15) fold();
         }
         fold();
@@ -539,7 +571,8 @@ k_dense_weight(const DenseWeight g)
     // threads that loaded the same columns, added in a fixed order
     if (owner && t < g.tile_out && o0 + t < n_out) {
         float sum = 0.f;
-        for (int k = 0; k < 32; k++) sum += s_bias[k * 128 + t];
+        const int length = g.tile_out > 64 ? 128 : 64, rows = kWeightBias / 4 / length;
+        for (int k = 0; k < rows; k++) sum += s_bias[k * length + t];
         g.part_b[(size_t)blockIdx.x * g.n_out + o0 + t] = sum;
     }
 }

@@ -18,27 +18,28 @@ namespace fgc {
 
 // Beyond this (2^60, infinities and NaN among it) a number is not split: parts of products could overflow where the product does not,
 // and an infinity times a part that is 0 is not a number.  Tiles that hold one are computed by scalar operations.
-constexpr uint32_t kUnsplit = 0x5d800000u;
+constexpr uint32_t kUnsplit = 0x5d800000u;         // (a number just below it may count as it: its first part is rounded)
 
-// Eight numbers into three units of eight parts; returns the largest pattern without sign.
+// Eight numbers into three units of eight parts; returns the largest first part without sign, as the upper half of the pattern of an fp32 number.
 __device__ __forceinline__ uint32_t split8(const float (&v)[8], uint4 (&part)[3])
 {
     uint32_t p[3][4], most = 0;
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         float a = v[2 * i], b = v[2 * i + 1];
-        most = max(most, max(__float_as_uint(a) & 0x7fffffffu, __float_as_uint(b) & 0x7fffffffu));
 #pragma unroll
         for (int k = 0; k < 3; k++) {
             const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
             const uint32_t u = *reinterpret_cast<const uint32_t *>(&h);
             p[k][i] = u;
+            if (k == 0) most = __vmaxu2(most, u & 0x7fff7fffu);
             if (k < 2) {
                 a -= __uint_as_float(u << 16);
                 b -= __uint_as_float(u & 0xffff0000u);
             }
         }
     }
+    most = max(most & 0xffffu, most >> 16) << 16;
 #pragma unroll
     for (int k = 0; k < 3; k++) part[k] = make_uint4(p[k][0], p[k][1], p[k][2], p[k][3]);
     return most;
