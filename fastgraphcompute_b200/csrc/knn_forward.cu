@@ -94,16 +94,19 @@ static int knn_forward_launch(const float *coords, int64_t n_vert, int32_t n_coo
 {
     const bool tree = (flags & FGC_FORWARD_TREE) != 0;
     int rc;
-    bool done = false;                     // status words and cell order are written by the build
-    if (tree) rc = fgc_knn_build_tree(coords, n_vert, n_coords, row_splits, n_rs, K, direction, ws, ws_bytes, stream);
+    bool words = false, order = tree;      // status words and cell order are written by the build
+    if (tree)
+        rc = knn_build_tree_forward(coords, n_vert, n_coords, row_splits, n_rs, K, direction, status ? status->words : nullptr, out_order, &words, ws,
+                                    ws_bytes, stream);
     else {
         const int dims = flags & FGC_SEARCH_GRID3 ? 3 : (flags & FGC_SEARCH_GRID4 ? 4 : 0);
         rc = knn_build_grid_forward(coords, n_vert, n_coords, row_splits, n_rs, K, direction, target_occupancy, dims,
-                                    status ? status->words : nullptr, out_order, &done, ws, ws_bytes, stream);
+                                    status ? status->words : nullptr, out_order, &words, ws, ws_bytes, stream);
+        order = words;
     }
     if (rc != FGC_OK) return rc;
     if (status) {
-        if (!done) rc = fgc_knn_publish_grid_info(ws, status->words, stream);
+        if (!words) rc = fgc_knn_publish_grid_info(ws, status->words, stream);
         if (rc != FGC_OK) return rc;
         *published = true;
         FGC_RETURN_IF_CUDA(cudaEventRecord(status->ready, (cudaStream_t)stream));
@@ -124,7 +127,7 @@ static int knn_forward_launch(const float *coords, int64_t n_vert, int32_t n_coo
                              (flags & (FGC_SEARCH_COUNT | FGC_SEARCH_GRID3 | FGC_SEARCH_GRID4)) | FGC_SEARCH_FRESH, out_idx,
                              out_distsq, ws, ws_bytes, stream);
     if (rc != FGC_OK) return rc;
-    if (out_order && n_vert > 0 && !done)
+    if (out_order && n_vert > 0 && !order)
         FGC_RETURN_IF_CUDA(cudaMemcpyAsync(out_order, fgc_knn_cell_order(ws, n_vert, n_coords, n_rs, K),
                                            sizeof(int32_t) * (size_t)n_vert, cudaMemcpyDeviceToDevice, (cudaStream_t)stream));
     if (ties && n_vert > 0) {

@@ -7,53 +7,16 @@
 // written as soon as the checks are done and the form of the grid is known, and the cell order goes to the caller's array on the way.
 #include <cstddef>
 
+#include "cluster.cuh"
 #include "knn_grid_build.cuh"
 
 namespace fgc {
 
-constexpr int kSmallCtas = 8, kSmallThreads = kSortWarps * 32, kSmallAll = kSmallCtas * kSmallThreads;
-constexpr int kSmallPoints = (int)(kSmallBuild / kSmallAll);           // of a thread
-static_assert(kSmallPoints * kSmallAll == kSmallBuild, "points do not fill the threads");
+constexpr int kSmallPoints = (int)(kSmallBuild / kClusterAll);         // of a thread
+static_assert(kSmallPoints * kClusterAll == kSmallBuild, "points do not fill the threads");
+static_assert(kSortWarps == kClusterWarps, "large cells are sorted by the CTAs of the cluster");
 constexpr int kSmallScan = 4;                                          // table entries of a thread per scan step
-
-__device__ __forceinline__ void cluster_barrier()
-{
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
-constexpr int kSmallSplits = kSmallThreads;                            // row splits that are kept in shared memory
-
-// Exclusive scan over the threads of a CTA; total: of all of them.
-__device__ __forceinline__ int cta_scan(int x, int *s_part, int &total)
-{
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    int incl = x;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(FGC_FULL_MASK, incl, o);
-        if (lane >= o) incl += y;
-    }
-    __syncthreads();
-    if (lane == 31) s_part[wib] = incl;
-    __syncthreads();
-    int before = incl - x;
-    total = 0;
-#pragma unroll
-    for (int k = 0; k < kSortWarps; k++) {
-        if (k == wib) before += total;
-        total += s_part[k];
-    }
-    return before;
-}
-
-// A word of another CTA's shared memory.
-__device__ __forceinline__ uint32_t cluster_word(const void *mine, int cta)
-{
-    uint32_t at, v;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"((uint32_t)__cvta_generic_to_shared(mine)), "r"(cta));
-    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(at) : "memory");
-    return v;
-}
+constexpr int kSmallSplits = kClusterThreads;                          // row splits that are kept in shared memory
 
 // What a CTA has found, read by all others.
 struct SmallPart {
@@ -63,31 +26,31 @@ struct SmallPart {
 };
 constexpr int kSmallWords = sizeof(SmallPart) / 4;
 
-__global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(kSmallThreads)
+__global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterThreads)
 k_build_small(const GridBuild a)
 {
     chain_wait();
     chain_release();
     extern __shared__ int s_sort[];
     __shared__ SmallPart s_mine;
-    __shared__ uint32_t s_all[kSmallCtas][kSmallWords];
+    __shared__ uint32_t s_all[kClusterCtas][kSmallWords];
     __shared__ unsigned long long s_sq;
     __shared__ int s_part[kSortWarps];
     __shared__ int s_splits[kSmallSplits];
     __shared__ KnnGrid s_grid;
-    const int t = threadIdx.x, lane = t & 31, wib = t >> 5, cta = blockIdx.x, first = cta * kSmallThreads + t;
+    const int t = threadIdx.x, lane = t & 31, wib = t >> 5, cta = blockIdx.x, first = cta * kClusterThreads + t;
     const int n = a.n_vert;
     KnnGrid *g = a.grid;
     auto gather = [&]() {
-        if (t < kSmallCtas * kSmallWords) s_all[t / kSmallWords][t % kSmallWords] = cluster_word((uint32_t *)&s_mine + t % kSmallWords, t / kSmallWords);
+        if (t < kClusterCtas * kSmallWords) s_all[t / kSmallWords][t % kSmallWords] = cluster_word((uint32_t *)&s_mine + t % kSmallWords, t / kSmallWords);
         __syncthreads();
     };
 
     // extents, checks and the number of possible neighbours; tickets and the first table cleared
-    for (int i = first; i < (int)((kGridHeaderBytes + kHardTicketBytes) / sizeof(int)); i += kSmallAll) ((int *)g)[i] = 0;
+    for (int i = first; i < (int)((kGridHeaderBytes + kHardTicketBytes) / sizeof(int)); i += kClusterAll) ((int *)g)[i] = 0;
     {
         const int n_counts = a.bins_cap_first * (a.n_rs - 1) * a.mirror + 1;
-        for (int i = first; i < n_counts; i += kSmallAll) a.counts[i] = 0;
+        for (int i = first; i < n_counts; i += kClusterAll) a.counts[i] = 0;
     }
     if (t < kSmallWords) ((uint32_t *)&s_mine)[t] = 0;
     if (t < (int)(sizeof(KnnGrid) / sizeof(int))) ((int *)&s_grid)[t] = 0;
@@ -97,7 +60,7 @@ k_build_small(const GridBuild a)
         uint32_t bad = 0, n_may = 0, lmin[4] = {0, 0, 0, 0}, lmax[4] = {0, 0, 0, 0};
 #pragma unroll
         for (int k = 0; k < kSmallPoints; k++) {
-            const int v = first + k * kSmallAll;
+            const int v = first + k * kClusterAll;
             if (v < n) {
                 const float *row = a.coords + (size_t)v * a.n_coords;
                 if (a.mirror > 1) {
@@ -122,7 +85,7 @@ k_build_small(const GridBuild a)
         }
         // row_splits must start at 0, end at n_vert and never decrease
         if (t < a.n_rs && t < kSmallSplits) s_splits[t] = (int)min(max(a.row_splits[t], (int64_t)0), (int64_t)n);
-        for (int i = first; i < a.n_rs; i += kSmallAll)
+        for (int i = first; i < a.n_rs; i += kClusterAll)
             if (i == 0 ? a.row_splits[0] != 0 : (a.row_splits[i] < a.row_splits[i - 1] || (i == a.n_rs - 1 && a.row_splits[i] != (int64_t)n))) bad |= 2;
         bad = __reduce_or_sync(FGC_FULL_MASK, bad);
         n_may = __reduce_add_sync(FGC_FULL_MASK, n_may);
@@ -145,7 +108,7 @@ k_build_small(const GridBuild a)
         for (int w = 0; w < 10; w++) {
             uint32_t x = s_all[0][w];
 #pragma unroll
-            for (int k = 1; k < kSmallCtas; k++) x = w < 8 ? max(x, s_all[k][w]) : (w == 8 ? x | s_all[k][w] : x + s_all[k][w]);
+            for (int k = 1; k < kClusterCtas; k++) x = w < 8 ? max(x, s_all[k][w]) : (w == 8 ? x | s_all[k][w] : x + s_all[k][w]);
             ((uint32_t *)&p)[w] = x;
         }
         int mirror = a.mirror, bins_target = a.bins_target, bins_cap = a.bins_cap;
@@ -162,14 +125,14 @@ k_build_small(const GridBuild a)
         // (pass p follows the p-th density pass that changed the grid)
         const bool look = good && (pass == 0 ? a.adaptive != 0 : (pass == 1 && a.allow_fallback && s_grid.fallback3));
         if (pass > 0) {
-            for (int i = first; i < s_grid.total_bins + 1; i += kSmallAll) a.counts[i] = 0;
+            for (int i = first; i < s_grid.total_bins + 1; i += kClusterAll) a.counts[i] = 0;
             if (t == 0) s_sq = 0;
             cluster_barrier();
         }
         unsigned may = 0;                  // of the thread's points
 #pragma unroll
         for (int k = 0; k < kSmallPoints; k++) {
-            const int v = first + k * kSmallAll;
+            const int v = first + k * kClusterAll;
             bin[k] = -1;
             if (good && v < n) {
                 int e;
@@ -224,7 +187,7 @@ k_build_small(const GridBuild a)
         if (t == 0) {
             unsigned long long sum = 0;
 #pragma unroll
-            for (int k = 0; k < kSmallCtas; k++) sum += (unsigned long long)s_all[k][11 + 2 * pass] << 32 | s_all[k][10 + 2 * pass];
+            for (int k = 0; k < kClusterCtas; k++) sum += (unsigned long long)s_all[k][11 + 2 * pass] << 32 | s_all[k][10 + 2 * pass];
             grid_refine(&s_grid, sum, n, a.seen_target, a.seen_target3, a.bins_target, pass, pass == 0 && a.allow_fallback);
         }
         __syncthreads();
@@ -247,8 +210,8 @@ k_build_small(const GridBuild a)
     // exclusive scan: a share of the table per CTA, in registers where it fits
     {
         const int entries = s_grid.total_bins + 1;
-        const int share = ((entries + kSmallCtas - 1) / kSmallCtas + 3) & ~3, lo = min(entries, cta * share), hi = min(entries, lo + share);
-        const bool once = share <= kSmallThreads * kSmallScan;
+        const int share = ((entries + kClusterCtas - 1) / kClusterCtas + 3) & ~3, lo = min(entries, cta * share), hi = min(entries, lo + share);
+        const bool once = share <= kClusterThreads * kSmallScan;
         int x[kSmallScan], sum = 0, all, before;
         if (once) {
 #pragma unroll
@@ -258,7 +221,7 @@ k_build_small(const GridBuild a)
                 sum += x[k];
             }
         } else {
-            for (int i = lo + t; i < hi; i += kSmallThreads) sum += a.counts[i];
+            for (int i = lo + t; i < hi; i += kClusterThreads) sum += a.counts[i];
         }
         before = cta_scan(sum, s_part, all);
         if (t == 0) s_mine.entries = all;
@@ -266,7 +229,7 @@ k_build_small(const GridBuild a)
         gather();
         int carry = 0;
         for (int k = 0; k < cta; k++) carry += s_all[k][14];
-        for (int i0 = lo; i0 < hi; i0 += kSmallThreads * kSmallScan) {
+        for (int i0 = lo; i0 < hi; i0 += kClusterThreads * kSmallScan) {
             const int at = i0 + t * kSmallScan;
             if (!once) {
                 sum = 0;
@@ -297,7 +260,7 @@ k_build_small(const GridBuild a)
     }
 #pragma unroll
     for (int k = 0; k < kSmallPoints; k++)
-        if (bin[k] >= 0 && FGC_DBG_OK(beg[k] + rank[k] >= 0 && beg[k] + rank[k] < n, &g->status)) a.stmp[beg[k] + rank[k]] = first + k * kSmallAll;
+        if (bin[k] >= 0 && FGC_DBG_OK(beg[k] + rank[k] >= 0 && beg[k] + rank[k] < n, &g->status)) a.stmp[beg[k] + rank[k]] = first + k * kClusterAll;
     cluster_barrier();
     int smaller[kSmallPoints] = {}, most = 0;
 #pragma unroll
@@ -307,11 +270,11 @@ k_build_small(const GridBuild a)
         for (int k = 0; k < kSmallPoints; k++)
 #pragma unroll
             for (int i = i0; i < i0 + 4; i++)
-                if (i < len[k] && len[k] <= kRankMax) smaller[k] += a.stmp[beg[k] + i] < first + k * kSmallAll ? 1 : 0;
+                if (i < len[k] && len[k] <= kRankMax) smaller[k] += a.stmp[beg[k] + i] < first + k * kClusterAll ? 1 : 0;
     }
 #pragma unroll
     for (int k = 0; k < kSmallPoints; k++) {
-        const int v = first + k * kSmallAll, at = beg[k] + smaller[k];
+        const int v = first + k * kClusterAll, at = beg[k] + smaller[k];
         if (bin[k] < 0) continue;
         if (len[k] <= kRankMax) {
             if (FGC_DBG_OK(beg[k] >= 0 && smaller[k] < len[k] && at < n, &g->status)) {
@@ -328,7 +291,7 @@ k_build_small(const GridBuild a)
     }
     cluster_barrier();
     const int n_big = __ldcg(&g->n_big_cells), n_huge = __ldcg(&g->n_huge_cells);
-    for (int w = cta * kSortWarps + wib; w < n_big; w += kSmallCtas * kSortWarps) {
+    for (int w = cta * kSortWarps + wib; w < n_big; w += kClusterCtas * kSortWarps) {
         const int cell = a.biglist[w], from = bounds[cell], many = bounds[cell + 1] - from;
         warp_sort_segment(a.sorig + from, many, s_sort + wib * kWarpSortMaxShared, lane);
         __syncwarp();
@@ -340,10 +303,10 @@ k_build_small(const GridBuild a)
         __syncwarp();
     }
     __syncthreads();
-    for (int w = cta; w < n_huge; w += kSmallCtas) {
+    for (int w = cta; w < n_huge; w += kClusterCtas) {
         const int cell = a.hugelist[w], from = bounds[cell], many = bounds[cell + 1] - from;
         sort_cell_by_cta(from, many, a.stmp, a.sorig, s_sort, kSortShared / 4, &g->status);
-        for (int i = t; i < many; i += kSmallThreads) {
+        for (int i = t; i < many; i += kClusterThreads) {
             const int v = a.sorig[from + i];
             place_point(from + i, v, grid_cell(&s_grid, cell), a.coords, a.n_coords, a.nv, a.direction, a.sorig, a.scoords, a.sbin, a.sflag);
             if (a.out_order) a.out_order[from + i] = v;
@@ -355,7 +318,7 @@ k_build_small(const GridBuild a)
 cudaError_t launch_small_build(const GridBuild &b, cudaStream_t s)
 {
     static_assert(kSortShared <= 48 * 1024, "needs an attribute");
-    k_build_small<<<kSmallCtas, kSmallThreads, kSortShared, s>>>(b);
+    k_build_small<<<kClusterCtas, kClusterThreads, kSortShared, s>>>(b);
     return cudaGetLastError();
 }
 

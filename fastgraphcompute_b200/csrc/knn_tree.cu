@@ -1,6 +1,7 @@
 // binned_select_knn forward for sm_100a: building the search tree (see knn_tree.cuh).
 //
-//   k_tree_extent   bounding box of the points, checks of coordinates and row splits
+//   k_tree_extent   bounding box of the points, checks of coordinates and row splits (small batches take everything up to the
+//                   sorted ids in one launch, knn_tree_small.cu)
 //   k_tree_keys     64-bit key of every point (row split, place on the Hilbert curve) and the first
 //                   radix histogram
 //   k_tree_hist     histogram of a later pass;  scan.cuh: its exclusive scan
@@ -11,7 +12,7 @@
 // The sort is stable and starts from the original order, so the tree is the same on every run.
 // Launch latency bounds the build of small batches (0.15 ms for 200 k points), scattered writes that
 // of large ones (0.31 ms for 1.6 M points, against 8 ms and more for their search).
-#include "knn_tree.cuh"
+#include "knn_tree_build.cuh"
 
 namespace fgc {
 
@@ -73,62 +74,12 @@ k_tree_extent(const float *__restrict__ coords, int n_vert, int n_coords, int ke
         int status = 0;
         if (__ldcg(&t->nonfinite)) status |= FGC_STATUS_NONFINITE;
         if (bad_rs) status |= FGC_STATUS_BAD_ROW_SPLITS;
-        float ext = 0.f;
-        for (int c = 0; c < key_dims; c++) {
-            const float lo = ordered_to_float(~__ldcg(&t->min_key[c])), hi = ordered_to_float(__ldcg(&t->max_key[c]));
-            t->origin[c] = lo;
-            ext = fmaxf(ext, hi - lo);
-        }
-        // equal cells in all dimensions; an extent of zero or one that overflows puts every point
-        // into cell 0 (any order gives a valid tree)
-        const float s = (float)(1u << bits) / ext;
-        t->scale = ext > 0.f && is_finite_bits(s) ? s : 0.f;
-        t->magic = kTreeMagic;
+        uint32_t min_key[kTreeKeyDims], max_key[kTreeKeyDims];
+#pragma unroll
+        for (int c = 0; c < kTreeKeyDims; c++) { min_key[c] = __ldcg(&t->min_key[c]); max_key[c] = __ldcg(&t->max_key[c]); }
+        tree_setup(t, min_key, max_key, key_dims, bits);
         g->n_events = n_rs - 1;
         g->status = status;
-    }
-}
-
-// Place of a cell on the Hilbert curve over ND dimensions of `bits` bits: J. Skilling, "Programming
-// the Hilbert curve", AIP Conf. Proc. 707 (2004), the transform from axes to the transposed index,
-// whose bits are then interleaved.
-template <int ND>
-__device__ __forceinline__ uint32_t hilbert_index(uint32_t (&x)[kTreeKeyDims], int bits)
-{
-    for (uint32_t q = 1u << (bits - 1); q > 1; q >>= 1) {
-        const uint32_t p = q - 1;
-#pragma unroll
-        for (int i = 0; i < ND; i++) {
-            if (x[i] & q) x[0] ^= p;
-            else { const uint32_t d = (x[0] ^ x[i]) & p; x[0] ^= d; x[i] ^= d; }
-        }
-    }
-#pragma unroll
-    for (int i = 1; i < ND; i++) x[i] ^= x[i - 1];
-    uint32_t e = 0;
-    for (uint32_t q = 1u << (bits - 1); q > 1; q >>= 1)
-        if (x[ND - 1] & q) e ^= q - 1;
-    uint32_t key = 0;
-    for (int b = bits - 1; b >= 0; b--)
-#pragma unroll
-        for (int i = 0; i < ND; i++) key = (key << 1) | (((x[i] ^ e) >> b) & 1u);
-    return key;
-}
-
-__device__ __forceinline__ uint32_t tree_key(const KnnTree *__restrict__ t, const float *__restrict__ row, int key_dims, int bits)
-{
-    const uint32_t top = (1u << bits) - 1;
-    uint32_t x[kTreeKeyDims];
-    const float scale = t->scale;
-#pragma unroll
-    for (int c = 0; c < kTreeKeyDims; c++)
-        x[c] = c < key_dims ? min(__float2uint_rz((__ldg(row + c) - t->origin[c]) * scale), top) : 0u;
-    switch (key_dims) {
-    case 2: return hilbert_index<2>(x, bits);
-    case 3: return hilbert_index<3>(x, bits);
-    case 4: return hilbert_index<4>(x, bits);
-    case 5: return hilbert_index<5>(x, bits);
-    default: return hilbert_index<6>(x, bits);
     }
 }
 
@@ -254,7 +205,7 @@ __global__ void __launch_bounds__(256)
 k_tree_leaves(const float *__restrict__ coords, int n_vert, int n_coords, const int64_t *__restrict__ direction,
               const int64_t *__restrict__ row_splits, int n_rs, KnnGrid *__restrict__ g, const int *__restrict__ ids,
               int *__restrict__ sorig, float4 *__restrict__ scoords, uint8_t *__restrict__ sflag,
-              float4 *__restrict__ leaf_box, float4 *__restrict__ node_box, float4 *__restrict__ half_box)
+              float4 *__restrict__ leaf_box, float4 *__restrict__ node_box, float4 *__restrict__ half_box, int *__restrict__ out_order)
 {
     chain_wait();
     chain_release();
@@ -279,6 +230,7 @@ k_tree_leaves(const float *__restrict__ coords, int n_vert, int n_coords, const 
         for (int c = 0; c < 4 * NV; c++) x[c] = act && c < n_coords ? __ldg(coords + (size_t)id * n_coords + c) : 0.f;
         if (act) {
             sorig[j] = id;
+            if (out_order) out_order[j] = id;
 #pragma unroll
             for (int v = 0; v < NV; v++)
                 scoords[(size_t)j * NV + v] = make_float4(x[4 * v], x[4 * v + 1], x[4 * v + 2], x[4 * v + 3]);
@@ -390,14 +342,14 @@ static cudaError_t sort_points(const float *coords, int n, int n_coords, const i
 
 template <int NV>
 static cudaError_t launch_boxes(const float *coords, int n, int n_coords, const int64_t *direction,
-                                const int64_t *row_splits, int n_rs, const KnnWorkspace &L, const TreeLayout &T,
-                                char *ws, cudaStream_t s)
+                                const int64_t *row_splits, int n_rs, const KnnWorkspace &L, const TreeLayout &T, const int *ids,
+                                int *out_order, char *ws, cudaStream_t s)
 {
     KnnGrid *g = (KnnGrid *)(ws + L.header);
     FGC_TRY(launch_chained(k_tree_leaves<NV>, (unsigned)T.n_box[1], 256, 0, s, coords, n, n_coords, direction,
-                           row_splits, n_rs, g, (const int *)(ws + T.ids[T.passes & 1]), (int *)(ws + L.sorig),
+                           row_splits, n_rs, g, ids, (int *)(ws + L.sorig),
                            (float4 *)(ws + L.scoords), (uint8_t *)(ws + L.sflag), (float4 *)(ws + T.box[0]),
-                           (float4 *)(ws + T.box[1]), n_coords == kHalfDims && T.groups ? (float4 *)(ws + T.half_box) : nullptr));
+                           (float4 *)(ws + T.box[1]), n_coords == kHalfDims && T.groups ? (float4 *)(ws + T.half_box) : nullptr, out_order));
     if (n <= 32768) return cudaSuccess;                  // no row split has more than one top node: never read
     return launch_chained(k_tree_top<NV>, (unsigned)((T.n_box[2] + 7) / 8), 256, 0, s, row_splits, n_rs, g,
                           (const float4 *)(ws + T.box[1]), (float4 *)(ws + T.box[2]), T.n_box[2]);
@@ -523,21 +475,22 @@ extern "C" int fgc_knn_groups_preferred(int64_t n_vert, int32_t n_coords, int64_
 //                      0.74 / 0.78 / 1.12, 200 k 1.00 / 0.51 / 0.72 and 0.97 / 0.78 / 0.96;  K = 32: 200 k in 40 0.85 / 0.84 / 1.30;  K = 40: 100 k 0.94 /
 //                      0.48 / 0.81 and 0.89 / 0.74 / 1.01;  K = 66: 50 k 0.85 / 0.38 / 0.51
 //   five               K = 16: 200 k in one 0.83 / 0.84 / 0.89, 800 k in eight 0.80 / 1.03 / 0.90;  K = 32: 200 k in eight 0.62 / 0.99 / 1.04
-//   learned, three     K = 8: 20 k in one 0.97, 50 k 0.84;  K = 16: 50 k in ten 0.78, 200 k in 40 0.96, 10 k in one 0.82, 3 k 0.82;  K = 24: 20 k in
-//                      ten 0.92, 50 k in 25 0.84
-//   learned, four      K = 8: 50 k in ten 0.87, 200 k in 40 0.97;  K = 10: 10 k in one 0.73, 3 k 0.87;  K = 16: 20 k in ten 0.91, 50 k in 25 0.84
+//   learned, three     K = 8: 50 k in one 0.84;  K = 16: 50 k in ten 0.78, 200 k in 40 0.96;  K = 24: 50 k in 25 0.84
+//   learned, four      K = 8: 50 k in ten 0.87, 200 k in 40 0.97;  K = 16: 50 k in 25 0.84
+//   learned, sorted in one launch (up to kSmallTree points; three / four)  K = 10: 3 k in one row split 0.63 / 0.64, 5 k in five 0.90 / 0.90, 10 k in
+//                      thirty 0.92 / 0.98, 16 k in fifty 0.84 / 0.89;  K = 40: 10 k in ten 0.76 / 0.68, 20 k in one 0.69 / 0.38;  K = 16: 1000 in one 0.88 / 0.91
 // In row splits of 5000 points in 50 clusters, a hundred each, the grid is ahead by 0.1 to 0.3 of its time at K = 24 to 40.
 extern "C" int fgc_knn_groups_ahead(int64_t n_vert, int32_t n_coords, int64_t n_rs, int32_t K, int32_t long_tails)
 {
     using namespace fgc;
-    if (n_vert < 3000 || n_vert > 0x7fffffff || n_coords < 3 || n_coords > kGroupDims || n_rs < 2 || n_rs > 0x7fffffff || K < 1 ||
+    if (n_vert < 1000 || n_vert > 0x7fffffff || n_coords < 3 || n_coords > kGroupDims || n_rs < 2 || n_rs > 0x7fffffff || K < 1 ||
         K > FGC_MAX_K)
         return 0;
     const int64_t mean = n_vert / (n_rs - 1);
     const bool large = mean >= 10000;
     int least = FGC_MAX_K + 1;                   // shortest list
     if (long_tails && n_coords <= 4) {
-        if (n_vert < 16384) least = mean >= 3000 ? (n_coords == 4 ? 10 : 16) : least;
+        if (n_vert <= kSmallTree) least = n_vert >= 3000 ? 8 : (mean >= 1000 ? 16 : least);
         else if (n_coords == 4) least = mean >= 4000 ? 8 : (mean >= 1500 ? 16 : least);
         else least = mean >= 15000 ? 8 : (mean >= 4000 ? 16 : (mean >= 1500 ? 24 : least));
     } else if (n_coords == 5) {
@@ -561,12 +514,13 @@ extern "C" int fgc_knn_groups_ahead(int64_t n_vert, int32_t n_coords, int64_t n_
     return tree_layout(knn_workspace_layout(n_vert, n_coords, n_rs, K), n_vert, n_coords, n_rs).groups ? 1 : 0;
 }
 
-extern "C" int fgc_knn_build_tree(const float *coords, int64_t n_vert, int32_t n_coords, const int64_t *row_splits,
-                                  int64_t n_rs, int32_t K, const int64_t *direction_or_null, void *workspace,
-                                  size_t workspace_bytes, fgc_stream_t stream)
+namespace fgc {
+
+int knn_build_tree_forward(const float *coords, int64_t n_vert, int32_t n_coords, const int64_t *row_splits, int64_t n_rs, int32_t K,
+                           const int64_t *direction_or_null, int32_t *info_mapped, int32_t *out_order, bool *words, void *workspace,
+                           size_t workspace_bytes, fgc_stream_t stream)
 {
     FGC_NVTX("fgc_knn_build_tree");
-    using namespace fgc;
     KnnWorkspace L;
     if (!row_splits) return FGC_ERR_BAD_ARGUMENT;
     const int rc = check_knn_args(n_vert, n_coords, n_rs, K, workspace, workspace_bytes, &L);
@@ -575,21 +529,38 @@ extern "C" int fgc_knn_build_tree(const float *coords, int64_t n_vert, int32_t n
     char *ws = (char *)workspace;
     KnnGrid *g = (KnnGrid *)(ws + L.header);
     KnnTree *t = (KnnTree *)(ws + L.tickets);
-    FGC_RETURN_IF_CUDA(cudaMemsetAsync(g, 0, kGridHeaderBytes + kHardTicketBytes, s));
+    int key_dims, bits, passes;
+    const bool small = n_vert > 0 && small_tree_bits(n_vert, n_coords, n_rs, &key_dims, &bits, &passes);
+    if (!small) FGC_RETURN_IF_CUDA(cudaMemsetAsync(g, 0, kGridHeaderBytes + kHardTicketBytes, s));
     if (n_vert == 0) return FGC_OK;
     if (!coords || n_rs < 2) return FGC_ERR_BAD_ARGUMENT;
     const TreeLayout T = tree_layout(L, n_vert, n_coords, n_rs);
     if (!T.fits) return FGC_ERR_TOO_LARGE;
     const int n = (int)n_vert, nrs = (int)n_rs;
-    const int64_t pt_blocks = (n_vert + 255) / 256;
-    const int red_blocks = pt_blocks < sm_count() * 4 ? (int)pt_blocks : sm_count() * 4;
-    k_tree_extent<<<red_blocks, 256, 0, s>>>(coords, n, n_coords, T.key_dims, T.bits, row_splits, nrs, g, t);
-    FGC_CHECK_LAUNCH();
-    FGC_RETURN_IF_CUDA(T.rounds == 16 ? sort_points<16>(coords, n, n_coords, row_splits, nrs, L, T, ws, s)
-                                      : sort_points<4>(coords, n, n_coords, row_splits, nrs, L, T, ws, s));
-    if (L.nv == 1) FGC_RETURN_IF_CUDA(launch_boxes<1>(coords, n, n_coords, direction_or_null, row_splits, nrs, L, T, ws, s));
-    else if (L.nv == 2) FGC_RETURN_IF_CUDA(launch_boxes<2>(coords, n, n_coords, direction_or_null, row_splits, nrs, L, T, ws, s));
-    else if (L.nv == 3) FGC_RETURN_IF_CUDA(launch_boxes<3>(coords, n, n_coords, direction_or_null, row_splits, nrs, L, T, ws, s));
-    else FGC_RETURN_IF_CUDA(launch_boxes<4>(coords, n, n_coords, direction_or_null, row_splits, nrs, L, T, ws, s));
+    const int *ids = (const int *)(ws + T.ids[small ? 1 : T.passes & 1]);
+    if (small) {
+        FGC_RETURN_IF_CUDA(launch_tree_small(coords, n, n_coords, key_dims, bits, passes, row_splits, nrs, g, t, (uint32_t *)(ws + T.keys[0]),
+                                             (int *)(ws + T.ids[0]), (int *)(ws + T.ids[1]), info_mapped, s));
+        if (words) *words = true;
+    } else {
+        const int64_t pt_blocks = (n_vert + 255) / 256;
+        const int red_blocks = pt_blocks < sm_count() * 4 ? (int)pt_blocks : sm_count() * 4;
+        k_tree_extent<<<red_blocks, 256, 0, s>>>(coords, n, n_coords, T.key_dims, T.bits, row_splits, nrs, g, t);
+        FGC_CHECK_LAUNCH();
+        FGC_RETURN_IF_CUDA(T.rounds == 16 ? sort_points<16>(coords, n, n_coords, row_splits, nrs, L, T, ws, s)
+                                          : sort_points<4>(coords, n, n_coords, row_splits, nrs, L, T, ws, s));
+    }
+    auto boxes = L.nv == 1 ? launch_boxes<1> : (L.nv == 2 ? launch_boxes<2> : (L.nv == 3 ? launch_boxes<3> : launch_boxes<4>));
+    FGC_RETURN_IF_CUDA(boxes(coords, n, n_coords, direction_or_null, row_splits, nrs, L, T, ids, out_order, ws, s));
     return FGC_OK;
+}
+
+}  // namespace fgc
+
+extern "C" int fgc_knn_build_tree(const float *coords, int64_t n_vert, int32_t n_coords, const int64_t *row_splits,
+                                  int64_t n_rs, int32_t K, const int64_t *direction_or_null, void *workspace,
+                                  size_t workspace_bytes, fgc_stream_t stream)
+{
+    return fgc::knn_build_tree_forward(coords, n_vert, n_coords, row_splits, n_rs, K, direction_or_null, nullptr, nullptr, nullptr, workspace,
+                                       workspace_bytes, stream);
 }

@@ -155,6 +155,11 @@ constexpr int kTieShare = 16;
 // the kernels of the grid return at once.
 constexpr int32_t kStatusNoGrid = 1 << 30;
 
+// fgc_knn_build_tree; out_order: original ids in curve order, or null; small batches write the two words that the host reads on the way
+// (*words is set then).
+int knn_build_tree_forward(const float *coords, int64_t n_vert, int32_t n_coords, const int64_t *row_splits, int64_t n_rs, int32_t K,
+                           const int64_t *direction_or_null, int32_t *info_mapped, int32_t *out_order, bool *words, void *workspace,
+                           size_t workspace_bytes, fgc_stream_t stream);
 // fgc_knn_search_tree; mark_ties: such rows are marked (and have to be searched again on a grid).
 int knn_search_tree(int64_t n_vert, int32_t n_coords, const int64_t *row_splits, int64_t n_rs, int32_t K,
                     int32_t has_direction, int32_t tf_compat, TieMarks mark_ties, int64_t *out_idx, float *out_distsq,

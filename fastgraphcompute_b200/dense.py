@@ -22,6 +22,8 @@ max_sum = 512
 # without ReLU 230 / 160, with it 264 / 161; 131 072 rows, 128 to 64 98 / 95 and 106 / 96).  Below, the pass and its
 # launch cost more than they save (200 000 rows, 128 to 10 85 / 91; 32 768 rows, 128 to 128 59 / 64).
 pass_from = 1 << 23
+# Forward alone, module with ReLU / own kernel, us: 66 000 rows, 128 to 64 71 / 45; 64 to 128 92 / 46; 100 000 rows, 128 to 64 91 / 52.
+forward_from = (1 << 22) + 1
 
 
 class _Linear(torch.autograd.Function):
@@ -129,7 +131,7 @@ def _pays(linear, x) -> bool:
         return False
     n, n_in, n_out = x.shape[0], linear.in_features, linear.out_features
     if not (torch.is_grad_enabled() and (x.requires_grad or linear.weight.requires_grad)):
-        return n * n_out >= pass_from            # nothing but the forward's pass to gain
+        return n * n_out >= (forward_from if n_in <= max_sum else pass_from)           # nothing but the forward to gain
     # A small weight: the library's product for its gradient is a good one.  800 000 rows, 64 to 4 451 / 560 and 32 to 16
     # 470 / 547; 200 000 rows, 32 to 32 710 / 239.
     if n_in * n_out < min_rows // 32:

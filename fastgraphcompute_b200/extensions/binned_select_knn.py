@@ -92,7 +92,7 @@ def _forward(coords, row_splits, K, direction, tf_compat, count_evals, order, lo
     grid_order = False
     if tree and search_tree is None:
         tree = False
-        if direction is None and n_vert >= (3000 if long_tails else 16384):      # (below, the rules say no: calls less, 3 us)
+        if direction is None and n_vert >= (1000 if long_tails else 16384):      # (below, the rules say no: calls less, 3 us)
             size = (n_vert, n_coords, n_rs, K, int(long_tails))
             tree = _cabi.lib.fgc_knn_tree_preferred(*size) == 1
             if not tree and (_cabi.lib.fgc_knn_groups_ahead(*size) == 1 or _cabi.lib.fgc_knn_groups_preferred(*size) == 1):

@@ -499,8 +499,9 @@ def test_lists_of_eight_queries(kind, sizes, D, K, flags):
     (100000, 4, 10, 40, 0, 1), (200000, 4, 10, 24, 0, 1), (200000, 4, 11, 24, 0, 0), (200000, 4, 50, 32, 0, 1), (400000, 4, 20, 16, 0, 1),
     (400000, 4, 100, 24, 0, 1), (800000, 4, 200, 16, 0, 1), (800000, 4, 200, 15, 0, 0), (50000, 4, 400, 66, 0, 0),
     (200000, 5, 2, 16, 0, 1), (200000, 5, 3, 16, 0, 0), (200000, 5, 13, 32, 0, 1), (200000, 5, 14, 32, 0, 0),
-    (2999, 4, 1, 16, 1, 0), (3000, 4, 1, 10, 1, 1), (3000, 4, 1, 9, 1, 0), (6001, 3, 2, 16, 1, 1), (5999, 3, 2, 16, 1, 0),
-    (16384, 3, 1, 8, 1, 1), (16384, 3, 4, 15, 1, 0), (20000, 4, 5, 8, 1, 1), (20000, 4, 13, 16, 1, 1), (20000, 4, 14, 16, 1, 0),
+    (999, 4, 1, 16, 1, 0), (1000, 4, 1, 16, 1, 1), (1000, 4, 1, 15, 1, 0), (2999, 3, 3, 16, 1, 0), (3000, 3, 10, 8, 1, 1), (3000, 3, 11, 8, 1, 0),
+    (24576, 3, 80, 8, 1, 1), (24577, 3, 16, 15, 1, 0), (24577, 3, 6, 16, 1, 1), (24577, 4, 6, 8, 1, 1), (24577, 4, 16, 16, 1, 1),
+    (24577, 4, 17, 16, 1, 0), (24576, 3, 1, 7, 1, 0),
     (400000, 2, 1, 200, 0, 0), (400000, 6, 1, 40, 0, 0), (400000, 3, 1, 0, 0, 0), (400000, 3, 1, 258, 0, 0)])
 def test_groups_ahead_by_size(n, D, row_splits, K, long_tails, ahead):
     """The edges of the ranges where the search by groups is ahead of the grid with its lists divided among eight queries."""
@@ -530,3 +531,48 @@ def test_large_cells_are_in_order(n, cloud):
     assert km.read_counters(runs[0][2])[0][7] >= 1
     _, dist, _ = _forward(km, x, rs, 9, True)
     assert torch.equal(dist.sort(dim=1).values, runs[0][1].sort(dim=1).values)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sizes,D,K", [([400, 0, 2], 3, 3), ([512, 33], 2, 9), ([4096, 1], 3, 17), ([4097], 4, 40), ([24576], 3, 16), ([24577], 3, 16),
+                                       ([20] * 700, 3, 9), ([300] * 33, 4, 24), ([5000, 0, 3000], 7, 20), ([6000], 9, 66), ([2] * 5000, 4, 4)])
+@pytest.mark.parametrize("kind", ["uniform", "equal", "far"])
+def test_tree_of_a_small_batch(sizes, D, K, kind):
+    """The sort in one launch and the chain beyond it: rounds of 4096 points, two and three radix passes, row splits that leave too few
+    bits, equal points, an extent that overflows; distances of the grid, a permutation as order, the same rows twice."""
+    km = importlib.import_module("fastgraphcompute_b200.extensions.binned_select_knn")
+    g = torch.Generator().manual_seed(sum(sizes) + D)
+    n = sum(sizes)
+    x = torch.rand((n, D), generator=g)
+    if kind == "equal":
+        x[torch.rand(n, generator=g) < 0.4] = 0.25
+    if kind == "far":
+        x = torch.randn((n, D), generator=g) * 1e18
+        x[: n // 50] *= 1e19
+    x, rs = x.to(DEV), torch.tensor([0] + sizes).cumsum(0).to(DEV)
+    _, gd, _ = _forward(km, x, rs, K, False)
+    old = km.search_tree
+    try:
+        km.search_tree = True
+        found = [km.knn_forward_with_order(x, rs, K, None, False, True) for _ in range(2)]
+    finally:
+        km.search_tree = old
+    for idx, dist, order in found:
+        assert torch.equal(gd.sort(dim=1).values, dist.sort(dim=1).values)
+        assert torch.equal(order.long().sort().values, torch.arange(n, device=DEV))
+        assert torch.equal(idx, found[0][0]) and torch.equal(order, found[0][2])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1200, 24576, 30000])
+def test_bad_input_of_a_small_tree(n):
+    km = importlib.import_module("fastgraphcompute_b200.extensions.binned_select_knn")
+    x = torch.rand((n, 4), generator=torch.Generator().manual_seed(n)).to(DEV)
+    x[n // 2, 3] = float("inf")
+    with pytest.raises(RuntimeError, match="non-finite"):
+        _forward(km, x, torch.tensor([0, n], device=DEV), 20, True)
+    x[n // 2, 3] = 0.5
+    for bad in ([1, n], [0, n - 1], [0, n, n - 2, n]):
+        with pytest.raises(RuntimeError, match="row_splits"):
+            _forward(km, x, torch.tensor(bad, device=DEV), 20, True)
+    assert int(_forward(km, x, torch.tensor([0, n], device=DEV), 20, True)[0].min()) >= 0
