@@ -199,13 +199,20 @@ __device__ __forceinline__ int tree_event_of(const int64_t *__restrict__ rs, int
     return lo;
 }
 
+// What the search by groups reads beside the tree (TreeLayout); null: it is not taken.
+struct LeafArrays {
+    float4 *box_lo, *box_hi, *half_lo, *half_hi, *point_a;
+    float2 *box_e, *half_e;
+    float *point_e;
+};
+
 // One CTA per node slot (32 leaves): points in curve order, the boxes of the leaves and the node's.
 template <int NV>
 __global__ void __launch_bounds__(256)
 k_tree_leaves(const float *__restrict__ coords, int n_vert, int n_coords, const int64_t *__restrict__ direction,
               const int64_t *__restrict__ row_splits, int n_rs, KnnGrid *__restrict__ g, const int *__restrict__ ids,
               int *__restrict__ sorig, float4 *__restrict__ scoords, uint8_t *__restrict__ sflag,
-              float4 *__restrict__ leaf_box, float4 *__restrict__ node_box, float4 *__restrict__ half_box, int *__restrict__ out_order)
+              float4 *__restrict__ leaf_box, float4 *__restrict__ node_box, const LeafArrays arrays, int *__restrict__ out_order)
 {
     chain_wait();
     chain_release();
@@ -257,12 +264,23 @@ k_tree_leaves(const float *__restrict__ coords, int n_vert, int n_coords, const 
             half_hi[c] = low ? ordered_to_float(b0) : (a1 <= b1 ? ordered_to_float(b1) : __uint_as_float(0xff800000u));
             if (lane == 0) { atomicMin(&s_lo[c], a); atomicMax(&s_hi[c], b); }
         }
-        if (NV == 2 && half_box && (lane & 15) == 0) {
-            float4 *out = half_box + (size_t)((leaf0 + l) * 2 + (lane >> 4)) * 2 * NV;
-#pragma unroll
-            for (int v = 0; v < NV; v++) {
-                out[v] = make_float4(half_lo[4 * v], half_lo[4 * v + 1], half_lo[4 * v + 2], half_lo[4 * v + 3]);
-                out[NV + v] = make_float4(half_hi[4 * v], half_hi[4 * v + 1], half_hi[4 * v + 2], half_hi[4 * v + 3]);
+        if constexpr (NV == 2) {
+            if (arrays.box_lo) {
+                const size_t at = (size_t)(leaf0 + l), half = 2 * at + (lane >> 4);
+                if (lane == 0) {
+                    arrays.box_lo[at] = make_float4(lo[0], lo[1], lo[2], lo[3]);
+                    arrays.box_hi[at] = make_float4(hi[0], hi[1], hi[2], hi[3]);
+                    arrays.box_e[at] = make_float2(lo[4], hi[4]);
+                }
+                if ((lane & 15) == 0) {
+                    arrays.half_lo[half] = make_float4(half_lo[0], half_lo[1], half_lo[2], half_lo[3]);
+                    arrays.half_hi[half] = make_float4(half_hi[0], half_hi[1], half_hi[2], half_hi[3]);
+                    arrays.half_e[half] = make_float2(half_lo[4], half_hi[4]);
+                }
+                if (act) {
+                    arrays.point_a[j] = make_float4(x[0], x[1], x[2], x[3]);
+                    arrays.point_e[j] = x[4];
+                }
             }
         }
         if (lane == 0) {
@@ -346,10 +364,16 @@ static cudaError_t launch_boxes(const float *coords, int n, int n_coords, const 
                                 int *out_order, char *ws, cudaStream_t s)
 {
     KnnGrid *g = (KnnGrid *)(ws + L.header);
+    LeafArrays arrays = {};
+    if (T.groups && n_coords == kApartDims) {
+        arrays.box_lo = (float4 *)(ws + T.box_lo); arrays.box_hi = (float4 *)(ws + T.box_hi); arrays.box_e = (float2 *)(ws + T.box_e);
+        arrays.half_lo = (float4 *)(ws + T.half_lo); arrays.half_hi = (float4 *)(ws + T.half_hi); arrays.half_e = (float2 *)(ws + T.half_e);
+        arrays.point_a = (float4 *)(ws + T.point_a); arrays.point_e = (float *)(ws + T.point_e);
+    }
     FGC_TRY(launch_chained(k_tree_leaves<NV>, (unsigned)T.n_box[1], 256, 0, s, coords, n, n_coords, direction,
                            row_splits, n_rs, g, ids, (int *)(ws + L.sorig),
                            (float4 *)(ws + L.scoords), (uint8_t *)(ws + L.sflag), (float4 *)(ws + T.box[0]),
-                           (float4 *)(ws + T.box[1]), n_coords == kHalfDims && T.groups ? (float4 *)(ws + T.half_box) : nullptr, out_order));
+                           (float4 *)(ws + T.box[1]), arrays, out_order));
     if (n <= 32768) return cudaSuccess;                  // no row split has more than one top node: never read
     return launch_chained(k_tree_top<NV>, (unsigned)((T.n_box[2] + 7) / 8), 256, 0, s, row_splits, n_rs, g,
                           (const float4 *)(ws + T.box[1]), (float4 *)(ws + T.box[2]), T.n_box[2]);
@@ -474,7 +498,9 @@ extern "C" int fgc_knn_groups_preferred(int64_t n_vert, int32_t n_coords, int64_
 //   four               K = 12: 1.6 M in 16 0.85 / 0.74 / 0.61, K = 8 1.03;  K = 16: 400 k 0.95 / 0.43 / 0.61 and 0.90 / 0.75 / 0.76;  K = 24: 400 k in 80
 //                      0.74 / 0.78 / 1.12, 200 k 1.00 / 0.51 / 0.72 and 0.97 / 0.78 / 0.96;  K = 32: 200 k in 40 0.85 / 0.84 / 1.30;  K = 40: 100 k 0.94 /
 //                      0.48 / 0.81 and 0.89 / 0.74 / 1.01;  K = 66: 50 k 0.85 / 0.38 / 0.51
-//   five               K = 16: 200 k in one 0.83 / 0.84 / 0.89, 800 k in eight 0.80 / 1.03 / 0.90;  K = 32: 200 k in eight 0.62 / 0.99 / 1.04
+//   five               K = 4: 800 k 0.75 / 0.42 / 0.58 and 0.77 / 0.65 / 0.72;  K = 8: 200 k 0.78 / 0.48 / 0.65 and 0.89 / 0.69 / 1.06, 800 k in 160 0.70 /
+//                      0.79 / 1.07;  K = 16: 50 k 0.84 / 0.53 / 1.16 and 0.84 / 0.90 / 1.15, in 25 0.86 / 0.81 / 1.36;  K = 24: 20 k 0.86 / 0.49 / 1.04 and
+//                      0.78 / 0.78 / 1.65
 //   learned, three     K = 8: 50 k in one 0.84;  K = 16: 50 k in ten 0.78, 200 k in 40 0.96;  K = 24: 50 k in 25 0.84
 //   learned, four      K = 8: 50 k in ten 0.87, 200 k in 40 0.97;  K = 16: 50 k in 25 0.84
 //   learned, sorted in one launch (up to kSmallTree points; three / four)  K = 10: 3 k in one row split 0.63 / 0.64, 5 k in five 0.90 / 0.90, 10 k in
@@ -494,7 +520,9 @@ extern "C" int fgc_knn_groups_ahead(int64_t n_vert, int32_t n_coords, int64_t n_
         else if (n_coords == 4) least = mean >= 4000 ? 8 : (mean >= 1500 ? 16 : least);
         else least = mean >= 15000 ? 8 : (mean >= 4000 ? 16 : (mean >= 1500 ? 24 : least));
     } else if (n_coords == 5) {
-        if (n_vert >= 200000) least = mean >= 100000 ? 16 : (mean >= 15000 ? 32 : least);
+        if (n_vert >= 20000 && mean >= 2000) least = n_vert >= 50000 ? 16 : 24;
+        if (n_vert >= 200000 && large) least = 8;
+        if (n_vert >= 800000 && mean >= 4000) least = large ? 4 : 8;
     } else if (n_coords == 4) {
         if (n_vert >= 50000) least = 66;
         if (n_vert >= 100000 && large) least = 40;

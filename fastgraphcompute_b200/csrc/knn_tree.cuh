@@ -48,18 +48,21 @@ constexpr int kRadixBins = 1 << kRadixBits;
 __host__ __device__ inline int64_t tree_base(int64_t ev_begin, int64_t e, int shift) { return (ev_begin >> shift) + e; }
 
 constexpr int kGroupDims = 5;          // searches by groups take up to so many coordinates,
-constexpr int kHalfDims = 5;           // and in so many they look at boxes of 16 points
+constexpr int kApartDims = 5;          // and in so many they look at boxes of 16 points, and read from arrays apart
 
 struct TreeLayout {
     size_t keys[2], ids[2], hist, hist_sums, box[3], end;
-    size_t listed, half_box, leaf_info;      // of the search by groups, in the place of the keys when they are sorted
+    size_t listed, leaf_info;                // of the search by groups, in the place of the keys when they are sorted
+    // in five coordinates the boxes of leaves and of their halves and the points once more, lower corners, upper corners and what is fifth
+    // apart: a warp that reads 32 in a row touches a quarter of the lines
+    size_t box_lo, box_hi, box_e, half_lo, half_hi, half_e, point_a, point_e;
     int64_t n_box[3];      // slots per level: leaves, nodes, top nodes
     int rounds;            // a CTA of a radix pass takes 256 * rounds keys
     int tiles;
     int key_dims, bits;    // Hilbert curve: dimensions and bits per dimension
     int passes;
     bool fits;
-    bool groups;           // room for half_box and leaf_info: row splits of thirty points or more, or few of them
+    bool groups;           // room for these: row splits of thirty points or more, or few of them
 };
 
 inline TreeLayout tree_layout(const KnnWorkspace &w, int64_t n_vert, int n_coords, int64_t n_rs)
@@ -94,9 +97,20 @@ inline TreeLayout tree_layout(const KnnWorkspace &w, int64_t n_vert, int n_coord
     // the sections from the cell table up to the original ids are the tree's to use
     t.fits = t.end <= w.sorig && t.bits >= 1 && entries < ((size_t)1 << 31);
     t.listed = t.keys[0];
-    t.half_box = align_up(t.listed + 4 * (size_t)n_vert, 256);
-    t.leaf_info = align_up(t.half_box + (n_coords == kHalfDims ? sizeof(float4) * 4 * w.nv * (size_t)t.n_box[0] : 0), 256);
-    t.groups = n_coords <= kGroupDims && t.leaf_info + (sizeof(int4) + 4 * sizeof(int2)) * (size_t)t.n_box[0] <= t.ids[0];
+    t.leaf_info = align_up(t.listed + 4 * (size_t)n_vert, 256);
+    const size_t leaves = n_coords == kApartDims ? (size_t)t.n_box[0] : 0, halves = 2 * leaves, points = n_coords == kApartDims ? (size_t)n_vert : 0;
+    off = t.end;
+    auto section = [&](size_t bytes) { const size_t at = off; off = align_up(off + bytes, 256); return at; };
+    t.box_lo = section(sizeof(float4) * leaves);
+    t.box_hi = section(sizeof(float4) * leaves);
+    t.box_e = section(sizeof(float2) * leaves);
+    t.half_lo = section(sizeof(float4) * halves);
+    t.half_hi = section(sizeof(float4) * halves);
+    t.half_e = section(sizeof(float2) * halves);
+    t.point_a = section(sizeof(float4) * points);
+    t.point_e = section(sizeof(float) * points);
+    t.groups = n_coords <= kGroupDims && t.fits && off <= w.sorig &&
+               t.leaf_info + (sizeof(int4) + 4 * sizeof(int2)) * (size_t)t.n_box[0] <= t.ids[0];
     return t;
 }
 

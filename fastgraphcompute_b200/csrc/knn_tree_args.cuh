@@ -5,12 +5,21 @@
 
 namespace fgc {
 
+// Boxes of up to five coordinates: corners of the first four, both of the fifth.
+struct BoxArrays {
+    const float4 *lo, *hi;
+    const float2 *e;
+};
+
 struct TreeArgs {
     const float4 *scoords;
     const int *sorig;
     const uint8_t *sflag;      // nullptr: no direction restriction
     const float4 *box[3];      // leaves, nodes, top nodes
-    const float4 *half_box;    // halves of leaves (16 points)
+    // in five coordinates: boxes of leaves and of their halves (16 points), points in curve order
+    BoxArrays leaves, halves;
+    const float4 *point_a;
+    const float *point_e;
     const int64_t *row_splits;
     KnnGrid *grid;
     KnnTree *tree;

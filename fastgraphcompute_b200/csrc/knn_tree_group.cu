@@ -22,10 +22,12 @@
 // instructions a query: some 250 for its list and its boxes, 350 for 16 leaves, 400 for the sort and the row) and the latency of list, box and
 // point one after the other, hence the many warps; k_tree_groups the shared-memory pipe (0.83; the counting's atomics) and issue slots
 // (0.71; 240 instructions a query; 72 registers, some of them spilled, 28 one-warp CTAs an SM).
-// Whole forward in ms, before this split of the lists and of the visits / now / one query at a time / the grid, without a second look in the
-// first three: 6.4 M uniform points in three coordinates, K = 64 13.5 / 10.1 / 21.5 / 18.3; 1.6 M learned ones in four, K = 40 6.6 / 4.8 / 9.4 /
-// 8.4; 800 k skewed in three, K = 128 3.0 / 2.3 / 4.6 / 18.8; a million normal ones in five, K = 40 15.0 / 13.4 / 18.2 / 26.4.  The second look adds
-// 0.85, 0.4, 1.5 and 0.4.
+// In five coordinates k_tree_rows was bound by the lines that its reads touch (shared-memory and L1 pipe 0.97, issue slots 0.40): boxes of 64 bytes and
+// points of 32, of which 40 and 20 are used.  Boxes, halves and points in arrays apart: a million normal points, K = 40 12.0 -> 7.7 ms.
+// Whole forward in ms, before the lists for eight queries / now / one query at a time / the grid, without a second look in the
+// first three: 6.4 M uniform points in three coordinates, K = 64 13.5 / 10.1 / 21.5 / 18.3; 1.6 M learned ones in four, K = 40 6.6 / 4.5 / 9.4 /
+// 8.4; 800 k skewed in three, K = 128 3.0 / 2.2 / 4.6 / 18.8; a million normal ones in five, K = 40 15.0 / 7.5 / 18.2 / 26.4.  The second look adds
+// 0.85, 0.4, 1.0 and 0.4.
 //
 // Other splits of the work, measured on the first and the third of these when they took 13.9 and 3.2: one kernel, a lane per query, the points of a leaf read from
 // shared memory by all 32 lanes (15.5; broadcast 16-byte loads write 512 bytes back each, four cycles an SM); candidates of all
@@ -74,6 +76,26 @@ __device__ __forceinline__ float box_box_sq(const float4 (&lo)[NV], const float4
         acc = __fadd_rn(acc, __fmul_rn(g3, g3));
     }
     return acc;
+}
+
+// The same for a leaf; in five coordinates from the arrays apart.
+template <int NV, int DC>
+__device__ __forceinline__ float leaf_box_sq(const float4 (&lo)[NV], const float4 (&hi)[NV], const TreeArgs &a, int64_t at)
+{
+    if constexpr (DC < kApartDims) {
+        return box_box_sq<NV>(lo, hi, a.box[0] + 2 * at);
+    } else {
+        const float4 bl = __ldg(a.leaves.lo + at), bh = __ldg(a.leaves.hi + at);
+        const float2 e = __ldg(a.leaves.e + at);
+        const float g0 = fmaxf(fmaxf(__fsub_rn(bl.x, hi[0].x), __fsub_rn(lo[0].x, bh.x)), 0.f);
+        const float g1 = fmaxf(fmaxf(__fsub_rn(bl.y, hi[0].y), __fsub_rn(lo[0].y, bh.y)), 0.f);
+        const float g2 = fmaxf(fmaxf(__fsub_rn(bl.z, hi[0].z), __fsub_rn(lo[0].z, bh.z)), 0.f);
+        const float g3 = fmaxf(fmaxf(__fsub_rn(bl.w, hi[0].w), __fsub_rn(lo[0].w, bh.w)), 0.f);
+        const float g4 = fmaxf(fmaxf(__fsub_rn(e.x, hi[NV - 1].x), __fsub_rn(lo[NV - 1].x, e.y)), 0.f);
+        float acc = __fadd_rn(__fadd_rn(__fmul_rn(g0, g0), __fmul_rn(g1, g1)), __fmul_rn(g2, g2));
+        acc = __fadd_rn(acc, __fmul_rn(g3, g3));
+        return __fadd_rn(acc, __fmul_rn(g4, g4));
+    }
 }
 
 // ----------------------------------------------------------------------------- bounds and lists
@@ -136,7 +158,8 @@ __device__ __forceinline__ void bound_leaf(const TreeArgs &a, const int slot)
         return;
     }
     const int n_leaf = (n_e + 31) >> 5, n_node = (n_e + 1023) >> 10, n_top = (n_e + 32767) >> 15;
-    const float4 *leaf_box = a.box[0] + (size_t)tree_base(ev_begin, e, 5) * (2 * NV);
+    const int64_t leaf0 = tree_base(ev_begin, e, 5);
+    const float4 *leaf_box = a.box[0] + (size_t)leaf0 * (2 * NV);
     const float4 *node_box = a.box[1] + (size_t)tree_base(ev_begin, e, 10) * (2 * NV);
     const float4 *top_box = a.box[2] + (size_t)tree_base(ev_begin, e, 15) * (2 * NV);
     const int rel_q = own_leaf * 32 + lane;
@@ -223,7 +246,7 @@ __device__ __forceinline__ void bound_leaf(const TreeArgs &a, const int slot)
                 if (lane == (int)(m & 31u)) nkey = kNoBox;
                 const int leaf = node_of[k] * 32 + lane;
                 if (leaf < n_leaf)
-                    lkey[k] = (__float_as_uint(box_box_sq<NV>(mid, mid, leaf_box + (size_t)leaf * (2 * NV))) & ~255u) |
+                    lkey[k] = (__float_as_uint(leaf_box_sq<NV, DC>(mid, mid, a, leaf0 + leaf)) & ~255u) |
                               (uint32_t)(k << 5 | lane);
             }
         }
@@ -353,7 +376,7 @@ __device__ __forceinline__ void bound_leaf(const TreeArgs &a, const int slot)
     auto take_node = [&](int node) {
         const int leaf = node * 32 + lane;
         bool want = false;
-        if (leaf < n_leaf) want = box_box_sq<NV>(glo, ghi, leaf_box + (size_t)leaf * (2 * NV)) <= tmax;
+        if (leaf < n_leaf) want = leaf_box_sq<NV, DC>(glo, ghi, a, leaf0 + leaf) <= tmax;
         const unsigned m = __ballot_sync(FGC_FULL_MASK, want);
         const int at = n + __popc(m & lanemask_lt());
         if (want && at < a.list_cap) list[at] = leaf;
@@ -416,19 +439,24 @@ __device__ __forceinline__ void bound_leaf(const TreeArgs &a, const int slot)
         for (int i0 = 0; i0 < n; i0 += 32) {
             const bool in = i0 + lane < n;
             const int leaf = in ? list[i0 + lane] : 0;
-            float box[8 * NV];
-#pragma unroll
-            for (int v = 0; v < 2 * NV; v++) {
-                const float4 b = __ldg(leaf_box + (size_t)leaf * (2 * NV) + v);
-                box[4 * v] = b.x; box[4 * v + 1] = b.y; box[4 * v + 2] = b.z; box[4 * v + 3] = b.w;
+            float4 bl, bh;
+            float2 be = make_float2(0.f, 0.f);
+            if constexpr (DC < kApartDims) {
+                bl = __ldg(leaf_box + 2 * (size_t)leaf);
+                bh = __ldg(leaf_box + 2 * (size_t)leaf + 1);
+            } else {
+                bl = __ldg(a.leaves.lo + leaf0 + leaf);
+                bh = __ldg(a.leaves.hi + leaf0 + leaf);
+                be = __ldg(a.leaves.e + leaf0 + leaf);
             }
+            const float box_lo[5] = {bl.x, bl.y, bl.z, bl.w, be.x}, box_hi[5] = {bh.x, bh.y, bh.z, bh.w, be.y};
             int bits = 0;
 #pragma unroll
             for (int p = 0; p < 4; p++) {
                 float acc = 0.f;
 #pragma unroll
                 for (int c = 0; c < DC; c++) {
-                    const float g = fmaxf(fmaxf(__fsub_rn(box[c], s_part[p][DC + c]), __fsub_rn(s_part[p][c], box[4 * NV + c])), 0.f);
+                    const float g = fmaxf(fmaxf(__fsub_rn(box_lo[c], s_part[p][DC + c]), __fsub_rn(s_part[p][c], box_hi[c])), 0.f);
                     acc = c == 0 ? __fmul_rn(g, g) : __fadd_rn(acc, __fmul_rn(g, g));
                 }
                 const bool want = in && acc <= s_part[p][2 * DC];
@@ -644,15 +672,15 @@ struct RowPoint {
     float e;              // the fifth
 };
 template <int DC>
-__device__ __forceinline__ RowPoint<DC> row_point(const float4 *__restrict__ scoords, int j)
+__device__ __forceinline__ RowPoint<DC> row_point(const TreeArgs &a, int j)
 {
     RowPoint<DC> p;
     p.e = 0.f;
-    if constexpr (DC <= 4) {
-        p.a = read_four(scoords + j);
+    if constexpr (DC < kApartDims) {
+        p.a = read_four(a.scoords + j);
     } else {
-        p.a = read_four(scoords + 2 * (size_t)j);
-        p.e = __ldg(reinterpret_cast<const float *>(scoords + 2 * (size_t)j + 1));
+        p.a = read_four(a.point_a + j);
+        p.e = __ldg(a.point_e + j);
     }
     return p;
 }
@@ -682,14 +710,24 @@ __device__ __forceinline__ float gap_sq(float lo, float hi, float x)
     return __fmul_rn(g, g);
 }
 template <int DC>
-__device__ __forceinline__ float row_box(const RowPoint<DC> &q, const float4 *__restrict__ box)
+__device__ __forceinline__ float row_gap(const RowPoint<DC> &q, const float4 &lo, const float4 &hi)
 {
-    constexpr int NV = DC <= 4 ? 1 : 2;
-    const float4 lo = read_four(box), hi = read_four(box + NV);
     float acc = __fadd_rn(__fadd_rn(gap_sq(lo.x, hi.x, q.a.x), gap_sq(lo.y, hi.y, q.a.y)), gap_sq(lo.z, hi.z, q.a.z));
     if constexpr (DC >= 4) acc = __fadd_rn(acc, gap_sq(lo.w, hi.w, q.a.w));
-    if constexpr (DC >= 5) acc = __fadd_rn(acc, gap_sq(__ldg(&box[1].x), __ldg(&box[3].x), q.e));
     return acc;
+}
+// (with up to four coordinates the corners of a box lie side by side: one address; apart they cost a register, 7.15 -> 8.0 ms for 6.4 M
+// uniform points in three, K = 64)
+template <int DC>
+__device__ __forceinline__ float row_box(const RowPoint<DC> &q, const float4 *__restrict__ box)
+{
+    return row_gap<DC>(q, read_four(box), read_four(box + 1));
+}
+template <int DC>
+__device__ __forceinline__ float row_box(const RowPoint<DC> &q, const BoxArrays &box, int64_t at)
+{
+    const float2 e = __ldg(box.e + at);
+    return __fadd_rn(row_gap<DC>(q, read_four(box.lo + at), read_four(box.hi + at)), gap_sq(e.x, e.y, q.e));
 }
 
 // A store, or a count, in shared memory under a predicate (as a branch it takes three instructions more).
@@ -714,9 +752,8 @@ k_tree_rows(const TreeArgs a)
 {
     chain_wait();
     chain_release();
-    constexpr int NV = DC <= 4 ? 1 : 2;
     constexpr int ROWS = RowShape<R>::ROWS, MOST = ROWS * 32;
-    constexpr bool HALVES = DC >= kHalfDims;
+    constexpr bool HALVES = DC >= kApartDims;
     constexpr int STEP = HALVES ? 8 : 4;
     __shared__ float2 s_pairs[kRowWarps][MOST];
     __shared__ __align__(16) int s_wanted[kRowWarps][kWanted];
@@ -750,13 +787,12 @@ k_tree_rows(const TreeArgs a)
     t = writes ? fminf(t, 3.402823466e38f) : kNoQuery;
     const int qi = ev_begin + min(rel_q, n_e - 1);
     const int *__restrict__ list = a.list + (size_t)(row >> 5) * a.list_room + part.x;
-    const float4 *__restrict__ leaf_box = a.box[0] + (size_t)(slot - (info.x >> 5)) * (2 * NV);
-    const float4 *__restrict__ half_box = a.half_box + (size_t)(slot - (info.x >> 5)) * (4 * NV);
-    const float4 *__restrict__ scoords = a.scoords;
+    const int64_t leaf0 = slot - (info.x >> 5);                  // first of the row split
+    const float4 *__restrict__ leaf_box = a.box[0] + 2 * leaf0;  // (not in five coordinates)
     float2 *pairs = s_pairs[w];
     const uint32_t pairs_at = (uint32_t)__cvta_generic_to_shared(pairs);
     int *wanted = s_wanted[w], *near = s_near[HALVES ? w : 0];
-    const RowPoint<DC> x = row_point<DC>(scoords, qi);
+    const RowPoint<DC> x = row_point<DC>(a, qi);
     int m = 0;                               // points kept
     uint32_t left_out = kNoBox;              // the last distance at which a point was left out that equals the bound
     auto keep = [&](const RowPoint<DC> &c, int j) {
@@ -800,7 +836,7 @@ k_tree_rows(const TreeArgs a)
         j = first + (HALVES ? lane & 15 : lane);
         j = j < ev_end ? j : qi;
         if (!FGC_DBG_OK(j >= ev_begin && j < a.n_vert, &a.grid->status)) j = qi;
-        c = row_point<DC>(scoords, j);
+        c = row_point<DC>(a, j);
         if constexpr (FLAGS) { const uint8_t f = a.sflag[j]; if (f == 1 || f == 2) j = qi; }
     };
     auto visit_wanted = [&]() {
@@ -836,7 +872,7 @@ k_tree_rows(const TreeArgs a)
         if (i < n_near) {
             const int half = near[(near0 + i) & 63] * 2 + (lane & 1);
             first = ev_begin + half * 16;
-            want = row_box<DC>(x, half_box + (size_t)half * (2 * NV)) <= t;
+            if constexpr (HALVES) want = row_box<DC>(x, a.halves, 2 * leaf0 + half) <= t;
         }
         const unsigned mask = __ballot_sync(FGC_FULL_MASK, want);
         const int at = n_wanted + __popc(mask & lanemask_lt());
@@ -851,7 +887,8 @@ k_tree_rows(const TreeArgs a)
         bool want = false;
         if (base + lane < n_list) {
             leaf = __ldg(list + base + lane);
-            want = row_box<DC>(x, leaf_box + (size_t)leaf * (2 * NV)) <= t;
+            if constexpr (DC < kApartDims) want = row_box<DC>(x, leaf_box + 2 * (size_t)leaf) <= t;
+            else want = row_box<DC>(x, a.leaves, leaf0 + leaf) <= t;
         }
         const unsigned mask = __ballot_sync(FGC_FULL_MASK, want);
         if constexpr (HALVES) {
@@ -1023,7 +1060,11 @@ int fgc::knn_search_tree_groups(int64_t n_vert, int32_t n_coords, const int64_t 
     a.n_slots = (int)T.n_box[0];
     if (!T.groups) return FGC_ERR_WORKSPACE;
     a.listed = (int *)((char *)workspace + T.listed);
-    a.half_box = (const float4 *)((char *)workspace + T.half_box);
+    const char *ws = (const char *)workspace;                    // (empty with up to four coordinates)
+    a.leaves = {(const float4 *)(ws + T.box_lo), (const float4 *)(ws + T.box_hi), (const float2 *)(ws + T.box_e)};
+    a.halves = {(const float4 *)(ws + T.half_lo), (const float4 *)(ws + T.half_hi), (const float2 *)(ws + T.half_e)};
+    a.point_a = (const float4 *)(ws + T.point_a);
+    a.point_e = (const float *)(ws + T.point_e);
     a.leaf_info = (int4 *)((char *)workspace + T.leaf_info);
     a.leaf_part = (int2 *)(a.leaf_info + T.n_box[0]);
     if (n_coords <= 3) FGC_RETURN_IF_CUDA((launch_tree<1, 3>(a, scratch, s)));
