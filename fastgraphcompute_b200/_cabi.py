@@ -40,7 +40,7 @@ KERNELS_KNN_BWD_SORTED = 7   # reverse graph (6) + gather (1)
 KERNELS_GRAVNET_PROJECT = 2    # forward + backward of the fused input projections
 KERNELS_GRAVNET_FWD = 1
 KERNELS_GRAVNET_BWD = 1
-KERNELS_OC_PREPARE = 8          # + the radix sort's own kernels
+KERNELS_OC_PREPARE = 15         # eight of them passes of the sort, which return at once where no digit differs
 
 STATUS_NONFINITE = 1
 STATUS_BAD_ROW_SPLITS = 2

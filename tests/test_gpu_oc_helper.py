@@ -127,3 +127,25 @@ def test_select_with_default_gradient():
             if ic[a, b] >= 0:
                 ref[ic[a, b]] += uc[a, b]
     parity.assert_grad_close(feat.grad.cpu().numpy(), ref.numpy(), what="select_with_default grad")
+
+
+@pytest.mark.parametrize("n", [1, 4095, 4096, 4097, 40961, 300001])
+@pytest.mark.parametrize("kind", ["one byte", "all bytes", "largest", "noise", "one object", "ascending", "gaps"])
+def test_sort_of_the_truth_indexes(n, kind):
+    """Passes of the sort that are taken and left out, at the edges of its tiles and with more tiles than one look-back reads."""
+    rng = np.random.RandomState(n % 1000)
+    ids = {"one byte": rng.randint(-3, 200, n), "all bytes": rng.randint(0, 2 ** 62, 300)[rng.randint(0, 300, n)] * 2 + 1,
+           "largest": np.where(rng.rand(n) < 0.3, 2 ** 63 - 1, rng.randint(-2, 4, n)), "noise": np.full(n, -1),
+           "one object": np.zeros(n), "ascending": np.arange(n) * 255 // n, "gaps": rng.randint(0, 5, n) << 24}[kind].astype(np.int64)
+    rs = np.array([0, n // 3, n // 3, n], np.int64)
+    M, _, per = run(ids, rs, calc_m_not=False)
+    split = (np.arange(n) >= n // 3).astype(np.int64) * 2
+    order = np.lexsort((np.arange(n), split, ids))
+    order = order[ids[order] >= 0]
+    head = np.ones(len(order), bool)
+    head[1:] = (ids[order][1:] != ids[order][:-1]) | (split[order][1:] != split[order][:-1])
+    rows = np.split(order, np.nonzero(head)[0][1:]) if len(order) else []
+    assert M.shape[0] == len(rows) and M.shape[1] == max([len(r) for r in rows], default=0)
+    for got, want in zip(M, rows):
+        assert np.array_equal(got[:len(want)], want) and (got[len(want):] == -1).all()
+    assert np.array_equal(per, [sum(split[r[0]] == e for r in rows) for e in range(3)])
