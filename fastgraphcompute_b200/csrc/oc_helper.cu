@@ -398,88 +398,108 @@ k_oc_fill_m(const OcHeader *__restrict__ h, const int *__restrict__ vals_a, cons
     }
 }
 
-// M_not, one warp per run of kOcRun tiles of kOcTile consecutive columns of one row.  The j-th
-// non-member is  row start + j + t(j),  t(j) = number of members with at most j non-members
-// before them.  t is non-decreasing in j: the warp searches it once for the first column of
-// its run (uniform loads) and then walks the member list forward, tile by tile -- every member
-// that falls into the tile raises t by one from its column on.  A tile with more than
-// kOcLinear members (a dense object) lets every column search between the tile's bounds
-// instead.  VEC2: rows are 16-byte aligned (even row length, aligned base) and a lane stores
-// two adjacent columns at once.
-constexpr int kOcTile = 512;
-constexpr int kOcRun = 4;
-constexpr int kOcLinear = 16;
+// M_not, one warp per run of kOcRun consecutive columns of one row, kOcStep at a time.  The j-th non-member is  row start + j + t(j),
+// t(j) = number of members with at most j non-members before them, which is non-decreasing in j: the warp searches it once for
+// the first column of its run and then walks the member list forward.  The lanes hold the next 32 members: a vote says how many of
+// them fall into the step's columns, and each of those is compared with a lane's columns.  Where 32 members are not enough for
+// a step (a dense object) every column searches instead.  VEC2: rows are 16-byte aligned (even row length, aligned base) and a
+// lane stores two adjacent columns at once.
+// Writing bounds it: 3200 rows of 100 000 columns 350 us = 7.3 TB/s (a plain fill of the matrix 339 us).  With every member compared
+// with all columns of 512 and 64-bit sums it was 413 us, bound by its 34 instructions a column, with 64 columns a step 396; the search by
+// 32 probes instead of halves, which a run waits for: 384 -> 350.  Runs of 2048 / 4096 / 8192 columns 358 / 369 / 382, 512 columns a
+// step (runs of 2048) 353.
+constexpr int kOcRun = 1024, kOcStep = 256;
 
 template <bool VEC2>
 __global__ void __launch_bounds__(256)
 k_oc_fill_m_not(const OcHeader *__restrict__ h, const int *__restrict__ vals_a, const int *__restrict__ vals_b,
-                const int *__restrict__ obj_start,
-                const int *__restrict__ obj_split, const int64_t *__restrict__ rs, int64_t n_unique,
+                const int *__restrict__ obj_start, const int *__restrict__ obj_split, const int64_t *__restrict__ rs, int64_t n_unique,
                 int n_maxrs, int64_t *__restrict__ M_not)
 {
     const int lane = threadIdx.x & 31;
     const int *__restrict__ vals = oc_in_b(h) ? vals_b : vals_a;
-    constexpr int kSpan = kOcTile * kOcRun;
-    const int runs_per_row = (n_maxrs + kSpan - 1) / kSpan;
+    const int runs_per_row = (int)(((int64_t)n_maxrs + kOcRun - 1) / kOcRun);
     const int64_t n_runs = n_unique * runs_per_row;
     const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (int64_t run = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; run < n_runs; run += n_warps) {
         const int64_t k = run / runs_per_row;
-        const int run0 = (int)(run - k * runs_per_row) * kSpan;
+        const int64_t run0 = (run - k * runs_per_row) * kOcRun;
         const int beg = obj_start[k], cnt = obj_start[k + 1] - beg;
         const int e = obj_split[k];
-        const int64_t row_start = rs[e];
-        const int n_non = (int)(rs[e + 1] - row_start) - cnt;
+        const int row_start = (int)rs[e];                                 // ids have 31 bits
+        const int n_non = (int)rs[e + 1] - row_start - cnt;
         // member i (a global point id) has  members[i] - row_start - i  non-members before it
         const int *__restrict__ members = vals + beg;
-        const int rs32 = (int)row_start;
         auto members_up_to = [&](int j, int lo, int hi) {
             while (lo < hi) {
                 const int mid = (lo + hi) >> 1;
-                if (members[mid] - rs32 - mid <= j) lo = mid + 1; else hi = mid;
+                if (members[mid] - row_start - mid <= j) lo = mid + 1; else hi = mid;
             }
             return lo;
         };
         int64_t *__restrict__ row = M_not + k * (int64_t)n_maxrs;
-        int t_first = members_up_to(run0, 0, cnt);
-        for (int j0 = run0; j0 < run0 + kSpan && j0 < n_maxrs; j0 += kOcTile) {
-            const int j_end = j0 + kOcTile < n_maxrs ? j0 + kOcTile : n_maxrs;
-            constexpr int PER = kOcTile / 32;           // columns per lane
-            auto column = [&](int u) { return VEC2 ? j0 + 2 * lane + 64 * (u >> 1) + (u & 1) : j0 + lane + 32 * u; };
-            int t_of[PER];
-#pragma unroll
-            for (int u = 0; u < PER; u++) t_of[u] = t_first;
-            int t = t_first;
-            for (; t < cnt && t - t_first <= kOcLinear; t++) {
-                const int b = members[t] - rs32 - t;
-                if (b >= j_end) break;
-#pragma unroll
-                for (int u = 0; u < PER; u++) t_of[u] += column(u) >= b ? 1 : 0;
+        const int run_end = (int)min(run0 + kOcRun, (int64_t)n_maxrs);
+        // members before the columns, found by 32 probes at a time
+        int t = 0;
+        for (int end = cnt; t < end;) {
+            const int step = (end - t + 31) >> 5, at = t + lane * step;
+            const bool up_to = at < end && members[at] - row_start - at < (int)run0;
+            const int found = __popc(__ballot_sync(FGC_FULL_MASK, up_to));
+            if (found == 0) break;
+            if (step == 1) { t += found; break; }
+            end = min(end, t + found * step);
+            t += (found - 1) * step + 1;
+        }
+        int held = t;                                                     // the first member that a lane holds
+        auto hold = [&]() { return held + lane < cnt ? members[held + lane] - row_start - held - lane : 0x7fffffff; };
+        int next = hold();
+        for (int j0 = (int)run0; j0 < run_end; j0 += kOcStep) {
+            constexpr int PER = kOcStep / 32;                             // columns per lane
+            const int j1 = run_end - j0 < kOcStep ? run_end : j0 + kOcStep;
+            const int c0 = j0 + (VEC2 ? 2 * lane : lane);
+            auto column = [&](int u) { return VEC2 ? c0 + 64 * (u >> 1) + (u & 1) : c0 + 32 * u; };
+            int in = __popc(__ballot_sync(FGC_FULL_MASK, next < j1));
+            if (in == 32 && held < t) {
+                held = t;
+                next = hold();
+                in = __popc(__ballot_sync(FGC_FULL_MASK, next < j1));
             }
-            if (t - t_first > kOcLinear) {
-                t = members_up_to(j_end - 1, t, cnt);
+            int id[PER];
 #pragma unroll
-                for (int u = 0; u < PER; u++) t_of[u] = members_up_to(column(u), t_first, t);
+            for (int u = 0; u < PER; u++) id[u] = row_start + t + column(u);
+            if (in < 32) {
+                for (int i = t - held; i < in; i++) {
+                    const int b = __shfl_sync(FGC_FULL_MASK, next, i) - c0;
+#pragma unroll
+                    for (int u = 0; u < PER; u++) id[u] += column(u) - c0 >= b ? 1 : 0;
+                }
+                t = held + in;
+            } else {
+                const int t1 = members_up_to(j1 - 1, t, cnt);
+#pragma unroll
+                for (int u = 0; u < PER; u++) id[u] += members_up_to(column(u), t, t1) - t;
+                held = t = t1;
+                next = hold();
             }
-            if (VEC2) {
+            int64_t *__restrict__ out = row + c0;
+            if (j0 + kOcStep <= min(run_end, n_non)) {
 #pragma unroll
-                for (int u = 0; u < PER; u += 2) {
-                    const int j = column(u);
-                    if (j < j_end) {    // j_end is even here, so j + 1 < j_end as well
-                        longlong2 v;
-                        v.x = j < n_non ? row_start + j + t_of[u] : -1;
-                        v.y = j + 1 < n_non ? row_start + j + 1 + t_of[u + 1] : -1;
-                        *reinterpret_cast<longlong2 *>(row + j) = v;
-                    }
+                for (int u = 0; u < PER; u += VEC2 ? 2 : 1) {
+                    if (VEC2) *reinterpret_cast<uint4 *>(out + 32 * u) = make_uint4((uint32_t)id[u], 0u, (uint32_t)id[u + 1], 0u);
+                    else out[32 * u] = (int64_t)(uint32_t)id[u];
                 }
             } else {
 #pragma unroll
-                for (int u = 0; u < PER; u++) {
-                    const int j = column(u);
-                    if (j < j_end) row[j] = j < n_non ? row_start + j + t_of[u] : -1;
+                for (int u = 0; u < PER; u += VEC2 ? 2 : 1) {
+                    const int64_t v = column(u) < n_non ? (int64_t)(uint32_t)id[u] : (int64_t)-1;
+                    if (column(u) >= j1) continue;
+                    if (VEC2)                      // an even row length: the second column is in the row if the first is
+                        *reinterpret_cast<longlong2 *>(out + 32 * u) =
+                            make_longlong2(v, column(u + 1) < n_non ? (int64_t)(uint32_t)id[u + 1] : (int64_t)-1);
+                    else
+                        out[32 * u] = v;
                 }
             }
-            t_first = t;
         }
     }
 }
@@ -590,9 +610,9 @@ extern "C" int fgc_oc_fill(const void *workspace, size_t workspace_bytes, int64_
     }
     if (out_M_not_or_null && mn_total > 0) {
         if (n_maxrs > 0x7fffffff) return FGC_ERR_TOO_LARGE;
-        const int64_t runs = n_unique * ceil_div64(n_maxrs, kOcTile * kOcRun);
-        int64_t blocks = ceil_div64(runs, 8);           // 8 warps per CTA, one run of tiles per warp and pass
-        if (blocks > fgc::sm_count() * 32) blocks = fgc::sm_count() * 32;
+        const int64_t runs = n_unique * ceil_div64(n_maxrs, kOcRun);
+        int64_t blocks = ceil_div64(runs, 8);           // 8 warps per CTA, one run per warp and pass
+        if (blocks > 0x7fffffff) blocks = 0x7fffffff;
         if ((n_maxrs & 1) == 0 && ((uintptr_t)out_M_not_or_null & 15) == 0)
             k_oc_fill_m_not<true><<<(unsigned)blocks, 256, 0, s>>>(h, vals_a, vals_b, obj_start, obj_split, row_splits, n_unique,
                                                                    (int)n_maxrs, out_M_not_or_null);

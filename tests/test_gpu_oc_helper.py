@@ -149,3 +149,19 @@ def test_sort_of_the_truth_indexes(n, kind):
     for got, want in zip(M, rows):
         assert np.array_equal(got[:len(want)], want) and (got[len(want):] == -1).all()
     assert np.array_equal(per, [sum(split[r[0]] == e for r in rows) for e in range(3)])
+
+
+@pytest.mark.parametrize("n", [255, 256, 257, 1023, 1025, 2049, 70002])
+@pytest.mark.parametrize("share", [0.002, 0.1, 0.13, 0.5, 0.95])
+def test_points_of_no_object(n, share):
+    """M_not with few members in the columns that are written at a time, with about as many as the lanes hold, and with more."""
+    rng = np.random.RandomState(n)
+    ids = np.where(rng.rand(n) < share, 0, 1 + rng.randint(0, 2, n)).astype(np.int64)
+    ids[n // 2:n // 2 + n // 8] = 0                                     # members without others between them
+    for rs in ([0, n], [0, n // 3, n]):
+        M, M_not, _ = run(ids, np.array(rs))
+        for k in range(M.shape[0]):
+            members = M[k][M[k] >= 0]
+            e = np.searchsorted(rs, members[0], side="right") - 1
+            want = np.setdiff1d(np.arange(rs[e], rs[e + 1]), members)
+            assert np.array_equal(M_not[k][:len(want)], want) and (M_not[k][len(want):] == -1).all()
