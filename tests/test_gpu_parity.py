@@ -1135,3 +1135,47 @@ def test_tree_search_in_a_cuda_graph(forward_flags, monkeypatch):
         graph.replay()
         torch.cuda.synchronize()
         assert torch.equal(idx, ei) and torch.equal(dist, ed)
+
+
+@pytest.mark.parametrize("n", [1, 255, 512, 513, 5001])
+@pytest.mark.parametrize("dims", [1, 2, 3, 5, 8])
+def test_binning_of_odd_sizes(n, dims):
+    """One vote and a search for the row split (32 and 33 of them, empty ones too), arrays that are and are not aligned to 16 bytes,
+    remainders of four numbers and of a CTA's points."""
+    rng = np.random.RandomState(100 * dims + n)
+    x = rng.randn(n, dims).astype(np.float32)
+    for n_splits in (1, 32, 33):
+        rs = np.concatenate([[0], np.sort(rng.randint(0, n + 1, n_splits - 1)), [n]]).astype(np.int64)
+        want = oracle.bin_by_coordinates(x, rs, n_bins=np.array([3], np.int64))
+        for shift in (0, 1):
+            part = torch.zeros(n * dims + 4, device=DEV)[shift:shift + n * dims].view(n, dims)
+            part.copy_(torch.from_numpy(x))
+            got = fgc.bin_by_coordinates(part, cu(rs), n_bins=torch.tensor([3], device=DEV))
+            for g, w in zip(got, want):
+                assert np.array_equal(g.cpu().numpy(), w)
+
+
+@pytest.mark.parametrize("bins", [40000, 70000, 2 ** 31 - 1, 2 ** 31 + 5])
+def test_binning_of_wide_tables(bins):
+    """Flat indexes below and above 32 bits, by the C interface (without a table to count in)."""
+    from fastgraphcompute_b200 import _cabi
+    n = 1000
+    rng = np.random.RandomState(3)
+    x = cu(rng.rand(n, 2).astype(np.float32))
+    rs, nb = cu(np.array([0, 300, n])), cu(np.array([bins, 5]))
+    params = torch.empty(256, dtype=torch.uint8, device=DEV)
+    idx, flat = torch.full((n, 3), -7, device=DEV), torch.full((n,), -7, device=DEV)
+    stream = torch.cuda.current_stream().cuda_stream
+    total = bins * 5 * 2
+    assert _cabi.lib.fgc_bin_prepare(_cabi.ptr(x), n, 2, 0, None, _cabi.ptr(nb), 2, _cabi.ptr(params), stream) == 0
+    host = _cabi.BinParams.from_buffer_copy(params.cpu().numpy().tobytes())
+    for limit in (total, total - bins):                               # the second: a table that ends early
+        assert _cabi.lib.fgc_bin_assign(_cabi.ptr(x), n, 2, _cabi.ptr(rs), 3, _cabi.ptr(params), 0, limit, _cabi.ptr(idx),
+                                        _cabi.ptr(flat), None, stream) == 0
+        q = (x.cpu().numpy() - np.array(host.shift[:2], np.float32)) / np.float32(host.bin_width) + np.float32(1e-3)
+        b = np.minimum(np.floor(q).astype(np.int64), np.array([bins, 5]) - 1)
+        split = (np.arange(n) >= 300).astype(np.int64)
+        want = (split * bins + b[:, 0]) * 5 + b[:, 1]
+        rows = np.stack([split, b[:, 0], b[:, 1]], 1)
+        rows[want >= limit], want[want >= limit] = 0, 0
+        assert np.array_equal(flat.cpu().numpy(), want) and np.array_equal(idx.cpu().numpy(), rows)
