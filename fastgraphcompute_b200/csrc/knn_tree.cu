@@ -496,11 +496,11 @@ extern "C" int fgc_knn_groups_preferred(int64_t n_vert, int32_t n_coords, int64_
 //                      K = 48: 200 k 0.98 / 0.52 / 0.86 / 0.53 and 0.97 / 0.74 / 0.95 / 0.64, K = 40 1.01;  K = 64: 100 k 0.99 / 0.55 / 0.93 / 0.61 and
 //                      0.97 / 0.63 / 1.06 / 0.60;  K = 66: 50 k 0.83 / 0.59 / 0.82 / 0.63
 //   four               K = 12: 1.6 M in 16 0.85 / 0.74 / 0.61, K = 8 1.03;  K = 16: 400 k 0.95 / 0.43 / 0.61 and 0.90 / 0.75 / 0.76;  K = 24: 400 k in 80
-//                      0.74 / 0.78 / 1.12, 200 k 1.00 / 0.51 / 0.72 and 0.97 / 0.78 / 0.96;  K = 32: 200 k in 40 0.85 / 0.84 / 1.30;  K = 40: 100 k 0.94 /
+//                      0.74 / 0.78 / 1.12, 200 k 1.00 / 0.51 / 0.72 and 0.97 / 0.78 / 0.96;  K = 32: 200 k in 40 0.85 / 0.84 / 1.30 (not taken);  K = 40: 100 k 0.94 /
 //                      0.48 / 0.81 and 0.89 / 0.74 / 1.01;  K = 66: 50 k 0.85 / 0.38 / 0.51
-//   five               K = 4: 800 k 0.75 / 0.42 / 0.58 and 0.77 / 0.65 / 0.72;  K = 8: 200 k 0.78 / 0.48 / 0.65 and 0.89 / 0.69 / 1.06, 800 k in 160 0.70 /
-//                      0.79 / 1.07;  K = 16: 50 k 0.84 / 0.53 / 1.16 and 0.84 / 0.90 / 1.15, in 25 0.86 / 0.81 / 1.36;  K = 24: 20 k 0.86 / 0.49 / 1.04 and
-//                      0.78 / 0.78 / 1.65
+//   five               K = 4: 800 k 0.75 / 0.42 / 0.58 and 0.77 / 0.65 / 0.72;  K = 8: 200 k in eight 0.88 / 0.70 / 1.06, 800 k in 160 0.70 / 0.79 / 1.07;  K = 24:
+//                      50 k in one 0.65 / 0.57 / 1.12;  not taken, since clusters lose more than a tenth: K = 16 there 0.84 / 0.52 / 1.18, 50 k in
+//                      five, K = 40 0.65 / 0.65 / 1.24, in twelve 0.62 / 0.75 / 1.50;  200 k in 40 0.45 / 0.64 / 1.25;  20 k in four 0.74 / 0.59 / 1.55
 //   learned, three     K = 8: 50 k in one 0.84;  K = 16: 50 k in ten 0.78, 200 k in 40 0.96;  K = 24: 50 k in 25 0.84
 //   learned, four      K = 8: 50 k in ten 0.87, 200 k in 40 0.97;  K = 16: 50 k in 25 0.84
 //   learned, sorted in one launch (up to kSmallTree points; three / four)  K = 10: 3 k in one row split 0.63 / 0.64, 5 k in five 0.90 / 0.90, 10 k in
@@ -520,13 +520,12 @@ extern "C" int fgc_knn_groups_ahead(int64_t n_vert, int32_t n_coords, int64_t n_
         else if (n_coords == 4) least = mean >= 4000 ? 8 : (mean >= 1500 ? 16 : least);
         else least = mean >= 15000 ? 8 : (mean >= 4000 ? 16 : (mean >= 1500 ? 24 : least));
     } else if (n_coords == 5) {
-        if (n_vert >= 20000 && mean >= 2000) least = n_vert >= 50000 ? 16 : 24;
-        if (n_vert >= 200000 && large) least = 8;
+        if (n_vert >= 50000 && mean >= 20000) least = n_vert >= 200000 ? 8 : 24;
         if (n_vert >= 800000 && mean >= 4000) least = large ? 4 : 8;
     } else if (n_coords == 4) {
         if (n_vert >= 50000) least = 66;
         if (n_vert >= 100000 && large) least = 40;
-        if (n_vert >= 200000 && mean >= 4000) least = mean >= 20000 ? 24 : 32;
+        if (n_vert >= 200000 && large) least = mean >= 20000 ? 24 : 32;
         if (n_vert >= 400000 && mean >= 4000) least = mean >= 20000 ? 16 : 24;
         if (n_vert >= 800000 && mean >= 4000) least = 16;
         if (n_vert >= 1500000 && large) least = 12;

@@ -496,10 +496,10 @@ def test_lists_of_eight_queries(kind, sizes, D, K, flags):
     (49999, 3, 1, 66, 0, 0), (50000, 3, 1, 66, 0, 1), (50000, 3, 1, 65, 0, 0), (100000, 3, 10, 64, 0, 1), (100000, 3, 11, 64, 0, 0),
     (200000, 3, 20, 48, 0, 1), (200000, 3, 20, 47, 0, 0), (400000, 3, 40, 32, 0, 1), (400000, 3, 100, 32, 0, 0), (400000, 3, 100, 40, 0, 1),
     (800000, 3, 200, 16, 0, 1), (800000, 3, 201, 16, 0, 0), (1500000, 3, 150, 12, 0, 1), (1500000, 3, 150, 11, 0, 0),
-    (100000, 4, 10, 40, 0, 1), (200000, 4, 10, 24, 0, 1), (200000, 4, 11, 24, 0, 0), (200000, 4, 50, 32, 0, 1), (400000, 4, 20, 16, 0, 1),
+    (100000, 4, 10, 40, 0, 1), (200000, 4, 10, 24, 0, 1), (200000, 4, 11, 24, 0, 0), (200000, 4, 20, 32, 0, 1), (200000, 4, 21, 32, 0, 0), (400000, 4, 20, 16, 0, 1),
     (400000, 4, 100, 24, 0, 1), (800000, 4, 200, 16, 0, 1), (800000, 4, 200, 15, 0, 0), (50000, 4, 400, 66, 0, 0),
-    (20000, 5, 10, 24, 0, 1), (20000, 5, 11, 24, 0, 0), (19999, 5, 1, 24, 0, 0), (50000, 5, 25, 16, 0, 1), (50000, 5, 25, 15, 0, 0), (200000, 5, 20, 8, 0, 1),
-    (200000, 5, 21, 8, 0, 0), (800000, 5, 80, 4, 0, 1), (800000, 5, 81, 4, 0, 0), (800000, 5, 200, 8, 0, 1), (800000, 5, 201, 8, 0, 0),
+    (50000, 5, 2, 24, 0, 1), (50000, 5, 3, 24, 0, 0), (49999, 5, 1, 24, 0, 0), (50000, 5, 2, 23, 0, 0), (200000, 5, 10, 8, 0, 1), (200000, 5, 11, 8, 0, 0),
+    (200000, 5, 10, 7, 0, 0), (800000, 5, 80, 4, 0, 1), (800000, 5, 81, 4, 0, 0), (800000, 5, 200, 8, 0, 1), (800000, 5, 201, 8, 0, 0),
     (999, 4, 1, 16, 1, 0), (1000, 4, 1, 16, 1, 1), (1000, 4, 1, 15, 1, 0), (2999, 3, 3, 16, 1, 0), (3000, 3, 10, 8, 1, 1), (3000, 3, 11, 8, 1, 0),
     (24576, 3, 80, 8, 1, 1), (24577, 3, 16, 15, 1, 0), (24577, 3, 6, 16, 1, 1), (24577, 4, 6, 8, 1, 1), (24577, 4, 16, 16, 1, 1),
     (24577, 4, 17, 16, 1, 0), (24576, 3, 1, 7, 1, 0),
