@@ -21,7 +21,7 @@
 // mask and dW / now: 1018 / 640 / 270.  Relative error against 64 bits, library / now: forward 2.0e-7 / 1.2e-7, input gradient 1.4e-7 / 0.8e-7,
 // dW 1.1e-6 (3.5e-7 summed in fp32 by 148 CTAs) / 1.4e-7.
 //
-// What bounds them is the latency of the splitting warps between loads and buffers (0.35 of the issue slots, tensor pipe 0.25).  With four warps instead of
+// What bounds them is the latency of the splitting warps between loads and buffers (400 k rows, 128 to 128: 0.38 to 0.43 of the issue slots, tensor pipe 0.21 to 0.36).  With four warps instead of
 // eight to write results a forward took 80 instead of 59 us (they read, added and wrote one sixteen of columns after the other); with
 // loads of a whole step issued when the last one had been split dW took 126 instead of 106, and 105 instead of 60 for 64 to 64,
 // where half of the threads had no columns.

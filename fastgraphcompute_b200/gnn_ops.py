@@ -1,7 +1,8 @@
 """GravNetOp -- drop-in for fastgraphcompute.gnn_ops.GravNetOp (gnn_ops.py:8-109).
 
 Same constructor, sub-module names (so state_dicts are interchangeable) and
-returned tuple.  The three Linear layers stay torch (cuBLAS); neighbour search
+returned tuple.  The input projections and, on large batches, the output
+layer run in kernels of their own; neighbour search
 and the weighted mean/max aggregation with their backward passes run in
 libfgc_b200.so.
 """
