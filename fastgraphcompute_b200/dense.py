@@ -33,11 +33,12 @@ class _Linear(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, bias, relu):
         if max_sum >= x.shape[1]:
-            x, weight = x.contiguous(), weight.contiguous()
+            # (a copy is the kernel's alone: what is saved below are the inputs, which second derivatives go through)
+            rows, columns = x.contiguous(), weight.contiguous()
             y = torch.empty((x.shape[0], weight.shape[0]), dtype=torch.float32, device=x.device)
             with _cabi.on_device(x.device):
                 _cabi.check(_cabi.lib.fgc_dense_forward(
-                    _cabi.ptr(x), _cabi.ptr(weight), _cabi.ptr(bias.contiguous()), x.shape[0], x.shape[1], weight.shape[0], int(relu),
+                    _cabi.ptr(rows), _cabi.ptr(columns), _cabi.ptr(bias.contiguous()), x.shape[0], x.shape[1], weight.shape[0], int(relu),
                     _cabi.ptr(y), _cabi.current_stream(x.device)), "fgc_dense_forward")
         elif x.shape[0] * weight.shape[0] < pass_from:
             y = torch.addmm(bias, x, weight.t())

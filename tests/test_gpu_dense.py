@@ -79,6 +79,32 @@ def test_dense_layer_special_values_and_plain_calls(monkeypatch):
     assert not torch.vmap(lambda v: torch.tensor(float(dense.fused_ok(lin, v))))(xs[:, None, :]).any()
 
 
+@pytest.mark.parametrize("strided", ["x", "weight", "both"])
+@pytest.mark.parametrize("relu", [False, True])
+def test_second_derivatives_through_strided_operands(monkeypatch, strided, relu):
+    """A slice of columns as input and a transposed weight: the derivatives of the first derivatives are those of the modules.  Sums of up
+    to 60 x 8 products of fp32 numbers of size 10 or so, each rounded a few times: 1e-4 of the largest."""
+    from fastgraphcompute_b200 import dense
+    monkeypatch.setattr(dense, "min_rows", 1)
+    monkeypatch.setattr(dense, "_pays", lambda *a: True)
+    torch.manual_seed(7)
+    lin, act = nn.Linear(12, 8).to(DEV), nn.ReLU()
+    if strided != "x":
+        lin.weight = nn.Parameter(torch.randn((12, 8), device=DEV).t())
+        assert not lin.weight.is_contiguous()
+    wide = torch.randn((60, 20), device=DEV, requires_grad=True)
+
+    def second(layer):
+        x = wide[:, 3:15] if strided != "weight" else wide[:, :12].clone()
+        out = layer(x)
+        dx, dw = torch.autograd.grad((out ** 2).sum(), [x, lin.weight], create_graph=True)
+        return out, torch.autograd.grad((dw ** 2).sum() + (dx ** 2).sum(), [wide, lin.weight])
+    out, got = second(lambda x: dense.linear_relu(lin, act, x) if relu else dense.linear(lin, x))
+    assert type(out.grad_fn).__name__ == "_LinearBackward"
+    for a, b in zip(got, second(lambda x: act(lin(x)) if relu else lin(x))[1]):
+        assert (a - b).abs().max() <= 1e-4 * b.abs().max()
+
+
 def test_forward_mode_derivatives_of_dense_layers(monkeypatch):
     """An input that carries a tangent goes through the modules, which have forward-mode derivatives: as one layer, and
     where the tangent starts at an inner layer's weight."""
