@@ -14,7 +14,7 @@
 //   k_dense_reduce  adds the CTAs' partial results in a fixed order: the result is the same on
 //                   every run.
 //
-// Tiles with numbers that cannot be split (infinities, NaN, 2^60 and more) are computed by scalar operations.
+// Tiles with numbers that cannot be split (infinities, NaN, 2^43 and more) are computed by scalar operations.
 //
 // Kernels with ReLU, us (read and written once): 200 k rows, 128 to 128: forward 59 (31), input gradient 71 (47), dW 106 (47); 1.6 M rows, 128 to
 // 64: 270 (188), 391 (250), 476 (250).  Forward and backward of the first, modules / library products with passes of our own for bias,
@@ -267,7 +267,7 @@ k_dense_rows(const DenseRows g)
                 if (!plain) {
                     tmem_wait_read();
 #pragma unroll
-                    for (int k = 0; k < 16; k++) v[k] = __uint_as_float(big[k]) + __uint_as_float(small[k]);
+                    for (int k = 0; k < 16; k++) v[k] = (__uint_as_float(big[k]) + __uint_as_float(small[k])) * kSplitUndo;
                     if (c + 32 < NT) read16(c + 32);
                 } else {
                     const long long row = row0 + lane;
@@ -533,7 +533,7 @@ k_dense_weight(const DenseWeight g)
                         tmem_read16(acc + NT + n_half + 16 * h, small);
                         tmem_wait_read();
 #pragma unroll
-                        for (int k = 0; k < 16; k++) total[16 * h + k] += __uint_as_float(big[k]) + __uint_as_float(small[k]);
+                        for (int k = 0; k < 16; k++) total[16 * h + k] = fmaf(__uint_as_float(big[k]) + __uint_as_float(small[k]), kSplitUndo, total[16 * h + k]);
                     }
                 }
             } else {

@@ -1,9 +1,14 @@
 // Tensor-core products of fp32 matrices at fp32 accuracy (sm_100a: tcgen05.mma, accumulators in TMEM).
 //
-// An fp32 number is the sum of three bfloat16 numbers, exactly: each takes the eight leading bits of what is left.  Of the nine
+// An fp32 number is the sum of three bfloat16 numbers: each takes the eight leading bits of what is left.  The third of a number below
+// 2^-110 would have bits below bfloat16's smallest, 2^-133, so numbers are multiplied by 2^16 first: then the smallest fp32 number, 2^-149, is
+// that one, and the three parts are exact for all of them (the tensor core keeps subnormal operands and sums: 2^-133 times 2^40, and
+// 2^-126 + 2^-140 from two products, came out exactly).  Results are divided by 2^32.  Of the nine
 // products of two such sums the six with the first part of either, or the second of both, are formed; the other three are below
 // 2^-24 of the result.  Products of bfloat16 numbers are exact in the fp32 accumulators.  The product of the two first parts has an
 // accumulator of its own, so that it is rounded only as often as it is added to.
+// (Sums of bfloat16 numbers for fp32 products: Henry, Tang and Heinecke, "Leveraging the bfloat16 artificial intelligence datatype for
+// higher-precision computations", 2019.)
 //
 // Operands lie in shared memory as rows of 64 numbers (128 bytes) in the 128-byte swizzle: eight rows make an atom of 1024 bytes,
 // 16-byte unit u of row r is at u ^ (r & 7).  The same bytes are a K-major operand (a row is a row or column of the result) and an
@@ -16,27 +21,31 @@
 
 namespace fgc {
 
-// Beyond this (2^60, infinities and NaN among it) a number is not split: parts of products could overflow where the product does not,
-// and an infinity times a part that is 0 is not a number.  Tiles that hold one are computed by scalar operations.
-constexpr uint32_t kUnsplit = 0x5d800000u;         // (a number just below it may count as it: its first part is rounded)
+constexpr float kSplitScale = 65536.f, kSplitUndo = 1.f / 65536.f / 65536.f;
+// From here on (2^59 when scaled, 2^43 as it was; infinities and NaN among it) a number is not split: sums of 512 products could overflow where
+// the result does not, and an infinity times a part that is 0 is not a number.  Tiles that hold one are computed by scalar operations.
+constexpr uint32_t kUnsplit = 0x5d000000u;         // (a number just below it may count as it: its first part is rounded)
 
 // Eight numbers into three units of eight parts; returns the largest first part without sign, as the upper half of the pattern of an fp32 number.
+// (Two at a time: the scaling costs nothing beside the differences one by one.)
 __device__ __forceinline__ uint32_t split8(const float (&v)[8], uint4 (&part)[3])
 {
     uint32_t p[3][4], most = 0;
+    const unsigned long long scale = pack_f32x2(kSplitScale, kSplitScale);
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-        float a = v[2 * i], b = v[2 * i + 1];
+        unsigned long long ab;
+        asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(ab) : "l"(pack_f32x2(v[2 * i], v[2 * i + 1])), "l"(scale));
 #pragma unroll
         for (int k = 0; k < 3; k++) {
+            float a, b;
+            unpack_f32x2(ab, a, b);
             const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
             const uint32_t u = *reinterpret_cast<const uint32_t *>(&h);
             p[k][i] = u;
             if (k == 0) most = __vmaxu2(most, u & 0x7fff7fffu);
-            if (k < 2) {
-                a -= __uint_as_float(u << 16);
-                b -= __uint_as_float(u & 0xffff0000u);
-            }
+            if (k < 2)
+                asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(ab) : "l"(ab), "l"(pack_f32x2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u))));
         }
     }
     most = max(most & 0xffffu, most >> 16) << 16;

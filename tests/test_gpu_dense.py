@@ -216,3 +216,34 @@ def test_numbers_that_are_not_split(monkeypatch, where, value):
         assert _cabi.lib.fgc_dense_forward(_cabi.ptr(x), _cabi.ptr(lin.weight.detach()), None, n, n_in, n_out, 0, _cabi.ptr(own),
                                            _cabi.current_stream(x.device)) == 0
         torch.testing.assert_close(own[700].double(), bias_free, rtol=1e-6, atol=0.0)
+
+
+@pytest.mark.parametrize("exponent", [-108, -112, -118, -122, -126, -135, -149, 42])
+@pytest.mark.parametrize("where", ["x", "weight"])
+def test_operands_keep_all_their_bits(exponent, where):
+    """Numbers from fp32's smallest on, all of one matrix of that size, the other of a size that is still split and keeps the results above
+    fp32's subnormals.  The operands are exact in both, so that only sums are rounded: of 40 or 24 products, or of 64 rows and then of five such
+    sums, sixteen at a time -- at most nine additions, by 2^-23 of the sum of the products' sizes each -- and products of 2^-24 are left out."""
+    from fastgraphcompute_b200 import _cabi
+    torch.manual_seed(5)
+    n, n_in, n_out, other = 300, 40, 24, min(max(-exponent - 20, -40), 38)
+    small = torch.randn((n, n_in) if where == "x" else (n_out, n_in), device=DEV) * 2.0 ** (exponent / 2) * 2.0 ** (exponent - exponent / 2)
+    large = torch.randn((n_out, n_in) if where == "x" else (n, n_in), device=DEV) * 2.0 ** other
+    x, weight = (small, large) if where == "x" else (large, small)
+    assert small.abs().max() > 0 and torch.isfinite(large).all()
+    stream, lib, ptr = _cabi.current_stream(x.device), _cabi.lib, _cabi.ptr
+
+    def close(a, ref, mag):
+        assert ((a.double() - ref).abs() <= 20 * 2.0 ** -24 * mag + 2.0 ** -149).all()
+    out = torch.empty((n, n_out), device=DEV)
+    assert lib.fgc_dense_forward(ptr(x), ptr(weight), None, n, n_in, n_out, 0, ptr(out), stream) == 0
+    close(out, x.double() @ weight.double().t(), x.double().abs() @ weight.double().abs().t())
+    # x as a gradient of n_in outputs: dx = x @ weight^T, and dw = x^T @ (large or small numbers)
+    turned, dx = weight.t().contiguous(), torch.empty((n, n_out), device=DEV)
+    assert lib.fgc_dense_input_gradient(ptr(x), None, ptr(turned), n, n_out, n_in, ptr(dx), stream) == 0
+    close(dx, x.double() @ turned.double(), x.double().abs() @ turned.double().abs())
+    y = (torch.randn((n, n_out), device=DEV) * 2.0 ** (other if where == "x" else exponent)).contiguous()
+    nbytes = lib.fgc_dense_backward_bytes(n, n_in, n_out)
+    dw, db, ws = torch.empty((n_out, n_in), device=DEV), torch.empty((n_out,), device=DEV), torch.empty(nbytes, dtype=torch.uint8, device=DEV)
+    assert lib.fgc_dense_backward(ptr(x), ptr(y), None, n, n_in, n_out, None, ptr(dw), ptr(db), ptr(ws), nbytes, stream) == 0
+    close(dw, y.double().t() @ x.double(), y.double().abs().t() @ x.double().abs())
