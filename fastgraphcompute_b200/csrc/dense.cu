@@ -14,7 +14,9 @@
 //   k_dense_reduce  adds the CTAs' partial results in a fixed order: the result is the same on
 //                   every run.
 //
-// Tiles with numbers that cannot be split (infinities, NaN, 2^43 and more) are computed by scalar operations.
+// Tiles of rows, and sixteens of the weight's columns, with numbers that cannot be split (infinities, 2^43 and more) are computed by scalar
+// operations: 200 k rows, 128 to 128 with ReLU, forward and backward 0.25 ms without such numbers, 0.51 with one in x, 1.06 with one in the weight,
+// 4.4 with all of x (every result summed on its own 2.0, 43 and 27; modules 0.99).  NaN costs nothing.
 //
 // Kernels with ReLU, us (read and written once): 200 k rows, 128 to 128: forward 59 (31), input gradient 71 (47), dW 106 (47); 1.6 M rows, 128 to
 // 64: 270 (188), 391 (250), 476 (250).  Forward and backward of the first, modules / library products with passes of our own for bias,
@@ -85,11 +87,11 @@ __device__ __forceinline__ void mask8(float4 (&g)[2], const float4 (&y)[2])
         if (y[i].w <= 0.f) g[i].w = 0.f;
     }
 }
-__device__ __forceinline__ uint32_t split_to(char *operand, int part_bytes, int row, int unit, const float4 (&v)[2])
+__device__ __forceinline__ float split_to(char *operand, int part_bytes, int row, int unit, const float4 (&v)[2])
 {
     const float f[8] = {v[0].x, v[0].y, v[0].z, v[0].w, v[1].x, v[1].y, v[1].z, v[1].w};
     uint4 part[3];
-    const uint32_t most = split8(f, part);
+    const float most = split8(f, part);
     char *to = operand + operand_at(row, unit);
 #pragma unroll
     for (int k = 0; k < 3; k++) *reinterpret_cast<uint4 *>(to + k * part_bytes) = part[k];
@@ -128,7 +130,8 @@ k_dense_rows(const DenseRows g)
     float *s_bias = s_stage + kRowsWrite * (kRowsStage / 4);                               // of the CTA's columns
     uint64_t *s_bar = reinterpret_cast<uint64_t *>(s_bias + 128);
     uint32_t *s_tmem = reinterpret_cast<uint32_t *>(s_bar + 10);
-    volatile int *s_late = reinterpret_cast<int *>(s_tmem + 1), *s_bad = s_late + 1;       // a wait that gave up; tiles not to be split
+    volatile int *s_late = reinterpret_cast<int *>(s_tmem + 1), *s_bad = s_late + 1;       // a wait that gave up; tiles not to be split,
+    int *s_bad_cols = const_cast<int *>(s_bad) + kRowsBad;                                 // sixteens of columns, a bit each
     const uint32_t bar = smem_at(s_bar), full = bar, empty = bar + 24, done = bar + 48, read = bar + 64;
     const int t = threadIdx.x, lane = t & 31, w = __shfl_sync(FGC_FULL_MASK, t >> 5, 0);
     const int col0 = blockIdx.y * g.tile_cols, NT = g.tile_cols;
@@ -143,13 +146,13 @@ k_dense_rows(const DenseRows g)
             mbar_init(done + 8 * i, 1);
             mbar_init(read + 8 * i, kRowsWrite);
         }
-        *s_late = 0;
+        *s_late = *s_bad_cols = 0;
         for (int i = 0; i < kRowsBad; i++) s_bad[i] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    __syncthreads();
     if (t < NT) s_bias[t] = g.bias && col0 + t < g.n_cols ? __ldg(g.bias + col0 + t) : 0.f;
     // the weight: row n of the operand is output column col0 + n
-    uint32_t most = 0;
     for (int i = t; i < g.chunks * NT * 8; i += kRowsThreads) {
         const int unit = i & 7, n = (i >> 3) % NT, chunk = (i >> 3) / NT;
         float4 v[2];
@@ -159,11 +162,11 @@ k_dense_rows(const DenseRows g)
             const int at = chunk * 64 + unit * 8 + k;
             f[k] = col0 + n < g.n_cols && at < g.n_sum ? __ldg(g.w + (size_t)at * g.w_sum + (size_t)(col0 + n) * g.w_col) : 0.f;
         }
-        most = max(most, split_to(s_w + chunk * NT * 128, w_part, n, unit, v));
+        if (split_to(s_w + chunk * NT * 128, w_part, n, unit, v) >= kUnsplit) atomicOr(s_bad_cols, 1 << (n >> 4));
     }
     smem_to_tensor_core();
     tc_before_sync();
-    const bool plain_all = __syncthreads_or(most >= kUnsplit);
+    __syncthreads();
     tc_after_sync();
     const uint32_t tmem = *s_tmem;
     const long long n_tiles = (g.n_rows + kRowsTile - 1) / kRowsTile;
@@ -191,11 +194,11 @@ k_dense_rows(const DenseRows g)
         // (a register is loaded again as soon as it has been split; beyond the last row nothing is read)
         auto split_step = [&](float4 (&a)[2][2], float4 (&m)[2][2]) {
             if (round > 0 && !__all_sync(FGC_FULL_MASK, wait_unless(empty + 8 * b, (round - 1) & 1, s_late))) return;
-            uint32_t top = 0;
+            float top = 0.f;
 #pragma unroll
             for (int i = 0; i < 2; i++) {
                 if constexpr (MASK) mask8(a[i], m[i]);
-                top = max(top, split_to(s_a + b * kRowsBuffer, kRowsTile * 128, row_in + 64 * i, unit, a[i]));
+                top = fmaxf(top, split_to(s_a + b * kRowsBuffer, kRowsTile * 128, row_in + 64 * i, unit, a[i]));
                 fetch(i, a, m);
             }
             advance();
@@ -253,38 +256,53 @@ k_dense_rows(const DenseRows g)
             const long long row0 = ((long long)blockIdx.x + (long long)tile * gridDim.x) * kRowsTile + 32 * quarter;
             const uint32_t acc = tmem + (uint32_t)((tile & 1) * 2 * NT) + ((uint32_t)(32 * quarter) << 16);
             bool plain = !__all_sync(FGC_FULL_MASK, wait_unless(done + 8 * (tile & 1), (tile >> 1) & 1, s_late));
-            plain = plain || plain_all || s_bad[tile & (kRowsBad - 1)];
-            plain = __any_sync(FGC_FULL_MASK, plain);
+            plain = plain || s_bad[tile & (kRowsBad - 1)];
+            const int scalar = __any_sync(FGC_FULL_MASK, plain) ? 0xff : *s_bad_cols;      // sixteens that the tensor core has not formed
             tc_after_sync();
             uint32_t big[16], small[16];
             auto read16 = [&](int c) {
+                if (c >= NT || (scalar >> (c >> 4) & 1)) return;
                 tmem_read16(acc + c, big);
                 tmem_read16(acc + NT + c, small);
             };
-            if (!plain && 16 * odd < NT) read16(16 * odd);
+            read16(16 * odd);
             for (int c = 16 * odd; c < NT; c += 32) {
                 float v[16];
-                if (!plain) {
+                if (!(scalar >> (c >> 4) & 1)) {
                     tmem_wait_read();
 #pragma unroll
                     for (int k = 0; k < 16; k++) v[k] = (__uint_as_float(big[k]) + __uint_as_float(small[k])) * kSplitUndo;
-                    if (c + 32 < NT) read16(c + 32);
                 } else {
-                    const long long row = row0 + lane;
-#pragma unroll 1
-                    for (int k = 0; k < 16; k++) {
-                        float sum = 0.f;
-                        if (row < g.n_rows && col0 + c + k < g.n_cols)
-                            for (int i = 0; i < g.n_sum; i++) {
-                                float a = __ldg(g.a + (size_t)row * g.n_sum + i);
-                                if (MASK && __ldg(g.mask + (size_t)row * g.n_sum + i) <= 0.f) a = 0.f;
-                                sum = fmaf(a, __ldg(g.w + (size_t)i * g.w_sum + (size_t)(col0 + c + k) * g.w_col), sum);
-                            }
-                        stage[lane * 20 + k] = sum;
-                    }
+                    // A row a lane, its 16 columns side by side; rows and columns beyond the last are read as the last and not written.  Two
+                    // numbers of the sum at a time, the next two on their way: the lanes hold their 32 of the weight.
+                    const size_t row = (size_t)min(row0 + lane, g.n_rows - 1) * g.n_sum;
+                    const int col = min(col0 + c + (lane & 15), g.n_cols - 1), mine = lane >> 4;
+                    const float *w = g.w + (size_t)col * g.w_col + (size_t)mine * g.w_sum;
+                    float a[2], b, next_a[2], next_b;
+                    auto load = [&](int i) {
 #pragma unroll
-                    for (int k = 0; k < 16; k++) v[k] = stage[lane * 20 + k];
+                        for (int j = 0; j < 2; j++) {
+                            next_a[j] = i + j < g.n_sum ? __ldg(g.a + row + i + j) : 0.f;
+                            if (MASK && i + j < g.n_sum && __ldg(g.mask + row + i + j) <= 0.f) next_a[j] = 0.f;
+                        }
+                        next_b = i + mine < g.n_sum ? __ldg(w + (size_t)i * g.w_sum) : 0.f;
+                    };
+#pragma unroll
+                    for (int k = 0; k < 16; k++) v[k] = 0.f;
+                    load(0);
+                    for (int i = 0; i < g.n_sum; i += 2) {
+                        a[0] = next_a[0];
+                        a[1] = next_a[1];
+                        b = next_b;
+                        load(i + 2);
+#pragma unroll
+                        for (int k = 0; k < 16; k++) v[k] = fmaf(a[0], __shfl_sync(FGC_FULL_MASK, b, k), v[k]);
+                        if (i + 1 >= g.n_sum) break;
+#pragma unroll
+                        for (int k = 0; k < 16; k++) v[k] = fmaf(a[1], __shfl_sync(FGC_FULL_MASK, b, 16 + k), v[k]);
+                    }
                 }
+                read16(c + 32);
 #pragma unroll
                 for (int k = 0; k < 4; k++) {
                     const float4 bias = *reinterpret_cast<const float4 *>(s_bias + c + 4 * k);
@@ -454,7 +472,7 @@ k_dense_weight(const DenseWeight g)
         }
         for (int step = 0; step < steps; step++) {
             const int b = step & 1;
-            uint32_t top = 0;
+            float top = 0.f;
             if (step >= 2 && !__all_sync(FGC_FULL_MASK, wait_unless(done + 8 * b, ((step >> 1) - 1) & 1, s_late))) top = kUnsplit;
             // (the rows of the next step from here on; beyond the last nothing is read)
             const long long row_now = row0;
@@ -465,7 +483,7 @@ k_dense_weight(const DenseWeight g)
 #pragma unroll
             for (int i = 0; i < 2; i++) {
                 if (i == 0 || wide_x) {
-                    top = max(top, split_to(s_x + b * kWeightBuffer, kWeightRows * 128, row_x + 32 * i, unit_x & 7, vx[i]));
+                    top = fmaxf(top, split_to(s_x + b * kWeightBuffer, kWeightRows * 128, row_x + 32 * i, unit_x & 7, vx[i]));
                     fetch_x(i);
                 }
             }
@@ -481,7 +499,7 @@ k_dense_weight(const DenseWeight g)
                     }
 #pragma unroll
                     for (int k = 0; k < 8; k++) sum[k] += v[k];
-                    top = max(top, split_to(s_y + b * kWeightBuffer, kWeightRows * 128, row_y + 32 * i, unit_y & 7, vy[i]));
+                    top = fmaxf(top, split_to(s_y + b * kWeightBuffer, kWeightRows * 128, row_y + 32 * i, unit_y & 7, vy[i]));
                     fetch_y(i);
                 }
             }
@@ -537,15 +555,25 @@ k_dense_weight(const DenseWeight g)
                     }
                 }
             } else {
-                const long long row0 = first + (long long)step * kWeightRows;
-                for (long long row = row0; row < min(last, row0 + kWeightRows); row++) {
-                    const float a = g.swap ? (m < n_in ? __ldg(g.x + (size_t)row * g.n_in + m) : 0.f) : (m < n_out ? masked_dy(row, m) : 0.f);
+                // a row of the matrices at a time, the next one on its way: the lanes hold its 64 numbers of the one, and theirs of the other
+                const long long row0 = first + (long long)step * kWeightRows, end = min(last, row0 + kWeightRows);
+                float a, v[2], next_a, next_v[2];
+                auto load = [&](long long row) {
+                    next_a = row >= end ? 0.f : (g.swap ? (m < n_in ? __ldg(g.x + (size_t)row * g.n_in + m) : 0.f) : (m < n_out ? masked_dy(row, m) : 0.f));
 #pragma unroll
-                    for (int k = 0; k < 64; k++) {
-                        const int n = n0 + k;
-                        const float v = g.swap ? (n < n_out ? masked_dy(row, n) : 0.f) : (n < n_in ? __ldg(g.x + (size_t)row * g.n_in + n) : 0.f);
-                        total[k] = fmaf(a, v, total[k]);
+                    for (int j = 0; j < 2; j++) {
+                        const int n = n0 + 32 * j + lane;
+                        next_v[j] = row >= end ? 0.f : (g.swap ? (n < n_out ? masked_dy(row, n) : 0.f) : (n < n_in ? __ldg(g.x + (size_t)row * g.n_in + n) : 0.f));
                     }
+                };
+                load(row0);
+                for (long long row = row0; row < end; row++) {
+                    a = next_a;
+                    v[0] = next_v[0];
+                    v[1] = next_v[1];
+                    load(row + 1);
+#pragma unroll
+                    for (int k = 0; k < 64; k++) total[k] = fmaf(a, __shfl_sync(FGC_FULL_MASK, v[k >> 5], k & 31), total[k]);
                 }
             }
             tc_before_sync();

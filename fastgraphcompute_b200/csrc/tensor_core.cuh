@@ -22,15 +22,17 @@
 namespace fgc {
 
 constexpr float kSplitScale = 65536.f, kSplitUndo = 1.f / 65536.f / 65536.f;
-// From here on (2^59 when scaled, 2^43 as it was; infinities and NaN among it) a number is not split: sums of 512 products could overflow where
-// the result does not, and an infinity times a part that is 0 is not a number.  Tiles that hold one are computed by scalar operations.
-constexpr uint32_t kUnsplit = 0x5d000000u;         // (a number just below it may count as it: its first part is rounded)
+// From here on (2^43 before the scaling; infinities among it) a number is not split: sums of 512 products could overflow where
+// the result does not, and an infinity times a part that is 0 is not a number.  What holds one is computed by scalar operations.  NaN is split
+// like any number: its parts are NaN, and so is what it is multiplied with or added to.
+constexpr float kUnsplit = 5.764607523034235e17f;          // 2^59
 
-// Eight numbers into three units of eight parts; returns the largest first part without sign, as the upper half of the pattern of an fp32 number.
+// Eight numbers into three units of eight parts; returns the largest size of the scaled numbers, NaN left out.
 // (Two at a time: the scaling costs nothing beside the differences one by one.)
-__device__ __forceinline__ uint32_t split8(const float (&v)[8], uint4 (&part)[3])
+__device__ __forceinline__ float split8(const float (&v)[8], uint4 (&part)[3])
 {
-    uint32_t p[3][4], most = 0;
+    uint32_t p[3][4];
+    float most = 0.f;
     const unsigned long long scale = pack_f32x2(kSplitScale, kSplitScale);
 #pragma unroll
     for (int i = 0; i < 4; i++) {
@@ -43,12 +45,11 @@ __device__ __forceinline__ uint32_t split8(const float (&v)[8], uint4 (&part)[3]
             const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
             const uint32_t u = *reinterpret_cast<const uint32_t *>(&h);
             p[k][i] = u;
-            if (k == 0) most = __vmaxu2(most, u & 0x7fff7fffu);
+            if (k == 0) most = fmaxf(most, fmaxf(fabsf(a), fabsf(b)));
             if (k < 2)
                 asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(ab) : "l"(ab), "l"(pack_f32x2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u))));
         }
     }
-    most = max(most & 0xffffu, most >> 16) << 16;
 #pragma unroll
     for (int k = 0; k < 3; k++) part[k] = make_uint4(p[k][0], p[k][1], p[k][2], p[k][3]);
     return most;
