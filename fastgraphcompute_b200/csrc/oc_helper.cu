@@ -193,7 +193,7 @@ k_oc_pass(int p, int n_vert, uint64_t *keys_a, uint64_t *keys_b, int *vals_a, in
     chain_wait();
     chain_release();
     const int active = h->active;
-    if ((active >> p & 1) == 0 || *(volatile int *)&h->status != 0) return;
+    if ((active >> p & 1) == 0) return;
     const bool from_b = __popc(active & ((1 << p) - 1)) & 1;
     const uint64_t *__restrict__ keys_in = from_b ? keys_b : keys_a;
     uint64_t *__restrict__ keys_out = from_b ? keys_a : keys_b;
@@ -203,10 +203,12 @@ k_oc_pass(int p, int n_vert, uint64_t *keys_a, uint64_t *keys_b, int *vals_a, in
     __shared__ int s_off[kOcBins], s_sum[8], s_tile;
     __shared__ __align__(8) uint64_t s_keys[kOcSortTile];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, shift = 8 * p;
-    if (threadIdx.x == 0) s_tile = atomicAdd(&h->tile[p], 1);
+    // (a status may be set by other CTAs of this pass: one thread looks, so that all of a CTA stay or leave)
+    if (threadIdx.x == 0) s_tile = *(volatile int *)&h->status != 0 ? -1 : atomicAdd(&h->tile[p], 1);
     for (int i = threadIdx.x; i < kOcWarps * kOcBins / 2; i += kOcWarps * 32) ((uint32_t *)s_cnt)[i] = 0;
     __syncthreads();
     const int tile = s_tile;
+    if (tile < 0) return;
     const int64_t first = (int64_t)tile * kOcSortTile, base = first + w * (kOcRounds * 32) + lane;
     const int n_here = (int)min((int64_t)kOcSortTile, n_vert - first);
     if (n_here <= 0) return;
@@ -287,7 +289,8 @@ k_oc_pass(int p, int n_vert, uint64_t *keys_a, uint64_t *keys_b, int *vals_a, in
                 }
             }
             if (t >= 0) t -= taken;
-            if (taken == 0 && ++spins >= kOcSpins) break;
+            spins = taken > 0 ? 0 : spins + 1;
+            if (spins >= kOcSpins) break;
         }
         if (spins >= kOcSpins) atomicOr(&h->status, FGC_STATUS_INTERNAL);
         else if (tile > 0) oc_store_tile(mine, tag | all | (unsigned long long)(before + count));

@@ -165,3 +165,14 @@ def test_points_of_no_object(n, share):
             e = np.searchsorted(rs, members[0], side="right") - 1
             want = np.setdiff1d(np.arange(rs[e], rs[e + 1]), members)
             assert np.array_equal(M_not[k][:len(want)], want) and (M_not[k][len(want):] == -1).all()
+
+
+@pytest.mark.parametrize("n", [4097, 300001])
+def test_a_status_ends_every_pass_of_the_sort(n):
+    """A status that is set when the passes begin: all CTAs of all of them leave, and nothing is kept from it for the next call."""
+    ids = torch.arange(n, device=DEV) % 70000
+    for _ in range(3):
+        with pytest.raises(RuntimeError, match="row_splits"):
+            fgc.oc_helper_matrices(ids, torch.tensor([0, n, n - 1, n], device=DEV))
+        M, _, per = run(ids.cpu(), [0, n], calc_m_not=False)
+        assert M.shape[0] == min(n, 70000) == per[0] and np.array_equal(M[:, 0], np.arange(M.shape[0]))
