@@ -39,6 +39,9 @@ struct OcHeader {
 
 constexpr size_t kOcHeaderBytes = 256;
 
+// Positions are counted in 31 bits, by up to a scan tile of 2048 at a time.
+constexpr int64_t kOcMostPoints = 0x7ffff000;
+
 // The sort: eight passes of eight bits over 64-bit keys, one launch each, 4096 keys a CTA.
 constexpr int kOcPasses = 8, kOcBins = 256, kOcWarps = 16, kOcRounds = 8, kOcSortTile = 32 * kOcWarps * kOcRounds;
 inline int oc_sort_tiles(int64_t n) { return (int)((n + kOcSortTile - 1) / kOcSortTile); }
@@ -430,18 +433,18 @@ k_oc_fill_m_not(const OcHeader *__restrict__ h, const int *__restrict__ vals_a, 
         const int beg = obj_start[k], cnt = obj_start[k + 1] - beg;
         const int e = obj_split[k];
         const int row_start = (int)rs[e];                                 // ids have 31 bits
-        const int n_non = (int)rs[e + 1] - row_start - cnt;
+        const uint32_t n_non = (uint32_t)((int)rs[e + 1] - row_start - cnt);
         // member i (a global point id) has  members[i] - row_start - i  non-members before it
         const int *__restrict__ members = vals + beg;
-        auto members_up_to = [&](int j, int lo, int hi) {
+        auto members_up_to = [&](uint32_t j, int lo, int hi) {
             while (lo < hi) {
                 const int mid = (lo + hi) >> 1;
-                if (members[mid] - row_start - mid <= j) lo = mid + 1; else hi = mid;
+                if ((uint32_t)(members[mid] - row_start - mid) <= j) lo = mid + 1; else hi = mid;
             }
             return lo;
         };
         int64_t *__restrict__ row = M_not + k * (int64_t)n_maxrs;
-        const int run_end = (int)min(run0 + kOcRun, (int64_t)n_maxrs);
+        const uint32_t run_end = (uint32_t)min(run0 + kOcRun, (int64_t)n_maxrs);
         // members before the columns, found by 32 probes at a time
         int t = 0;
         for (int end = cnt; t < end;) {
@@ -454,27 +457,28 @@ k_oc_fill_m_not(const OcHeader *__restrict__ h, const int *__restrict__ vals_a, 
             t += (found - 1) * step + 1;
         }
         int held = t;                                                     // the first member that a lane holds
-        auto hold = [&]() { return held + lane < cnt ? members[held + lane] - row_start - held - lane : 0x7fffffff; };
-        int next = hold();
-        for (int j0 = (int)run0; j0 < run_end; j0 += kOcStep) {
+        auto hold = [&]() { return held + lane < cnt ? (uint32_t)(members[held + lane] - row_start - held - lane) : 0x7fffffffu; };
+        uint32_t next = hold();
+        // (columns up to a step beyond the last: more than 31 bits)
+        for (uint32_t j0 = (uint32_t)run0; j0 < run_end; j0 += kOcStep) {
             constexpr int PER = kOcStep / 32;                             // columns per lane
-            const int j1 = run_end - j0 < kOcStep ? run_end : j0 + kOcStep;
-            const int c0 = j0 + (VEC2 ? 2 * lane : lane);
-            auto column = [&](int u) { return VEC2 ? c0 + 64 * (u >> 1) + (u & 1) : c0 + 32 * u; };
+            const uint32_t j1 = run_end - j0 < kOcStep ? run_end : j0 + kOcStep;
+            const uint32_t c0 = j0 + (VEC2 ? 2 * lane : lane);
+            auto column = [&](int u) { return c0 + (VEC2 ? 64 * (u >> 1) + (u & 1) : 32 * u); };
             int in = __popc(__ballot_sync(FGC_FULL_MASK, next < j1));
             if (in == 32 && held < t) {
                 held = t;
                 next = hold();
                 in = __popc(__ballot_sync(FGC_FULL_MASK, next < j1));
             }
-            int id[PER];
+            uint32_t id[PER];
 #pragma unroll
             for (int u = 0; u < PER; u++) id[u] = row_start + t + column(u);
             if (in < 32) {
                 for (int i = t - held; i < in; i++) {
-                    const int b = __shfl_sync(FGC_FULL_MASK, next, i) - c0;
+                    const int b = (int)(__shfl_sync(FGC_FULL_MASK, next, i) - c0);
 #pragma unroll
-                    for (int u = 0; u < PER; u++) id[u] += column(u) - c0 >= b ? 1 : 0;
+                    for (int u = 0; u < PER; u++) id[u] += (int)(column(u) - c0) >= b ? 1 : 0;
                 }
                 t = held + in;
             } else {
@@ -488,17 +492,17 @@ k_oc_fill_m_not(const OcHeader *__restrict__ h, const int *__restrict__ vals_a, 
             if (j0 + kOcStep <= min(run_end, n_non)) {
 #pragma unroll
                 for (int u = 0; u < PER; u += VEC2 ? 2 : 1) {
-                    if (VEC2) *reinterpret_cast<uint4 *>(out + 32 * u) = make_uint4((uint32_t)id[u], 0u, (uint32_t)id[u + 1], 0u);
-                    else out[32 * u] = (int64_t)(uint32_t)id[u];
+                    if (VEC2) *reinterpret_cast<uint4 *>(out + 32 * u) = make_uint4(id[u], 0u, id[u + 1], 0u);
+                    else out[32 * u] = (int64_t)id[u];
                 }
             } else {
 #pragma unroll
                 for (int u = 0; u < PER; u += VEC2 ? 2 : 1) {
-                    const int64_t v = column(u) < n_non ? (int64_t)(uint32_t)id[u] : (int64_t)-1;
+                    const int64_t v = column(u) < n_non ? (int64_t)id[u] : (int64_t)-1;
                     if (column(u) >= j1) continue;
                     if (VEC2)                      // an even row length: the second column is in the row if the first is
                         *reinterpret_cast<longlong2 *>(out + 32 * u) =
-                            make_longlong2(v, column(u + 1) < n_non ? (int64_t)(uint32_t)id[u + 1] : (int64_t)-1);
+                            make_longlong2(v, column(u + 1) < n_non ? (int64_t)id[u + 1] : (int64_t)-1);
                     else
                         out[32 * u] = v;
                 }
@@ -526,7 +530,7 @@ k_select_with_default(const int64_t *__restrict__ idx, const W *__restrict__ fea
 
 extern "C" size_t fgc_oc_workspace_bytes(int64_t n_vert)
 {
-    if (n_vert < 0 || n_vert > 0x7ffffff0) return 0;
+    if (n_vert < 0 || n_vert > fgc::kOcMostPoints) return 0;
     return fgc::oc_workspace_layout(n_vert).total;
 }
 
@@ -537,7 +541,7 @@ extern "C" int fgc_oc_prepare(const int64_t *asso_idx, int64_t n_vert, const int
     FGC_NVTX("fgc_oc_prepare");
     using namespace fgc;
     if (n_vert < 0 || n_rs < 1 || !row_splits || (!objects_per_split && n_rs > 1)) return FGC_ERR_BAD_ARGUMENT;
-    if (n_vert > 0x7ffffff0 || n_rs > 0x7fffffff) return FGC_ERR_TOO_LARGE;
+    if (n_vert > kOcMostPoints || n_rs > 0x7fffffff) return FGC_ERR_TOO_LARGE;
     const OcWorkspace L = oc_workspace_layout(n_vert);
     if (!workspace || workspace_bytes < L.total || ((uintptr_t)workspace & 255)) return FGC_ERR_WORKSPACE;
     cudaStream_t s = (cudaStream_t)stream;
@@ -594,7 +598,7 @@ extern "C" int fgc_oc_fill(const void *workspace, size_t workspace_bytes, int64_
     FGC_NVTX("fgc_oc_fill");
     using namespace fgc;
     if (n_vert < 0 || n_unique < 0 || n_maxuq < 0 || n_maxrs < 0 || !row_splits) return FGC_ERR_BAD_ARGUMENT;
-    if (n_vert > 0x7ffffff0) return FGC_ERR_TOO_LARGE;
+    if (n_vert > kOcMostPoints) return FGC_ERR_TOO_LARGE;
     const OcWorkspace L = oc_workspace_layout(n_vert);
     if (!workspace || workspace_bytes < L.total || ((uintptr_t)workspace & 255)) return FGC_ERR_WORKSPACE;
     cudaStream_t s = (cudaStream_t)stream;

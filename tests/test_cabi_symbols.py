@@ -97,3 +97,14 @@ def test_search_by_size(n, D, row_splits, K, long_tails, tree):
     """The tree at the edges of the ranges where it was measured ahead of the grid."""
     from fastgraphcompute_b200 import _cabi
     assert _cabi.lib.fgc_knn_tree_preferred(n, D, row_splits + 1, K, long_tails) == tree
+
+
+def test_object_matrices_refuse_more_points_than_they_can_count():
+    """(positions of the last tile of 2048 are counted in 31 bits)"""
+    from fastgraphcompute_b200 import _cabi
+    lib, most = _cabi.lib, 0x7ffff000
+    assert lib.fgc_oc_workspace_bytes(most) > 0
+    for n in (most + 1, 0x7ffffff0, 1 << 31):
+        assert lib.fgc_oc_workspace_bytes(n) == 0
+        assert lib.fgc_oc_prepare(256, n, 256, 2, 256, 1 << 60, 256, None) == _cabi.ERR_TOO_LARGE
+        assert lib.fgc_oc_fill(256, 1 << 60, n, 256, 1, 1, 1, 256, None, None) == _cabi.ERR_TOO_LARGE

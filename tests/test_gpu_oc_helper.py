@@ -176,3 +176,27 @@ def test_a_status_ends_every_pass_of_the_sort(n):
             fgc.oc_helper_matrices(ids, torch.tensor([0, n, n - 1, n], device=DEV))
         M, _, per = run(ids.cpu(), [0, n], calc_m_not=False)
         assert M.shape[0] == 40 == per[0] and np.array_equal(M[:, 0], np.arange(40))
+
+
+@pytest.mark.parametrize("n_maxrs", [0x7fffffff, 0x7ffffffe, 0x7fffff01])
+def test_columns_up_to_31_bits(n_maxrs):
+    """Rows as long as fgc_oc_fill takes them: the last steps reach beyond 31 bits.  Nothing before or behind the row is written."""
+    import ctypes
+    from fastgraphcompute_b200 import _cabi
+    if torch.cuda.mem_get_info()[0] < 40 << 30:
+        pytest.skip("needs 17 GB")
+    lib, ptr = _cabi.lib, _cabi.ptr
+    asso, rs = torch.tensor([-1, 3, -1, 3, -1], device=DEV), torch.tensor([0, 5], device=DEV)
+    nbytes, stream = lib.fgc_oc_workspace_bytes(5), _cabi.current_stream(asso.device)
+    ws, per = torch.empty(nbytes, dtype=torch.uint8, device=DEV), torch.empty(1, dtype=torch.int64, device=DEV)
+    assert lib.fgc_oc_prepare(ptr(asso), 5, ptr(rs), 2, ptr(ws), nbytes, ptr(per), stream) == 0
+    status, sizes = ctypes.c_int32(0), (ctypes.c_int64 * 3)()
+    assert lib.fgc_oc_read_sizes(ptr(ws), ctypes.byref(status), sizes, stream) == 0 and list(sizes) == [1, 2, 5]
+    M = torch.empty((1, 2), dtype=torch.int64, device=DEV)
+    room = torch.full((n_maxrs + 64,), -7, dtype=torch.int64, device=DEV)
+    row = room[32:32 + n_maxrs]
+    assert lib.fgc_oc_fill(ptr(ws), nbytes, 5, ptr(rs), 1, 2, n_maxrs, ptr(M), ptr(row), stream) == 0
+    assert M.tolist() == [[1, 3]] and row[:4].tolist() == [0, 2, 4, -1]
+    assert (room[:32] == -7).all() and (room[32 + n_maxrs:] == -7).all()
+    for part in row[3:].split(1 << 28):
+        assert int(part.min()) == -1 == int(part.max())
