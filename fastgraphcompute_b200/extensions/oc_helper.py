@@ -104,6 +104,8 @@ def oc_helper_matrices(truth_idxs: torch.Tensor, row_splits: torch.Tensor,
         if status.value & _cabi.STATUS_BAD_ROW_SPLITS:
             raise RuntimeError("oc_helper_matrices: row_splits must start at 0, end at len(truth_idxs) "
                                "and never decrease")
+        if status.value:
+            raise RuntimeError("oc_helper_matrices: internal error, status %d" % status.value)
         n_unique, n_maxuq, n_maxrs = int(sizes[0]), int(sizes[1]), int(sizes[2])
         M = torch.empty((n_unique, n_maxuq), dtype=torch.int64, device=dev)
         if calc_m_not:

@@ -200,3 +200,17 @@ def test_columns_up_to_31_bits(n_maxrs):
     assert (room[:32] == -7).all() and (room[32 + n_maxrs:] == -7).all()
     for part in row[3:].split(1 << 28):
         assert int(part.min()) == -1 == int(part.max())
+
+
+def test_an_internal_status_is_an_error(monkeypatch):
+    """(a sort that gave up leaves no objects, which would look like a result)"""
+    from fastgraphcompute_b200 import _cabi
+    read = _cabi.lib.fgc_oc_read_sizes
+
+    def gave_up(ws, status, sizes, stream):
+        rc = read(ws, status, sizes, stream)
+        status._obj.value |= _cabi.STATUS_INTERNAL
+        return rc
+    monkeypatch.setattr(_cabi.lib, "fgc_oc_read_sizes", gave_up)
+    with pytest.raises(RuntimeError, match="status 32"):
+        fgc.oc_helper_matrices(torch.zeros(5, dtype=torch.int64, device=DEV), torch.tensor([0, 5], device=DEV))
