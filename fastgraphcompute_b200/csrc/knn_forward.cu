@@ -35,7 +35,7 @@ static StatusPool &status_pool()
     return *pool;
 }
 
-// Allocations that are harmless to a graph capture of another thread.
+// Allocations, and queries of an event, that are harmless to a graph capture of another thread.
 struct RelaxedCapture {
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
     RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
@@ -171,6 +171,7 @@ extern "C" int fgc_knn_forward(const float *coords, int64_t n_vert, int32_t n_co
     }
     // The words are on their way (also after an error of a later launch), and here long before the build has ended: looked for until the
     // event behind the build says that it has.
+    const RelaxedCapture relaxed;          // (a query of an event would end another thread's capture)
     volatile int64_t *const words = (volatile int64_t *)slot.words;
     cudaError_t e = cudaErrorNotReady;
     for (int i = 1; *words == kNoWords && e == cudaErrorNotReady; i++)

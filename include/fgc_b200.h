@@ -233,8 +233,8 @@ int fgc_knn_search_tree(int64_t n_vert, int32_t n_coords, const int64_t *row_spl
  * the search on it, and -- where out_order_or_null is given -- a copy of fgc_knn_cell_order [n_vert].
  * flags: FGC_SEARCH_COUNT, FGC_SEARCH_GRID3, FGC_SEARCH_GRID4 as for fgc_knn_search.
  * info_host_or_null [2], host memory: receives what fgc_knn_publish_grid_info stores.  The call then WAITS
- * until the build is done (not for the search, which is enqueued by then) and must not be captured into a graph;
- * it takes two page-locked words and an event from a pool that all threads share (64 of them are kept).  Without it
+ * until the device has stored them -- the checks are done and the form of the grid is known by then, the build itself may still be
+ * running -- and must not be captured into a graph; it takes two page-locked words and an event from a pool that all threads share (64 of them are kept).  Without it
  * nothing waits.
  */
 #define FGC_FORWARD_TREE 64    /* flags: search on a tree instead of a grid */

@@ -1096,6 +1096,46 @@ def test_forward_from_threads_that_come_and_go():
     assert bool((x == 2.0).all())
 
 
+@pytest.mark.parametrize("n,D,K", [(4000, 3, 8), (400000, 3, 16), (400000, 3, 64), (300000, 5, 40)])
+def test_forward_waits_beside_another_threads_capture(n, D, K):
+    """The call looks for its status words while another thread captures a graph: neither notices the other.  Grid built by one launch and by
+    many, tree."""
+    import threading
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    coords = torch.rand((n, D), generator=gen, device="cuda")
+    rs = torch.tensor([0, n], device="cuda")
+    want = fgc.binned_select_knn(K, coords, rs)
+    stream, got, errors = torch.cuda.Stream(), [], []
+
+    def work():
+        try:
+            with torch.cuda.stream(stream):
+                for _ in range(3):
+                    got.append(fgc.binned_select_knn(K, coords, rs))
+        except Exception as e:          # noqa: BLE001
+            errors.append(e)
+    work()                              # (so that the stream's memory is there: allocating any ends a capture)
+    got.clear()
+    torch.cuda.synchronize()
+    x, graph, side = torch.zeros(8, device="cuda"), torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        graph.capture_begin(capture_error_mode="global")      # (sees unsafe calls of all threads)
+        y = x + 1
+        thread = threading.Thread(target=work)
+        thread.start()
+        thread.join()
+        y = y + 1
+        graph.capture_end()
+    torch.cuda.synchronize()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert not errors and y.tolist() == [2.0] * 8
+    for idx, dist in got:
+        assert torch.equal(idx, want[0]) and torch.equal(dist, want[1])
+
+
+
 def test_grid_form_is_remembered_with_and_without_flags_apart(forward_flags):
     """Four coordinates: the form that a call with direction flags chose says nothing about one without."""
     import importlib
