@@ -308,3 +308,46 @@ def test_a_diverged_run_is_not_much_slower(value, where):
         else:
             lin.weight[3, 4] = value
     assert time() <= 25 * plain
+
+
+@pytest.mark.parametrize("n_in,n_out", [(128, 128), (64, 64), (72, 40), (96, 200), (200, 24), (130, 70)])
+@pytest.mark.parametrize("relu", [False, True])
+def test_every_part_of_a_product_counts(n_in, n_out, relu):
+    """One product per result, over several steps of many CTAs: nothing averages out.  Of the nine products of parts the three left out are below
+    2^-25, 2^-25 and 2^-33 of the result, and what is added is rounded by 2^-24 a few times; a third part that is lost, or left from the step
+    before, is 2^-17 and more."""
+    from fastgraphcompute_b200 import _cabi
+    lib, ptr, n = _cabi.lib, _cabi.ptr, 148 * 64 * 5 + 17
+    gen = torch.Generator(device=DEV).manual_seed(n_in)
+    stream, rnd = _cabi.current_stream(torch.device(DEV)), lambda *size: torch.randn(size, generator=gen, device=DEV)
+    weight, rows = rnd(n_out, n_in), torch.arange(n, device=DEV)
+    y = torch.where(rnd(n, n_out) < 0, 0.0, 1.0) if relu else None
+
+    def close(got, ref):
+        assert ((got.double() - ref).abs() <= 4 * 2.0 ** -24 * ref.abs()).all()
+    # forward: one number a row of x
+    x, col, v = torch.zeros((n, n_in), device=DEV), torch.randint(0, n_in, (n,), generator=gen, device=DEV), rnd(n)
+    x[rows, col] = v
+    out = torch.empty((n, n_out), device=DEV)
+    assert lib.fgc_dense_forward(ptr(x), ptr(weight), None, n, n_in, n_out, int(relu), ptr(out), stream) == 0
+    ref = v.double()[:, None] * weight.t()[col].double()
+    close(out, ref.relu() if relu else ref)
+    # input gradient: one number a row of dy
+    dy, col = torch.zeros((n, n_out), device=DEV), torch.randint(0, n_out, (n,), generator=gen, device=DEV)
+    dy[rows, col] = v
+    passes = torch.ones(n, device=DEV) if y is None else y[rows, col]
+    dx = torch.empty((n, n_in), device=DEV)
+    assert lib.fgc_dense_input_gradient(ptr(dy), ptr(y), ptr(weight), n, n_in, n_out, ptr(dx), stream) == 0
+    close(dx, (v * passes).double()[:, None] * weight[col].double())
+    # weight gradient: a dense x, one row of dy for every output
+    x = rnd(n, n_in)
+    nbytes = lib.fgc_dense_backward_bytes(n, n_in, n_out)
+    dw, db, ws = torch.empty((n_out, n_in), device=DEV), torch.empty((n_out,), device=DEV), torch.empty(nbytes, dtype=torch.uint8, device=DEV)
+    for _ in range(6):
+        row, outputs, g = torch.randperm(n, generator=gen, device=DEV)[:n_out], torch.arange(n_out, device=DEV), rnd(n_out)
+        dy.zero_()
+        dy[row, outputs] = g
+        passes = torch.ones(n_out, device=DEV) if y is None else y[row, outputs]
+        assert lib.fgc_dense_backward(ptr(x), ptr(dy), ptr(y), n, n_in, n_out, None, ptr(dw), ptr(db), ptr(ws), nbytes, stream) == 0
+        close(dw, (g * passes).double()[:, None] * x[row].double())
+        assert torch.equal(db, g * passes)
