@@ -34,11 +34,9 @@ UNIT = "points/s"
 WORKLOAD = "c2: single-event binned kNN fwd+bwd, N=200000, D=4, K=32, 50-component Gaussian mixture sigma=0.02"
 L2_FLUSH_BYTES = 256 << 20
 
-# DRAM traffic of one k_knn launch on this workload: dram__bytes_read.sum (8.54 MB) +
-# dram__bytes_write.sum (53.18 MB) of the ncu capture summarised in
-# profiles/k_knn_c2_ncu_full.md.  Below the 80 MB of algorithmic bytes because part of the
-# output is still in the 126 MB L2 when the kernel ends.
-KNN_KERNEL_DRAM_TRAFFIC_BYTES = 60018432
+# DRAM traffic of the 33 launches of one forward on this workload (search by groups): dram__bytes_read.sum +
+# dram__bytes_write.sum of the ncu capture summarised in profiles/knn_c2_step_launch_list.md, caches cold for every launch.
+FORWARD_DRAM_TRAFFIC_BYTES = 133900000
 
 
 def env_int(name, default):
@@ -243,8 +241,6 @@ def run_b200(args):
 
     import fastgraphcompute_b200 as fgc
     from fastgraphcompute_b200 import _cabi, synthetic
-    import importlib
-    knn_mod = importlib.import_module("fastgraphcompute_b200.extensions.binned_select_knn")
 
     sections = set() if args.no_gravnet else {x for x in args.sections.split(",") if x and x != "none"}
 
@@ -305,45 +301,10 @@ def run_b200(args):
     total_ms = max_over_ranks(sum(step_ms))
     value = world * n * args.steps / (total_ms * 1e-3)
 
-    # The dominant kernel alone, for the roofline: the search half of the forward through the
-    # split C ABI (fgc_knn_build_grid_dims once, then fgc_knn_search per step on that grid; the
-    # grid form is the one the public call settles on for this data), same inputs, L2 flushed
-    # before every launch, CUDA events on the launching stream around the launch.
-    def time_search_kernel(reps):
-        nb = _cabi.lib.fgc_knn_workspace_bytes(n, d_coords.shape[1], d_rs.numel(), K)
-        ws = torch.empty(nb, dtype=torch.uint8, device=dev)
-        s_idx = torch.empty((n, K), dtype=torch.int64, device=dev)
-        s_dsq = torch.empty((n, K), dtype=torch.float32, device=dev)
-        stream = _cabi.current_stream(dev)
-        info = torch.empty(2, dtype=torch.int32, pin_memory=True)
-        _cabi.check(_cabi.lib.fgc_knn_build_grid_dims(_cabi.ptr(d_coords), n, d_coords.shape[1], _cabi.ptr(d_rs),
-                                                      d_rs.numel(), K, None, 0.0, 0, _cabi.ptr(ws), nb, stream), "build")
-        _cabi.check(_cabi.lib.fgc_knn_publish_grid_info(_cabi.ptr(ws), info.data_ptr(), stream), "info")
-        torch.cuda.synchronize(dev)
-        form = int(info[1]) & 15
-        _cabi.check(_cabi.lib.fgc_knn_build_grid_dims(_cabi.ptr(d_coords), n, d_coords.shape[1], _cabi.ptr(d_rs),
-                                                      d_rs.numel(), K, None, 0.0, form, _cabi.ptr(ws), nb, stream), "build")
-        flags = 8 if form == 3 else 16 if form == 4 else 0
-        out = []
-        for i in range(reps + 2):
-            flush.zero_()
-            a0 = torch.cuda.Event(enable_timing=True)
-            a1 = torch.cuda.Event(enable_timing=True)
-            a0.record()
-            _cabi.check(_cabi.lib.fgc_knn_search(n, d_coords.shape[1], d_rs.numel(), K, 0, 0, flags, _cabi.ptr(s_idx),
-                                                 _cabi.ptr(s_dsq), _cabi.ptr(ws), nb, stream), "search")
-            a1.record()
-            if i >= 2:
-                out.append((a0, a1))
-        torch.cuda.synchronize(dev)
-        return [a.elapsed_time(b) for a, b in out]
-
-    knn_ms = time_search_kernel(args.steps)
-    knn_ms_avg = sum(knn_ms) / len(knn_ms)
-    phases = {"fwd_ms_median": statistics.median(a.elapsed_time(m_) for (a, _), m_ in zip(pairs, fwd_marks)),
+    fwd_ms = statistics.median(a.elapsed_time(m_) for (a, _), m_ in zip(pairs, fwd_marks))
+    phases = {"fwd_ms_median": fwd_ms,
               "bwd_ms_median": statistics.median(m_.elapsed_time(b) for (_, b), m_ in zip(pairs, fwd_marks)),
-              "fwd_bwd_ms_median": statistics.median(step_ms),
-              "search_kernel_ms_median": statistics.median(knn_ms)}
+              "fwd_bwd_ms_median": statistics.median(step_ms)}
 
     # ---- end to end from host buffers ("e2e") --------------------------------------------------
     o_idx = torch.empty((n, K), dtype=torch.int64).pin_memory()
@@ -472,12 +433,6 @@ def run_b200(args):
     clocks = sampler.summary(t_load0, t_load1) if sampler else None
     if sampler:
         sampler.stop()
-
-    # ---- candidate count of the search (for the FP32 view of the roofline) -------------------
-    idx, dsq, ws = knn_mod.knn_forward_raw(d_coords, d_rs, K, None, False, count_evals=True)
-    counters, grid_shape, cell_w = knn_mod.read_counters(ws)
-    n_evals = counters[0]
-    del idx, dsq, ws
 
     # ---- GravNet layer (second half of the headline metric) -------------------------------
     gravnet = None
@@ -786,7 +741,7 @@ def run_b200(args):
                         "aten_threads": torch.get_num_threads(),
                         "note": "the reference's kNN, binning and gradient loops are single-threaded"}
         # distance evaluations of the reference's own shell walk at its default binning, counted
-        # by the instrumented C restatement on the same workload (beside the count of this search)
+        # by the instrumented C restatement on the same workload
         try:
             from oracle import oracle as _oracle
             t0 = time.time()
@@ -801,13 +756,9 @@ def run_b200(args):
     if rank == 0:
         peak, peak_kind = measured_peaks()
         d = w.coords.shape[1]
-        props = torch.cuda.get_device_properties(dev)
-        max_mhz = (clocks or {}).get("sm_max_mhz") or 1965.0
-        fp32_peak_tflops = props.multi_processor_count * 128 * 2 * max_mhz * 1e6 / 1e12
         alg_bytes = n * (4 * d + 8 * K + 4 * K)          # coords read + int64 idx + fp32 distsq written
-        achieved = alg_bytes / (knn_ms_avg * 1e-3) / 1e9
-        launches_per_step = (_cabi.KERNELS_BUILD_GRID + _cabi.KERNELS_PUBLISH_STATUS + _cabi.KERNELS_SEARCH +
-                             _cabi.KERNELS_KNN_BWD)
+        achieved = alg_bytes / (fwd_ms * 1e-3) / 1e9
+        launches_per_step = _cabi.KERNELS_TREE_FORWARD + _cabi.KERNELS_TREE_SECOND_LOOK + _cabi.KERNELS_KNN_BWD
         line = {
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
             "warmup": max(args.warmup, 3), "ms_per_step": total_ms / args.steps,
@@ -823,19 +774,12 @@ def run_b200(args):
                             "first input copy until the last result has landed, L2 flush of every step included",
                     "single_batch_ms": e2e_single_ms},
             "gpu_launches": launches_per_step * args.steps,
-            "roofline": {"bound": "hbm", "kernel": "k_knn (neighbour search)", "achieved": achieved,
+            "roofline": {"bound": "hbm", "kernel": "binned_select_knn forward: search by groups, 33 launches", "achieved": achieved,
                          "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                         "peak_source": "of " + peak_kind, "traffic": KNN_KERNEL_DRAM_TRAFFIC_BYTES,
-                         "algorithmic_bytes_per_launch": alg_bytes, "kernel_ms": knn_ms_avg,
-                         "note": "not HBM-bound: ncu shows 85 % of issue slots busy, DRAM at 0.9 % "
-                                 "(profiles/k_knn_c2_ncu_full.md)"},
-            "roofline_fp32": {"note": "the search is bound by CUDA-core issue, not by HBM: distance evaluations x 3*D flops",
-                              "distance_evals_per_launch": n_evals, "evals_per_query": n_evals / n,
-                              "achieved_tflops": n_evals * 3 * d / (knn_ms_avg * 1e-3) / 1e12,
-                              "peak_tflops": fp32_peak_tflops,
-                              "peak_source": "computed, not measured: SMs x 128 FP32 lanes x 2 flop x max SM clock",
-                              "frac": n_evals * 3 * d / (knn_ms_avg * 1e-3) / 1e12 / fp32_peak_tflops,
-                              "grid_shape": grid_shape, "cell_width": cell_w},
+                         "peak_source": "of " + peak_kind, "traffic": FORWARD_DRAM_TRAFFIC_BYTES,
+                         "algorithmic_bytes_per_launch": alg_bytes, "kernel_ms": fwd_ms,
+                         "note": "not HBM-bound: k_tree_rows, its longest kernel, keeps 86 % of the issue slots busy "
+                                 "(profiles/knn_c2_step_launch_list.md); tree and second look are chains of short launches"},
             "clocks": clocks,
         }
         line["phases"] = phases

@@ -35,6 +35,10 @@ KERNELS_BUILD_GRID = 9
 KERNELS_BUILD_GRID_D4 = 11      # D = 4: a second density pass may follow a fallback to three binned coordinates
 KERNELS_PUBLISH_STATUS = 1   # the wrapper's status check after the grid build
 KERNELS_SEARCH = 2             # k_knn + k_knn_hard (the queries that gave up their walk)
+# binned_select_knn by groups beyond 24576 points: tree 15 (three radix passes), status words, bounds, rows, listed queries; and
+# the second look at rows with equal distances: gate, grid, search, queries that gave up their walk (D = 4 and eager calls; D = 3 two less)
+KERNELS_TREE_FORWARD = 19
+KERNELS_TREE_SECOND_LOOK = 14
 KERNELS_KNN_BWD = 1
 KERNELS_KNN_BWD_SORTED = 7   # reverse graph (6) + gather (1)
 KERNELS_GRAVNET_PROJECT = 2    # forward + backward of the fused input projections

@@ -3,7 +3,8 @@
 // Small batches are bound by the host.  A caller in an interpreter pays for every call into the
 // library and for the event and the pinned word of the status check; here they cost one call, and the
 // wait for the status word happens without the interpreter (two row splits of 5000 points, K = 16, forward and
-// backward, B200, timed in turn: 196 -> 168 us; a GravNet layer on ten small events: 303 -> 289 us).
+// backward, B200, timed in turn: 196 -> 168 us; a GravNet layer on ten small events: 303 -> 289 us;
+// with the build in one launch and the words looked for 128 and 240 since).
 #include <mutex>
 #include <thread>
 

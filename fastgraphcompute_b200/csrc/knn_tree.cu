@@ -505,7 +505,12 @@ extern "C" int fgc_knn_groups_preferred(int64_t n_vert, int32_t n_coords, int64_
 //   learned, four      K = 8: 50 k in ten 0.87, 200 k in 40 0.97;  K = 16: 50 k in 25 0.84
 //   learned, sorted in one launch (up to kSmallTree points; three / four)  K = 10: 3 k in one row split 0.63 / 0.64, 5 k in five 0.90 / 0.90, 10 k in
 //                      thirty 0.92 / 0.98, 16 k in fifty 0.84 / 0.89;  K = 40: 10 k in ten 0.76 / 0.68, 20 k in one 0.69 / 0.38;  K = 16: 1000 in one 0.88 / 0.91
-// In row splits of 5000 points in 50 clusters, a hundred each, the grid is ahead by 0.1 to 0.3 of its time at K = 24 to 40.
+// The ranges weigh uniform, normal and skewed points most.  Clusters of about as many points as K, for which the grid's cells are right, lose:
+// uniform / normal / mixture / skewed again, three coordinates, 800 k in 200, K = 16 0.91 / 0.90 / 1.11 / 0.81; four, 200 k in 20, K = 32 0.88 / 0.80 /
+// 1.12 / 0.20, 400 k in 100, K = 24 and 31 0.72 / 0.79 / 1.19 / 0.44 and 0.71 / 0.84 / 1.24 / 0.26; five, 50 k in two, K = 24 0.72 / 0.54 / 1.28 / 0.25, 100 k in five
+// 0.61 / 0.62 / 1.15 / 0.19, 800 k in 200, K = 8 0.70 / 0.80 / 1.12 / 0.80.  So do layers whose coordinates are not what long_tails says, learned / mixture /
+// uniform: three, 5000 in one, K = 8 0.94 / 1.18 / 1.46, 50 k in one, K = 8 0.97 / 1.34 / 1.57; four, 5000 in one 0.67 / 1.10 / 1.65, 50 k in 33, K = 16 0.86 /
+// 1.43 / 1.02.
 extern "C" int fgc_knn_groups_ahead(int64_t n_vert, int32_t n_coords, int64_t n_rs, int32_t K, int32_t long_tails)
 {
     using namespace fgc;

@@ -9,9 +9,9 @@ from torch.autograd import forward_ad
 
 from . import _cabi
 
-
-# Fewer rows are bound by launches, of which the fused form has more: forward and backward of a 128 to 64 layer
-# with ReLU take 186 us as modules and 197 fused at 16 384 rows, 247 and 193 at 32 768, 604 and 360 at 200 000.
+# Fewer rows: launches outweigh most of what is saved.  Forward and backward with ReLU, modules / own kernels, us: 32 768 rows, 64 to 64 171 / 134, 128 to
+# 128 247 / 133, 64 to 24 154 / 133; 16 384 rows 164 / 146, 141 / 133 and 137 / 133, but 256 to 256 259 / 137.  (Drawn with scalar kernels; these
+# are ahead on both sides of it.)
 min_rows = 32768
 
 # Sums over more columns (FGC_DENSE_MAX_SUM) stay with the library.
@@ -22,7 +22,9 @@ max_sum = 512
 # without ReLU 230 / 160, with it 264 / 161; 131 072 rows, 128 to 64 98 / 95 and 106 / 96).  Below, the pass and its
 # launch cost more than they save (200 000 rows, 128 to 10 85 / 91; 32 768 rows, 128 to 128 59 / 64).
 pass_from = 1 << 23
-# Forward alone, module with ReLU / own kernel, us: 66 000 rows, 128 to 64 71 / 45; 64 to 128 92 / 46; 100 000 rows, 128 to 64 91 / 52.
+# Forward alone, module with ReLU / own kernel, us: 66 000 rows, 128 to 64 71 / 45; 64 to 128 92 / 46; 100 000 rows, 128 to 64 91 / 52; several
+# shares of the columns, 200 000 rows: 256 to 256 789 / 246, 512 to 128 636 / 461, 512 to 512 2381 / 1825; 16 384 rows, 512 to 512 217 / 168.
+# (Ahead below it too, 32 768 rows, 128 to 128 50 / 21: not measured to its edge.)
 forward_from = (1 << 22) + 1
 
 
@@ -133,16 +135,16 @@ def _pays(linear, x) -> bool:
     n, n_in, n_out = x.shape[0], linear.in_features, linear.out_features
     if not (torch.is_grad_enabled() and (x.requires_grad or linear.weight.requires_grad)):
         return n * n_out >= (forward_from if n_in <= max_sum else pass_from)           # nothing but the forward to gain
-    # A small weight: the library's product for its gradient is a good one.  800 000 rows, 64 to 4 451 / 560 and 32 to 16
-    # 470 / 547; 200 000 rows, 32 to 32 710 / 239.
+    # A small weight: the library's product for its gradient is a good one, and little is gained: 200 000 rows, 32 to 16 158 / 134, 65 536
+    # rows 137 / 133, but 32 to 32 657 / 134.
     if n_in * n_out < min_rows // 32:
         return False
-    # Few outputs fill a sixth of a tile, which takes twice the rows to pay: 128 to 10 at 32 768 rows 165 / 177, at
-    # 65 536 214 / 188; 64 to 24 at 32 768 226 / 198.
+    # Few outputs fill a part of a tile, which takes twice the rows to gain from: 128 to 10 at 32 768 rows 133 / 132, at
+    # 65 536 156 / 133; 64 to 24 at 32 768 154 / 133.
     if n_out < 24 and (n + 1) // 2 < min_rows:
         return False
-    # Many tiles of a weight read x and the gradient again and again: 200 000 rows, 256 to 256 2129 / 1956, 512 to 128 2048 /
-    # 1974, but 384 to 160 (padded to 384 x 256) 2196 / 2370, 2048 to 64 3490 / 3798, 512 to 512 6591 / 6891.
+    # Many tiles of a weight read x and the gradient again and again, and gain less: 200 000 rows, 256 to 256 2106 / 840, 512 to 128 2026 /
+    # 1004, 384 to 160 2155 / 1034, 512 to 512 6550 / 4909.  (Drawn with scalar kernels, which lost on the last two.)
     return _padded(n_in) * _padded(n_out) <= 65536
 
 

@@ -132,7 +132,7 @@ def _forward(coords, row_splits, K, direction, tf_compat, count_evals, order, lo
     # build only, the GPU never idles while the host checks, and -- unlike a device-to-host copy -- the store
     # does not queue behind bulk result copies that other streams have in flight.
     # One call into the library for all of it (two row splits of 5000 points, K = 16, forward and backward:
-    # 196 us with four calls, a pinned tensor and an event from here, 168 us so).
+    # 196 us with four calls, a pinned tensor and an event from here, 168 us so; 128 with the build in one launch).
     info = (ctypes.c_int32 * 2)() if check else None
     _cabi.check(_cabi.lib.fgc_knn_forward(
         coords.data_ptr(), n_vert, n_coords, row_splits.data_ptr(), n_rs, K,

@@ -568,6 +568,8 @@ int fgc_strict_batch_from_row_splits(const int64_t *row_splits, int64_t n_rs, in
 /*
  * Dense layers around the message passing (torch.nn.Linear and ReLU in the reference, gnn_ops.py:60-68), fp32 matrices
  * row by row, on the tensor cores at fp32 accuracy.
+ * Numbers keep all their bits down to fp32's smallest; rows, and columns of the weight, near infinities or numbers of 2^43 and more take
+ * scalar operations, which are slower.
  *
  * fgc_dense_forward: out [n_rows, n_out] = act(x weight^T + bias), weight [n_out, n_in]; act is ReLU when relu != 0.
  * fgc_dense_input_gradient: dx [n_rows, n_in] = dY weight, with dY the gradient of a layer's output, masked where y_or_null, the
