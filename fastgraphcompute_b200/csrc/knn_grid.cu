@@ -254,7 +254,12 @@ k_rank_place(const float *__restrict__ coords, int n_vert, int n_coords, int nv,
     chain_wait();
     chain_release();
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= n_vert || g->status != 0) return;
+    if (v >= n_vert) return;
+    const int status = g->status;
+    if (status != 0) {
+        if (status & kNotBuilt) sorig[v] = v;
+        return;
+    }
     const int bin = pbin[v];
     const int beg = bounds[bin], len = bounds[bin + 1] - beg;
     if (len <= kRankMax) {

@@ -204,6 +204,10 @@ int knn_build_grid_forward(const float *coords, int64_t n_vert, int32_t n_coords
                            fgc_stream_t stream);
 
 // Argument checks shared by the kNN entry points.
+// Status of a build that did not take place.  Points are in the order of their ids then, so that what goes by the cell order of a caller who
+// does not look at the status (backward, aggregation) never reads uninitialised ids.
+constexpr int kNotBuilt = FGC_STATUS_NONFINITE | FGC_STATUS_BAD_ROW_SPLITS | FGC_STATUS_INTERNAL;
+
 inline int check_knn_args(int64_t n_vert, int32_t n_coords, int64_t n_rs, int32_t K,
                           const void *workspace, size_t workspace_bytes, KnnWorkspace *L)
 {

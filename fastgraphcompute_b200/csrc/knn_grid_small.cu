@@ -203,6 +203,10 @@ k_build_small(const GridBuild a)
         if (t == 0 && a.info_mapped && late_words) store_info(a.info_mapped, s_grid.status, s_grid.gdims + 16 * s_grid.fallback3);
     }
     if (!good) {
+        for (int v = first; v < n; v += kClusterAll) {
+            a.sorig[v] = v;
+            if (a.out_order) a.out_order[v] = v;
+        }
         cluster_barrier();               // (a CTA that has left can not be read)
         return;
     }

@@ -216,7 +216,13 @@ k_tree_leaves(const float *__restrict__ coords, int n_vert, int n_coords, const 
 {
     chain_wait();
     chain_release();
-    if (g->status != 0) return;
+    if (g->status != 0) {                                   // kNotBuilt
+        for (int v = blockIdx.x * 256 + threadIdx.x; v < n_vert; v += gridDim.x * 256) {
+            sorig[v] = v;
+            if (out_order) out_order[v] = v;
+        }
+        return;
+    }
     __shared__ uint32_t s_lo[4 * NV], s_hi[4 * NV];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     if (threadIdx.x < 4 * NV) { s_lo[threadIdx.x] = 0xffffffffu; s_hi[threadIdx.x] = 0; }

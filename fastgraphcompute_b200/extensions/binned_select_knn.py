@@ -18,8 +18,8 @@ from .. import _cabi
 target_occupancy = 0.0
 # Read the device status word after every forward (one small device->host copy).
 # The reference synchronises several times per call; switching this off makes the
-# call fully asynchronous but turns bad inputs (NaN, malformed row_splits) into
-# silently unwritten outputs.
+# call fully asynchronous but turns bad inputs (NaN, malformed row_splits) silently into
+# rows without neighbours.
 check_status = True
 # Backward by sorted-segment reductions over a reverse neighbour graph instead of float atomics:
 # bit-identical gradients from run to run (the atomic version, like the reference's CUDA path,

@@ -1219,3 +1219,25 @@ def test_binning_of_wide_tables(bins):
         rows = np.stack([split, b[:, 0], b[:, 1]], 1)
         rows[want >= limit], want[want >= limit] = 0, 0
         assert np.array_equal(flat.cpu().numpy(), want) and np.array_equal(idx.cpu().numpy(), rows)
+
+
+@pytest.mark.parametrize("n,D,K,long_tails", [(1000, 3, 8, False), (20000, 3, 8, False), (400000, 4, 16, False), (5000, 4, 16, True),
+                                              (30000, 3, 40, True), (400000, 5, 40, False)])
+@pytest.mark.parametrize("bad", ["nan", "row_splits"])
+def test_order_of_a_call_with_bad_input(monkeypatch, n, D, K, long_tails, bad):
+    """Without the status check, as in a captured graph: rows without neighbours, and an order that the backward and the aggregation can
+    go by.  Grids and trees built by one launch and by many."""
+    import importlib
+    km = importlib.import_module("fastgraphcompute_b200.extensions.binned_select_knn")
+    monkeypatch.setattr(km, "check_status", False)
+    coords = torch.rand((n, D), generator=torch.Generator().manual_seed(n)).to(DEV)
+    if bad == "nan":
+        coords[n // 3, D - 1] = float("nan")
+    rs = torch.tensor([0, n] if bad == "nan" else [0, n // 2, n // 4, n], device=DEV)
+    ids = torch.arange(n, device=DEV)
+    torch.cuda.synchronize()
+    stale = [torch.full((n,), 1 << 30, dtype=torch.int32, device=DEV) for _ in range(4)]      # what memory may hold
+    del stale
+    idx, dist, order = km.knn_forward_with_order(coords, rs, K, None, False, long_tails)
+    assert torch.equal(order.long().sort().values, ids)
+    assert torch.equal(idx[:, 0], ids) and bool((idx[:, 1:] == -1).all()) and not dist.any()
